@@ -35,7 +35,7 @@ struct Workspace {
   float* ksq;        // backward: c|k|^2 per row
   float* row_bias;   // query norms (non-softmax) or the forward's L re-pitched to n_pad (softmax backward)
   float* delta;      // backward only
-  void* lslab;       // single-kernel backward only: L and delta bias slabs, fp32 (B, H, N, D) dQ accumulator
+  void* lslab;       // single-kernel backward only: L and delta bias slabs, fp32 dQ accumulator (D floats per padded row)
   void* dslab;
   float* dq_acc;
   size_t bytes;
@@ -86,7 +86,7 @@ Workspace carve(void* base, int B, int H, int N, int D, int softmax, int backwar
       w.dslab = p + off;
       off += slab;
       w.dq_acc = reinterpret_cast<float*>(p + off);
-      off += align256(static_cast<size_t>(B) * H * N * D * sizeof(float));
+      off += align256(rows * D * sizeof(float));
     }
   }
   w.bytes = off;
@@ -359,7 +359,10 @@ int rbf_b200_bwd_phases(const void* q, const void* k, const void* v, const void*
     if (t1 != 0 || t2 != 0)
       return fail(RBF_B200_ERR_TENSOR_MAP, "cuTensorMapEncodeTiled failed for the bias slabs (codes %d, %d)", t1, t2);
     if (D == 64) {
-      const int t3 = rbf::make_tmap_f32_bhnd(&f.tm_dq_acc, ws.dq_acc, B, H, N, D, 32);
+      // the kernel's drain warps store 32 rows of dK and dV each
+      if ((rc = make_map(&f.tm_dk, "dk", dk, dk_strides, bf16, B, H, N, D, 32))) return rc;
+      if ((rc = make_map(&f.tm_dv, "dv", dv, dv_strides, bf16, B, H, N, D, 32))) return rc;
+      const int t3 = rbf::make_tmap_f32_bhnd(&f.tm_dq_acc, ws.dq_acc, B, H, N, n_pad, D, 32);
       if (t3 != 0)
         return fail(RBF_B200_ERR_TENSOR_MAP, "cuTensorMapEncodeTiled failed for the dQ accumulator (code %d)", t3);
     }

@@ -75,6 +75,20 @@ __device__ __forceinline__ uint32_t status_unit(const volatile int* unit_ptr) {
   return blockIdx.y * gridDim.x + blockIdx.x;
 }
 
+// Non-blocking look at a phase: issued ahead of independent work, it takes the barrier's latency off a wait that is
+// already over when the thread gets to it.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait. Returns false when the wait ran out (after `limit` SM clocks) or another thread of the CTA raised
 // `abort_flag`. The first wait of a launch that runs out records (site, work unit) in the status word.
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
@@ -157,9 +171,11 @@ __device__ __forceinline__ void tma_store_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
-// Fire-and-forget fp32 add into global memory (performed in L2).
-__device__ __forceinline__ void red_add_f32(float* dst, float v) {
-  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst), "f"(v) : "memory");
+// Fire-and-forget fp32 add of four consecutive floats into global memory (performed in L2; 16-byte aligned).
+__device__ __forceinline__ void red_add_v4(float* dst, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(v0)),
+               "f"(__uint_as_float(v1)), "f"(__uint_as_float(v2)), "f"(__uint_as_float(v3))
+               : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -243,6 +259,14 @@ __device__ __forceinline__ SmemDesc make_sdesc_slab32(uint32_t smem_addr) {
 }
 __device__ __forceinline__ uint64_t sdesc_at(const SmemDesc& d, uint32_t byte_offset) {
   return (static_cast<uint64_t>(d.hi) << 32) | static_cast<uint64_t>(d.lo + (byte_offset >> 4));
+}
+
+// True in one lane of a converged warp. A warp that issues MMAs runs its loops with all lanes and branches on this only
+// around the instructions: descriptors and addresses then stay warp-uniform.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
 }
 
 // D[tmem] (+)= A[smem] * B[smem]
