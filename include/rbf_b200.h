@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define RBF_B200_ABI_VERSION 3
+#define RBF_B200_ABI_VERSION 4
 
 enum {
   RBF_B200_OK = 0,
@@ -104,6 +104,25 @@ int rbf_b200_bwd_phases(const void* q, const void* k, const void* v, const void*
                         const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
                         const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides, int dtype,
                         int causal, int softmax, float sm_scale, void* stream, int phases);
+
+/* The same calls with `status_slot`: the device-side address (rbf_b200_map_status_slots) of a 4-byte word in mapped
+ * page-locked host memory, or NULL. The call's last kernel stores the launch's status word there when everything before
+ * it has finished (the forward: the last block to leave; the single-kernel backward: its dQ conversion), which saves the
+ * kernel of its own that rbf_b200_post_device_status enqueues; calls on other paths (fp32 tensors, the two-kernel
+ * backward) enqueue that kernel. Only a call whose phases include a main kernel posts. */
+int rbf_b200_fwd_posting(const void* q, const void* k, const void* v, void* out, float* lse, void* workspace,
+                        size_t workspace_bytes, int B, int H, int N, int D, const int64_t* q_strides,
+                        const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides, int dtype,
+                        int causal, int softmax, float sm_scale, void* stream, int phases, unsigned int* status_slot);
+int rbf_b200_bwd_posting(const void* q, const void* k, const void* v, const void* out, const float* lse,
+                        const void* dout, void* dq, void* dk, void* dv, void* workspace, size_t workspace_bytes, int B,
+                        int H, int N, int D, const int64_t* q_strides, const int64_t* k_strides,
+                        const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
+                        const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides, int dtype,
+                        int causal, int softmax, float sm_scale, void* stream, int phases, unsigned int* status_slot);
+/* Device-side address of `host_slots` (page-locked host memory mapped into the current device's address space). */
+int rbf_b200_map_status_slots(unsigned int* host_slots, unsigned int** device_slots);
+
 
 /* Forward for callers that cannot hand over device memory of their own. It has no counterpart in the reference,
  * whose launchers allocate freely through torch. Some hosts of this library cannot do that: a plug-in running

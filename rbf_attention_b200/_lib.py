@@ -12,7 +12,7 @@ import os
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "librbf_b200.so")
 
-ABI_VERSION = 3
+ABI_VERSION = 4
 
 STATUS_NAMES = {
     0: "ok",
@@ -26,6 +26,7 @@ STATUS_NAMES = {
 
 # Every symbol include/rbf_b200.h declares, with its ctypes signature.
 _c_i64p = ctypes.POINTER(ctypes.c_int64)
+I64x3 = ctypes.c_int64 * 3
 SIGNATURES = {
     "rbf_b200_abi_version": (ctypes.c_int, []),
     "rbf_b200_last_error": (ctypes.c_char_p, []),
@@ -50,6 +51,17 @@ SIGNATURES = {
         [ctypes.c_void_p] * 10 + [ctypes.c_size_t] + [ctypes.c_int] * 4 + [_c_i64p] * 8
         + [ctypes.c_int] * 3 + [ctypes.c_float, ctypes.c_void_p, ctypes.c_int],
     ),
+    "rbf_b200_fwd_posting": (
+        ctypes.c_int,
+        [ctypes.c_void_p] * 6 + [ctypes.c_size_t] + [ctypes.c_int] * 4 + [_c_i64p] * 4
+        + [ctypes.c_int] * 3 + [ctypes.c_float, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p],
+    ),
+    "rbf_b200_bwd_posting": (
+        ctypes.c_int,
+        [ctypes.c_void_p] * 10 + [ctypes.c_size_t] + [ctypes.c_int] * 4 + [_c_i64p] * 8
+        + [ctypes.c_int] * 3 + [ctypes.c_float, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p],
+    ),
+    "rbf_b200_map_status_slots": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p)]),
     "rbf_b200_static_scratch_bytes": (ctypes.c_size_t, []),
     "rbf_b200_fwd_static": (
         ctypes.c_int,
@@ -145,7 +157,7 @@ def load() -> ctypes.CDLL:
 def strides3(t) -> ctypes.Array:
     """Element strides of dims (b, h, n) of a (B, H, N, D) tensor as an int64[3]."""
     s = t.stride()
-    return (ctypes.c_int64 * 3)(s[0], s[1], s[2])
+    return I64x3(s[0], s[1], s[2])
 
 
 def check(rc: int, what: str) -> None:

@@ -35,7 +35,7 @@ struct Workspace {
   float* ksq;        // backward: c|k|^2 per row
   float* row_bias;   // query norms (non-softmax) or the forward's L re-pitched to n_pad (softmax backward)
   float* delta;      // backward only
-  void* lslab;       // single-kernel backward only: L and delta bias slabs, fp32 dQ accumulator (D floats per padded row)
+  void* lslab;       // single-kernel backward only: L and delta bias slabs, fp32 (B, H, N, D) dQ accumulator
   void* dslab;
   float* dq_acc;
   size_t bytes;
@@ -86,7 +86,7 @@ Workspace carve(void* base, int B, int H, int N, int D, int softmax, int backwar
       w.dslab = p + off;
       off += slab;
       w.dq_acc = reinterpret_cast<float*>(p + off);
-      off += align256(rows * D * sizeof(float));
+      off += align256(static_cast<size_t>(B) * H * N * D * sizeof(float));
     }
   }
   w.bytes = off;
@@ -159,7 +159,7 @@ size_t rbf_b200_workspace_bytes(int B, int H, int N, int D, int softmax, int bac
 static int fwd_tf32(const void* q, const void* k, const void* v, void* out, float* lse, void* workspace,
                     size_t workspace_bytes, int B, int H, int N, int D, const int64_t* q_strides,
                     const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides, int causal,
-                    int softmax, float sm_scale, void* stream_v, int phases) {
+                    int softmax, float sm_scale, void* stream_v, int phases, unsigned int* status_slot) {
   int rc;
   if ((rc = check_common(B, H, N, 64, 0, sm_scale))) return rc;
   if (D != 64) return fail(RBF_B200_ERR_BAD_ARGUMENT, "fp32 tensors (TF32 operands) are supported at head dim 64, got %d", D);
@@ -209,19 +209,21 @@ static int fwd_tf32(const void* q, const void* k, const void* v, void* out, floa
   a.qsq = ws.row_bias; a.lse = lse; a.status = ws.status;
   a.B = B; a.H = H; a.N = N; a.n_pad = n_pad; a.causal = causal ? 1 : 0; a.scale2 = 2.f * c; a.slab_w = 1.0f;
   e = rbf::launch_fwd_tf32(a, softmax != 0, stream);
+  if (e == cudaSuccess && status_slot != nullptr) e = rbf::launch_post_status(ws.status, status_slot, stream);
   if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "forward launch failed: %s", cudaGetErrorString(e));
   return RBF_B200_OK;
 }
 
-int rbf_b200_fwd_phases(const void* q, const void* k, const void* v, void* out, float* lse, void* workspace,
-                        size_t workspace_bytes, int B, int H, int N, int D, const int64_t* q_strides,
-                        const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides, int dtype,
-                        int causal, int softmax, float sm_scale, void* stream_v, int phases) {
+int rbf_b200_fwd_posting(const void* q, const void* k, const void* v, void* out, float* lse, void* workspace,
+                         size_t workspace_bytes, int B, int H, int N, int D, const int64_t* q_strides,
+                         const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides, int dtype,
+                         int causal, int softmax, float sm_scale, void* stream_v, int phases,
+                         unsigned int* status_slot) {
   g_last_error[0] = 0;
   int rc;
   if (dtype == 2)
     return fwd_tf32(q, k, v, out, lse, workspace, workspace_bytes, B, H, N, D, q_strides, k_strides, v_strides,
-                    o_strides, causal, softmax, sm_scale, stream_v, phases);
+                    o_strides, causal, softmax, sm_scale, stream_v, phases, status_slot);
   if ((rc = check_common(B, H, N, D, dtype, sm_scale))) return rc;
   if ((rc = check_tensor("q", q, q_strides, B, H, N, D))) return rc;
   if ((rc = check_tensor("k", k, k_strides, B, H, N, D))) return rc;
@@ -265,9 +267,18 @@ int rbf_b200_fwd_phases(const void* q, const void* k, const void* v, void* out, 
   a.slab_w = slab_w(bf16);
   a.qsq = ws.row_bias; a.lse = lse; a.status = ws.status;
   a.B = B; a.H = H; a.N = N; a.n_pad = n_pad; a.causal = causal ? 1 : 0; a.scale2 = 2.f * c;
+  a.status_slot = status_slot;
   e = rbf::launch_fwd(a, bf16, D, softmax != 0, stream);
   if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "forward launch failed: %s", cudaGetErrorString(e));
   return RBF_B200_OK;
+}
+
+int rbf_b200_fwd_phases(const void* q, const void* k, const void* v, void* out, float* lse, void* workspace,
+                        size_t workspace_bytes, int B, int H, int N, int D, const int64_t* q_strides,
+                        const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides, int dtype,
+                        int causal, int softmax, float sm_scale, void* stream_v, int phases) {
+  return rbf_b200_fwd_posting(q, k, v, out, lse, workspace, workspace_bytes, B, H, N, D, q_strides, k_strides, v_strides,
+                              o_strides, dtype, causal, softmax, sm_scale, stream_v, phases, nullptr);
 }
 
 int rbf_b200_fwd(const void* q, const void* k, const void* v, void* out, float* lse, void* workspace,
@@ -278,12 +289,13 @@ int rbf_b200_fwd(const void* q, const void* k, const void* v, void* out, float* 
                              v_strides, o_strides, dtype, causal, softmax, sm_scale, stream_v, RBF_B200_PHASE_ALL);
 }
 
-int rbf_b200_bwd_phases(const void* q, const void* k, const void* v, const void* out, const float* lse,
-                        const void* dout, void* dq, void* dk, void* dv, void* workspace, size_t workspace_bytes, int B,
-                        int H, int N, int D, const int64_t* q_strides, const int64_t* k_strides,
-                        const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
-                        const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides, int dtype,
-                        int causal, int softmax, float sm_scale, void* stream_v, int phases) {
+int rbf_b200_bwd_posting(const void* q, const void* k, const void* v, const void* out, const float* lse,
+                         const void* dout, void* dq, void* dk, void* dv, void* workspace, size_t workspace_bytes, int B,
+                         int H, int N, int D, const int64_t* q_strides, const int64_t* k_strides,
+                         const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
+                         const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides, int dtype,
+                         int causal, int softmax, float sm_scale, void* stream_v, int phases,
+                          unsigned int* status_slot) {
   g_last_error[0] = 0;
   int rc;
   if ((rc = check_common(B, H, N, D, dtype, sm_scale))) return rc;
@@ -362,7 +374,7 @@ int rbf_b200_bwd_phases(const void* q, const void* k, const void* v, const void*
       // the kernel's drain warps store 32 rows of dK and dV each
       if ((rc = make_map(&f.tm_dk, "dk", dk, dk_strides, bf16, B, H, N, D, 32))) return rc;
       if ((rc = make_map(&f.tm_dv, "dv", dv, dv_strides, bf16, B, H, N, D, 32))) return rc;
-      const int t3 = rbf::make_tmap_f32_bhnd(&f.tm_dq_acc, ws.dq_acc, B, H, N, n_pad, D, 32);
+      const int t3 = rbf::make_tmap_f32_bhnd(&f.tm_dq_acc, ws.dq_acc, B, H, N, D, 32);
       if (t3 != 0)
         return fail(RBF_B200_ERR_TENSOR_MAP, "cuTensorMapEncodeTiled failed for the dQ accumulator (code %d)", t3);
     }
@@ -375,6 +387,7 @@ int rbf_b200_bwd_phases(const void* q, const void* k, const void* v, const void*
     if (!softmax) { f.q_rows = q; set_strides(f.q_strides, q_strides); f.delta = ws.delta; }
     f.B = B; f.H = H; f.N = N; f.n_pad = n_pad; f.causal = causal ? 1 : 0;
     f.scale2 = 2.f * c; f.grad_scale = 2.f * sm_scale; f.slab_w = slab_w(bf16);
+    f.status_slot = status_slot;
     e = D == 128 ? rbf::launch_bwd_fused128(f, bf16, stream) : rbf::launch_bwd_fused(f, bf16, stream);
     if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "backward launch failed: %s", cudaGetErrorString(e));
     return RBF_B200_OK;
@@ -395,7 +408,22 @@ int rbf_b200_bwd_phases(const void* q, const void* k, const void* v, const void*
     e = rbf::launch_bwd_dq(a, bf16, D, softmax != 0, stream);
     if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "dQ launch failed: %s", cudaGetErrorString(e));
   }
+  if (status_slot != nullptr && (phases & (RBF_B200_PHASE_MAIN | RBF_B200_PHASE_MAIN2))) {
+    e = rbf::launch_post_status(ws.status, status_slot, stream);
+    if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "status launch failed: %s", cudaGetErrorString(e));
+  }
   return RBF_B200_OK;
+}
+
+int rbf_b200_bwd_phases(const void* q, const void* k, const void* v, const void* out, const float* lse,
+                        const void* dout, void* dq, void* dk, void* dv, void* workspace, size_t workspace_bytes, int B,
+                        int H, int N, int D, const int64_t* q_strides, const int64_t* k_strides,
+                        const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
+                        const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides, int dtype,
+                        int causal, int softmax, float sm_scale, void* stream_v, int phases) {
+  return rbf_b200_bwd_posting(q, k, v, out, lse, dout, dq, dk, dv, workspace, workspace_bytes, B, H, N, D, q_strides,
+                              k_strides, v_strides, o_strides, do_strides, dq_strides, dk_strides, dv_strides, dtype,
+                              causal, softmax, sm_scale, stream_v, phases, nullptr);
 }
 
 int rbf_b200_bwd(const void* q, const void* k, const void* v, const void* out, const float* lse, const void* dout,
@@ -765,6 +793,20 @@ int rbf_b200_scale_unless_one(void* x, const float* factor, int64_t n, int dtype
   if (sms <= 0) return fail(RBF_B200_ERR_LAUNCH, "cannot read the SM count of the current device");
   const cudaError_t e = rbf::launch_scale_unless_one(x, factor, n, dtype, sms, static_cast<cudaStream_t>(stream_v));
   if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "scale launch failed: %s", cudaGetErrorString(e));
+  return RBF_B200_OK;
+}
+
+int rbf_b200_map_status_slots(unsigned int* host_slots, unsigned int** device_slots) {
+  g_last_error[0] = 0;
+  if (host_slots == nullptr || device_slots == nullptr)
+    return fail(RBF_B200_ERR_BAD_ARGUMENT, "host_slots and device_slots must not be NULL");
+  void* dev_ptr = nullptr;
+  const cudaError_t e = cudaHostGetDevicePointer(&dev_ptr, host_slots, 0);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(RBF_B200_ERR_BAD_ARGUMENT, "host_slots is not mapped page-locked host memory: %s", cudaGetErrorString(e));
+  }
+  *device_slots = static_cast<unsigned int*>(dev_ptr);
   return RBF_B200_OK;
 }
 

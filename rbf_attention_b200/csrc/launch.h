@@ -27,7 +27,7 @@ struct RowStatsArgs {
   void* kslab_out;        // -ksq / (scale2 * slab_w); -slab_big on padding rows
   void* lslab_out;        // -lse / (scale2 * slab_w); -slab_big on padding rows
   void* dslab_out;        // -delta / slab_w; 0 on padding rows
-  float* zero_rows;       // optional (B*H, n_pad, D) fp32 array to clear (the backward's dQ accumulator)
+  float* zero_rows;       // optional (B*H, N, D) fp32 array to clear (the backward's dQ accumulator)
   int lslab_from_qsq;     // non-softmax variant: the L slab carries -qsq / (scale2 * slab_w) instead
   int dslab_zero;         // non-softmax variant: dS = P * dP, nothing is subtracted
   float scale2, slab_w, slab_big;
@@ -175,6 +175,7 @@ struct FwdArgs {
   int B, H, N, n_pad;
   int causal;
   float scale2;           // 2 * gamma * log2(e)
+  unsigned int* status_slot;   // optional: device-side address of a mapped host word that gets the status word
 };
 cudaError_t launch_fwd(const FwdArgs& a, bool bf16, int D, bool softmax, cudaStream_t stream);
 // fp32 tensors on TF32 operands, head dim 64 (tensor maps of fp32 tiles, slabs of 8 floats per row; slab_w unused)
@@ -217,7 +218,7 @@ struct BwdFusedArgs {
   CUtensorMap tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv;
   CUtensorMap tm_lslab, tm_dslab;  // (B*H, n_pad, 16) bias slabs of -L / scale2 and -delta, box 16 x 128
   CUtensorMap tm_dq_acc;  // head dim 64: the accumulator as 32-float x 32-row boxes, 128-byte swizzle
-  float* dq_acc;          // fp32 accumulator, n_pad x D floats per (batch, head): rows at D = 64, see the kernel at D = 128
+  float* dq_acc;          // fp32 (B, H, N, D) contiguous accumulator
   void* dq;               // final dQ in the operand type
   int64_t dq_strides[3];
   const float* ksq;       // (B*H, n_pad); head dim 64 only (the head-dim-128 kernel takes the norms from its K tile)
@@ -231,6 +232,7 @@ struct BwdFusedArgs {
   int B, H, N, n_pad;
   int causal;
   float scale2, grad_scale, slab_w;
+  unsigned int* status_slot;   // optional, as in FwdArgs: posted by the dQ conversion, which runs after the main kernel
 };
 cudaError_t launch_bwd_fused(const BwdFusedArgs& a, bool bf16, cudaStream_t stream);      // D = 64
 cudaError_t launch_bwd_fused128(const BwdFusedArgs& a, bool bf16, cudaStream_t stream);   // D = 128

@@ -20,6 +20,13 @@ struct DeviceStatus {
   unsigned int code;   // 0 = ok; otherwise (site << 24) | (work unit & 0xffffff), see status_unit()
 };
 
+// Hands the status word to the host: a plain store into page-locked host memory mapped into the device's address space,
+// so that no copy engine takes part and the word arrives even while the engines are busy with bulk transfers.
+__device__ __forceinline__ void post_status_word(const DeviceStatus* status, unsigned int* host_slot) {
+  *reinterpret_cast<volatile unsigned int*>(host_slot) = *reinterpret_cast<const volatile unsigned int*>(&status->code);
+  __threadfence_system();
+}
+
 static constexpr long long kWaitCycleLimit = 2000000000ll;  // about one second of SM clocks
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -171,11 +178,9 @@ __device__ __forceinline__ void tma_store_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
-// Fire-and-forget fp32 add of four consecutive floats into global memory (performed in L2; 16-byte aligned).
-__device__ __forceinline__ void red_add_v4(float* dst, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
-  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(v0)),
-               "f"(__uint_as_float(v1)), "f"(__uint_as_float(v2)), "f"(__uint_as_float(v3))
-               : "memory");
+// Fire-and-forget fp32 add into global memory (performed in L2).
+__device__ __forceinline__ void red_add_f32(float* dst, float v) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst), "f"(v) : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -95,7 +95,7 @@ enum Site : uint32_t {
 
 struct Params {
   const float* ksq;      // (B*H, n_pad), +inf on padding rows
-  float* dq_acc;         // fp32 (B*H, n_pad, 64), zero-initialised
+  float* dq_acc;         // fp32 (B*H, N, 64), zero-initialised
   DeviceStatus* status;
   unsigned int* work;    // [0] items taken beyond the CTAs' first, [1] CTAs that have left; zero at launch and at its end
   int total_items;       // key tiles x (batch, head) pairs
@@ -688,13 +688,15 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
   }
 }
 
-// dq[b,h,n,:] = scale * acc[b,h,n,:]  (acc fp32 (B*H, n_pad, D), dq 16-bit with strides)
+// dq[b,h,n,:] = scale * acc[b,h,n,:]  (acc fp32 contiguous, dq 16-bit with strides)
 template <bool kBf16>
 __global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict__ acc, void* __restrict__ dq, int H,
                                                          int N, int64_t sb, int64_t sh, int64_t sn, float scale,
                                                          int64_t total_chunks, const void* __restrict__ q,
                                                          int64_t qsb, int64_t qsh, int64_t qsn,
-                                                         const float* __restrict__ delta, int n_pad) {
+                                                         const float* __restrict__ delta, int n_pad,
+                                                         const DeviceStatus* status, unsigned int* status_slot) {
+  if (status_slot != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) post_status_word(status, status_slot);
   // one thread per 8 consecutive elements of a row (D = 64: 8 chunks per row)
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total_chunks) return;
@@ -703,7 +705,7 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict
   const int64_t n = row % N;
   const int64_t bh = row / N;
   const int64_t b = bh / H, h = bh % H;
-  const float4* src = reinterpret_cast<const float4*>(acc + (bh * n_pad + n) * D + ch * 8);
+  const float4* src = reinterpret_cast<const float4*>(acc + row * D + ch * 8);
   float4 a = src[0], c = src[1];
   if (q != nullptr) {
     // non-softmax variant: subtract delta[row] * q[row, :]
@@ -748,7 +750,7 @@ static cudaError_t launch_t(const BwdFusedArgs& a, cudaStream_t stream) {
   const int64_t chunks = static_cast<int64_t>(a.B) * a.H * a.N * 8;
   dq_convert_kernel<kBf16><<<static_cast<unsigned>((chunks + 255) / 256), 256, 0, stream>>>(
       a.dq_acc, a.dq, a.H, a.N, a.dq_strides[0], a.dq_strides[1], a.dq_strides[2], a.grad_scale, chunks, a.q_rows,
-      a.q_strides[0], a.q_strides[1], a.q_strides[2], a.delta, a.n_pad);
+      a.q_strides[0], a.q_strides[1], a.q_strides[2], a.delta, a.n_pad, a.status, a.status_slot);
   return cudaGetLastError();
 }
 

@@ -11,10 +11,10 @@
 //   dK  [128 x 128] += dS^T Q          TMEM x smem (dS^T: 32 TMEM columns of 16-bit pairs)
 //   dQ^T[128 d x 64 q] = K^T dS^T      smem x smem (K read M-major; dS^T a second time, as a [key][query]
 //                                      shared-memory tile of 128-byte rows read N-major)
-// dQ^T leaves the CTA straight from registers: a drain thread owns one head-dim index, and the fp32 accumulator is laid
-// out as [64-query step][query / 4][head dim][query % 4], so that one red.global.add.v4 per four queries covers 512
-// consecutive bytes per warp (with one scalar red per query - 128 bytes - a pass at B2 H32 N16384 took 17.06 ms, now
-// 16.89). No shared-memory staging: shared-memory bandwidth is what bounds this kernel (the MMA operand fetch alone runs at about 120 of the 128 bytes per clock). A small
+// dQ^T leaves the CTA straight from registers: a drain thread owns one head-dim index, so for every query of the
+// step the 32 lanes of a warp hold 32 consecutive floats of the (B, H, N, D) fp32 accumulator and one scalar
+// red.global.add per query is a coalesced 128-byte line. No shared-memory staging: shared-memory bandwidth is
+// what bounds this kernel (the MMA operand fetch alone runs at about 120 of the 128 bytes per clock). A small
 // kernel scales and converts the accumulator afterwards. (Every SM can push about 25 bytes per clock of
 // reduce-adds into L2, measured; a step's 32 KB of dQ therefore takes as long as its MMAs and must overlap them.)
 //
@@ -84,7 +84,7 @@ enum Site : uint32_t {
 };
 
 struct Params {
-  float* dq_acc;         // fp32 (B*H, n_pad / 64, 16, 128, 4), zero-initialised
+  float* dq_acc;         // fp32 (B, H, N, 128), zero-initialised
   DeviceStatus* status;
   int H, N, n_pad, causal;
   float scale2, grad_scale, slab_w;
@@ -333,14 +333,14 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     setmaxnreg_dec<kDrainRegs>();
     const int wq = warp & 3;                                // TMEM lane quadrant = 32 head-dim rows
     const uint32_t lane_sel = static_cast<uint32_t>(wq * 32) << 16;
-    float* acc_col = p.dq_acc + static_cast<int64_t>(bh) * p.n_pad * D + (wq * 32 + lane) * 4;
+    float* acc_col = p.dq_acc + static_cast<int64_t>(bh) * p.N * D + wq * 32 + lane;
     bool ok = true;
     for (int n = 0; n < cnt; ++n) {
       ok = mbar_wait(dq_full, n & 1, abort_flag, p.status, kSiteDQFull);
       if (!ok) break;
       tc_fence_after_sync();
       const int q0 = (first + n) * kQStep;
-      const int groups = (p.N - q0 + 3) >> 2;               // groups of four queries inside the sequence (the rest is 0)
+      const int valid = p.N - q0;                           // queries of this step inside the sequence
       float* dst = acc_col + static_cast<int64_t>(q0) * D;
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
@@ -351,10 +351,14 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
           tc_fence_before_sync();
           mbar_arrive_warp(dq_drained);   // the next dQ^T MMA may overwrite TMEM
         }
+        if (valid >= kQStep) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (hh * 8 + i < groups)
-            red_add_v4(dst + (hh * 8 + i) * (4 * D), v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          for (int i = 0; i < 32; ++i) red_add_f32(dst + (hh * 32 + i) * D, __uint_as_float(v[i]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (hh * 32 + i < valid) red_add_f32(dst + (hh * 32 + i) * D, __uint_as_float(v[i]));
+        }
       }
     }
   } else {
@@ -532,47 +536,41 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   if (warp == kMmaWarpA) tmem_dealloc(tmem, 512);
 }
 
-// dq[b,h,n,:] = scale * acc[b,h,n,:]  (dq 16-bit with strides). A block converts 64 queries; a thread takes two
-// head-dim columns of four queries (32 consecutive bytes of the accumulator), so that a warp reads 1 KB and writes half
-// a row (128 bytes) of four queries.
+// dq[b,h,n,:] = scale * acc[b,h,n,:]  (acc fp32 contiguous, dq 16-bit with strides); one thread per 8 elements
 template <bool kBf16>
 __global__ void __launch_bounds__(256) dq_convert128_kernel(const float* __restrict__ acc, void* __restrict__ dq,
                                                             int H, int N, int64_t sb, int64_t sh, int64_t sn,
-                                                            float scale, const void* __restrict__ q, int64_t qsb,
-                                                            int64_t qsh, int64_t qsn,
-                                                            const float* __restrict__ delta, int n_pad) {
-  const int bh = blockIdx.y, b = bh / H, h = bh % H;
-  const int col = (threadIdx.x & 63) * 2;                     // two columns; 64 threads per group of four queries
-  const int q0 = blockIdx.x * kQStep;
-  const float* src = acc + (static_cast<int64_t>(bh) * n_pad + q0) * D + col * 4;
-  float4 x[4], y[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {                               // all loads first; the accumulator is padded to whole tiles
-    const int g = (threadIdx.x >> 6) + i * 4;
-    x[i] = *reinterpret_cast<const float4*>(src + g * (4 * D));
-    y[i] = *reinterpret_cast<const float4*>(src + g * (4 * D) + 4);
+                                                            float scale, int64_t total_chunks,
+                                                            const void* __restrict__ q, int64_t qsb, int64_t qsh,
+                                                            int64_t qsn, const float* __restrict__ delta, int n_pad,
+                                                            const DeviceStatus* status, unsigned int* status_slot) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (status_slot != nullptr && i == 0) post_status_word(status, status_slot);
+  if (i >= total_chunks) return;
+  const int64_t row = i >> 4;
+  const int ch = static_cast<int>(i & 15);
+  const int64_t n = row % N;
+  const int64_t bh = row / N;
+  const int64_t b = bh / H, h = bh % H;
+  const float4* src = reinterpret_cast<const float4*>(acc + row * D + ch * 8);
+  float4 a = src[0], c = src[1];
+  if (q != nullptr) {
+    // non-softmax variant: subtract delta[row] * q[row, :]
+    const float w = delta[bh * n_pad + n];
+    const uint4 qv = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(q) + b * qsb + h * qsh +
+                                                     n * qsn + ch * 8);
+    const float2 q0 = unpack2<kBf16>(qv.x), q1 = unpack2<kBf16>(qv.y), q2 = unpack2<kBf16>(qv.z),
+                 q3 = unpack2<kBf16>(qv.w);
+    a.x = fmaf(-w, q0.x, a.x); a.y = fmaf(-w, q0.y, a.y); a.z = fmaf(-w, q1.x, a.z); a.w = fmaf(-w, q1.y, a.w);
+    c.x = fmaf(-w, q2.x, c.x); c.y = fmaf(-w, q2.y, c.y); c.z = fmaf(-w, q3.x, c.z); c.w = fmaf(-w, q3.y, c.w);
   }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int n0 = q0 + ((threadIdx.x >> 6) + i * 4) * 4;
-    const float xs[4] = {x[i].x, x[i].y, x[i].z, x[i].w}, ys[4] = {y[i].x, y[i].y, y[i].z, y[i].w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + j;
-      if (n >= N) break;
-      float a = xs[j], c = ys[j];
-      if (q != nullptr) {
-        // non-softmax variant: subtract delta[row] * q[row, :]
-        const float w = delta[static_cast<int64_t>(bh) * n_pad + n];
-        const float2 f = unpack2<kBf16>(*reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(q) +
-                                                                           b * qsb + h * qsh + n * qsn + col));
-        a = fmaf(-w, f.x, a);
-        c = fmaf(-w, f.y, c);
-      }
-      *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(dq) + b * sb + h * sh + n * sn + col) =
-          pack2<kBf16>(a * scale, c * scale);
-    }
-  }
+  uint4 o;
+  o.x = pack2<kBf16>(a.x * scale, a.y * scale);
+  o.y = pack2<kBf16>(a.z * scale, a.w * scale);
+  o.z = pack2<kBf16>(c.x * scale, c.y * scale);
+  o.w = pack2<kBf16>(c.z * scale, c.w * scale);
+  uint16_t* dst = reinterpret_cast<uint16_t*>(dq) + b * sb + h * sh + n * sn + ch * 8;
+  *reinterpret_cast<uint4*>(dst) = o;
 }
 
 template <bool kBf16>
@@ -595,9 +593,10 @@ static cudaError_t launch_t(const BwdFusedArgs& a, cudaStream_t stream) {
                                            p);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  dq_convert128_kernel<kBf16><<<dim3((a.N + kQStep - 1) / kQStep, a.B * a.H), 256, 0, stream>>>(
-      a.dq_acc, a.dq, a.H, a.N, a.dq_strides[0], a.dq_strides[1], a.dq_strides[2], a.grad_scale, a.q_rows,
-      a.q_strides[0], a.q_strides[1], a.q_strides[2], a.delta, a.n_pad);
+  const int64_t chunks = static_cast<int64_t>(a.B) * a.H * a.N * (D / 8);
+  dq_convert128_kernel<kBf16><<<static_cast<unsigned>((chunks + 255) / 256), 256, 0, stream>>>(
+      a.dq_acc, a.dq, a.H, a.N, a.dq_strides[0], a.dq_strides[1], a.dq_strides[2], a.grad_scale, chunks, a.q_rows,
+      a.q_strides[0], a.q_strides[1], a.q_strides[2], a.delta, a.n_pad, a.status, a.status_slot);
   return cudaGetLastError();
 }
 

@@ -65,9 +65,9 @@ __global__ void __launch_bounds__(256) row_stats_kernel(const RowStatsArgs a) {
 
   if (a.zero_rows != nullptr) {
     // clear this block's rows of the fp32 accumulator: the writes ride along with a kernel that mostly reads
-    const int rows_here = min(rows_per_block, a.n_pad - row_begin);
+    const int rows_here = min(rows_per_block, a.N - row_begin);
     if (rows_here > 0) {
-      float4* dst = reinterpret_cast<float4*>(a.zero_rows + (out_base + row_begin) * D);
+      float4* dst = reinterpret_cast<float4*>(a.zero_rows + (static_cast<int64_t>(bh) * a.N + row_begin) * D);
       const int n4 = rows_here * (D / 4);
       for (int i = threadIdx.x; i < n4; i += 256) dst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -512,12 +512,7 @@ __global__ void __launch_bounds__(32) wait_selftest_kernel(DeviceStatus* status,
 }
 
 __global__ void __launch_bounds__(32) post_status_kernel(const DeviceStatus* status, unsigned int* host_slot) {
-  // a plain store into page-locked host memory mapped into the device's address space: no copy engine takes part,
-  // so the word arrives even while the engines are busy with the caller's own bulk transfers
-  if (threadIdx.x == 0) {
-    *reinterpret_cast<volatile unsigned int*>(host_slot) = status->code;
-    __threadfence_system();
-  }
+  if (threadIdx.x == 0) post_status_word(status, host_slot);
 }
 
 cudaError_t launch_post_status(const DeviceStatus* status, unsigned int* host_slot_device_ptr, cudaStream_t stream) {

@@ -100,15 +100,14 @@ inline int make_tmap_slab8_f32(CUtensorMap* out, const void* base, int BH, int n
   return static_cast<int>(r);
 }
 
-// Tensor map over an fp32 (B, H, n_pad, D) accumulator of which the first N rows count; box = 32 floats (128 bytes) x
-// `box_rows`.
-inline int make_tmap_f32_bhnd(CUtensorMap* out, const void* base, int B, int H, int N, int n_pad, int D, int box_rows) {
+// Tensor map over a contiguous fp32 (B, H, N, D) accumulator; box = 32 floats (128 bytes) x `box_rows`.
+inline int make_tmap_f32_bhnd(CUtensorMap* out, const void* base, int B, int H, int N, int D, int box_rows) {
   EncodeTiledFn enc = get_encode_tiled();
   if (enc == nullptr) return -1;
   cuuint64_t gdim[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(H),
                         static_cast<cuuint64_t>(B)};
-  cuuint64_t gstr[3] = {static_cast<cuuint64_t>(D) * 4, static_cast<cuuint64_t>(n_pad) * D * 4,
-                        static_cast<cuuint64_t>(H) * n_pad * D * 4};
+  cuuint64_t gstr[3] = {static_cast<cuuint64_t>(D) * 4, static_cast<cuuint64_t>(N) * D * 4,
+                        static_cast<cuuint64_t>(H) * N * D * 4};
   cuuint32_t box[4] = {32, static_cast<cuuint32_t>(box_rows), 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base), gdim, gstr, box, estr,

@@ -10,16 +10,45 @@ Reference counterparts (paths inside the reference project):
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
+import threading
 import time
 
 import torch
+from torch.autograd import forward_ad
+from torch.autograd.function import once_differentiable
 
 from . import _lib
 
 _DTYPE_CODE = {torch.bfloat16: 0, torch.float16: 1}
 _F32_CODE = 2          # forward only: fp32 tensors on TF32 operands, head dim 64
+
+
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+
+
+def _direct(*tensors) -> bool:
+    """Whether a call may run its implementation right here instead of going through the registered operator: plain
+    CUDA tensors in eager mode, with nothing active that has to see the operator (tracing or compilation, dispatch and
+    function modes, functorch transforms, forward-mode differentiation). The operator layer - schema, fake kernels,
+    dispatch keys, aliasing checks - costs 70 to 100 us of host time per call, more than the device time of a training
+    step's attention below about 1500 tokens (B4 H8 D64: 76 us of kernels in a pass of 280 us); where the question is
+    open the operator is used."""
+    if torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack():
+        return False
+    if (torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None
+            or forward_ad._current_level >= 0):
+        return False
+    for t in tensors:
+        if t is not None and not (type(t) in _PLAIN_TYPES and t.is_cuda):
+            return False
+    return True
+
+
+def _needs_grad(*tensors) -> bool:
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
 
 
 def _validate(name: str, t: torch.Tensor, like: torch.Tensor | None = None) -> None:
@@ -45,6 +74,8 @@ def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     B, H, N, D = t.shape
     per16 = 16 // t.element_size()
     ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0
+    if ok and D % per16 == 0 and t.is_contiguous():
+        return t
     for ext, s in zip((B, H, N), t.stride()[:3]):
         if ext > 1 and (s <= 0 or s % per16 != 0):
             ok = False
@@ -114,9 +145,18 @@ class _OnDevice:
         return False
 
 
+@functools.lru_cache(maxsize=256)
+def _workspace_bytes(B, H, N, D, softmax, backward) -> int:
+    return _lib.load().rbf_b200_workspace_bytes(B, H, N, D, int(softmax), int(backward))
+
+
+@functools.lru_cache(maxsize=256)
+def _dense_strides3(H, N, D) -> ctypes.Array:
+    return _lib.I64x3(H * N * D, N * D, D)
+
+
 def _workspace(B, H, N, D, softmax, backward, device) -> torch.Tensor:
-    lib = _lib.load()
-    nbytes = lib.rbf_b200_workspace_bytes(B, H, N, D, int(softmax), int(backward))
+    nbytes = _workspace_bytes(B, H, N, D, bool(softmax), backward)
     # torch's caching allocator returns 512-byte aligned blocks, which satisfies the 256-byte rule
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
@@ -125,11 +165,11 @@ class _StatusMonitor:
     """Surfaces device-side wait timeouts of the operator path without synchronising.
 
     Every kernel bounds its waits; one that runs out leaves a non-zero status word at the start of the call's
-    workspace and the kernels return with incomplete results. After each launch a one-thread kernel on the launch
-    stream stores the word into a ring of pinned host slots (a store through the mapped host address: a copy would
-    queue on the copy engine behind the caller's own device-to-host transfers and hold the launch stream up for
-    their duration); a slot holds -1 until its word has arrived, so no event is needed to see that it has. Later
-    calls look at the slots that have been written and raise ``RuntimeError`` for a non-zero one. A timeout is therefore reported by a later operator call or by
+    workspace and the kernels return with incomplete results. Each call's last kernel stores the word into a ring of
+    pinned host slots (a store through the mapped host address: a copy would queue on the copy engine behind the
+    caller's own device-to-host transfers and hold the launch stream up for their duration); a slot holds -1 until its
+    word has arrived, so no event is needed to see that it has. Later calls look at the slots that have been written and
+    raise ``RuntimeError`` for a non-zero one. A timeout is therefore reported by a later operator call or by
     ``check_device_status()``, not by the call that suffered it. ``RBF_B200_SYNC_STATUS=1`` makes every call
     synchronise and check its own status (for debugging). Nothing is recorded while a CUDA graph is being captured.
     """
@@ -142,6 +182,11 @@ class _StatusMonitor:
         self.host = torch.zeros(self.SLOTS, dtype=torch.int32).pin_memory()
         self.slots = self.host.numpy()          # same memory: reading a slot costs 0.1 us instead of 3
         self.base = self.host.data_ptr()
+        mapped = ctypes.c_void_p()
+        with _OnDevice(device):
+            _lib.check(_lib.load().rbf_b200_map_status_slots(self.base, ctypes.byref(mapped)), "rbf_b200_map_status_slots")
+        self.mapped = mapped.value              # the ring's address on the device
+        self.lock = threading.RLock()           # forward and backward run on different threads
         self.what = [""] * self.SLOTS
         self.oldest = 0        # the pending entries are the slots oldest, oldest + 1, ..., next - 1 (mod SLOTS)
         self.next = 0
@@ -169,12 +214,13 @@ class _StatusMonitor:
         when ``wait``)."""
         if wait and self.pending:
             torch.cuda.synchronize(self.device)
-        while self.pending:
-            if self.slots[self.oldest] == self._NOT_YET:
-                if wait:
-                    raise RuntimeError(f"{self.what[self.oldest]}: the status word did not arrive")
-                break
-            self._retire_oldest()
+        with self.lock:
+            while self.pending:
+                if self.slots[self.oldest] == self._NOT_YET:
+                    if wait:
+                        raise RuntimeError(f"{self.what[self.oldest]}: the status word did not arrive")
+                    break
+                self._retire_oldest()
 
     def record_range_check(self, tensors, what):
         """fp32 tensors narrowed to fp16 operands: records (asynchronously, like the status word) whether the
@@ -186,28 +232,50 @@ class _StatusMonitor:
         flag[0] = bad
         self.record(flag, "range:" + what)
 
+    def _reserve(self, what) -> int:
+        with self.lock:
+            if self.pending == self.SLOTS:      # the ring is full: wait for its oldest entry, and for that one only
+                self.poll()
+                if self.pending == self.SLOTS:
+                    # (its kernel was enqueued SLOTS calls ago: the word arrives without any help from this thread. A
+                    # device-wide synchronisation here would also drain the caller's copy streams.)
+                    deadline = time.monotonic() + 10.0
+                    while self.slots[self.oldest] == self._NOT_YET:
+                        if time.monotonic() > deadline:
+                            torch.cuda.synchronize(self.device)
+                            break
+                        time.sleep(0)
+                    self._retire_oldest()
+            i = self.next
+            self.slots[i] = self._NOT_YET
+            self.what[i] = what
+            self.next = (i + 1) % self.SLOTS
+            self.pending += 1
+            return i
+
+    def launch(self, what, call) -> None:
+        """``call(slot address)`` enqueues a call whose last kernel posts its status word there (0: no posting, while a
+        CUDA graph is being captured) and returns its error code."""
+        if torch._C._cuda_isCurrentStreamCapturing():
+            _lib.check(call(0), what)
+            return
+        i = self._reserve(what)
+        rc = call(self.mapped + 4 * i)
+        if rc != 0:
+            self.slots[i] = 0                   # nothing was enqueued that could post
+            _lib.check(rc, what)
+        if _SYNC_STATUS:
+            self.poll(wait=True)
+
     def record(self, ws, what):
+        """Posts the status word at the start of ``ws`` with a kernel of its own."""
         if torch.cuda.is_current_stream_capturing():
             return
-        if self.pending == self.SLOTS:          # the ring is full: wait for its oldest entry, and for that one only
-            self.poll()
-            if self.pending == self.SLOTS:
-                # (its kernel was enqueued SLOTS calls ago: the word arrives without any help from this thread. A
-                # device-wide synchronisation here would also drain the caller's copy streams.)
-                deadline = time.monotonic() + 10.0
-                while self.slots[self.oldest] == self._NOT_YET:
-                    if time.monotonic() > deadline:
-                        torch.cuda.synchronize(self.device)
-                        break
-                    time.sleep(0)
-                self._retire_oldest()
-        i = self.next
-        self.slots[i] = self._NOT_YET
-        _lib.check(_lib.load().rbf_b200_post_device_status(ws.data_ptr(), self.base + 4 * i, _stream_ptr(ws.device)),
-                   "rbf_b200_post_device_status")
-        self.what[i] = what
-        self.next = (i + 1) % self.SLOTS
-        self.pending += 1
+        i = self._reserve(what)
+        rc = _lib.load().rbf_b200_post_device_status(ws.data_ptr(), self.base + 4 * i, _stream_ptr(ws.device))
+        if rc != 0:
+            self.slots[i] = 0
+            _lib.check(rc, "rbf_b200_post_device_status")
         if _SYNC_STATUS:
             self.poll(wait=True)
 
@@ -232,6 +300,13 @@ def check_device_status(device=None) -> None:
     _monitor(torch.device(device)).poll(wait=True)
 
 
+_PHASE_ALL = 7          # pre-pass and both main kernels (include/rbf_b200.h)
+
+
+def _strides3(t: torch.Tensor, dense) -> ctypes.Array:
+    return dense if t.is_contiguous() else _lib.strides3(t)
+
+
 def _forward(q, k, v, is_causal: bool, softmax: bool):
     _validate("q", q)
     _validate("k", k, q)
@@ -249,15 +324,14 @@ def _forward(q, k, v, is_causal: bool, softmax: bool):
     ws = _workspace(B, H, N, D, softmax, False, q.device)
     mon = _monitor(q.device)
     mon.poll()
+    dense = _dense_strides3(H, N, D)
     with _OnDevice(q.device):
-        rc = lib.rbf_b200_fwd(
+        mon.launch("rbf_b200_fwd", lambda slot: lib.rbf_b200_fwd_posting(
             qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(),
             lse.data_ptr() if softmax else None, ws.data_ptr(), ws.numel(),
-            B, H, N, D, _lib.strides3(qc), _lib.strides3(kc), _lib.strides3(vc), _lib.strides3(out),
-            code, int(bool(is_causal)), int(softmax), 1.0 / math.sqrt(D0), _stream_ptr(q.device),
-        )
-        _lib.check(rc, "rbf_b200_fwd")
-        mon.record(ws, "rbf_b200_fwd")
+            B, H, N, D, _strides3(qc, dense), _strides3(kc, dense), _strides3(vc, dense), dense,
+            code, int(bool(is_causal)), int(softmax), 1.0 / math.sqrt(D0), _stream_ptr(q.device), _PHASE_ALL, slot,
+        ))
         if q.dtype == torch.float32 and not tf32:
             mon.record_range_check((qc, kc, vc), "rbf_b200_fwd")
     if D != D0:
@@ -284,23 +358,22 @@ def _backward(q, k, v, out, lse, dout, is_causal: bool, sm_scale: float, softmax
     dk = torch.empty_like(dq)
     dv = torch.empty_like(dq)
     ws = _workspace(B, H, N, D, softmax, True, q.device)
-    z3 = (ctypes.c_int64 * 3)(0, 0, 0)
+    z3 = _lib.I64x3(0, 0, 0)
     mon = _monitor(q.device)
     mon.poll()
     # torch.use_deterministic_algorithms(True) selects the backward whose summation order is fixed
     lib.rbf_b200_set_deterministic(int(torch.are_deterministic_algorithms_enabled()))
+    dense = _dense_strides3(H, N, D)
     with _OnDevice(q.device):
-        rc = lib.rbf_b200_bwd(
+        mon.launch("rbf_b200_bwd", lambda slot: lib.rbf_b200_bwd_posting(
             qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
             oc.data_ptr() if have_out else None, lse.data_ptr() if softmax else None, doc.data_ptr(),
             dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(),
-            B, H, N, D, _lib.strides3(qc), _lib.strides3(kc), _lib.strides3(vc),
-            _lib.strides3(oc) if have_out else z3, _lib.strides3(doc),
-            _lib.strides3(dq), _lib.strides3(dk), _lib.strides3(dv),
-            _DTYPE_CODE[cdt], int(bool(is_causal)), int(softmax), float(sm_scale), _stream_ptr(q.device),
-        )
-        _lib.check(rc, "rbf_b200_bwd")
-        mon.record(ws, "rbf_b200_bwd")
+            B, H, N, D, _strides3(qc, dense), _strides3(kc, dense), _strides3(vc, dense),
+            _strides3(oc, dense) if have_out else z3, _strides3(doc, dense),
+            dense, dense, dense,
+            _DTYPE_CODE[cdt], int(bool(is_causal)), int(softmax), float(sm_scale), _stream_ptr(q.device), _PHASE_ALL, slot,
+        ))
         if q.dtype == torch.float32:
             mon.record_range_check((qc, kc, vc, doc), "rbf_b200_bwd")
     if D != D0:
@@ -497,11 +570,11 @@ def susie_block_fwd(
     if table.shape[0] < S - R:
         raise ValueError(f"the position table holds {table.shape[0]} rows, {S - R} text positions are needed")
     qk = torch.empty((2, B, S, H, D), dtype=qkv.dtype, device=dev)
-    out = torch.empty((B, S, H, D), dtype=qkv.dtype, device=dev)
+    out = torch.empty((B, S, E), dtype=qkv.dtype, device=dev)
     lse = torch.empty((B, H, S) if softmax else (0,), dtype=torch.float32, device=dev)
     q, k = _bhsd_view(qk[0]), _bhsd_view(qk[1])
     v = _bhsd_view(qkv.view(B, S, 3, H, D)[:, :, 2])
-    o = _bhsd_view(out)
+    o = _bhsd_view(out.view(B, S, H, D))
     ws = _workspace(B, H, S, D, softmax, False, dev)
     scale = 1.0 / math.sqrt(D)
     mon = _monitor(dev)
@@ -513,13 +586,11 @@ def susie_block_fwd(
             q.data_ptr(), k.data_ptr(), _lib.strides3(q), _lib.strides3(k), ws.data_ptr(), ws.numel(),
             B, S, H, D, R, _DTYPE_CODE[qkv.dtype], int(softmax), scale, stream)
         _lib.check(rc, "rbf_b200_qkv_prep")
-        rc = lib.rbf_b200_fwd_phases(
+        mon.launch("rbf_b200_fwd (attention block)", lambda slot: lib.rbf_b200_fwd_posting(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr() if softmax else None,
             ws.data_ptr(), ws.numel(), B, H, S, D, _lib.strides3(q), _lib.strides3(k), _lib.strides3(v),
-            _lib.strides3(o), _DTYPE_CODE[qkv.dtype], 1, int(softmax), scale, stream, 2)
-        _lib.check(rc, "rbf_b200_fwd")
-        mon.record(ws, "rbf_b200_fwd (attention block)")
-    return out.view(B, S, E), lse, qk
+            _lib.strides3(o), _DTYPE_CODE[qkv.dtype], 1, int(softmax), scale, stream, 2, slot))
+    return out, lse, qk
 
 
 @susie_block_fwd.register_fake
@@ -571,13 +642,12 @@ def susie_block_bwd(
     lib.rbf_b200_set_deterministic(int(torch.are_deterministic_algorithms_enabled()))
     with _OnDevice(dev):
         stream = _stream_ptr(dev)
-        rc = lib.rbf_b200_bwd(
+        mon.launch("rbf_b200_bwd (attention block)", lambda slot: lib.rbf_b200_bwd_posting(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr() if softmax else None,
             do.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(), B, H, S, D,
             _lib.strides3(q), _lib.strides3(k), _lib.strides3(v), _lib.strides3(o), _lib.strides3(do),
-            _lib.strides3(dq), _lib.strides3(dk), _lib.strides3(dv), dt, 1, int(softmax), 1.0 / math.sqrt(D), stream)
-        _lib.check(rc, "rbf_b200_bwd")
-        mon.record(ws, "rbf_b200_bwd (attention block)")
+            _lib.strides3(dq), _lib.strides3(dk), _lib.strides3(dv), dt, 1, int(softmax), 1.0 / math.sqrt(D), stream,
+            _PHASE_ALL, slot))
         rc = lib.rbf_b200_qkv_prep_bwd(
             dq.data_ptr(), dk.data_ptr(), _lib.strides3(dq), _lib.strides3(dk), table.data_ptr(), d_pw.data_ptr(),
             d_rp.data_ptr() if R > 0 else None, ws2.data_ptr(), nb2, B, S, H, D, R, dt, stream)

@@ -115,6 +115,7 @@ def test_training_step_entries_validate_before_any_launch(built_library):
     assert lib.rbf_b200_column_sums(p, None, p, 1 << 20, 8, 16, 16, 0, None) == 1
     assert lib.rbf_b200_post_device_status(None, p, None) == 1
     assert lib.rbf_b200_post_device_status(p, None, None) == 1
+    assert lib.rbf_b200_map_status_slots(None, None) == 1
 
 
 def test_gelu_entries_validate_before_any_launch(built_library):

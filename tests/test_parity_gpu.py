@@ -806,3 +806,43 @@ def test_backward_items_of_every_short_length_overlap(N, causal):
         for name, a, b in zip(("dQ", "dK", "dV"), got, want):
             # measured 1e-4; one flipped bf16 rounding in a thousand elements
             assert oracle.error_report(a.float().cpu(), b.float().cpu())["rel_l2"] <= 1e-3, name
+
+
+@pytest.mark.parametrize("D,N,softmax,deterministic", [(64, 200, True, False), (64, 3000, False, False),
+                                                       (128, 200, True, False), (64, 200, True, True)])
+def test_calls_post_their_status_word(D, N, softmax, deterministic):
+    """The posting entry points: the slot in mapped host memory gets the launch's status word (0) from the call's last
+    kernel - single- and many-item launches, both head dims, the two-kernel backward -, also when a block finds the word
+    already set and leaves at once (the word is then what was planted)."""
+    lib = _lib.load()
+    B, H = 2, 3
+    q, k, v, do = (t.to(DEV) for t in oracle.make_inputs(B, H, N, D, seed=4, dtype=torch.bfloat16))
+    out, lse = cabi_forward(q, k, v, True, softmax)
+    slots = torch.full((4,), -1, dtype=torch.int32).pin_memory()
+    mapped = ctypes.c_void_p()
+    assert lib.rbf_b200_map_status_slots(slots.data_ptr(), ctypes.byref(mapped)) == 0, lib.rbf_b200_last_error()
+    stream = torch.cuda.current_stream().cuda_stream
+    ws = torch.empty(lib.rbf_b200_workspace_bytes(B, H, N, D, int(softmax), 0), dtype=torch.uint8, device=DEV)
+
+    def forward(phases, slot):
+        return lib.rbf_b200_fwd_posting(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr() if softmax else None,
+                                        ws.data_ptr(), ws.numel(), B, H, N, D, _s3(q), _s3(k), _s3(v), _s3(out), 0, 1,
+                                        int(softmax), 1.0 / math.sqrt(D), stream, phases, mapped.value + 4 * slot)
+
+    assert forward(7, 0) == 0
+    ws[:4] = torch.tensor([7, 0, 0, 1], dtype=torch.uint8)        # site 1, unit 7
+    assert forward(2, 1) == 0                                     # main kernel alone: every block leaves at once
+    ws2 = torch.empty(lib.rbf_b200_workspace_bytes(B, H, N, D, int(softmax), 1), dtype=torch.uint8, device=DEV)
+    dq, dk, dv = (torch.empty_like(q) for _ in range(3))
+    lib.rbf_b200_set_deterministic(int(deterministic))
+    try:
+        rc = lib.rbf_b200_bwd_posting(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
+                                      lse.data_ptr() if softmax else None, do.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+                                      dv.data_ptr(), ws2.data_ptr(), ws2.numel(), B, H, N, D, _s3(q), _s3(k), _s3(v),
+                                      _s3(out), _s3(do), _s3(dq), _s3(dk), _s3(dv), 0, 1, int(softmax),
+                                      1.0 / math.sqrt(D), stream, 7, mapped.value + 8)
+    finally:
+        lib.rbf_b200_set_deterministic(0)
+    assert rc == 0, lib.rbf_b200_last_error()
+    torch.cuda.synchronize()
+    assert slots.tolist() == [0, (1 << 24) | 7, 0, -1]
