@@ -536,8 +536,7 @@ def _bhsd_view(t: torch.Tensor) -> torch.Tensor:
     return t.permute(0, 2, 1, 3)
 
 
-@torch.library.custom_op("rbf_attn_b200::susie_block_fwd", mutates_args=())
-def susie_block_fwd(
+def _susie_block_fwd(
     qkv: torch.Tensor,
     pos_weight: torch.Tensor,
     reg_pos_emb: torch.Tensor | None,
@@ -593,6 +592,9 @@ def susie_block_fwd(
     return out, lse, qk
 
 
+susie_block_fwd = torch.library.custom_op("rbf_attn_b200::susie_block_fwd", mutates_args=())(_susie_block_fwd)
+
+
 @susie_block_fwd.register_fake
 def _(qkv, pos_weight, reg_pos_emb, table, num_heads, softmax):
     B, S, E3 = qkv.shape
@@ -605,8 +607,7 @@ def _(qkv, pos_weight, reg_pos_emb, table, num_heads, softmax):
     )
 
 
-@torch.library.custom_op("rbf_attn_b200::susie_block_bwd", mutates_args=())
-def susie_block_bwd(
+def _susie_block_bwd(
     qkv: torch.Tensor,
     qk: torch.Tensor,
     out: torch.Tensor,
@@ -655,6 +656,9 @@ def susie_block_bwd(
     return dqkv.view(B, S, 3 * E), d_pw, d_rp
 
 
+susie_block_bwd = torch.library.custom_op("rbf_attn_b200::susie_block_bwd", mutates_args=())(_susie_block_bwd)
+
+
 @susie_block_bwd.register_fake
 def _(qkv, qk, out, lse, dout, table, num_registers, softmax):
     _, B, S, H, D = qk.shape
@@ -681,8 +685,8 @@ def _susie_block_backward(ctx, dout, dlse, dqk):
     qkv, qk, out, lse, table = ctx.saved_tensors
     if dout is None:
         return None, None, None, None, None, None
-    dqkv, d_pw, d_rp = torch.ops.rbf_attn_b200.susie_block_bwd(
-        qkv, qk, out, lse, dout, table, ctx.num_registers, ctx.softmax)
+    bwd = _susie_block_bwd if _direct(qkv, qk, out, lse, dout, table) else torch.ops.rbf_attn_b200.susie_block_bwd
+    dqkv, d_pw, d_rp = bwd(qkv, qk, out, lse, dout, table, ctx.num_registers, ctx.softmax)
     d_rp = None if ctx.rp_dtype is None else d_rp.to(ctx.rp_dtype)
     return dqkv, d_pw.to(ctx.pw_dtype), d_rp, None, None, None
 
@@ -692,9 +696,28 @@ torch.library.register_autograd(
 )
 
 
+class _SusieBlock(torch.autograd.Function):
+    """``rbf_attn_b200::susie_block_fwd`` and its autograd formula for calls that go around the operator (``_direct``)."""
+
+    @staticmethod
+    def forward(ctx, qkv, pos_weight, reg_pos_emb, table, num_heads, softmax):
+        out, lse, qk = _susie_block_fwd(qkv, pos_weight, reg_pos_emb, table, num_heads, softmax)
+        _susie_block_setup_context(ctx, (qkv, pos_weight, reg_pos_emb, table, num_heads, softmax), (out, lse, qk))
+        return out
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dout):
+        return _susie_block_backward(ctx, dout, None, None)
+
+
 def susie_block_attention(qkv, pos_weight, reg_pos_emb, table, num_heads, softmax=True):
     """Attention of one block from the fused projection output: (B, S, 3 H D) -> (B, S, H D), causal, with the SuSiE
     position term and the register-position rows added to q and k inside the operator."""
+    if type(softmax) is bool and type(num_heads) is int and _direct(qkv, pos_weight, reg_pos_emb, table):
+        if _needs_grad(qkv, pos_weight, reg_pos_emb):
+            return _SusieBlock.apply(qkv, pos_weight, reg_pos_emb, table, num_heads, softmax)
+        return _susie_block_fwd(qkv, pos_weight, reg_pos_emb, table, num_heads, softmax)[0]
     return torch.ops.rbf_attn_b200.susie_block_fwd(qkv, pos_weight, reg_pos_emb, table, num_heads, softmax)[0]
 
 
@@ -767,8 +790,7 @@ def exclusive_self_attention(o, v):
 # Linear layers whose bias gradient is the library's column sum (nn.Linear in train_rbf_transformer.py:143, 216 and
 # rbf_attention.py:1625-1626)
 # ---------------------------------------------------------------------------------------------
-@torch.library.custom_op("rbf_attn_b200::column_sums", mutates_args=())
-def column_sums(x: torch.Tensor) -> torch.Tensor:
+def _column_sums(x: torch.Tensor) -> torch.Tensor:
     """fp32 sums over the rows of a 16-bit CUDA matrix (rows, cols), cols a multiple of 8."""
     if x.dim() != 2 or not x.is_cuda or x.dtype not in _DTYPE_CODE or x.shape[1] % 8 != 0:
         raise ValueError("column_sums: a 16-bit CUDA matrix whose width is a multiple of 8")
@@ -784,6 +806,9 @@ def column_sums(x: torch.Tensor) -> torch.Tensor:
                                       xc.stride(0) if rows > 1 else cols, _DTYPE_CODE[x.dtype], _stream_ptr(x.device))
     _lib.check(rc, "rbf_b200_column_sums")
     return out
+
+
+column_sums = torch.library.custom_op("rbf_attn_b200::column_sums", mutates_args=())(_column_sums)
 
 
 @column_sums.register_fake
@@ -809,12 +834,12 @@ class _LinearBiasSum(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             dw = g2.t().mm(x.reshape(-1, x.shape[-1]))
         if ctx.needs_input_grad[2]:
-            db = torch.ops.rbf_attn_b200.column_sums(g2).to(g.dtype)
+            sums = _column_sums if _direct(g2) else torch.ops.rbf_attn_b200.column_sums
+            db = sums(g2).to(g.dtype)
         return dx, dw, db
 
 
-@torch.library.custom_op("rbf_attn_b200::gelu_fwd", mutates_args=())
-def gelu_fwd(h: torch.Tensor) -> torch.Tensor:
+def _gelu_fwd(h: torch.Tensor) -> torch.Tensor:
     """Exact (erf) GELU of a 16-bit CUDA tensor whose element count is a multiple of 8."""
     if not h.is_cuda or h.dtype not in _DTYPE_CODE or h.numel() % 8 != 0:
         raise ValueError("gelu_fwd: a 16-bit CUDA tensor with a multiple of 8 elements")
@@ -827,13 +852,15 @@ def gelu_fwd(h: torch.Tensor) -> torch.Tensor:
     return out
 
 
+gelu_fwd = torch.library.custom_op("rbf_attn_b200::gelu_fwd", mutates_args=())(_gelu_fwd)
+
+
 @gelu_fwd.register_fake
 def _(h):
     return torch.empty_like(h, memory_format=torch.contiguous_format)
 
 
-@torch.library.custom_op("rbf_attn_b200::gelu_bwd", mutates_args=())
-def gelu_bwd(h: torch.Tensor, dy: torch.Tensor, with_bias: bool) -> tuple[torch.Tensor, torch.Tensor]:
+def _gelu_bwd(h: torch.Tensor, dy: torch.Tensor, with_bias: bool) -> tuple[torch.Tensor, torch.Tensor]:
     """dh = dy * gelu'(h) for (..., cols) tensors and, with ``with_bias``, its fp32 sum over all leading dims."""
     cols = h.shape[-1]
     hc, gc = h.contiguous(), dy.to(h.dtype).contiguous()
@@ -850,6 +877,9 @@ def gelu_bwd(h: torch.Tensor, dy: torch.Tensor, with_bias: bool) -> tuple[torch.
     return dh, dbias
 
 
+gelu_bwd = torch.library.custom_op("rbf_attn_b200::gelu_bwd", mutates_args=())(_gelu_bwd)
+
+
 @gelu_bwd.register_fake
 def _(h, dy, with_bias):
     return (torch.empty_like(h, memory_format=torch.contiguous_format),
@@ -864,12 +894,13 @@ class _LinearGelu(torch.autograd.Function):
     def forward(ctx, x, weight, bias):
         h = torch.nn.functional.linear(x, weight, bias)
         ctx.save_for_backward(x, weight, h)
-        return torch.ops.rbf_attn_b200.gelu_fwd(h)
+        return (_gelu_fwd if _direct(h) else torch.ops.rbf_attn_b200.gelu_fwd)(h)
 
     @staticmethod
     def backward(ctx, g):
         x, weight, h = ctx.saved_tensors
-        dh, dbias = torch.ops.rbf_attn_b200.gelu_bwd(h, g, ctx.needs_input_grad[2])
+        bwd = _gelu_bwd if _direct(h, g) else torch.ops.rbf_attn_b200.gelu_bwd
+        dh, dbias = bwd(h, g, ctx.needs_input_grad[2])
         dh2 = dh.reshape(-1, dh.shape[-1])
         dx = dh.matmul(weight) if ctx.needs_input_grad[0] else None
         dw = dh2.t().mm(x.reshape(-1, x.shape[-1])) if ctx.needs_input_grad[1] else None
@@ -905,8 +936,7 @@ def layer_norm_supported(x: torch.Tensor, weight, bias) -> bool:
             and x.shape[-1] % 256 == 0 and 0 < x.shape[-1] <= 1024)
 
 
-@torch.library.custom_op("rbf_attn_b200::layer_norm_fwd", mutates_args=())
-def layer_norm_fwd(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
+def _layer_norm_fwd(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
                    eps: float) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """y = (x - mean) * rstd * weight + bias over the last dim; returns (y, mean, rstd), the statistics in fp32."""
     if not layer_norm_supported(x, weight, bias):
@@ -926,6 +956,9 @@ def layer_norm_fwd(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
     return y, mean, rstd
 
 
+layer_norm_fwd = torch.library.custom_op("rbf_attn_b200::layer_norm_fwd", mutates_args=())(_layer_norm_fwd)
+
+
 @layer_norm_fwd.register_fake
 def _(x, weight, bias, eps):
     rows = x.numel() // x.shape[-1]
@@ -933,8 +966,7 @@ def _(x, weight, bias, eps):
             x.new_empty(rows, dtype=torch.float32))
 
 
-@torch.library.custom_op("rbf_attn_b200::layer_norm_bwd", mutates_args=())
-def layer_norm_bwd(x: torch.Tensor, dy: torch.Tensor, weight: torch.Tensor, mean: torch.Tensor,
+def _layer_norm_bwd(x: torch.Tensor, dy: torch.Tensor, weight: torch.Tensor, mean: torch.Tensor,
                    rstd: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     cols = x.shape[-1]
     xc, dyc, wc = x.contiguous(), dy.to(x.dtype).contiguous(), weight.contiguous()
@@ -953,6 +985,9 @@ def layer_norm_bwd(x: torch.Tensor, dy: torch.Tensor, weight: torch.Tensor, mean
     return dx, dgamma.to(weight.dtype), dbeta.to(weight.dtype)
 
 
+layer_norm_bwd = torch.library.custom_op("rbf_attn_b200::layer_norm_bwd", mutates_args=())(_layer_norm_bwd)
+
+
 @layer_norm_bwd.register_fake
 def _(x, dy, weight, mean, rstd):
     return (torch.empty_like(x, memory_format=torch.contiguous_format), torch.empty_like(weight),
@@ -969,20 +1004,39 @@ def _ln_backward(ctx, g_y, _g_mean, _g_rstd):
     if g_y is None:
         return None, None, None, None
     x, weight, mean, rstd = ctx.saved_tensors
-    dx, dgamma, dbeta = torch.ops.rbf_attn_b200.layer_norm_bwd(x, g_y, weight, mean, rstd)
+    bwd = _layer_norm_bwd if _direct(x, g_y, weight, mean, rstd) else torch.ops.rbf_attn_b200.layer_norm_bwd
+    dx, dgamma, dbeta = bwd(x, g_y, weight, mean, rstd)
     return dx, dgamma, dbeta, None
 
 
 torch.library.register_autograd("rbf_attn_b200::layer_norm_fwd", _ln_backward, setup_context=_ln_setup_context)
 
 
+class _LayerNorm(torch.autograd.Function):
+    """``rbf_attn_b200::layer_norm_fwd`` and its autograd formula for calls that go around the operator (``_direct``)."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias, eps):
+        output = _layer_norm_fwd(x, weight, bias, eps)
+        _ln_setup_context(ctx, (x, weight, bias, eps), output)
+        return output[0]
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, g_y):
+        return _ln_backward(ctx, g_y, None, None)
+
+
 def layer_norm(x, weight, bias, eps: float = 1e-5):
     """``F.layer_norm(x, (x.shape[-1],), weight, bias, eps)`` on the library's kernels (see layer_norm_supported)."""
+    if type(eps) is float and _direct(x, weight, bias):
+        if _needs_grad(x, weight, bias):
+            return _LayerNorm.apply(x, weight, bias, eps)
+        return _layer_norm_fwd(x, weight, bias, eps)[0]
     return torch.ops.rbf_attn_b200.layer_norm_fwd(x, weight, bias, eps)[0]
 
 
-@torch.library.custom_op("rbf_attn_b200::add_layer_norm_fwd", mutates_args=())
-def add_layer_norm_fwd(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
+def _add_layer_norm_fwd(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
                        eps: float) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """s = x + residual (rounded to the dtype, as the separate addition leaves it) and y = LayerNorm(s) from one pass;
     returns (s, y, mean, rstd)."""
@@ -1006,6 +1060,9 @@ def add_layer_norm_fwd(x: torch.Tensor, residual: torch.Tensor, weight: torch.Te
     return s, y, mean, rstd
 
 
+add_layer_norm_fwd = torch.library.custom_op("rbf_attn_b200::add_layer_norm_fwd", mutates_args=())(_add_layer_norm_fwd)
+
+
 @add_layer_norm_fwd.register_fake
 def _(x, residual, weight, bias, eps):
     rows = x.numel() // x.shape[-1]
@@ -1014,8 +1071,7 @@ def _(x, residual, weight, bias, eps):
             x.new_empty(rows, dtype=torch.float32))
 
 
-@torch.library.custom_op("rbf_attn_b200::layer_norm_bwd_add", mutates_args=())
-def layer_norm_bwd_add(x: torch.Tensor, dy: torch.Tensor, dres: torch.Tensor, weight: torch.Tensor, mean: torch.Tensor,
+def _layer_norm_bwd_add(x: torch.Tensor, dy: torch.Tensor, dres: torch.Tensor, weight: torch.Tensor, mean: torch.Tensor,
                        rstd: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """The LayerNorm backward with ``dres`` (the gradient reaching x along the skip path) added to dx before the
     rounding: (dx, dgamma, dbeta)."""
@@ -1040,6 +1096,9 @@ def layer_norm_bwd_add(x: torch.Tensor, dy: torch.Tensor, dres: torch.Tensor, we
     return dx, dgamma.to(weight.dtype), dbeta.to(weight.dtype)
 
 
+layer_norm_bwd_add = torch.library.custom_op("rbf_attn_b200::layer_norm_bwd_add", mutates_args=())(_layer_norm_bwd_add)
+
+
 @layer_norm_bwd_add.register_fake
 def _(x, dy, dres, weight, mean, rstd):
     return (torch.empty_like(x, memory_format=torch.contiguous_format), torch.empty_like(weight),
@@ -1057,10 +1116,13 @@ def _add_ln_backward(ctx, g_s, g_y, _g_mean, _g_rstd):
     if g_y is None:
         return g_s, g_s, None, None, None
     s, weight, mean, rstd = ctx.saved_tensors
+    direct = _direct(s, g_y, g_s, weight, mean, rstd)
     if g_s is None:
-        dx, dgamma, dbeta = torch.ops.rbf_attn_b200.layer_norm_bwd(s, g_y, weight, mean, rstd)
+        bwd = _layer_norm_bwd if direct else torch.ops.rbf_attn_b200.layer_norm_bwd
+        dx, dgamma, dbeta = bwd(s, g_y, weight, mean, rstd)
     else:
-        dx, dgamma, dbeta = torch.ops.rbf_attn_b200.layer_norm_bwd_add(s, g_y, g_s, weight, mean, rstd)
+        bwd = _layer_norm_bwd_add if direct else torch.ops.rbf_attn_b200.layer_norm_bwd_add
+        dx, dgamma, dbeta = bwd(s, g_y, g_s, weight, mean, rstd)
     return dx, dx, dgamma, dbeta, None
 
 
@@ -1068,9 +1130,28 @@ torch.library.register_autograd("rbf_attn_b200::add_layer_norm_fwd", _add_ln_bac
                                 setup_context=_add_ln_setup_context)
 
 
+class _AddLayerNorm(torch.autograd.Function):
+    """``rbf_attn_b200::add_layer_norm_fwd`` and its autograd formula for calls that go around the operator."""
+
+    @staticmethod
+    def forward(ctx, x, residual, weight, bias, eps):
+        output = _add_layer_norm_fwd(x, residual, weight, bias, eps)
+        _add_ln_setup_context(ctx, (x, residual, weight, bias, eps), output)
+        return output[0], output[1]
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, g_s, g_y):
+        return _add_ln_backward(ctx, g_s, g_y, None, None)
+
+
 def add_layer_norm(x, residual, weight, bias, eps: float = 1e-5):
     """``s = x + residual; y = F.layer_norm(s, (s.shape[-1],), weight, bias, eps)`` in one pass over the activations
     (and one in the backward, which takes the skip path's gradient with it): returns (s, y)."""
+    if type(eps) is float and _direct(x, residual, weight, bias):
+        if _needs_grad(x, residual, weight, bias):
+            return _AddLayerNorm.apply(x, residual, weight, bias, eps)
+        return _add_layer_norm_fwd(x, residual, weight, bias, eps)[:2]
     s, y, _mean, _rstd = torch.ops.rbf_attn_b200.add_layer_norm_fwd(x, residual, weight, bias, eps)
     return s, y
 
@@ -1082,8 +1163,7 @@ def add_layer_norm(x, residual, weight, bias, eps: float = 1e-5):
 _CE_DTYPE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
-@torch.library.custom_op("rbf_attn_b200::cross_entropy_fwd", mutates_args=())
-def cross_entropy_fwd(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int) -> tuple[torch.Tensor, torch.Tensor]:
+def _cross_entropy_fwd(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int) -> tuple[torch.Tensor, torch.Tensor]:
     """Mean cross entropy over the rows whose target is not ``ignore_index`` (fp32 scalar) and its gradient with
     respect to ``logits`` (same shape and dtype), from one pass: logits (rows, cols) with unit column stride,
     targets (rows,) int64."""
@@ -1110,13 +1190,15 @@ def cross_entropy_fwd(logits: torch.Tensor, targets: torch.Tensor, ignore_index:
     return loss_rows.sum() * grad_scale, dlogits
 
 
+cross_entropy_fwd = torch.library.custom_op("rbf_attn_b200::cross_entropy_fwd", mutates_args=())(_cross_entropy_fwd)
+
+
 @cross_entropy_fwd.register_fake
 def _(logits, targets, ignore_index):
     return logits.new_empty((), dtype=torch.float32), torch.empty_like(logits, memory_format=torch.contiguous_format)
 
 
-@torch.library.custom_op("rbf_attn_b200::scale_unless_one_", mutates_args=("x",))
-def scale_unless_one_(x: torch.Tensor, factor: torch.Tensor) -> None:
+def _scale_unless_one(x: torch.Tensor, factor: torch.Tensor) -> None:
     """x *= factor (a one-element tensor) unless factor == 1, decided on the device."""
     if not x.is_contiguous():
         raise ValueError("x must be contiguous")
@@ -1125,6 +1207,9 @@ def scale_unless_one_(x: torch.Tensor, factor: torch.Tensor) -> None:
         rc = _lib.load().rbf_b200_scale_unless_one(x.data_ptr(), f.data_ptr(), x.numel(), _CE_DTYPE[x.dtype],
                                                    _stream_ptr(x.device))
     _lib.check(rc, "rbf_b200_scale_unless_one")
+
+
+scale_unless_one_ = torch.library.custom_op("rbf_attn_b200::scale_unless_one_", mutates_args=("x",))(_scale_unless_one)
 
 
 def _ce_setup_context(ctx, inputs, output):
@@ -1138,27 +1223,98 @@ def _ce_backward(ctx, g_loss, _g_dlogits):
     if g_loss is None:
         return None, None, None
     (dlogits,) = ctx.saved_tensors
-    torch.ops.rbf_attn_b200.scale_unless_one_(dlogits, g_loss)
+    if _direct(dlogits, g_loss):
+        _scale_unless_one(dlogits, g_loss)
+        torch.autograd.graph.increment_version(dlogits)     # as the operator layer does for what it mutates
+    else:
+        torch.ops.rbf_attn_b200.scale_unless_one_(dlogits, g_loss)
     return dlogits, None, None
 
 
 torch.library.register_autograd("rbf_attn_b200::cross_entropy_fwd", _ce_backward, setup_context=_ce_setup_context)
 
 
+class _CrossEntropy(torch.autograd.Function):
+    """``rbf_attn_b200::cross_entropy_fwd`` and its autograd formula for calls that go around the operator."""
+
+    @staticmethod
+    def forward(ctx, logits, targets, ignore_index):
+        output = _cross_entropy_fwd(logits, targets, ignore_index)
+        _ce_setup_context(ctx, (logits, targets, ignore_index), output)
+        return output[0]
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, g_loss):
+        return _ce_backward(ctx, g_loss, None)
+
+
 def cross_entropy(logits, targets, ignore_index: int = -100):
     """``F.cross_entropy(logits, targets, ignore_index=ignore_index)`` (mean reduction) for 2-D CUDA logits, with the
     gradient produced by the forward kernel."""
+    if type(ignore_index) is int and _direct(logits, targets):
+        if _needs_grad(logits):
+            return _CrossEntropy.apply(logits, targets, ignore_index)
+        return _cross_entropy_fwd(logits, targets, ignore_index)[0]
     return torch.ops.rbf_attn_b200.cross_entropy_fwd(logits, targets, ignore_index)[0]
 
 
 # ---------------------------------------------------------------------------------------------
 # Wrappers with the reference's names (rbf_attention.py:848-853)
 # ---------------------------------------------------------------------------------------------
+class _ScaledAttention(torch.autograd.Function):
+    """``rbf_attn_v5::scaled_fwd`` and its autograd formula for calls that go around the operator (``_direct``)."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, is_causal):
+        out, lse = _forward(q, k, v, is_causal, softmax=True)
+        ctx.save_for_backward(q, k, v, out, lse)
+        ctx.is_causal = is_causal
+        return out
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dout):
+        q, k, v, out, lse = ctx.saved_tensors
+        sm_scale = 1.0 / math.sqrt(q.shape[-1])
+        if _direct(q, k, v, out, lse, dout):
+            return *_backward(q, k, v, out, lse, dout, ctx.is_causal, sm_scale, softmax=True), None
+        return *torch.ops.rbf_attn_v5.scaled_bwd(q, k, v, out, lse, dout, ctx.is_causal, sm_scale), None
+
+
+class _NonSoftmaxAttention(torch.autograd.Function):
+    """``rbf_attn_v5::non_softmax_fwd`` and its autograd formula for calls that go around the operator (``_direct``)."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, is_causal):
+        out = _forward(q, k, v, is_causal, softmax=False)[0]
+        ctx.save_for_backward(q, k, v, out)
+        ctx.is_causal = is_causal
+        return out
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dout):
+        q, k, v, out = ctx.saved_tensors
+        sm_scale = 1.0 / math.sqrt(q.shape[-1])
+        if _direct(q, k, v, out, dout):
+            return *_backward(q, k, v, out, None, dout, ctx.is_causal, sm_scale, softmax=False), None
+        return *torch.ops.rbf_attn_v5.non_softmax_bwd_with_out(q, k, v, out, dout, ctx.is_causal, sm_scale), None
+
+
 def run_triton_rbf(q, k, v, is_causal=True):
     """Softmax RBF attention. The name is the reference's; nothing here uses Triton."""
+    if type(is_causal) is bool and _direct(q, k, v):
+        if _needs_grad(q, k, v):
+            return _ScaledAttention.apply(q, k, v, is_causal)
+        return _forward(q, k, v, is_causal, softmax=True)[0]
     return torch.ops.rbf_attn_v5.scaled_fwd(q, k, v, is_causal)[0]
 
 
 def run_triton_non_softmax_rbf(q, k, v, is_causal=True):
     """Non-softmax RBF attention ``exp(-g|q-k|^2) V``. The name is the reference's."""
+    if type(is_causal) is bool and _direct(q, k, v):
+        if _needs_grad(q, k, v):
+            return _NonSoftmaxAttention.apply(q, k, v, is_causal)
+        return _forward(q, k, v, is_causal, softmax=False)[0]
     return torch.ops.rbf_attn_v5.non_softmax_fwd(q, k, v, is_causal)
