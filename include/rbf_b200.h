@@ -109,14 +109,16 @@ int rbf_b200_bwd_phases(const void* q, const void* k, const void* v, const void*
  * page-locked host memory, or NULL. The call's last kernel stores the launch's status word there when everything before
  * it has finished (the forward: the last block to leave; the single-kernel backward: its dQ conversion), which saves the
  * kernel of its own that rbf_b200_post_device_status enqueues; calls on other paths (fp32 tensors, the two-kernel
- * backward) enqueue that kernel. Only a call whose phases include a main kernel posts. */
+ * backward) enqueue that kernel. Only a call whose phases include a main kernel posts. Unlike the calls above these take
+ * 16-bit tensors of any head dim that is a multiple of 8 up to 128, in place; the workspace is that of D = 64 (up to 64)
+ * or D = 128. */
 int rbf_b200_fwd_posting(const void* q, const void* k, const void* v, void* out, float* lse, void* workspace,
-                        size_t workspace_bytes, int B, int H, int N, int D, const int64_t* q_strides,
+                        size_t workspace_bytes, int B, int H, int N, int head_dim, const int64_t* q_strides,
                         const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides, int dtype,
                         int causal, int softmax, float sm_scale, void* stream, int phases, unsigned int* status_slot);
 int rbf_b200_bwd_posting(const void* q, const void* k, const void* v, const void* out, const float* lse,
                         const void* dout, void* dq, void* dk, void* dv, void* workspace, size_t workspace_bytes, int B,
-                        int H, int N, int D, const int64_t* q_strides, const int64_t* k_strides,
+                        int H, int N, int head_dim, const int64_t* q_strides, const int64_t* k_strides,
                         const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
                         const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides, int dtype,
                         int causal, int softmax, float sm_scale, void* stream, int phases, unsigned int* status_slot);

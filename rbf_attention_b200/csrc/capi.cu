@@ -102,6 +102,17 @@ int check_common(int B, int H, int N, int D, int dtype, float sm_scale) {
   return 0;
 }
 
+// Head dims of the posting entry points: the kernels run at 64 or 128 columns, and tensor maps that end at the tensor's
+// last column make the loads fill the rest of a tile with zeros (which add nothing to any product) and the stores leave
+// it out. (Leaving the zero columns out of the products, with their count as a kernel argument, cost head dim 128 itself
+// 4 % on the forward and up to 10 % on the backward: a test per MMA on the issuing threads.)
+int padded_head_dim(int head_dim) { return head_dim <= 64 ? 64 : 128; }
+int check_head_dim(int head_dim) {
+  if (head_dim <= 0 || head_dim > 128 || head_dim % 8 != 0)
+    return fail(RBF_B200_ERR_BAD_ARGUMENT, "head dim %d is not supported (a multiple of 8 up to 128)", head_dim);
+  return 0;
+}
+
 int check_tensor(const char* name, const void* p, const int64_t* s, int B, int H, int N, int D) {
   if (p == nullptr) return fail(RBF_B200_ERR_BAD_ARGUMENT, "%s is NULL", name);
   if (s == nullptr) return fail(RBF_B200_ERR_BAD_ARGUMENT, "%s strides are NULL", name);
@@ -215,20 +226,22 @@ static int fwd_tf32(const void* q, const void* k, const void* v, void* out, floa
 }
 
 int rbf_b200_fwd_posting(const void* q, const void* k, const void* v, void* out, float* lse, void* workspace,
-                         size_t workspace_bytes, int B, int H, int N, int D, const int64_t* q_strides,
+                         size_t workspace_bytes, int B, int H, int N, int head_dim, const int64_t* q_strides,
                          const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides, int dtype,
                          int causal, int softmax, float sm_scale, void* stream_v, int phases,
                          unsigned int* status_slot) {
   g_last_error[0] = 0;
   int rc;
   if (dtype == 2)
-    return fwd_tf32(q, k, v, out, lse, workspace, workspace_bytes, B, H, N, D, q_strides, k_strides, v_strides,
+    return fwd_tf32(q, k, v, out, lse, workspace, workspace_bytes, B, H, N, head_dim, q_strides, k_strides, v_strides,
                     o_strides, causal, softmax, sm_scale, stream_v, phases, status_slot);
+  if ((rc = check_head_dim(head_dim))) return rc;
+  const int D = padded_head_dim(head_dim);
   if ((rc = check_common(B, H, N, D, dtype, sm_scale))) return rc;
-  if ((rc = check_tensor("q", q, q_strides, B, H, N, D))) return rc;
-  if ((rc = check_tensor("k", k, k_strides, B, H, N, D))) return rc;
-  if ((rc = check_tensor("v", v, v_strides, B, H, N, D))) return rc;
-  if ((rc = check_tensor("out", out, o_strides, B, H, N, D))) return rc;
+  if ((rc = check_tensor("q", q, q_strides, B, H, N, head_dim))) return rc;
+  if ((rc = check_tensor("k", k, k_strides, B, H, N, head_dim))) return rc;
+  if ((rc = check_tensor("v", v, v_strides, B, H, N, head_dim))) return rc;
+  if ((rc = check_tensor("out", out, o_strides, B, H, N, head_dim))) return rc;
   if (softmax && lse == nullptr) return fail(RBF_B200_ERR_BAD_ARGUMENT, "lse is NULL");
   if (workspace == nullptr || reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
     return fail(RBF_B200_ERR_WORKSPACE, "workspace is NULL or not 256-byte aligned");
@@ -241,17 +254,17 @@ int rbf_b200_fwd_posting(const void* q, const void* k, const void* v, void* out,
   rbf::FwdArgs a{};
   // the forward streams keys in tiles of 128 at D = 64 and of 64 at D = 128
   const int key_rows = D == 128 ? 64 : rbf::kTile;
-  if ((rc = make_map(&a.tm_q, "q", q, q_strides, bf16, B, H, N, D))) return rc;
-  if ((rc = make_map(&a.tm_k, "k", k, k_strides, bf16, B, H, N, D, key_rows))) return rc;
-  if ((rc = make_map(&a.tm_v, "v", v, v_strides, bf16, B, H, N, D, key_rows))) return rc;
-  if ((rc = make_map(&a.tm_o, "out", out, o_strides, bf16, B, H, N, D))) return rc;
+  if ((rc = make_map(&a.tm_q, "q", q, q_strides, bf16, B, H, N, head_dim))) return rc;
+  if ((rc = make_map(&a.tm_k, "k", k, k_strides, bf16, B, H, N, head_dim, key_rows))) return rc;
+  if ((rc = make_map(&a.tm_v, "v", v, v_strides, bf16, B, H, N, head_dim, key_rows))) return rc;
+  if ((rc = make_map(&a.tm_o, "out", out, o_strides, bf16, B, H, N, head_dim))) return rc;
 
   const int n_pad = rbf::padded_rows(N);
   const float c = sm_scale * rbf::kLog2e;
   cudaError_t e = cudaSuccess;
   if (phases & RBF_B200_PHASE_PREPASS) {
     rbf::RowStatsArgs r{};
-    r.B = B; r.H = H; r.N = N; r.n_pad = n_pad; r.scale = c; r.status_to_clear = ws.status;
+    r.B = B; r.H = H; r.N = N; r.n_pad = n_pad; r.scale = c; r.status_to_clear = ws.status; r.head_dim = head_dim;
     r.scale2 = 2.f * c; r.slab_w = slab_w(bf16); r.slab_big = slab_big(bf16);
     r.k = k; r.kslab_out = ws.kslab; set_strides(r.ks, k_strides);
     if (!softmax) {
@@ -277,6 +290,9 @@ int rbf_b200_fwd_phases(const void* q, const void* k, const void* v, void* out, 
                         size_t workspace_bytes, int B, int H, int N, int D, const int64_t* q_strides,
                         const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides, int dtype,
                         int causal, int softmax, float sm_scale, void* stream_v, int phases) {
+  g_last_error[0] = 0;
+  int rc;
+  if (dtype != 2 && (rc = check_common(B, H, N, D, dtype, sm_scale))) return rc;
   return rbf_b200_fwd_posting(q, k, v, out, lse, workspace, workspace_bytes, B, H, N, D, q_strides, k_strides, v_strides,
                               o_strides, dtype, causal, softmax, sm_scale, stream_v, phases, nullptr);
 }
@@ -291,23 +307,25 @@ int rbf_b200_fwd(const void* q, const void* k, const void* v, void* out, float* 
 
 int rbf_b200_bwd_posting(const void* q, const void* k, const void* v, const void* out, const float* lse,
                          const void* dout, void* dq, void* dk, void* dv, void* workspace, size_t workspace_bytes, int B,
-                         int H, int N, int D, const int64_t* q_strides, const int64_t* k_strides,
+                         int H, int N, int head_dim, const int64_t* q_strides, const int64_t* k_strides,
                          const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
                          const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides, int dtype,
                          int causal, int softmax, float sm_scale, void* stream_v, int phases,
                           unsigned int* status_slot) {
   g_last_error[0] = 0;
   int rc;
+  if ((rc = check_head_dim(head_dim))) return rc;
+  const int D = padded_head_dim(head_dim);
   if ((rc = check_common(B, H, N, D, dtype, sm_scale))) return rc;
-  if ((rc = check_tensor("q", q, q_strides, B, H, N, D))) return rc;
-  if ((rc = check_tensor("k", k, k_strides, B, H, N, D))) return rc;
-  if ((rc = check_tensor("v", v, v_strides, B, H, N, D))) return rc;
-  if ((rc = check_tensor("dout", dout, do_strides, B, H, N, D))) return rc;
-  if ((rc = check_tensor("dq", dq, dq_strides, B, H, N, D))) return rc;
-  if ((rc = check_tensor("dk", dk, dk_strides, B, H, N, D))) return rc;
-  if ((rc = check_tensor("dv", dv, dv_strides, B, H, N, D))) return rc;
+  if ((rc = check_tensor("q", q, q_strides, B, H, N, head_dim))) return rc;
+  if ((rc = check_tensor("k", k, k_strides, B, H, N, head_dim))) return rc;
+  if ((rc = check_tensor("v", v, v_strides, B, H, N, head_dim))) return rc;
+  if ((rc = check_tensor("dout", dout, do_strides, B, H, N, head_dim))) return rc;
+  if ((rc = check_tensor("dq", dq, dq_strides, B, H, N, head_dim))) return rc;
+  if ((rc = check_tensor("dk", dk, dk_strides, B, H, N, head_dim))) return rc;
+  if ((rc = check_tensor("dv", dv, dv_strides, B, H, N, head_dim))) return rc;
   if (softmax || out != nullptr) {
-    if ((rc = check_tensor("out", out, o_strides, B, H, N, D))) return rc;
+    if ((rc = check_tensor("out", out, o_strides, B, H, N, head_dim))) return rc;
   }
   if (softmax && lse == nullptr) return fail(RBF_B200_ERR_BAD_ARGUMENT, "lse is NULL");
   const bool fused = use_fused_backward(D, softmax, out != nullptr);
@@ -320,20 +338,22 @@ int rbf_b200_bwd_posting(const void* q, const void* k, const void* v, const void
   const bool bf16 = dtype == 0;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   rbf::BwdArgs a{};
-  if ((rc = make_map(&a.tm_q, "q", q, q_strides, bf16, B, H, N, D))) return rc;
-  if ((rc = make_map(&a.tm_k, "k", k, k_strides, bf16, B, H, N, D))) return rc;
-  if ((rc = make_map(&a.tm_v, "v", v, v_strides, bf16, B, H, N, D))) return rc;
-  if ((rc = make_map(&a.tm_do, "dout", dout, do_strides, bf16, B, H, N, D))) return rc;
-  if ((rc = make_map(&a.tm_dq, "dq", dq, dq_strides, bf16, B, H, N, D))) return rc;
-  if ((rc = make_map(&a.tm_dk, "dk", dk, dk_strides, bf16, B, H, N, D))) return rc;
-  if ((rc = make_map(&a.tm_dv, "dv", dv, dv_strides, bf16, B, H, N, D))) return rc;
+  if ((rc = make_map(&a.tm_q, "q", q, q_strides, bf16, B, H, N, head_dim))) return rc;
+  if ((rc = make_map(&a.tm_k, "k", k, k_strides, bf16, B, H, N, head_dim))) return rc;
+  if ((rc = make_map(&a.tm_v, "v", v, v_strides, bf16, B, H, N, head_dim))) return rc;
+  if ((rc = make_map(&a.tm_do, "dout", dout, do_strides, bf16, B, H, N, head_dim))) return rc;
+  // (the head-dim-64 single kernel's drain warps store 32 rows of dK and dV each)
+  const int dkv_rows = fused && D == 64 ? 32 : rbf::kTile;
+  if (!fused && (rc = make_map(&a.tm_dq, "dq", dq, dq_strides, bf16, B, H, N, head_dim))) return rc;
+  if ((rc = make_map(&a.tm_dk, "dk", dk, dk_strides, bf16, B, H, N, head_dim, dkv_rows))) return rc;
+  if ((rc = make_map(&a.tm_dv, "dv", dv, dv_strides, bf16, B, H, N, head_dim, dkv_rows))) return rc;
 
   const int n_pad = rbf::padded_rows(N);
   const float c = sm_scale * rbf::kLog2e;
   cudaError_t e = cudaSuccess;
   if (phases & RBF_B200_PHASE_PREPASS) {
     rbf::RowStatsArgs r{};
-    r.B = B; r.H = H; r.N = N; r.n_pad = n_pad; r.scale = c; r.status_to_clear = ws.status;
+    r.B = B; r.H = H; r.N = N; r.n_pad = n_pad; r.scale = c; r.status_to_clear = ws.status; r.head_dim = head_dim;
     r.scale2 = 2.f * c; r.slab_w = slab_w(bf16); r.slab_big = slab_big(bf16);
     if (fused) { r.lslab_out = ws.lslab; r.dslab_out = ws.dslab; r.zero_rows = ws.dq_acc; }
     // The head-dim-128 single kernel takes the key norms from its resident K tile, so K is not read here. (At head
@@ -363,17 +383,14 @@ int rbf_b200_bwd_posting(const void* q, const void* k, const void* v, const void
     // the head-dim-128 kernel streams the queries in steps of 64 rows
     const int q_rows = D == 128 ? 64 : rbf::kTile;
     if (q_rows != rbf::kTile) {
-      if ((rc = make_map(&f.tm_q, "q", q, q_strides, bf16, B, H, N, D, q_rows))) return rc;
-      if ((rc = make_map(&f.tm_do, "dout", dout, do_strides, bf16, B, H, N, D, q_rows))) return rc;
+      if ((rc = make_map(&f.tm_q, "q", q, q_strides, bf16, B, H, N, head_dim, q_rows))) return rc;
+      if ((rc = make_map(&f.tm_do, "dout", dout, do_strides, bf16, B, H, N, head_dim, q_rows))) return rc;
     }
     const int t1 = rbf::make_tmap_slab16(&f.tm_lslab, ws.lslab, bf16, B * H, n_pad, q_rows);
     const int t2 = rbf::make_tmap_slab16(&f.tm_dslab, ws.dslab, bf16, B * H, n_pad, q_rows);
     if (t1 != 0 || t2 != 0)
       return fail(RBF_B200_ERR_TENSOR_MAP, "cuTensorMapEncodeTiled failed for the bias slabs (codes %d, %d)", t1, t2);
     if (D == 64) {
-      // the kernel's drain warps store 32 rows of dK and dV each
-      if ((rc = make_map(&f.tm_dk, "dk", dk, dk_strides, bf16, B, H, N, D, 32))) return rc;
-      if ((rc = make_map(&f.tm_dv, "dv", dv, dv_strides, bf16, B, H, N, D, 32))) return rc;
       const int t3 = rbf::make_tmap_f32_bhnd(&f.tm_dq_acc, ws.dq_acc, B, H, N, D, 32);
       if (t3 != 0)
         return fail(RBF_B200_ERR_TENSOR_MAP, "cuTensorMapEncodeTiled failed for the dQ accumulator (code %d)", t3);
@@ -387,7 +404,7 @@ int rbf_b200_bwd_posting(const void* q, const void* k, const void* v, const void
     if (!softmax) { f.q_rows = q; set_strides(f.q_strides, q_strides); f.delta = ws.delta; }
     f.B = B; f.H = H; f.N = N; f.n_pad = n_pad; f.causal = causal ? 1 : 0;
     f.scale2 = 2.f * c; f.grad_scale = 2.f * sm_scale; f.slab_w = slab_w(bf16);
-    f.status_slot = status_slot;
+    f.head_dim = head_dim; f.status_slot = status_slot;
     e = D == 128 ? rbf::launch_bwd_fused128(f, bf16, stream) : rbf::launch_bwd_fused(f, bf16, stream);
     if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "backward launch failed: %s", cudaGetErrorString(e));
     return RBF_B200_OK;
@@ -421,6 +438,9 @@ int rbf_b200_bwd_phases(const void* q, const void* k, const void* v, const void*
                         const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
                         const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides, int dtype,
                         int causal, int softmax, float sm_scale, void* stream_v, int phases) {
+  g_last_error[0] = 0;
+  int rc;
+  if ((rc = check_common(B, H, N, D, dtype, sm_scale))) return rc;
   return rbf_b200_bwd_posting(q, k, v, out, lse, dout, dq, dk, dv, workspace, workspace_bytes, B, H, N, D, q_strides,
                               k_strides, v_strides, o_strides, do_strides, dq_strides, dk_strides, dv_strides, dtype,
                               causal, softmax, sm_scale, stream_v, phases, nullptr);

@@ -33,6 +33,7 @@ struct RowStatsArgs {
   float scale2, slab_w, slab_big;
   int64_t ks[3], qs[3], os[3], dos[3];   // element strides of dims b, h, n
   int B, H, N, n_pad;
+  int head_dim;           // columns of the tensors, a multiple of 8 up to the kernel's D
   float scale;
   float qsq_pad;
   int iters;              // set by the launcher
@@ -232,6 +233,7 @@ struct BwdFusedArgs {
   int B, H, N, n_pad;
   int causal;
   float scale2, grad_scale, slab_w;
+  int head_dim;                // columns of the tensors, a multiple of 8 up to the kernel's D (the maps end there)
   unsigned int* status_slot;   // optional, as in FwdArgs: posted by the dQ conversion, which runs after the main kernel
 };
 cudaError_t launch_bwd_fused(const BwdFusedArgs& a, bool bf16, cudaStream_t stream);      // D = 64

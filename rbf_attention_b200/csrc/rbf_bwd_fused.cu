@@ -695,13 +695,15 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict
                                                          int64_t total_chunks, const void* __restrict__ q,
                                                          int64_t qsb, int64_t qsh, int64_t qsn,
                                                          const float* __restrict__ delta, int n_pad,
-                                                         const DeviceStatus* status, unsigned int* status_slot) {
+                                                         const DeviceStatus* status, unsigned int* status_slot,
+                                                         int head_dim) {
   if (status_slot != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) post_status_word(status, status_slot);
   // one thread per 8 consecutive elements of a row (D = 64: 8 chunks per row)
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total_chunks) return;
   const int64_t row = i >> 3;
   const int ch = static_cast<int>(i & 7);
+  if (ch * 8 >= head_dim) return;
   const int64_t n = row % N;
   const int64_t bh = row / N;
   const int64_t b = bh / H, h = bh % H;
@@ -750,7 +752,7 @@ static cudaError_t launch_t(const BwdFusedArgs& a, cudaStream_t stream) {
   const int64_t chunks = static_cast<int64_t>(a.B) * a.H * a.N * 8;
   dq_convert_kernel<kBf16><<<static_cast<unsigned>((chunks + 255) / 256), 256, 0, stream>>>(
       a.dq_acc, a.dq, a.H, a.N, a.dq_strides[0], a.dq_strides[1], a.dq_strides[2], a.grad_scale, chunks, a.q_rows,
-      a.q_strides[0], a.q_strides[1], a.q_strides[2], a.delta, a.n_pad, a.status, a.status_slot);
+      a.q_strides[0], a.q_strides[1], a.q_strides[2], a.delta, a.n_pad, a.status, a.status_slot, a.head_dim);
   return cudaGetLastError();
 }
 

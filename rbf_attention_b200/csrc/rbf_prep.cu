@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) row_stats_kernel(const RowStatsArgs a) {
     const int row = row_begin + (it * 8 + warp) * kRowsPerWarp + sub;
     const bool valid = row < a.N;
     float ksq = 0.f, qsq = 0.f, delta = 0.f;
-    if (valid) {
+    if (valid && part * 8 < a.head_dim) {
       if (a.k != nullptr) {
         const uint4 v = load_chunk(a.k, a.ks, b, h, row, part);
         ksq = dot8<kBf16>(v, v);

@@ -100,12 +100,19 @@ def _padded_head_dim(D: int) -> int:
     """Head dim the kernels run at: 64 or 128. Other head dims up to 128 run zero-padded to the next of the two, which
     is exact: zero columns add nothing to q.k, to |k|^2 or to |q|^2, and zero value columns give zero output columns
     (the reference pads to the next power of two inside its kernels, rbf_attention.py:661). The softmax scale keeps
-    using the caller's D."""
+    using the caller's D. Multiples of 8 in 16-bit types are padded by the kernels' own loads (``_columns``)."""
     if D <= 64:
         return 64
     if D <= 128:
         return 128
     raise ValueError(f"head dim {D} is not supported (at most 128)")
+
+
+def _columns(D: int, dtype: torch.dtype) -> int:
+    """Columns the tensors of a call get: their own where the kernels' loads can pad them (16-bit rows of a multiple of 16
+    bytes), else those the kernels run at. At head dim 80 (B2 H12 N1500, fp16) padding and slicing with separate passes
+    were 20 of the 28 launches and half the device time of a training pass."""
+    return D if dtype != torch.float32 and D % 8 == 0 else _padded_head_dim(D)
 
 
 def _pad_d(t: torch.Tensor, Dp: int) -> torch.Tensor:
@@ -318,23 +325,24 @@ def _forward(q, k, v, is_causal: bool, softmax: bool):
     tf32 = q.dtype == torch.float32 and D == 64
     cdt = torch.float32 if tf32 else _compute_dtype(q)
     code = _F32_CODE if tf32 else _DTYPE_CODE[cdt]
-    qc, kc, vc = (_tma_ready(_pad_d(t.to(cdt), D)) for t in (q, k, v))
-    out = torch.empty((B, H, N, D), dtype=cdt, device=q.device)
+    Dc = _columns(D0, cdt)
+    qc, kc, vc = (_tma_ready(_pad_d(t.to(cdt), Dc)) for t in (q, k, v))
+    out = torch.empty((B, H, N, Dc), dtype=cdt, device=q.device)
     lse = torch.empty((B, H, N), dtype=torch.float32, device=q.device) if softmax else None
     ws = _workspace(B, H, N, D, softmax, False, q.device)
     mon = _monitor(q.device)
     mon.poll()
-    dense = _dense_strides3(H, N, D)
+    dense = _dense_strides3(H, N, Dc)
     with _OnDevice(q.device):
         mon.launch("rbf_b200_fwd", lambda slot: lib.rbf_b200_fwd_posting(
             qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(),
             lse.data_ptr() if softmax else None, ws.data_ptr(), ws.numel(),
-            B, H, N, D, _strides3(qc, dense), _strides3(kc, dense), _strides3(vc, dense), dense,
+            B, H, N, Dc, _strides3(qc, dense), _strides3(kc, dense), _strides3(vc, dense), dense,
             code, int(bool(is_causal)), int(softmax), 1.0 / math.sqrt(D0), _stream_ptr(q.device), _PHASE_ALL, slot,
         ))
         if q.dtype == torch.float32 and not tf32:
             mon.record_range_check((qc, kc, vc), "rbf_b200_fwd")
-    if D != D0:
+    if Dc != D0:
         out = out[..., :D0].contiguous()
     if cdt != q.dtype:
         out = out.to(q.dtype)
@@ -350,11 +358,12 @@ def _backward(q, k, v, out, lse, dout, is_causal: bool, sm_scale: float, softmax
     D = _padded_head_dim(D0)
     lib = _lib.load()
     cdt = _compute_dtype(q)
-    qc, kc, vc, doc = (_tma_ready(_pad_d(t.to(cdt), D)) for t in (q, k, v, dout))
+    Dc = _columns(D0, cdt)
+    qc, kc, vc, doc = (_tma_ready(_pad_d(t.to(cdt), Dc)) for t in (q, k, v, dout))
     # the non-softmax variant takes the forward output when the caller has it: the single-kernel backward needs it
     have_out = out is not None
-    oc = _tma_ready(_pad_d(out.to(cdt), D)) if have_out else None
-    dq = torch.empty((B, H, N, D), dtype=cdt, device=q.device)
+    oc = _tma_ready(_pad_d(out.to(cdt), Dc)) if have_out else None
+    dq = torch.empty((B, H, N, Dc), dtype=cdt, device=q.device)
     dk = torch.empty_like(dq)
     dv = torch.empty_like(dq)
     ws = _workspace(B, H, N, D, softmax, True, q.device)
@@ -363,20 +372,20 @@ def _backward(q, k, v, out, lse, dout, is_causal: bool, sm_scale: float, softmax
     mon.poll()
     # torch.use_deterministic_algorithms(True) selects the backward whose summation order is fixed
     lib.rbf_b200_set_deterministic(int(torch.are_deterministic_algorithms_enabled()))
-    dense = _dense_strides3(H, N, D)
+    dense = _dense_strides3(H, N, Dc)
     with _OnDevice(q.device):
         mon.launch("rbf_b200_bwd", lambda slot: lib.rbf_b200_bwd_posting(
             qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
             oc.data_ptr() if have_out else None, lse.data_ptr() if softmax else None, doc.data_ptr(),
             dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(),
-            B, H, N, D, _strides3(qc, dense), _strides3(kc, dense), _strides3(vc, dense),
+            B, H, N, Dc, _strides3(qc, dense), _strides3(kc, dense), _strides3(vc, dense),
             _strides3(oc, dense) if have_out else z3, _strides3(doc, dense),
             dense, dense, dense,
             _DTYPE_CODE[cdt], int(bool(is_causal)), int(softmax), float(sm_scale), _stream_ptr(q.device), _PHASE_ALL, slot,
         ))
         if q.dtype == torch.float32:
             mon.record_range_check((qc, kc, vc, doc), "rbf_b200_bwd")
-    if D != D0:
+    if Dc != D0:
         dq, dk, dv = (t[..., :D0].contiguous() for t in (dq, dk, dv))
     if cdt != q.dtype:
         dq, dk, dv = dq.to(q.dtype), dk.to(q.dtype), dv.to(q.dtype)

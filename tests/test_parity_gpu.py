@@ -846,3 +846,30 @@ def test_calls_post_their_status_word(D, N, softmax, deterministic):
     assert rc == 0, lib.rbf_b200_last_error()
     torch.cuda.synchronize()
     assert slots.tolist() == [0, (1 << 24) | 7, 0, -1]
+
+
+@pytest.mark.parametrize("D", [8, 24, 40, 56, 72, 80, 104, 120])
+@pytest.mark.parametrize("softmax,causal,dtype,deterministic", [(True, True, torch.bfloat16, False),
+                                                                (False, False, torch.float16, False),
+                                                                (True, False, torch.float16, True)])
+def test_head_dims_that_are_multiples_of_eight_run_in_place(D, softmax, causal, dtype, deterministic):
+    """No copy of the tensors: views into one (B, N, 3, H, D) buffer, ragged N, whose neighbours hold NaN - a column or row
+    read past the tensors' own would show -, and gradients whose neighbours are checked to stay untouched by the head
+    dims' padding (the stores are clipped)."""
+    B, H, N = 2, 3, 150
+    q, k, v, do = oracle.make_inputs(B, H, N, D, seed=D, dtype=dtype, std=1.0 if softmax else 0.5)
+    ref = oracle.torch_forward_backward(q, k, v, do, causal, softmax, dtype=torch.float32)
+    buf = torch.full((B, N + 1, 4, H, D), float("nan"), dtype=dtype, device=DEV)
+    for i, t in enumerate((q, k, v)):
+        buf[:, :N, i] = t.to(DEV).permute(0, 2, 1, 3)
+    qd, kd, vd = (buf[:, :N, i].permute(0, 2, 1, 3) for i in range(3))
+    out, lse = ops._forward(qd, kd, vd, causal, softmax)
+    torch.use_deterministic_algorithms(deterministic)
+    try:
+        grads = ops._backward(qd, kd, vd, out, lse, do.to(DEV), causal, 1.0 / math.sqrt(D), softmax)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    ops.check_device_status()
+    for name, got, want in zip(("O", "dQ", "dK", "dV"), (out, *grads), ref):
+        assert got.shape == want.shape
+        check(name, got.cpu().float(), want, REL_L2[dtype])
