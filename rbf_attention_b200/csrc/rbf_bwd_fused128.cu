@@ -214,7 +214,10 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     }
   } else if (warp == kMmaWarpA || warp == kMmaWarpB || warp == kMmaWarpC) {
     // ------------------------------------------------------------------ MMA issuers
-    if (lane == 0) {
+    // (whole warps run the loops and one lane issues, see elect_one(): backward call at B2 H16 N3333 full 510 -> 498 us,
+    // B4 H16 N2048 causal 275 -> 266 us against loops inside `if (lane == 0)`)
+    {
+      const bool el = elect_one();
       constexpr uint32_t idesc_s = make_idesc(kTile, kQStep, kBf16, false, false);  // 128 keys x 64 queries, K-major both
       constexpr uint32_t idesc_acc = make_idesc(kTile, D, kBf16, false, true);      // dV, dK: B read N-major
       constexpr uint32_t idesc_dq = make_idesc(D, kQStep, kBf16, true, true);       // dQ^T: A M-major, B N-major
@@ -247,9 +250,11 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         if (ok) ok = wait_q(0);
         if (ok) {
           tc_fence_after_sync();
-          issue_scores(tmem + kColS, k_kmaj, q_kmaj0, lslab0);
-          umma_commit(s_full);
-          umma_commit(&q_empty[0]);
+          if (el) {
+            issue_scores(tmem + kColS, k_kmaj, q_kmaj0, lslab0);
+            umma_commit(s_full);
+            umma_commit(&q_empty[0]);
+          }
         }
         for (int n = 0; n < cnt && ok; ++n) {
           if (n + 1 < cnt) {
@@ -257,21 +262,25 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
             ok = wait_q(n + 1) && mbar_wait(s_consumed, n & 1, abort_flag, p.status, kSiteSConsumed);
             if (!ok) break;
             tc_fence_after_sync();
-            issue_scores(tmem + kColS, k_kmaj, stage_of(q_kmaj0, st, kQTileBytes), stage_of(lslab0, st, kSlabBytes));
-            umma_commit(s_full);
-            umma_commit(&q_empty[st]);
+            if (el) {
+              issue_scores(tmem + kColS, k_kmaj, stage_of(q_kmaj0, st, kQTileBytes), stage_of(lslab0, st, kSlabBytes));
+              umma_commit(s_full);
+              umma_commit(&q_empty[st]);
+            }
           }
           // dV += P^T dO
           ok = mbar_wait(p_full, n & 1, abort_flag, p.status, kSitePFull);
           if (!ok) break;
           tc_fence_after_sync();
           const SmemDesc do_n = stage_of(do_nmaj0, n % kDoStages, kQTileBytes);
+          if (el) {
 #pragma unroll
-          for (int kk = 0; kk < kQStep / 16; ++kk)
-            umma_ts(tmem + kColDV, tmem + kColPT + kk * 8, sdesc_at(do_n, kk * 2048), idesc_acc,
-                    (n > 0 || kk > 0) ? 1u : 0u);
-          umma_commit(dv_done);
-          umma_commit(&do_empty[n % kDoStages]);
+            for (int kk = 0; kk < kQStep / 16; ++kk)
+              umma_ts(tmem + kColDV, tmem + kColPT + kk * 8, sdesc_at(do_n, kk * 2048), idesc_acc,
+                      (n > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(dv_done);
+            umma_commit(&do_empty[n % kDoStages]);
+          }
         }
       } else if (warp == kMmaWarpB) {
         const SmemDesc v_kmaj = make_sdesc_parts(smem_u32(s_v), 16, 1024);
@@ -281,9 +290,11 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         if (ok) ok = wait_do(0);
         if (ok) {
           tc_fence_after_sync();
-          issue_scores(tmem + kColDP, v_kmaj, do_kmaj0, dslab0);
-          umma_commit(dp_full);
-          umma_commit(&do_empty[0]);
+          if (el) {
+            issue_scores(tmem + kColDP, v_kmaj, do_kmaj0, dslab0);
+            umma_commit(dp_full);
+            umma_commit(&do_empty[0]);
+          }
         }
         for (int n = 0; n < cnt && ok; ++n) {
           if (n + 1 < cnt) {
@@ -291,9 +302,11 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
             ok = wait_do(n + 1) && mbar_wait(dp_consumed, n & 1, abort_flag, p.status, kSiteDPConsumed);
             if (!ok) break;
             tc_fence_after_sync();
-            issue_scores(tmem + kColDP, v_kmaj, stage_of(do_kmaj0, st, kQTileBytes), stage_of(dslab0, st, kSlabBytes));
-            umma_commit(dp_full);
-            umma_commit(&do_empty[st]);
+            if (el) {
+              issue_scores(tmem + kColDP, v_kmaj, stage_of(do_kmaj0, st, kQTileBytes), stage_of(dslab0, st, kSlabBytes));
+              umma_commit(dp_full);
+              umma_commit(&do_empty[st]);
+            }
           }
           // dK += dS^T Q
           ok = mbar_wait(&ds_full[n % kDsStages], (n / kDsStages) & 1, abort_flag, p.status, kSiteDSFull);
@@ -301,12 +314,14 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
           tc_fence_after_sync();
           // A = the TMEM copy of dS^T (16-bit pairs, 32 columns): only Q is fetched from shared memory
           const SmemDesc q_n = stage_of(q_nmaj0, n % kQStages, kQTileBytes);
+          if (el) {
 #pragma unroll
-          for (int kk = 0; kk < kQStep / 16; ++kk)
-            umma_ts(tmem + kColDK, tmem + kColDST + kk * 8, sdesc_at(q_n, kk * 2048), idesc_acc,
-                    (n > 0 || kk > 0) ? 1u : 0u);
-          umma_commit(&q_empty[n % kQStages]);
-          umma_commit(dk_done);
+            for (int kk = 0; kk < kQStep / 16; ++kk)
+              umma_ts(tmem + kColDK, tmem + kColDST + kk * 8, sdesc_at(q_n, kk * 2048), idesc_acc,
+                      (n > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(&q_empty[n % kQStages]);
+            umma_commit(dk_done);
+          }
         }
       } else {
         // dQ^T = K^T dS^T : A = K tile read M-major (rows = keys = reduction index, 64-wide d groups 16 KB apart),
@@ -318,15 +333,17 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
           if (ok && n > 0) ok = mbar_wait(dq_drained, (n - 1) & 1, abort_flag, p.status, kSiteDQDrained);
           if (!ok) break;
           tc_fence_after_sync();
+          if (el) {
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk)
-            umma_ss(tmem + kColDQ, sdesc_at(k_mmaj, kk * 2048),
-                    sdesc_at(ds_nmaj, (n % kDsStages) * kDsBytes + kk * 2048), idesc_dq, kk > 0);
-          umma_commit(dq_full);                    // dQ^T readable
-          umma_commit(&ds_free[n % kDsStages]);    // the shared-memory tile's reader is done
+            for (int kk = 0; kk < kTile / 16; ++kk)
+              umma_ss(tmem + kColDQ, sdesc_at(k_mmaj, kk * 2048),
+                      sdesc_at(ds_nmaj, (n % kDsStages) * kDsBytes + kk * 2048), idesc_dq, kk > 0);
+            umma_commit(dq_full);                    // dQ^T readable
+            umma_commit(&ds_free[n % kDsStages]);    // the shared-memory tile's reader is done
+          }
         }
       }
-      if (ok) umma_commit(acc_done);
+      if (ok && el) umma_commit(acc_done);
     }
   } else if (warp >= kDrainWarp0) {
     // ------------------------------------------------------------------ dQ^T drain (thread = head-dim index)

@@ -194,7 +194,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   // work item the CTA's producer is loading (the status word of a wait that runs out names it, not the block index)
   volatile int* s_unit = reinterpret_cast<volatile int*>(smem + L::kMisc + 8);
   constexpr int kItemSlots = L::kItemSlots;
-  constexpr int kItemReaders = 2 + 8 * kSplit;   // two issuing threads, one arrival per softmax warp
+  constexpr int kItemReaders = 2 + 8 * kSplit;   // two issuing warps, one arrival per softmax warp
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -227,7 +227,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   };
   // n-th item of the CTA as seen by the issuers and the softmax warps (whole warps call this together); false at the
   // end of the sequence
-  auto read_item = [&](uint32_t n, bool whole_warp, bool& ok_ref, Item& it) -> bool {
+  auto read_item = [&](uint32_t n, bool& ok_ref, Item& it) -> bool {
     if (n == 0) {
       it = first_item;
       if (!kPersistent) return true;
@@ -245,8 +245,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       it.h = s_items[slot].z;
       it.m0 = s_items[slot].w;
     }
-    if (whole_warp) mbar_arrive_warp(&item_empty[slot]);
-    else mbar_arrive(&item_empty[slot]);
+    mbar_arrive_warp(&item_empty[slot]);
     if (it.bh < 0) return false;
     if (n != 0) count_key_tiles<kKeys>(it, N, causal);
     return true;
@@ -402,7 +401,12 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   } else if (warp == kMmaWarp0 || warp == kMmaWarp0 + 1) {
     // ------------------------------------------------------------------ MMA issuer of query tile t
     setmaxnreg_dec<R::kOtherRegs>();
-    if (lane == 0) {
+    // The whole warp runs the loop and one lane issues: descriptors, addresses and barrier waits stay warp-uniform. With
+    // the loop inside `if (lane == 0)` the MMAs' operands went through vector registers, and at D = 128 - eleven or more
+    // MMAs per tile and thread - the issue itself held the tensor pipe up: B2 H16 N3333 D128 full 245 -> 226 us, B4 H8
+    // N1024 D64 23.5 -> 22.8 us, B8 H16 N4096 D64 unchanged.
+    {
+      const bool el = elect_one();
       const int t = warp - kMmaWarp0;
       constexpr uint32_t idesc_s = make_idesc(kTile, kKeys, kBf16, false, false);   // S = Q K^T
       constexpr uint32_t idesc_o = make_idesc(kTile, D, kBf16, false, true);        // O += P V (V is N-major)
@@ -416,21 +420,25 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         k_desc.lo += static_cast<uint32_t>(st) * (kKvBytes >> 4);
         SmemDesc slab = kslab_desc0;
         slab.lo += static_cast<uint32_t>(st) * (kSlabBytes >> 4);
+        if (el) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          umma_ss(tmem_s[t], sdesc_at(q_desc, (kk >> 2) * kBoxBytes + (kk & 3) * 32),
-                  sdesc_at(k_desc, (kk >> 2) * kKvBoxBytes + (kk & 3) * 32), idesc_s, kk > 0);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            umma_ss(tmem_s[t], sdesc_at(q_desc, (kk >> 2) * kBoxBytes + (kk & 3) * 32),
+                    sdesc_at(k_desc, (kk >> 2) * kKvBoxBytes + (kk & 3) * 32), idesc_s, kk > 0);
+          }
+          umma_ss(tmem_s[t], sdesc_at(ones_desc, 0), sdesc_at(slab, 0), idesc_s, 1u);   // + key-norm bias
+          umma_commit(&s_full[t]);
         }
-        umma_ss(tmem_s[t], sdesc_at(ones_desc, 0), sdesc_at(slab, 0), idesc_s, 1u);   // + key-norm bias
-        umma_commit(&s_full[t]);
       };
       auto issue_o = [&](int st, uint32_t accumulate) {
         SmemDesc v_desc = v_desc0;
         v_desc.lo += static_cast<uint32_t>(st) * (kKvBytes >> 4);
+        if (el) {
 #pragma unroll
-        for (int kk = 0; kk < kKeys / 16; ++kk)
-          umma_ts(tmem_o[t], tmem_p[t] + kk * 8, sdesc_at(v_desc, kk * 2048), idesc_o, kk > 0 ? 1u : accumulate);
-        umma_commit(&o_done[t]);
+          for (int kk = 0; kk < kKeys / 16; ++kk)
+            umma_ts(tmem_o[t], tmem_p[t] + kk * 8, sdesc_at(v_desc, kk * 2048), idesc_o, kk > 0 ? 1u : accumulate);
+          umma_commit(&o_done[t]);
+        }
       };
       auto wait_k = [&](uint32_t g) {
         return mbar_wait(&k_full[g % kStages], (g / kStages) & 1, abort_flag, status, kSiteKFull, s_unit);
@@ -442,7 +450,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       bool ok = true;
       for (uint32_t n = 0; ok && (kPersistent || n == 0); ++n) {
         Item it;
-        if (!read_item(n, false, ok, it)) break;
+        if (!read_item(n, ok, it)) break;
         const int my_nkt = it.nkt(t), nkt_max = it.nkt_max;
         // Every stage is released by both issuers: by a commit after this tile's last MMA that reads it, or - when
         // this tile has nothing (left) to do with it - by a plain arrival made only after the stage has been filled,
@@ -455,12 +463,12 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           if (!ok) break;
           tc_fence_after_sync();
           issue_s(G % kStages);
-          if (kPersistent && my_nkt == 1) umma_commit(&q_free[t]);
-          umma_commit(&k_empty[G % kStages]);
+          if (el && kPersistent && my_nkt == 1) umma_commit(&q_free[t]);
+          if (el) umma_commit(&k_empty[G % kStages]);
         } else {
           ok = wait_k(G);
           if (!ok) break;
-          mbar_arrive(&k_empty[G % kStages]);
+          if (el) mbar_arrive(&k_empty[G % kStages]);
         }
         for (int j = 0; j < nkt_max && ok; ++j) {
           const uint32_t g = G + j;
@@ -474,7 +482,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
               if (!ok) break;
               tc_fence_after_sync();
               issue_s(st_next);
-              if (kPersistent && j + 2 == my_nkt) umma_commit(&q_free[t]);   // the item's last read of Q_t
+              if (el && kPersistent && j + 2 == my_nkt) umma_commit(&q_free[t]);   // the item's last read of Q_t
               used_k_next = true;
             }
             ok = wait_v(g);
@@ -482,19 +490,19 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (!ok) break;
             tc_fence_after_sync();
             issue_o(st, j > 0 ? 1u : 0u);
-            umma_commit(&v_empty[st]);
+            if (el) umma_commit(&v_empty[st]);
           } else {
             ok = wait_v(g);
             if (!ok) break;
-            mbar_arrive(&v_empty[st]);
+            if (el) mbar_arrive(&v_empty[st]);
           }
           if (j + 1 < nkt_max) {
             if (used_k_next) {
-              umma_commit(&k_empty[st_next]);
+              if (el) umma_commit(&k_empty[st_next]);
             } else {
               ok = wait_k(g + 1);
               if (!ok) break;
-              mbar_arrive(&k_empty[st_next]);
+              if (el) mbar_arrive(&k_empty[st_next]);
             }
           }
         }
@@ -531,7 +539,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
     for (uint32_t n = 0; ok && (kPersistent || n == 0); ++n) {
       Item it;
-      if (!read_item(n, true, ok, it)) break;
+      if (!read_item(n, ok, it)) break;
       const int my_nkt = it.nkt(t);
       if (my_nkt == 0) continue;
       const int r0 = it.m0 + t * kTile;
