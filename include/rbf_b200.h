@@ -122,6 +122,14 @@ int rbf_b200_bwd_posting(const void* q, const void* k, const void* v, const void
                         const int64_t* v_strides, const int64_t* o_strides, const int64_t* do_strides,
                         const int64_t* dq_strides, const int64_t* dk_strides, const int64_t* dv_strides, int dtype,
                         int causal, int softmax, float sm_scale, void* stream, int phases, unsigned int* status_slot);
+/* fp32 tensors on the fp16-operand calls. Narrowing: `count` (at most 5) fp32 (B, H, N, D) tensors, D a multiple of 8, unit
+ * stride on D, 16-byte aligned, strides (count x 3, elements of dims b, h, n) multiples of 4, into dense fp16 tensors; when a
+ * converted value of one of the first `checked` is an infinity the kernel stores 1 in *flag (device memory, cleared by the
+ * caller). Widening: dense fp16 tensors of n elements each, n a multiple of 8, into fp32. */
+int rbf_b200_narrow_f32(int count, const void* const* src, void* const* dst, const int64_t* strides, int B, int H, int N,
+                        int D, int checked, unsigned int* flag, void* stream);
+int rbf_b200_widen_f16(int count, const void* const* src, void* const* dst, int64_t n, void* stream);
+
 /* Device-side address of `host_slots` (page-locked host memory mapped into the current device's address space). */
 int rbf_b200_map_status_slots(unsigned int* host_slots, unsigned int** device_slots);
 

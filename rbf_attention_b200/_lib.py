@@ -61,6 +61,15 @@ SIGNATURES = {
         [ctypes.c_void_p] * 10 + [ctypes.c_size_t] + [ctypes.c_int] * 4 + [_c_i64p] * 8
         + [ctypes.c_int] * 3 + [ctypes.c_float, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p],
     ),
+    "rbf_b200_narrow_f32": (
+        ctypes.c_int,
+        [ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p), _c_i64p] + [ctypes.c_int] * 5
+        + [ctypes.c_void_p, ctypes.c_void_p],
+    ),
+    "rbf_b200_widen_f16": (
+        ctypes.c_int,
+        [ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p), ctypes.c_int64, ctypes.c_void_p],
+    ),
     "rbf_b200_map_status_slots": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p)]),
     "rbf_b200_static_scratch_bytes": (ctypes.c_size_t, []),
     "rbf_b200_fwd_static": (

@@ -816,6 +816,58 @@ int rbf_b200_scale_unless_one(void* x, const float* factor, int64_t n, int dtype
   return RBF_B200_OK;
 }
 
+int rbf_b200_narrow_f32(int count, const void* const* src, void* const* dst, const int64_t* strides, int B, int H, int N,
+                        int D, int checked, unsigned int* flag, void* stream_v) {
+  g_last_error[0] = 0;
+  if (count <= 0 || count > rbf::kMaxNarrow || checked < 0 || checked > count)
+    return fail(RBF_B200_ERR_BAD_ARGUMENT, "1 to %d tensors, of which at most that many are checked", rbf::kMaxNarrow);
+  if (B <= 0 || H <= 0 || N <= 0 || D <= 0 || D % 8 != 0)
+    return fail(RBF_B200_ERR_BAD_ARGUMENT, "B, H, N must be positive and D a positive multiple of 8");
+  if (src == nullptr || dst == nullptr || strides == nullptr || (checked > 0 && flag == nullptr))
+    return fail(RBF_B200_ERR_BAD_ARGUMENT, "src, dst, strides and (with checked tensors) flag must not be NULL");
+  rbf::NarrowArgs a{};
+  const int ext[3] = {B, H, N};
+  for (int t = 0; t < count; ++t) {
+    if (src[t] == nullptr || dst[t] == nullptr) return fail(RBF_B200_ERR_BAD_ARGUMENT, "tensor %d is NULL", t);
+    if (reinterpret_cast<uintptr_t>(src[t]) % 16 != 0 || reinterpret_cast<uintptr_t>(dst[t]) % 16 != 0)
+      return fail(RBF_B200_ERR_BAD_LAYOUT, "tensor %d is not 16-byte aligned", t);
+    for (int i = 0; i < 3; ++i) {
+      if (ext[i] > 1 && strides[3 * t + i] % 4 != 0)
+        return fail(RBF_B200_ERR_BAD_LAYOUT, "stride[%d] of tensor %d must be a multiple of 4 elements", i, t);
+      a.strides[t][i] = ext[i] > 1 ? strides[3 * t + i] : 0;
+    }
+    a.src[t] = static_cast<const float*>(src[t]);
+    a.dst[t] = dst[t];
+  }
+  a.chunks = static_cast<int64_t>(B) * H * N * (D / 8);
+  if ((a.chunks + 255) / 256 > 0x7fffffffll) return fail(RBF_B200_ERR_BAD_ARGUMENT, "the tensors are too large");
+  a.H = H; a.N = N; a.D = D; a.count = count; a.checked = checked; a.flag = flag;
+  const cudaError_t e = rbf::launch_narrow(a, static_cast<cudaStream_t>(stream_v));
+  if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "narrowing launch failed: %s", cudaGetErrorString(e));
+  return RBF_B200_OK;
+}
+
+int rbf_b200_widen_f16(int count, const void* const* src, void* const* dst, int64_t n, void* stream_v) {
+  g_last_error[0] = 0;
+  if (count <= 0 || count > rbf::kMaxNarrow) return fail(RBF_B200_ERR_BAD_ARGUMENT, "1 to %d tensors", rbf::kMaxNarrow);
+  if (n < 0 || n % 8 != 0) return fail(RBF_B200_ERR_BAD_ARGUMENT, "n must be a multiple of 8");
+  if (src == nullptr || dst == nullptr) return fail(RBF_B200_ERR_BAD_ARGUMENT, "src and dst must not be NULL");
+  rbf::WidenArgs a{};
+  for (int t = 0; t < count; ++t) {
+    if (src[t] == nullptr || dst[t] == nullptr) return fail(RBF_B200_ERR_BAD_ARGUMENT, "tensor %d is NULL", t);
+    if (reinterpret_cast<uintptr_t>(src[t]) % 16 != 0 || reinterpret_cast<uintptr_t>(dst[t]) % 16 != 0)
+      return fail(RBF_B200_ERR_BAD_LAYOUT, "tensor %d is not 16-byte aligned", t);
+    a.src[t] = src[t];
+    a.dst[t] = static_cast<float*>(dst[t]);
+  }
+  if (n == 0) return RBF_B200_OK;
+  a.chunks = n / 8; a.count = count;
+  if ((a.chunks + 255) / 256 > 0x7fffffffll) return fail(RBF_B200_ERR_BAD_ARGUMENT, "the tensors are too large");
+  const cudaError_t e = rbf::launch_widen(a, static_cast<cudaStream_t>(stream_v));
+  if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "widening launch failed: %s", cudaGetErrorString(e));
+  return RBF_B200_OK;
+}
+
 int rbf_b200_map_status_slots(unsigned int* host_slots, unsigned int** device_slots) {
   g_last_error[0] = 0;
   if (host_slots == nullptr || device_slots == nullptr)

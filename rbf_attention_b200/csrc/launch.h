@@ -130,6 +130,26 @@ int layer_norm_bwd_blocks(int64_t rows, int sms);
 cudaError_t launch_layer_norm_fwd(const LayerNormArgs& a, int cols, bool bf16, int sms, cudaStream_t stream);
 cudaError_t launch_layer_norm_bwd(const LayerNormBwdArgs& a, int cols, bool bf16, int sms, cudaStream_t stream);
 
+// fp32 -> fp16 of up to kMaxNarrow (B, H, N, D) tensors (strides in elements, unit stride on D) into dense ones; the first
+// `checked` of them set *flag when a converted value is an infinity. fp16 -> fp32 of dense tensors: narrow.cu.
+static constexpr int kMaxNarrow = 5;
+struct NarrowArgs {
+  const float* src[kMaxNarrow];
+  void* dst[kMaxNarrow];
+  int64_t strides[kMaxNarrow][3];
+  int64_t chunks;            // B * H * N * D / 8
+  int H, N, D, count, checked;
+  unsigned int* flag;
+};
+struct WidenArgs {
+  const void* src[kMaxNarrow];
+  float* dst[kMaxNarrow];
+  int64_t chunks;            // elements / 8
+  int count;
+};
+cudaError_t launch_narrow(const NarrowArgs& a, cudaStream_t stream);
+cudaError_t launch_widen(const WidenArgs& a, cudaStream_t stream);
+
 // Column sums of a 16-bit (rows x cols) matrix, row pitch ld elements, into out (cols, fp32): col_sums.cu.
 // `partials` holds col_sums_bands() x cols floats.
 int col_sums_bands(int64_t rows, int cols, int sms);

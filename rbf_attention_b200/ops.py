@@ -307,6 +307,46 @@ def check_device_status(device=None) -> None:
     _monitor(torch.device(device)).poll(wait=True)
 
 
+def _narrow(tensors, checked: int, mon, what: str):
+    """fp32 (B, H, N, D) tensors as fp16 operands, in one launch that also looks whether one of the first ``checked``
+    leaves fp16's range (reported like a status word: by a later call). What the kernel's 16-byte loads cannot take goes
+    through PyTorch's conversion."""
+    B, H, N, D = tensors[0].shape
+    ok = D % 8 == 0 and D > 0 and all(
+        t.dtype == torch.float32 and t.shape == tensors[0].shape and t.device == tensors[0].device and t.stride(3) == 1 and t.data_ptr() % 16 == 0 and all(e <= 1 or st % 4 == 0 for e, st in zip((B, H, N), t.stride()))
+        for t in tensors)
+    if not ok:
+        halves = [t.to(torch.float16) for t in tensors]
+        mon.record_range_check(halves[:checked], what)
+        return halves
+    n = len(tensors)
+    dev = tensors[0].device
+    halves = [torch.empty((B, H, N, D), dtype=torch.float16, device=dev) for _ in tensors]
+    flag = torch.zeros(4, dtype=torch.uint8, device=dev)
+    pointers, strides = ctypes.c_void_p * n, (ctypes.c_int64 * (3 * n))(*(st for t in tensors for st in t.stride()[:3]))
+    with _OnDevice(dev):
+        rc = _lib.load().rbf_b200_narrow_f32(n, pointers(*(t.data_ptr() for t in tensors)),
+                                             pointers(*(t.data_ptr() for t in halves)), strides, B, H, N, D, checked,
+                                             flag.data_ptr(), _stream_ptr(dev))
+        _lib.check(rc, "rbf_b200_narrow_f32")
+        mon.record(flag, "range:" + what)
+    return halves
+
+
+def _widen(tensors):
+    """Dense fp16 tensors of one shape as fp32, in one launch."""
+    count = tensors[0].numel()
+    if count % 8 != 0:
+        return [t.float() for t in tensors]
+    out = [torch.empty(t.shape, dtype=torch.float32, device=t.device) for t in tensors]
+    pointers = ctypes.c_void_p * len(out)
+    with _OnDevice(out[0].device):
+        rc = _lib.load().rbf_b200_widen_f16(len(out), pointers(*(t.data_ptr() for t in tensors)),
+                                            pointers(*(t.data_ptr() for t in out)), count, _stream_ptr(out[0].device))
+    _lib.check(rc, "rbf_b200_widen_f16")
+    return out
+
+
 _PHASE_ALL = 7          # pre-pass and both main kernels (include/rbf_b200.h)
 
 
@@ -326,12 +366,14 @@ def _forward(q, k, v, is_causal: bool, softmax: bool):
     cdt = torch.float32 if tf32 else _compute_dtype(q)
     code = _F32_CODE if tf32 else _DTYPE_CODE[cdt]
     Dc = _columns(D0, cdt)
-    qc, kc, vc = (_tma_ready(_pad_d(t.to(cdt), Dc)) for t in (q, k, v))
+    mon = _monitor(q.device)
+    mon.poll()
+    narrowed = q.dtype == torch.float32 and not tf32
+    ins = _narrow((q, k, v), 3, mon, "rbf_b200_fwd") if narrowed else (q, k, v)
+    qc, kc, vc = (_tma_ready(_pad_d(t, Dc)) for t in ins)
     out = torch.empty((B, H, N, Dc), dtype=cdt, device=q.device)
     lse = torch.empty((B, H, N), dtype=torch.float32, device=q.device) if softmax else None
     ws = _workspace(B, H, N, D, softmax, False, q.device)
-    mon = _monitor(q.device)
-    mon.poll()
     dense = _dense_strides3(H, N, Dc)
     with _OnDevice(q.device):
         mon.launch("rbf_b200_fwd", lambda slot: lib.rbf_b200_fwd_posting(
@@ -340,12 +382,10 @@ def _forward(q, k, v, is_causal: bool, softmax: bool):
             B, H, N, Dc, _strides3(qc, dense), _strides3(kc, dense), _strides3(vc, dense), dense,
             code, int(bool(is_causal)), int(softmax), 1.0 / math.sqrt(D0), _stream_ptr(q.device), _PHASE_ALL, slot,
         ))
-        if q.dtype == torch.float32 and not tf32:
-            mon.record_range_check((qc, kc, vc), "rbf_b200_fwd")
     if Dc != D0:
         out = out[..., :D0].contiguous()
-    if cdt != q.dtype:
-        out = out.to(q.dtype)
+    if narrowed:
+        (out,) = _widen([out])
     return out, lse
 
 
@@ -359,17 +399,22 @@ def _backward(q, k, v, out, lse, dout, is_causal: bool, sm_scale: float, softmax
     lib = _lib.load()
     cdt = _compute_dtype(q)
     Dc = _columns(D0, cdt)
-    qc, kc, vc, doc = (_tma_ready(_pad_d(t.to(cdt), Dc)) for t in (q, k, v, dout))
+    mon = _monitor(q.device)
+    mon.poll()
     # the non-softmax variant takes the forward output when the caller has it: the single-kernel backward needs it
     have_out = out is not None
-    oc = _tma_ready(_pad_d(out.to(cdt), Dc)) if have_out else None
+    ins = (q, k, v, dout, out) if have_out else (q, k, v, dout)
+    if cdt != q.dtype:
+        ins = _narrow(ins, 4, mon, "rbf_b200_bwd")
+    elif have_out and out.dtype != cdt:
+        ins = (q, k, v, dout, out.to(cdt))
+    qc, kc, vc, doc, *oc = (_tma_ready(_pad_d(t, Dc)) for t in ins)
+    oc = oc[0] if have_out else None
     dq = torch.empty((B, H, N, Dc), dtype=cdt, device=q.device)
     dk = torch.empty_like(dq)
     dv = torch.empty_like(dq)
     ws = _workspace(B, H, N, D, softmax, True, q.device)
     z3 = _lib.I64x3(0, 0, 0)
-    mon = _monitor(q.device)
-    mon.poll()
     # torch.use_deterministic_algorithms(True) selects the backward whose summation order is fixed
     lib.rbf_b200_set_deterministic(int(torch.are_deterministic_algorithms_enabled()))
     dense = _dense_strides3(H, N, Dc)
@@ -383,12 +428,10 @@ def _backward(q, k, v, out, lse, dout, is_causal: bool, sm_scale: float, softmax
             dense, dense, dense,
             _DTYPE_CODE[cdt], int(bool(is_causal)), int(softmax), float(sm_scale), _stream_ptr(q.device), _PHASE_ALL, slot,
         ))
-        if q.dtype == torch.float32:
-            mon.record_range_check((qc, kc, vc, doc), "rbf_b200_bwd")
     if Dc != D0:
         dq, dk, dv = (t[..., :D0].contiguous() for t in (dq, dk, dv))
     if cdt != q.dtype:
-        dq, dk, dv = dq.to(q.dtype), dk.to(q.dtype), dv.to(q.dtype)
+        dq, dk, dv = _widen([dq, dk, dv])
     return dq, dk, dv
 
 

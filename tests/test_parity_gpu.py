@@ -873,3 +873,35 @@ def test_head_dims_that_are_multiples_of_eight_run_in_place(D, softmax, causal, 
     for name, got, want in zip(("O", "dQ", "dK", "dV"), (out, *grads), ref):
         assert got.shape == want.shape
         check(name, got.cpu().float(), want, REL_L2[dtype])
+
+
+@pytest.mark.parametrize("D,view", [(64, "dense"), (72, "dense"), (64, "bnhd"), (64, "odd"), (36, "dense"), (64, "mixed")])
+def test_fp32_conversions_equal_torchs(D, view):
+    """One launch for all tensors of a call, both ways: bitwise what .to() gives, and only an input that becomes infinite
+    is reported. Layouts that the kernel does not take (odd offsets, 36 columns, another dtype) go through PyTorch."""
+    B, H, N = 2, 3, 77
+    g = torch.Generator(device=DEV).manual_seed(D)
+    if view == "bnhd":
+        src = [torch.randn((B, N, H, D), generator=g, device=DEV).permute(0, 2, 1, 3) for _ in range(5)]
+    elif view == "odd":
+        src = [torch.randn(B * H * N * D + 1, generator=g, device=DEV)[1:].view(B, H, N, D) for _ in range(5)]
+    else:
+        src = [torch.randn((B, H, N, D), generator=g, device=DEV) for _ in range(5)]
+    if view == "mixed":
+        src[4] = src[4].half()
+    mon = ops._monitor(torch.device(DEV))
+    got = ops._narrow(src, 4, mon, "test")
+    for a, b in zip(got, src):
+        assert torch.equal(a, b.to(torch.float16))
+    for a, b in zip(ops._widen(got[:3]), got):
+        assert torch.equal(a, b.float())
+    ops.check_device_status()
+    src[0][1, 2, 76, D - 1] = float("nan")              # not an infinity
+    if view != "mixed":
+        src[4][0, 0, 0, 0] = 1e6                        # not among the checked
+    ops._narrow(src, 4, mon, "test")
+    ops.check_device_status()
+    src[3][1, 2, 76, D - 1] = -65520.0                  # the smallest magnitude that rounds to infinity
+    ops._narrow(src, 4, mon, "test")
+    with pytest.raises(RuntimeError, match="float16's range"):
+        ops.check_device_status()
