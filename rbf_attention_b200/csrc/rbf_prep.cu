@@ -187,6 +187,29 @@ __device__ __forceinline__ float load_param(const void* base, int64_t index, boo
   return __half2float(__ushort_as_half(raw));
 }
 
+// Eight consecutive parameters, index a multiple of 8: 16-byte loads where the array is aligned for them (it is unless the
+// caller passes a view), single ones otherwise. qkv_prep_kernel at B64 S1028 H8 D64: 65 -> 63 us, B4 S4100 fp16 14.0 -> 13.3.
+__device__ __forceinline__ void load_param8(const void* base, int64_t index, bool fp32, bool bf16, float (&out)[8]) {
+  const uint8_t* p = reinterpret_cast<const uint8_t*>(base) + index * (fp32 ? 4 : 2);
+  if (reinterpret_cast<uintptr_t>(base) % 16 != 0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) out[j] = load_param(base, index + j, fp32, bf16);
+  } else if (fp32) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w;
+    out[4] = b.x; out[5] = b.y; out[6] = b.z; out[7] = b.w;
+  } else {
+    const uint4 raw = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = bf16 ? unpack2<true>(w[i]) : unpack2<false>(w[i]);
+      out[2 * i] = f.x;
+      out[2 * i + 1] = f.y;
+    }
+  }
+}
+
 template <bool kBf16>
 __device__ __forceinline__ uint4 add_round8(const uint4& x, const float (&e)[8], float& sumsq) {
   const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
@@ -227,15 +250,14 @@ __global__ void __launch_bounds__(256) qkv_prep_kernel(const QkvPrepArgs a) {
     if (valid) {
       float e[8];
       if (s < a.R) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          e[j] = load_param(a.reg_pos, (static_cast<int64_t>(h) * a.R + s) * D + part * 8 + j, a.params_fp32, kBf16);
+        load_param8(a.reg_pos, (static_cast<int64_t>(h) * a.R + s) * D + part * 8, a.params_fp32, kBf16, e);
       } else {
-        const float* trow = a.table + static_cast<int64_t>(s - a.R) * D + part * 8;
-        const int i0 = (part * 8) % (D / 2);
+        const float4* trow = reinterpret_cast<const float4*>(a.table + static_cast<int64_t>(s - a.R) * D + part * 8);
+        const float4 t0 = trow[0], t1 = trow[1];
+        load_param8(a.pos_weight, static_cast<int64_t>(h) * (D / 2) + (part * 8) % (D / 2), a.params_fp32, kBf16, e);
+        const float tv[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          e[j] = trow[j] * load_param(a.pos_weight, static_cast<int64_t>(h) * (D / 2) + i0 + j, a.params_fp32, kBf16);
+        for (int j = 0; j < 8; ++j) e[j] *= tv[j];
       }
       const uint16_t* src = reinterpret_cast<const uint16_t*>(a.qkv) + (static_cast<int64_t>(b) * a.S + s) * 3 * E +
                             static_cast<int64_t>(h) * D + part * 8;

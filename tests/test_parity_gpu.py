@@ -905,3 +905,22 @@ def test_fp32_conversions_equal_torchs(D, view):
     ops._narrow(src, 4, mon, "test")
     with pytest.raises(RuntimeError, match="float16's range"):
         ops.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_block_parameters_at_odd_addresses(dtype):
+    """pos_weight and reg_pos_emb that are not 16-byte aligned take single loads: bitwise the aligned result."""
+    B, S, H, D, R = 2, 70, 3, 64, 4
+    g = torch.Generator(device=DEV).manual_seed(1)
+    qkv = torch.randn((B, S, 3 * H * D), generator=g, device=DEV).bfloat16()
+    pw, rp = (torch.randn(s, generator=g, device=DEV).to(dtype) for s in ((H, D // 2), (H, R, D)))
+    table = attention.get_unrotated_sinusoids(S - R, D, DEV)
+
+    def odd(t):
+        buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)[1:]
+        return buf.view(t.shape).copy_(t)
+
+    want = ops._susie_block_fwd(qkv, pw, rp, table, H, True)
+    got = ops._susie_block_fwd(qkv, odd(pw), odd(rp), table, H, True)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
