@@ -27,9 +27,9 @@
 // traced, their waits are over when they get to them), in which TMEM and shared-memory latencies stretch with the MMA
 // operand traffic; taking all MMAs out shortens the whole backward by 22 %, the exponentials by 4 %, the drain by 6 %.
 // Between items they only wait for the next scores: the drain warps finish dK and dV. Measured against one item at a
-// time with the epilogue on the compute warps (backward call, B8 H16 N4096 causal: 926 -> 898 us; B4 H12 N1000 full:
-// 67.0 -> 62.0 us; N8192 B4 H16 training pass 2.71 -> 2.64 ms; N1028 B64 H8 unchanged at 485 us, bound by how fast
-// loads and drains of items of five steps follow each other).
+// time with the epilogue on the compute warps (backward call, B8 H16 N4096 causal: 926 -> 897 us; B4 H12 N1000 full:
+// 67.0 -> 61.4 us; N8192 B4 H16 training pass 2.71 -> 2.64 ms; N1028 B64 H8 about 480 us as before, bound by how
+// fast loads and drains of items of five steps on average follow each other).
 // TMEM columns: S^T [0,128), dP^T [128,256), P^T [256,320), dV [320,384), dK [384,448), dQ_partial [448,512).
 #include "common.cuh"
 #include "launch.h"
@@ -49,11 +49,13 @@ static constexpr int kMmaWarpC = 3;
 static constexpr int kComputeWarp0 = 4;
 static constexpr int kDrainWarp0 = 20;
 // Register budget: the launch allocates 80 per thread (768 threads); setmaxnreg may only redistribute that
-// total: 512 * 96 + 128 * 40 + 128 * 56 = 768 * 80. (An increase beyond what the decreases released blocks
-// forever, with no timeout.)
+// total: 512 * 96 + 128 * 32 + 128 * 64 = 768 * 80. (An increase beyond what the decreases released blocks
+// forever, with no timeout.) The drain warps lag behind on short items; with 56 registers, dK finished after the last
+// dQ_partial and scalar arithmetic the backward call took 42.2 us (now 41.1) at B4 H8 N1024, 62.6 (61.4) at B4 H12 N1000
+// full, 907 (897) at B8 H16 N4096.
 static constexpr int kComputeRegs = 96;
-static constexpr int kOtherRegs = 40;
-static constexpr int kDrainRegs = 56;
+static constexpr int kOtherRegs = 32;
+static constexpr int kDrainRegs = 64;
 static_assert(512 * kComputeRegs + 128 * kOtherRegs + 128 * kDrainRegs <= 768 * 80, "setmaxnreg budget");
 static constexpr int kDqBoxBytes = 32 * 128;        // 4 KB: 32 rows of 128 bytes of one drain warp
 
@@ -130,7 +132,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
   const float* s_ksq = reinterpret_cast<const float*>(smem + Smem::kKsq);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Smem::kBars);
   uint64_t* k_full = bars;                   // [2] K tile and key norms of an item landed
-  uint64_t* k_free = k_full + 2;             // [2] the item's dK has been formed (all MMAs that read K are complete)
+  uint64_t* k_free = k_full + 2;             // [2] the item's last dQ_partial is drained (nothing reads K any more)
   uint64_t* v_full = k_free + 2;
   uint64_t* v_free = v_full + 1;             // the item's last dP^T has completed
   uint64_t* q_full = v_free + 1;             // [kQStages] Q tile + L slab landed
@@ -429,6 +431,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
             umma_ss(tmem + kColDK, sdesc_at(ds_kmaj, (kk >> 2) * (kTile * 128) + (kk & 3) * 32), sdesc_at(q_n, kk * 2048),
                     idesc_acc, (n > 0 || kk > 0) ? 1u : 0u);
           umma_commit(&q_empty[st]);
+          if (n == cnt - 1) umma_commit(dk_acc);   // the item's dK is complete
         }
         if (g > 0) ok = mbar_wait(dq_drained, (g - 1) & 1, abort_flag, p.status, kSiteDQDrained, s_item);
         if (!ok) break;
@@ -438,7 +441,6 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
           for (int kk = 0; kk < kTile / 16; ++kk)
             umma_ss(tmem + kColDQ, sdesc_at(ds_mmaj, kk * 2048), sdesc_at(k_nmaj, kk * 2048), idesc_dq, kk > 0);
           umma_commit(dq_full);                    // dQ_partial readable; the dS^T tile's readers are done
-          if (n == cnt - 1) umma_commit(dk_acc);   // the item's dK is complete, and K has no reader but the drain
         }
       }
     }
@@ -494,7 +496,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     while (ok && next_item()) {
     const int row0 = k_row0 + wq * 32;             // this warp's key rows
     for (int n = 0; n < cnt - 1 && ok; ++n) ok = drain_dq(n);
-    // dV is complete one product before the last dQ_partial
+    // dV and dK are complete before the last dQ_partial, and the next item's products wait for their columns
     if (ok) ok = mbar_wait(dv_acc, I & 1, abort_flag, p.status, kSiteDVAcc, s_item);
     if (!ok) break;
     tc_fence_after_sync();
@@ -525,7 +527,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
         tma_store_commit();
       }
     }
-    ok = drain_dq(cnt - 1) && mbar_wait(dk_acc, I & 1, abort_flag, p.status, kSiteDKAcc, s_item) &&
+    ok = mbar_wait(dk_acc, I & 1, abort_flag, p.status, kSiteDKAcc, s_item) &&
          mbar_wait(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item) &&
          mbar_wait(&rs_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteRowsum, s_item);
     if (!ok) break;
@@ -554,14 +556,14 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const float2 kv = unpack2<kBf16>(kw[i]);
-            const float x0 = p.grad_scale * fmaf(-w, kv.x, __uint_as_float(acc[q4 * 8 + 2 * i]));
-            const float x1 = p.grad_scale * fmaf(-w, kv.y, __uint_as_float(acc[q4 * 8 + 2 * i + 1]));
+            float x0, x1;
+            ffma2v(x0, x1, kv.x, kv.y, -w, -w, __uint_as_float(acc[q4 * 8 + 2 * i]), __uint_as_float(acc[q4 * 8 + 2 * i + 1]));
+            fmul2(x0, x1, x0, x1, p.grad_scale, p.grad_scale);
             o[i] = pack2<kBf16>(x0, x1);
           }
           *reinterpret_cast<uint4*>(box + sw128_offset(lane, hh * 4 + q4)) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
-      mbar_arrive_warp(&k_free[I & 1]);
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
@@ -569,6 +571,9 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
         tma_store_commit();
       }
     }
+    ok = drain_dq(cnt - 1);
+    if (!ok) break;
+    mbar_arrive_warp(&k_free[I & 1]);        // the last dQ_partial was K's last reader
     T += cnt;
     ++I;
     }
