@@ -18,7 +18,6 @@ import time
 
 import torch
 from torch.autograd import forward_ad
-from torch.autograd.function import once_differentiable
 
 from . import _lib
 
@@ -45,6 +44,28 @@ def _direct(*tensors) -> bool:
         if t is not None and not (type(t) in _PLAIN_TYPES and t.is_cuda):
             return False
     return True
+
+
+def _direct_backward(*tensors) -> bool:
+    """``_direct`` for a backward formula. Under ``create_graph`` (the only time a backward runs with grad mode on) the
+    registered operator computes the gradient: it has no autograd formula, so what it returns is linked to its inputs and
+    refuses to be differentiated, while a direct call's result would be a constant and a penalty on it would silently add
+    nothing."""
+    return not torch.is_grad_enabled() and _direct(*tensors)
+
+
+class _FirstOrderOnly(torch.autograd.Function):
+    """``grad`` itself, linked to the ``origins`` that it was computed from and refusing to be differentiated: for gradients
+    formed under ``create_graph`` from saved tensors that carry no graph of their own."""
+
+    @staticmethod
+    def forward(ctx, what, grad, *origins):
+        ctx.what = what
+        return grad.view_as(grad)
+
+    @staticmethod
+    def backward(ctx, *_grads):
+        raise RuntimeError(f"Trying to backward through the gradient of {ctx.what}, which has no second-order formula")
 
 
 def _needs_grad(*tensors) -> bool:
@@ -737,7 +758,7 @@ def _susie_block_backward(ctx, dout, dlse, dqk):
     qkv, qk, out, lse, table = ctx.saved_tensors
     if dout is None:
         return None, None, None, None, None, None
-    bwd = _susie_block_bwd if _direct(qkv, qk, out, lse, dout, table) else torch.ops.rbf_attn_b200.susie_block_bwd
+    bwd = _susie_block_bwd if _direct_backward(qkv, qk, out, lse, dout, table) else torch.ops.rbf_attn_b200.susie_block_bwd
     dqkv, d_pw, d_rp = bwd(qkv, qk, out, lse, dout, table, ctx.num_registers, ctx.softmax)
     d_rp = None if ctx.rp_dtype is None else d_rp.to(ctx.rp_dtype)
     return dqkv, d_pw.to(ctx.pw_dtype), d_rp, None, None, None
@@ -758,7 +779,6 @@ class _SusieBlock(torch.autograd.Function):
         return out
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, dout):
         return _susie_block_backward(ctx, dout, None, None)
 
@@ -886,7 +906,7 @@ class _LinearBiasSum(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             dw = g2.t().mm(x.reshape(-1, x.shape[-1]))
         if ctx.needs_input_grad[2]:
-            sums = _column_sums if _direct(g2) else torch.ops.rbf_attn_b200.column_sums
+            sums = _column_sums if _direct_backward(g2) else torch.ops.rbf_attn_b200.column_sums
             db = sums(g2).to(g.dtype)
         return dx, dw, db
 
@@ -946,13 +966,16 @@ class _LinearGelu(torch.autograd.Function):
     def forward(ctx, x, weight, bias):
         h = torch.nn.functional.linear(x, weight, bias)
         ctx.save_for_backward(x, weight, h)
+        ctx.bias = bias         # a link for create_graph: its value is not read again, so it may change in place
         return (_gelu_fwd if _direct(h) else torch.ops.rbf_attn_b200.gelu_fwd)(h)
 
     @staticmethod
     def backward(ctx, g):
         x, weight, h = ctx.saved_tensors
-        bwd = _gelu_bwd if _direct(h, g) else torch.ops.rbf_attn_b200.gelu_bwd
+        bwd = _gelu_bwd if _direct_backward(h, g) else torch.ops.rbf_attn_b200.gelu_bwd
         dh, dbias = bwd(h, g, ctx.needs_input_grad[2])
+        if torch.is_grad_enabled():         # h was saved without the graph that made it
+            dh, dbias = (_FirstOrderOnly.apply("linear_gelu", t, x, weight, ctx.bias, g) for t in (dh, dbias))
         dh2 = dh.reshape(-1, dh.shape[-1])
         dx = dh.matmul(weight) if ctx.needs_input_grad[0] else None
         dw = dh2.t().mm(x.reshape(-1, x.shape[-1])) if ctx.needs_input_grad[1] else None
@@ -1056,7 +1079,7 @@ def _ln_backward(ctx, g_y, _g_mean, _g_rstd):
     if g_y is None:
         return None, None, None, None
     x, weight, mean, rstd = ctx.saved_tensors
-    bwd = _layer_norm_bwd if _direct(x, g_y, weight, mean, rstd) else torch.ops.rbf_attn_b200.layer_norm_bwd
+    bwd = _layer_norm_bwd if _direct_backward(x, g_y, weight, mean, rstd) else torch.ops.rbf_attn_b200.layer_norm_bwd
     dx, dgamma, dbeta = bwd(x, g_y, weight, mean, rstd)
     return dx, dgamma, dbeta, None
 
@@ -1074,7 +1097,6 @@ class _LayerNorm(torch.autograd.Function):
         return output[0]
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, g_y):
         return _ln_backward(ctx, g_y, None, None)
 
@@ -1168,7 +1190,7 @@ def _add_ln_backward(ctx, g_s, g_y, _g_mean, _g_rstd):
     if g_y is None:
         return g_s, g_s, None, None, None
     s, weight, mean, rstd = ctx.saved_tensors
-    direct = _direct(s, g_y, g_s, weight, mean, rstd)
+    direct = _direct_backward(s, g_y, g_s, weight, mean, rstd)
     if g_s is None:
         bwd = _layer_norm_bwd if direct else torch.ops.rbf_attn_b200.layer_norm_bwd
         dx, dgamma, dbeta = bwd(s, g_y, weight, mean, rstd)
@@ -1192,7 +1214,6 @@ class _AddLayerNorm(torch.autograd.Function):
         return output[0], output[1]
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, g_s, g_y):
         return _add_ln_backward(ctx, g_s, g_y, None, None)
 
@@ -1265,7 +1286,7 @@ scale_unless_one_ = torch.library.custom_op("rbf_attn_b200::scale_unless_one_", 
 
 
 def _ce_setup_context(ctx, inputs, output):
-    ctx.save_for_backward(output[1])
+    ctx.save_for_backward(output[1])        # an output, so that under create_graph it is linked to the logits
     ctx.set_materialize_grads(False)        # no zero tensor of the logits' size for the unused second output
 
 
@@ -1275,12 +1296,15 @@ def _ce_backward(ctx, g_loss, _g_dlogits):
     if g_loss is None:
         return None, None, None
     (dlogits,) = ctx.saved_tensors
-    if _direct(dlogits, g_loss):
-        _scale_unless_one(dlogits, g_loss)
-        torch.autograd.graph.increment_version(dlogits)     # as the operator layer does for what it mutates
-    else:
-        torch.ops.rbf_attn_b200.scale_unless_one_(dlogits, g_loss)
-    return dlogits, None, None
+    with torch.no_grad():
+        if _direct(dlogits, g_loss):
+            _scale_unless_one(dlogits, g_loss)
+            torch.autograd.graph.increment_version(dlogits)     # as the operator layer does for what it mutates
+        else:
+            torch.ops.rbf_attn_b200.scale_unless_one_(dlogits, g_loss)
+    if torch.is_grad_enabled():
+        return _FirstOrderOnly.apply("cross_entropy", dlogits, g_loss), None, None
+    return dlogits.detach(), None, None
 
 
 torch.library.register_autograd("rbf_attn_b200::cross_entropy_fwd", _ce_backward, setup_context=_ce_setup_context)
@@ -1293,12 +1317,11 @@ class _CrossEntropy(torch.autograd.Function):
     def forward(ctx, logits, targets, ignore_index):
         output = _cross_entropy_fwd(logits, targets, ignore_index)
         _ce_setup_context(ctx, (logits, targets, ignore_index), output)
-        return output[0]
+        return output
 
     @staticmethod
-    @once_differentiable
-    def backward(ctx, g_loss):
-        return _ce_backward(ctx, g_loss, None)
+    def backward(ctx, g_loss, g_dlogits):
+        return _ce_backward(ctx, g_loss, g_dlogits)
 
 
 def cross_entropy(logits, targets, ignore_index: int = -100):
@@ -1306,7 +1329,7 @@ def cross_entropy(logits, targets, ignore_index: int = -100):
     gradient produced by the forward kernel."""
     if type(ignore_index) is int and _direct(logits, targets):
         if _needs_grad(logits):
-            return _CrossEntropy.apply(logits, targets, ignore_index)
+            return _CrossEntropy.apply(logits, targets, ignore_index)[0]
         return _cross_entropy_fwd(logits, targets, ignore_index)[0]
     return torch.ops.rbf_attn_b200.cross_entropy_fwd(logits, targets, ignore_index)[0]
 
@@ -1325,11 +1348,10 @@ class _ScaledAttention(torch.autograd.Function):
         return out
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, dout):
         q, k, v, out, lse = ctx.saved_tensors
         sm_scale = 1.0 / math.sqrt(q.shape[-1])
-        if _direct(q, k, v, out, lse, dout):
+        if _direct_backward(q, k, v, out, lse, dout):
             return *_backward(q, k, v, out, lse, dout, ctx.is_causal, sm_scale, softmax=True), None
         return *torch.ops.rbf_attn_v5.scaled_bwd(q, k, v, out, lse, dout, ctx.is_causal, sm_scale), None
 
@@ -1345,11 +1367,10 @@ class _NonSoftmaxAttention(torch.autograd.Function):
         return out
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, dout):
         q, k, v, out = ctx.saved_tensors
         sm_scale = 1.0 / math.sqrt(q.shape[-1])
-        if _direct(q, k, v, out, dout):
+        if _direct_backward(q, k, v, out, dout):
             return *_backward(q, k, v, out, None, dout, ctx.is_causal, sm_scale, softmax=False), None
         return *torch.ops.rbf_attn_v5.non_softmax_bwd_with_out(q, k, v, out, dout, ctx.is_causal, sm_scale), None
 

@@ -94,7 +94,7 @@ def test_direct_calls_equal_the_operators(name, monkeypatch):
 
 @pytest.mark.parametrize("name", sorted(CASES))
 def test_direct_calls_keep_autograds_rules(name):
-    """Saved tensors go through the hooks, and a second differentiation is refused as the operators refuse it."""
+    """Saved tensors go through the hooks."""
     torch.manual_seed(0)
     run = CASES[name][0]()
     want = _grads(run)
@@ -107,12 +107,22 @@ def test_direct_calls_keep_autograds_rules(name):
         assert (a.float() - b.float()).norm() <= 1e-3 * b.float().norm() + 1e-12
 
 
-def test_second_order_gradients_are_refused():
-    run = CASES["softmax"][0]()
-    out, (q, k, v) = run()
-    (dq,) = torch.autograd.grad(out.float().square().sum(), (q,), create_graph=True)
-    with pytest.raises(RuntimeError):
-        torch.autograd.grad(dq.float().sum(), (q,))
+@pytest.mark.parametrize("loss", ["linear", "quadratic"])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_second_order_gradients_are_refused(name, loss):
+    """A gradient taken with ``create_graph`` equals the plain one and refuses to be differentiated, as the registered
+    backward operators do (test_second_order_cpu.py has the cases of the graph alone)."""
+    torch.manual_seed(0)
+    run = CASES[name][0]()
+    reduce = (lambda t: t.float().sum()) if loss == "linear" else (lambda t: t.float().square().sum())
+    out, inputs = run()
+    (want,) = torch.autograd.grad(reduce(out), inputs[:1])
+    out, inputs = run()
+    (got,) = torch.autograd.grad(reduce(out), inputs[:1], create_graph=True)
+    assert not want.requires_grad and got.requires_grad
+    assert (got.float() - want.float()).norm() <= 1e-3 * want.float().norm() + 1e-12
+    with pytest.raises(RuntimeError, match="Trying to backward through"):
+        got.float().square().sum().backward()
 
 
 def test_what_is_not_a_plain_cuda_tensor_takes_the_operator():
