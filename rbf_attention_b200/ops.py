@@ -9,6 +9,7 @@ Reference counterparts (paths inside the reference project):
 
 from __future__ import annotations
 
+import collections
 import ctypes
 import functools
 import math
@@ -189,6 +190,18 @@ def _workspace(B, H, N, D, softmax, backward, device) -> torch.Tensor:
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
+# States of a status entry: its slot is taken but its call has not returned yet; the call's kernels are enqueued and will
+# post; the call was left by an exception and may or may not post.
+_RESERVED, _ENQUEUED, _ABANDONED = range(3)
+
+
+class _StatusEntry:
+    __slots__ = ("slot", "what", "state")
+
+    def __init__(self, slot, what):
+        self.slot, self.what, self.state = slot, what, _RESERVED
+
+
 class _StatusMonitor:
     """Surfaces device-side wait timeouts of the operator path without synchronising.
 
@@ -215,40 +228,91 @@ class _StatusMonitor:
             _lib.check(_lib.load().rbf_b200_map_status_slots(self.base, ctypes.byref(mapped)), "rbf_b200_map_status_slots")
         self.mapped = mapped.value              # the ring's address on the device
         self.lock = threading.RLock()           # forward and backward run on different threads
-        self.what = [""] * self.SLOTS
-        self.oldest = 0        # the pending entries are the slots oldest, oldest + 1, ..., next - 1 (mod SLOTS)
-        self.next = 0
-        self.pending = 0
+        self.free = collections.deque(range(self.SLOTS))
+        self.pending: dict = {}                 # slot -> entry, in the order of their reservation
 
-    def _retire_oldest(self):
-        i = self.oldest
-        self.oldest = (i + 1) % self.SLOTS
-        self.pending -= 1
-        code = int(self.slots[i]) & 0xFFFFFFFF
-        if code != 0:
-            self.slots[i] = 0
-            if self.what[i].startswith("range:"):
-                raise RuntimeError(
-                    f"{self.what[i][6:]}: float32 inputs exceed float16's range (|x| >= 65504) on a path that runs on "
-                    "float16 tensor-core operands; its results contain inf / nan. Scale the inputs or use bfloat16"
-                )
+    def _reserve(self, what) -> _StatusEntry:
+        deadline = time.monotonic() + 10.0
+        while True:
+            with self.lock:
+                if not self.free:
+                    self.poll()
+                if self.free:
+                    entry = _StatusEntry(self.free.popleft(), what)
+                    self.slots[entry.slot] = self._NOT_YET
+                    self.pending[entry.slot] = entry
+                    return entry
+            # The ring is full: the oldest word belongs to a call SLOTS calls ago and arrives without any help from this
+            # thread. (A device-wide synchronisation here would also drain the caller's copy streams: only when it is late.)
+            if time.monotonic() > deadline:
+                self.poll(wait=True)
+                deadline = time.monotonic() + 10.0
+            time.sleep(0)
+
+    def _retire(self, entry) -> None:
+        del self.pending[entry.slot]
+        self.free.append(entry.slot)
+
+    def _check(self, code, what) -> None:
+        if code == 0:
+            return
+        if what.startswith("range:"):
             raise RuntimeError(
-                f"{self.what[i]}: a device-side wait ran out (site {code >> 24}, work unit {code & 0xFFFFFF}); "
-                "the results of that call are incomplete"
+                f"{what[6:]}: float32 inputs exceed float16's range (|x| >= 65504) on a path that runs on "
+                "float16 tensor-core operands; its results contain inf / nan. Scale the inputs or use bfloat16"
             )
+        raise RuntimeError(
+            f"{what}: a device-side wait ran out (site {code >> 24}, work unit {code & 0xFFFFFF}); "
+            "the results of that call are incomplete"
+        )
 
     def poll(self, wait=False):
-        """Checks the entries whose status word has arrived, oldest first (all of them, after waiting for the device,
-        when ``wait``)."""
+        """Checks the entries whose status word has arrived, oldest first (when ``wait``: of all calls enqueued so far,
+        after waiting for the device; calls that other threads enqueue meanwhile are left to a later look)."""
+        due = set()
         if wait and self.pending:
+            with self.lock:
+                due.update(e for e in self.pending.values() if e.state != _RESERVED)
             torch.cuda.synchronize(self.device)
+        done, code, what = [], 0, ""
         with self.lock:
-            while self.pending:
-                if self.slots[self.oldest] == self._NOT_YET:
-                    if wait:
-                        raise RuntimeError(f"{self.what[self.oldest]}: the status word did not arrive")
+            for e in self.pending.values():
+                code, what = int(self.slots[e.slot]), e.what
+                if code == self._NOT_YET:
+                    code = 0
+                    if e not in due:
+                        if wait or e.state != _ENQUEUED:
+                            continue
+                        break
+                    if e.state == _ENQUEUED:
+                        done.append(e)
+                        code = self._NOT_YET
+                        break
+                done.append(e)
+                if code != 0:
                     break
-                self._retire_oldest()
+            for e in done:
+                self._retire(e)
+        if code == self._NOT_YET:
+            raise RuntimeError(f"{what}: the status word did not arrive")
+        self._check(code & 0xFFFFFFFF, what)
+
+    def _enqueue(self, what, call) -> None:
+        """``call(slot number)`` enqueues what posts a status word there and returns an error code."""
+        entry = self._reserve(what)
+        try:
+            rc = call(entry.slot)
+            entry.state = _ENQUEUED
+        except BaseException:
+            # whether something was enqueued is not known: the slot is not used again before the device has been waited for
+            entry.state = _ABANDONED
+            raise
+        if rc != 0:                             # nothing was enqueued that could post
+            with self.lock:
+                self._retire(entry)
+            _lib.check(rc, what)
+        if _SYNC_STATUS:
+            self.poll(wait=True)
 
     def record_range_check(self, tensors, what):
         """fp32 tensors narrowed to fp16 operands: records (asynchronously, like the status word) whether the
@@ -260,52 +324,20 @@ class _StatusMonitor:
         flag[0] = bad
         self.record(flag, "range:" + what)
 
-    def _reserve(self, what) -> int:
-        with self.lock:
-            if self.pending == self.SLOTS:      # the ring is full: wait for its oldest entry, and for that one only
-                self.poll()
-                if self.pending == self.SLOTS:
-                    # (its kernel was enqueued SLOTS calls ago: the word arrives without any help from this thread. A
-                    # device-wide synchronisation here would also drain the caller's copy streams.)
-                    deadline = time.monotonic() + 10.0
-                    while self.slots[self.oldest] == self._NOT_YET:
-                        if time.monotonic() > deadline:
-                            torch.cuda.synchronize(self.device)
-                            break
-                        time.sleep(0)
-                    self._retire_oldest()
-            i = self.next
-            self.slots[i] = self._NOT_YET
-            self.what[i] = what
-            self.next = (i + 1) % self.SLOTS
-            self.pending += 1
-            return i
-
     def launch(self, what, call) -> None:
         """``call(slot address)`` enqueues a call whose last kernel posts its status word there (0: no posting, while a
         CUDA graph is being captured) and returns its error code."""
         if torch._C._cuda_isCurrentStreamCapturing():
             _lib.check(call(0), what)
             return
-        i = self._reserve(what)
-        rc = call(self.mapped + 4 * i)
-        if rc != 0:
-            self.slots[i] = 0                   # nothing was enqueued that could post
-            _lib.check(rc, what)
-        if _SYNC_STATUS:
-            self.poll(wait=True)
+        self._enqueue(what, lambda slot: call(self.mapped + 4 * slot))
 
     def record(self, ws, what):
         """Posts the status word at the start of ``ws`` with a kernel of its own."""
         if torch.cuda.is_current_stream_capturing():
             return
-        i = self._reserve(what)
-        rc = _lib.load().rbf_b200_post_device_status(ws.data_ptr(), self.base + 4 * i, _stream_ptr(ws.device))
-        if rc != 0:
-            self.slots[i] = 0
-            _lib.check(rc, "rbf_b200_post_device_status")
-        if _SYNC_STATUS:
-            self.poll(wait=True)
+        self._enqueue(what, lambda slot: _lib.load().rbf_b200_post_device_status(
+            ws.data_ptr(), self.base + 4 * slot, _stream_ptr(ws.device)))
 
 
 _SYNC_STATUS = os.environ.get("RBF_B200_SYNC_STATUS", "0") not in ("", "0")
@@ -316,7 +348,7 @@ def _monitor(device) -> _StatusMonitor:
     key = device.index if device.index is not None else torch.cuda.current_device()
     m = _monitors.get(key)
     if m is None:
-        m = _monitors[key] = _StatusMonitor(device)
+        m = _monitors.setdefault(key, _StatusMonitor(device))
     return m
 
 
