@@ -253,9 +253,9 @@ class _StatusMonitor:
         del self.pending[entry.slot]
         self.free.append(entry.slot)
 
-    def _check(self, code, what) -> None:
-        if code == 0:
-            return
+    def _report(self, code, what) -> None:
+        if code == self._NOT_YET & 0xFFFFFFFF:
+            raise RuntimeError(f"{what}: the status word did not arrive")
         if what.startswith("range:"):
             raise RuntimeError(
                 f"{what[6:]}: float32 inputs exceed float16's range (|x| >= 65504) on a path that runs on "
@@ -269,10 +269,12 @@ class _StatusMonitor:
     def poll(self, wait=False):
         """Checks the entries whose status word has arrived, oldest first (when ``wait``: of all calls enqueued so far,
         after waiting for the device; calls that other threads enqueue meanwhile are left to a later look)."""
-        due = set()
-        if wait and self.pending:
+        if not self.pending:
+            return
+        due = ()
+        if wait:
             with self.lock:
-                due.update(e for e in self.pending.values() if e.state != _RESERVED)
+                due = {e for e in self.pending.values() if e.state != _RESERVED}
             torch.cuda.synchronize(self.device)
         done, code, what = [], 0, ""
         with self.lock:
@@ -293,9 +295,8 @@ class _StatusMonitor:
                     break
             for e in done:
                 self._retire(e)
-        if code == self._NOT_YET:
-            raise RuntimeError(f"{what}: the status word did not arrive")
-        self._check(code & 0xFFFFFFFF, what)
+        if code != 0:
+            self._report(code & 0xFFFFFFFF, what)
 
     def _enqueue(self, what, call) -> None:
         """``call(slot number)`` enqueues what posts a status word there and returns an error code."""
