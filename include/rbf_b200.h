@@ -278,7 +278,8 @@ int rbf_b200_set_deterministic(int on);
 int rbf_b200_get_deterministic(void);
 
 /* Self-test of the bounded device waits every kernel of the library relies on: launches one block that waits, with
- * the kernels' own wait routine, on a barrier that nothing arms. After `limit_cycles` SM clocks (at most 2e9) the
+ * the kernels' own wait routines (a warp's, whose lanes have to leave together, then one thread's), on a barrier that
+ * nothing arms. After `limit_cycles` SM clocks (at most 2e9) the
  * wait gives up, records site 250 in the status word at the start of `workspace` (at least 256 bytes, 256-byte
  * aligned) and the kernel returns by itself; rbf_b200_read_device_status then reports RBF_B200_ERR_DEVICE. A later
  * forward or backward call on the same workspace clears the word. Nothing traps, faults or spins without bound.

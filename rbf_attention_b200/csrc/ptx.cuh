@@ -82,7 +82,7 @@ __device__ __forceinline__ uint32_t status_unit(const volatile int* unit_ptr) {
   return blockIdx.y * gridDim.x + blockIdx.x;
 }
 
-// Non-blocking look at a phase: issued ahead of independent work, it takes the barrier's latency off a wait that is
+// Non-blocking look at a phase (lanes of a warp may see different answers): issued ahead of independent work, it takes the barrier's latency off a wait that is
 // already over when the thread gets to it.
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -96,7 +96,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait. Returns false when the wait ran out (after `limit` SM clocks) or another thread of the CTA raised
+// Bounded wait of one thread (the producers). Returns false when the wait ran out (after `limit` SM clocks) or another thread of the CTA raised
 // `abort_flag`. The first wait of a launch that runs out records (site, work unit) in the status word.
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                 DeviceStatus* status, uint32_t site, long long limit,
@@ -120,6 +120,36 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
                                           DeviceStatus* status, uint32_t site,
                                           const volatile int* unit_ptr = nullptr) {
   return mbar_wait_limit(bar, parity, abort_flag, status, site, kWaitCycleLimit, unit_ptr);
+}
+
+// The same wait by a whole converged warp: every lane gets the same answer. Lanes that decided for themselves could part
+// at a wait that runs out, one leaving for the end of the kernel while another goes on to a __syncwarp or a warp-wide
+// tensor-memory instruction and stands there without limit.
+__device__ __forceinline__ bool mbar_wait_warp_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                     DeviceStatus* status, uint32_t site, long long limit,
+                                                     const volatile int* unit_ptr = nullptr) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  uint32_t spins = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if ((++spins & 0x3f) == 0) {
+      const bool late = clock64() - t0 > limit;
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+      if (__any_sync(0xffffffffu, late)) {
+        if ((threadIdx.x & 31) == 0) {
+          *abort_flag = 1;
+          if (status != nullptr) atomicCAS(&status->code, 0u, (site << 24) | (status_unit(unit_ptr) & 0xffffffu));
+        }
+        return false;
+      }
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                               DeviceStatus* status, uint32_t site,
+                                               const volatile int* unit_ptr = nullptr) {
+  return mbar_wait_warp_limit(bar, parity, abort_flag, status, site, kWaitCycleLimit, unit_ptr);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -295,7 +295,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
     uint32_t grp_phase = 0;
     auto group_sync = [&]() -> bool {
       mbar_arrive_warp(grp_sync);
-      const bool done = mbar_wait(grp_sync, grp_phase & 1, abort_flag, p.status, kSiteGroup);
+      const bool done = mbar_wait_warp(grp_sync, grp_phase & 1, abort_flag, p.status, kSiteGroup);
       ++grp_phase;
       return done;
     };
@@ -317,7 +317,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
       const int sb = n % C::kSBufs;
       float cs_next = 0.f, cd_next = 0.f;
       if (n + 1 < cnt) fetch_col(n + 1, cs_next, cd_next);
-      ok = group_sync() && mbar_wait(&s_full[sb], (n / C::kSBufs) & 1, abort_flag, p.status, kSiteSFull);
+      ok = group_sync() && mbar_wait_warp(&s_full[sb], (n / C::kSBufs) & 1, abort_flag, p.status, kSiteSFull);
       if (!ok) break;
       tc_fence_after_sync();
       const float* vbuf = s_vec + (n & 1) * 2 * kTile;
@@ -360,7 +360,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
         mbar_arrive_warp(&p_full[sb]);
       }
 
-      ok = mbar_wait(dp_full, n & 1, abort_flag, p.status, kSiteDPFull);
+      ok = mbar_wait_warp(dp_full, n & 1, abort_flag, p.status, kSiteDPFull);
       if (!ok) break;
       tc_fence_after_sync();
       // dS = P * (dP - delta): read dP in four 32-column chunks, then write the packed dS over dP's columns
@@ -400,7 +400,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
       }
     }
 
-    if (ok) ok = mbar_wait(acc_done, 0, abort_flag, p.status, kSiteAccDone);
+    if (ok) ok = mbar_wait_warp(acc_done, 0, abort_flag, p.status, kSiteAccDone);
     if (ok) {
       tc_fence_after_sync();
       // All MMAs are complete: the B1 ring is free and serves as staging for the TMA stores.

@@ -255,12 +255,12 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         umma_ss(dst, sdesc_at(ones_desc, 0), sdesc_at(slab, 0), idesc_s, 1u);
       };
       auto wait_q = [&](int n) {
-        return mbar_wait(&q_full[n % kQStages], (n / kQStages) & 1, abort_flag, p.status, kSiteQFull);
+        return mbar_wait_warp(&q_full[n % kQStages], (n / kQStages) & 1, abort_flag, p.status, kSiteQFull);
       };
       auto wait_do = [&](int n) {
-        return mbar_wait(&do_full[n % kDoStages], (n / kDoStages) & 1, abort_flag, p.status, kSiteDoFull);
+        return mbar_wait_warp(&do_full[n % kDoStages], (n / kDoStages) & 1, abort_flag, p.status, kSiteDoFull);
       };
-      bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, kSiteKV);
+      bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status, kSiteKV);
 
       if (warp == kMmaWarpA) {
         const SmemDesc k_kmaj = make_sdesc_parts(smem_u32(s_k), 16, 1024);
@@ -279,7 +279,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         for (int n = 0; n < cnt && ok; ++n) {
           if (n + 1 < cnt) {
             const int st = (n + 1) % kQStages;
-            ok = wait_q(n + 1) && mbar_wait(s_consumed, n & 1, abort_flag, p.status, kSiteSConsumed);
+            ok = wait_q(n + 1) && mbar_wait_warp(s_consumed, n & 1, abort_flag, p.status, kSiteSConsumed);
             if (!ok) break;
             tc_fence_after_sync();
             if (el) {
@@ -289,7 +289,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
             }
           }
           // dV += P^T dO
-          ok = mbar_wait(p_full, n & 1, abort_flag, p.status, kSitePFull);
+          ok = mbar_wait_warp(p_full, n & 1, abort_flag, p.status, kSitePFull);
           if (!ok) break;
           tc_fence_after_sync();
           const SmemDesc do_n = stage_of(do_nmaj0, n % kDoStages, kQTileBytes);
@@ -319,7 +319,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         for (int n = 0; n < cnt && ok; ++n) {
           if (n + 1 < cnt) {
             const int st = (n + 1) % kDoStages;
-            ok = wait_do(n + 1) && mbar_wait(dp_consumed, n & 1, abort_flag, p.status, kSiteDPConsumed);
+            ok = wait_do(n + 1) && mbar_wait_warp(dp_consumed, n & 1, abort_flag, p.status, kSiteDPConsumed);
             if (!ok) break;
             tc_fence_after_sync();
             if (el) {
@@ -329,7 +329,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
             }
           }
           // dK += dS^T Q
-          ok = mbar_wait(&ds_full[n % kDsStages], (n / kDsStages) & 1, abort_flag, p.status, kSiteDSFull);
+          ok = mbar_wait_warp(&ds_full[n % kDsStages], (n / kDsStages) & 1, abort_flag, p.status, kSiteDSFull);
           if (!ok) break;
           tc_fence_after_sync();
           // A = the TMEM copy of dS^T (16-bit pairs, 32 columns): only Q is fetched from shared memory
@@ -349,8 +349,8 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         const SmemDesc k_mmaj = make_sdesc_parts(smem_u32(s_k), kBoxBytes, 1024);
         const SmemDesc ds_nmaj = make_sdesc_parts(smem_u32(s_ds), kBoxBytes, 1024);
         for (int n = 0; n < cnt && ok; ++n) {
-          ok = mbar_wait(&ds_full[n % kDsStages], (n / kDsStages) & 1, abort_flag, p.status, kSiteDSFull);
-          if (ok && n > 0) ok = mbar_wait(dq_drained, (n - 1) & 1, abort_flag, p.status, kSiteDQDrained);
+          ok = mbar_wait_warp(&ds_full[n % kDsStages], (n / kDsStages) & 1, abort_flag, p.status, kSiteDSFull);
+          if (ok && n > 0) ok = mbar_wait_warp(dq_drained, (n - 1) & 1, abort_flag, p.status, kSiteDQDrained);
           if (!ok) break;
           tc_fence_after_sync();
           if (el) {
@@ -373,7 +373,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     float* acc_col = p.dq_acc + static_cast<int64_t>(bh) * p.N * D + wq * 32 + lane;
     bool ok = true;
     for (int n = 0; n < cnt; ++n) {
-      ok = mbar_wait(dq_full, n & 1, abort_flag, p.status, kSiteDQFull);
+      ok = mbar_wait_warp(dq_full, n & 1, abort_flag, p.status, kSiteDQFull);
       if (!ok) break;
       tc_fence_after_sync();
       const int q0 = (first + n) * kQStep;
@@ -408,7 +408,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     // c |k_r|^2 of this thread's key row, from the resident K tile; rows past N (zero-filled by the load) get
     // +infinity, i.e. weight exp2(-inf) = 0
     float neg_ksq = -INFINITY;
-    bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, kSiteKV);
+    bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status, kSiteKV);
     if (ok && k_row0 + r < p.N) {
       float acc = 0.f;
 #pragma unroll 1
@@ -426,7 +426,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     }
 
     for (int n = 0; n < cnt && ok; ++n) {
-      ok = mbar_wait(s_full, n & 1, abort_flag, p.status, kSiteSFull);
+      ok = mbar_wait_warp(s_full, n & 1, abort_flag, p.status, kSiteSFull);
       if (!ok) break;
       tc_fence_after_sync();
       float pr[16];
@@ -457,7 +457,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 #pragma unroll
         for (int i = 0; i < 8; ++i) packed[i] = pack2<kBf16>(pr[2 * i], pr[2 * i + 1]);
         if (n > 0) {   // the P^T columns are free once dV of the previous step has completed
-          ok = mbar_wait(dv_done, (n - 1) & 1, abort_flag, p.status, kSiteDVDone);
+          ok = mbar_wait_warp(dv_done, (n - 1) & 1, abort_flag, p.status, kSiteDVDone);
           if (!ok) break;
           tc_fence_after_sync();
         }
@@ -467,7 +467,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         mbar_arrive_warp(p_full);
       }
 
-      ok = mbar_wait(dp_full, n & 1, abort_flag, p.status, kSiteDPFull);
+      ok = mbar_wait_warp(dp_full, n & 1, abort_flag, p.status, kSiteDPFull);
       if (!ok) break;
       tc_fence_after_sync();
       uint32_t ds_packed[8];
@@ -489,7 +489,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         ds_rowsum += rs0 + rs1;
       }
       if (n >= kDsStages) {   // the dS^T buffer is free once dK and dQ^T of its previous step have completed
-        ok = mbar_wait(&ds_free[n % kDsStages], ((n / kDsStages) - 1) & 1, abort_flag, p.status, kSiteDsFree);
+        ok = mbar_wait_warp(&ds_free[n % kDsStages], ((n / kDsStages) - 1) & 1, abort_flag, p.status, kSiteDsFree);
         if (!ok) break;
       }
       // row r of the [key][query] tile: 16-byte chunks 2g and 2g + 1
@@ -500,7 +500,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       fence_proxy_async_smem();
       // second copy for dK = dS^T Q, which takes its A operand from TMEM; free once dK of the previous step is done
       if (n > 0) {
-        ok = mbar_wait(dk_done, (n - 1) & 1, abort_flag, p.status, kSiteDsFree);
+        ok = mbar_wait_warp(dk_done, (n - 1) & 1, abort_flag, p.status, kSiteDsFree);
         if (!ok) break;
         tc_fence_after_sync();
       }
@@ -513,11 +513,11 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     uint32_t grp_phase = 0;
     auto group_sync = [&]() -> bool {
       mbar_arrive_warp(grp_sync);
-      const bool done = mbar_wait(grp_sync, grp_phase & 1, abort_flag, p.status, kSiteGroup);
+      const bool done = mbar_wait_warp(grp_sync, grp_phase & 1, abort_flag, p.status, kSiteGroup);
       ++grp_phase;
       return done;
     };
-    if (ok) ok = mbar_wait(acc_done, 0, abort_flag, p.status, kSiteAccDone);
+    if (ok) ok = mbar_wait_warp(acc_done, 0, abort_flag, p.status, kSiteAccDone);
     if (ok) {
       tc_fence_after_sync();
       s_rowsum[g * kTile + r] = ds_rowsum;      // every group holds a quarter of rowsum(dS^T)

@@ -235,7 +235,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       return false;
     }
     const int slot = n % kItemSlots;
-    if (!mbar_wait(&item_full[slot], (n / kItemSlots) & 1, abort_flag, status, kSiteItemFull, s_unit)) {
+    if (!mbar_wait_warp(&item_full[slot], (n / kItemSlots) & 1, abort_flag, status, kSiteItemFull, s_unit)) {
       ok_ref = false;
       return false;
     }
@@ -441,10 +441,10 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
       };
       auto wait_k = [&](uint32_t g) {
-        return mbar_wait(&k_full[g % kStages], (g / kStages) & 1, abort_flag, status, kSiteKFull, s_unit);
+        return mbar_wait_warp(&k_full[g % kStages], (g / kStages) & 1, abort_flag, status, kSiteKFull, s_unit);
       };
       auto wait_v = [&](uint32_t g) {
-        return mbar_wait(&v_full[g % kStages], (g / kStages) & 1, abort_flag, status, kSiteVFull, s_unit);
+        return mbar_wait_warp(&v_full[g % kStages], (g / kStages) & 1, abort_flag, status, kSiteVFull, s_unit);
       };
       uint32_t G = 0, ct = 0, qn = 0;
       bool ok = true;
@@ -458,8 +458,8 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (my_nkt > 0) {
           // first scores of the item: Q_t has landed, the first key tile has landed, and the group holds the last
           // scores of the previous item in registers (it is then busy with their exponentials and its output)
-          ok = mbar_wait(&q_full[t], qn & 1, abort_flag, status, kSiteQFull, s_unit) && wait_k(G);
-          if (ok && ct > 0) ok = mbar_wait(&s_consumed[t], (ct - 1) & 1, abort_flag, status, kSiteSConsumed, s_unit);
+          ok = mbar_wait_warp(&q_full[t], qn & 1, abort_flag, status, kSiteQFull, s_unit) && wait_k(G);
+          if (ok && ct > 0) ok = mbar_wait_warp(&s_consumed[t], (ct - 1) & 1, abort_flag, status, kSiteSConsumed, s_unit);
           if (!ok) break;
           tc_fence_after_sync();
           issue_s(G % kStages);
@@ -478,7 +478,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           if (j < my_nkt) {
             if (j + 1 < my_nkt) {
               // next scores first: they only need S_t(j) to have been read
-              ok = wait_k(g + 1) && mbar_wait(&s_consumed[t], (ct + j) & 1, abort_flag, status, kSiteSConsumed, s_unit);
+              ok = wait_k(g + 1) && mbar_wait_warp(&s_consumed[t], (ct + j) & 1, abort_flag, status, kSiteSConsumed, s_unit);
               if (!ok) break;
               tc_fence_after_sync();
               issue_s(st_next);
@@ -486,7 +486,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
               used_k_next = true;
             }
             ok = wait_v(g);
-            ok = ok && mbar_wait(&p_full[t], (ct + j) & 1, abort_flag, status, kSitePFull, s_unit);
+            ok = ok && mbar_wait_warp(&p_full[t], (ct + j) & 1, abort_flag, status, kSitePFull, s_unit);
             if (!ok) break;
             tc_fence_after_sync();
             issue_o(st, j > 0 ? 1u : 0u);
@@ -552,7 +552,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       float ub = INFINITY;
       bool safe = false;                             // warp-wide: no row of this warp can overflow any more
       if (kSkipMax) {
-        ok = mbar_wait(&q_full[t], qn & 1, abort_flag, status, kSiteQFull, s_unit);
+        ok = mbar_wait_warp(&q_full[t], qn & 1, abort_flag, status, kSiteQFull, s_unit);
         if (!ok) break;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};         // independent sums: the chain is on every item's critical path
 #pragma unroll
@@ -571,7 +571,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       }
       if (kPersistent) mbar_arrive_warp(&q_free[t]);   // this warp will not read Q_t of this item (again)
       for (int j = 0; j < my_nkt; ++j) {
-        ok = ok && mbar_wait(&s_full[t], (ct + j) & 1, abort_flag, status, kSiteSFull, s_unit);
+        ok = ok && mbar_wait_warp(&s_full[t], (ct + j) & 1, abort_flag, status, kSiteSFull, s_unit);
         if (!ok) break;
         tc_fence_after_sync();
 
@@ -621,7 +621,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (j > 0 && __any_sync(0xffffffffu, need)) {
               // O_t holds the sum over key tiles < j; wait until the last P V has landed, then rescale this thread's
               // share of the row.
-              ok = mbar_wait(&o_done[t], (ct + j - 1) & 1, abort_flag, status, kSiteODone, s_unit);
+              ok = mbar_wait_warp(&o_done[t], (ct + j - 1) & 1, abort_flag, status, kSiteODone, s_unit);
               if (!ok) break;
               tc_fence_after_sync();
 #pragma unroll
@@ -663,7 +663,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             packed[i + 1] = pack2<kBf16>(p2, p3);
           }
           if (!waited_o) {
-            ok = mbar_wait(&o_done[t], (ct + j - 1) & 1, abort_flag, status, kSitePFree, s_unit);
+            ok = mbar_wait_warp(&o_done[t], (ct + j - 1) & 1, abort_flag, status, kSitePFree, s_unit);
             if (!ok) break;
             tc_fence_after_sync();
             waited_o = true;
@@ -689,8 +689,8 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       }
       if (!ok) break;
 
-      ok = mbar_wait(&o_done[t], (ct + my_nkt - 1) & 1, abort_flag, status, kSiteODoneFinal, s_unit);
-      if (ok && kPersistent && qn > 0) ok = mbar_wait(&stage_free[t], (qn - 1) & 1, abort_flag, status, kSiteStageFree, s_unit);
+      ok = mbar_wait_warp(&o_done[t], (ct + my_nkt - 1) & 1, abort_flag, status, kSiteODoneFinal, s_unit);
+      if (ok && kPersistent && qn > 0) ok = mbar_wait_warp(&stage_free[t], (qn - 1) & 1, abort_flag, status, kSiteStageFree, s_unit);
       if (!ok) break;
       tc_fence_after_sync();
       const float inv = kSoftmax ? (1.0f / l_sum) : 1.0f;
@@ -714,7 +714,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       tc_fence_before_sync();                        // the output has been read: the next item may accumulate into O_t
       fence_proxy_async_smem();
       mbar_arrive_warp(&grp_sync[t]);
-      ok = mbar_wait(&grp_sync[t], qn & 1, abort_flag, status, kSiteGroup, s_unit);
+      ok = mbar_wait_warp(&grp_sync[t], qn & 1, abort_flag, status, kSiteGroup, s_unit);
       if (!ok) break;
       if (storer) {
         for (int x = 0; x < kBoxes; ++x) tma_store_4d(&tm_o, stage + x * kBoxBytes, x * 64, r0, it.h, it.b);

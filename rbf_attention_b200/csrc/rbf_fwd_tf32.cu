@@ -241,7 +241,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (!kSoftmax && nkt > 0) row_bias = qsq[static_cast<int64_t>(bh) * n_pad + row];
     bool ok = true;
     for (int j = 0; j < nkt; ++j) {
-      ok = mbar_wait(s_full, j & 1, abort_flag, status, kSiteSFull);
+      ok = mbar_wait_warp(s_full, j & 1, abort_flag, status, kSiteSFull);
       if (!ok) break;
       tc_fence_after_sync();
       uint32_t raw[kKeys];
@@ -268,7 +268,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           l_sum *= alpha;
         }
         if (j > 0 && __any_sync(0xffffffffu, need)) {
-          ok = mbar_wait(o_done, (j - 1) & 1, abort_flag, status, kSiteODone);
+          ok = mbar_wait_warp(o_done, (j - 1) & 1, abort_flag, status, kSiteODone);
           if (!ok) break;
           tc_fence_after_sync();
 #pragma unroll
@@ -295,7 +295,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       l_sum += ps;
       // P's columns are free once O += P V of the previous tile has completed
       if (j > 0) {
-        ok = mbar_wait(o_done, (j - 1) & 1, abort_flag, status, kSiteODone);
+        ok = mbar_wait_warp(o_done, (j - 1) & 1, abort_flag, status, kSiteODone);
         if (!ok) break;
         tc_fence_after_sync();
       }
@@ -305,7 +305,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // 128-byte swizzle; thread = (key, half of the d chunks); the previous tile's MMAs have released V^T (o_done)
       {
         const int st = j % kStages;
-        ok = mbar_wait(&v_full[st], (j / kStages) & 1, abort_flag, status, kSiteVFull);
+        ok = mbar_wait_warp(&v_full[st], (j / kStages) & 1, abort_flag, status, kSiteVFull);
         if (!ok) break;
         const int key = tid & 63, half = tid >> 6;
         const uint8_t* src = s_v + st * kKvBytes;
@@ -327,7 +327,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       tc_fence_before_sync();
       mbar_arrive_warp(p_full);
     }
-    if (ok && nkt > 0) ok = mbar_wait(o_done, (nkt - 1) & 1, abort_flag, status, kSiteODone);
+    if (ok && nkt > 0) ok = mbar_wait_warp(o_done, (nkt - 1) & 1, abort_flag, status, kSiteODone);
     if (ok && nkt > 0) {
       tc_fence_after_sync();
       const float inv = kSoftmax ? (1.0f / l_sum) : 1.0f;
@@ -345,7 +345,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       fence_proxy_async_smem();
       mbar_arrive_warp(grp_sync);
-      ok = mbar_wait(grp_sync, 0, abort_flag, status, kSiteGroup);
+      ok = mbar_wait_warp(grp_sync, 0, abort_flag, status, kSiteGroup);
       if (ok && r == 0) {
         for (int x = 0; x < 2; ++x) tma_store_4d(&tm_o, stage + x * kBoxBytes, x * 32, r0, h, b);
         tma_store_commit();

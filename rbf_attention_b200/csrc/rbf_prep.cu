@@ -526,9 +526,16 @@ __global__ void __launch_bounds__(32) wait_selftest_kernel(DeviceStatus* status,
     abort_flag = 0;
   }
   __syncwarp();
-  // nothing ever arrives on `bar`: the first lane whose limit runs out records the status and raises the flag, the
-  // other lanes leave on the flag, and the block returns
-  mbar_wait_limit(&bar, 0, &abort_flag, status, kSiteSelfTest, limit);
+  // Nothing ever arrives on `bar`. The warp's wait, with a limit of its own for every lane: all lanes leave it together,
+  // with the same answer and the status recorded (a unit of 0xffffff says that they did not agree).
+  const bool ran_out = !mbar_wait_warp_limit(&bar, 0, &abort_flag, status, kSiteSelfTest, limit + 64 * threadIdx.x);
+  const bool agree = __all_sync(0xffffffffu, ran_out);
+  // One thread's wait: it raises the flag again.
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    const bool second = !mbar_wait_limit(&bar, 0, &abort_flag, status, kSiteSelfTest, limit);
+    if (!agree || !second || abort_flag == 0) status->code = (kSiteSelfTest << 24) | 0xffffffu;
+  }
   __syncwarp();
   if (threadIdx.x == 0) mbar_inval(&bar);
 }

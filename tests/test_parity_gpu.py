@@ -290,6 +290,11 @@ def test_bounded_wait_runs_out_and_the_workspace_recovers():
     rc = lib.rbf_b200_read_device_status(ws.data_ptr(), stream, ctypes.byref(code))     # synchronises: the kernel is back
     assert rc == 6 and code.value >> 24 == 250 and code.value & 0xFFFFFF == 0
     assert b"wait ran out" in lib.rbf_b200_last_error()
+    # whatever the limit, the lanes of a warp leave together (a unit of 0xffffff would say that they did not)
+    for limit in (1, 300, 20_000, 1_000_000):
+        ws[:4] = 0
+        assert lib.rbf_b200_selftest_wait_timeout(ws.data_ptr(), nbytes, limit, stream) == 0, lib.rbf_b200_last_error()
+        assert lib.rbf_b200_read_device_status(ws.data_ptr(), stream, ctypes.byref(code)) == 6 and code.value == 250 << 24
     # the asynchronous form: a kernel stores the word into mapped pinned host memory; pageable memory is refused
     slot = torch.zeros(1, dtype=torch.int32).pin_memory()
     assert lib.rbf_b200_post_device_status(ws.data_ptr(), slot.data_ptr(), stream) == 0, lib.rbf_b200_last_error()
