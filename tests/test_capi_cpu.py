@@ -127,3 +127,53 @@ def test_gelu_entries_validate_before_any_launch(built_library):
     assert lib.rbf_b200_gelu_fwd(p, p, 0, 0, None) == 0
     assert lib.rbf_b200_gelu_bwd(p, p, p, None, None, 0, 8, 20, 0, None) == 1
     assert lib.rbf_b200_gelu_bwd(None, p, p, None, None, 0, 8, 16, 0, None) == 1
+
+
+def _call_posting(lib, backward, *, p=0x10000, head_dim=64, N=256, dtype=0, row=64, ws_bytes=1 << 24, lse=0x10000):
+    s = (ctypes.c_int64 * 3)(N * row, N * row, row)
+    tail = (lse,) + (p,) * (4 if backward else 0) + (0x10000, ws_bytes, 1, 1, N, head_dim) + (s,) * (8 if backward else 4)
+    fn = lib.rbf_b200_bwd_posting if backward else lib.rbf_b200_fwd_posting
+    return fn(p, p, p, p, *tail, dtype, 1, 1, 0.125, None, 7, None)
+
+
+@pytest.mark.parametrize("backward", [False, True])
+def test_posting_entries_validate_before_any_launch(backward, built_library):
+    lib = _lib.load()
+    for head_dim in (-8, 0, 12, 63, 136, 256):
+        assert _call_posting(lib, backward, head_dim=head_dim, row=256) == 1 and b"head dim" in lib.rbf_b200_last_error()
+    assert _call_posting(lib, backward, head_dim=40, dtype=3) == 1
+    assert _call_posting(lib, backward, head_dim=40, N=0) == 1
+    assert _call_posting(lib, backward, head_dim=40, p=0) == 1 and b"NULL" in lib.rbf_b200_last_error()
+    assert _call_posting(lib, backward, head_dim=40, p=0x10008) == 2 and b"16-byte" in lib.rbf_b200_last_error()
+    assert _call_posting(lib, backward, head_dim=40, row=44) == 2                # rows not a multiple of 16 bytes
+    assert _call_posting(lib, backward, head_dim=72, row=64) == 2                # rows overlap
+    assert _call_posting(lib, backward, head_dim=40, lse=0) == 1
+    # the workspace is that of the head dim that the kernels run at
+    for head_dim, columns in ((40, 64), (72, 128)):
+        need = lib.rbf_b200_workspace_bytes(1, 1, 256, columns, 1, int(backward))
+        assert _call_posting(lib, backward, head_dim=head_dim, row=columns, ws_bytes=need - 1) == 3
+        assert str(need).encode() in lib.rbf_b200_last_error()
+
+
+def test_conversion_entries_validate_before_any_launch(built_library):
+    lib = _lib.load()
+
+    def narrow(count=2, src=0x10000, dst=0x10000, strides=(64, 64, 64), B=2, H=2, N=2, D=64, checked=1, flag=0x10000):
+        pointers = lambda p: (ctypes.c_void_p * 6)(*[p] * 6)
+        return lib.rbf_b200_narrow_f32(count, pointers(src), pointers(dst), (ctypes.c_int64 * 18)(*strides * 6), B, H, N, D,
+                                       checked, flag, None)
+
+    assert narrow(count=0) == 1 and narrow(count=6) == 1 and narrow(checked=3) == 1 and narrow(checked=-1) == 1
+    assert narrow(B=0) == 1 and narrow(N=-1) == 1 and narrow(D=12) == 1 and narrow(D=0) == 1
+    assert narrow(src=0) == 1 and narrow(dst=0) == 1 and narrow(flag=None) == 1
+    assert narrow(src=0x10004) == 2 and narrow(dst=0x10008) == 2
+    assert narrow(strides=(64, 64, 66)) == 2 and b"multiple of 4" in lib.rbf_b200_last_error()
+    assert narrow(B=65536, H=65536, N=65536) == 1 and b"too large" in lib.rbf_b200_last_error()
+
+    def widen(count=2, src=0x10000, dst=0x10000, n=64):
+        pointers = lambda p: (ctypes.c_void_p * 6)(*[p] * 6)
+        return lib.rbf_b200_widen_f16(count, pointers(src), pointers(dst), n, None)
+
+    assert widen(count=0) == 1 and widen(count=6) == 1 and widen(n=-8) == 1 and widen(n=12) == 1
+    assert widen(src=0) == 1 and widen(dst=0) == 1 and widen(src=0x10002) == 2 and widen(dst=0x10004) == 2
+    assert widen(n=1 << 45) == 1 and widen(n=0) == 0

@@ -858,9 +858,8 @@ def test_calls_post_their_status_word(D, N, softmax, deterministic):
                                                                 (False, False, torch.float16, False),
                                                                 (True, False, torch.float16, True)])
 def test_head_dims_that_are_multiples_of_eight_run_in_place(D, softmax, causal, dtype, deterministic):
-    """No copy of the tensors: views into one (B, N, 3, H, D) buffer, ragged N, whose neighbours hold NaN - a column or row
-    read past the tensors' own would show -, and gradients whose neighbours are checked to stay untouched by the head
-    dims' padding (the stores are clipped)."""
+    """No copy of the tensors: views into one (B, N, 4, H, D) buffer, ragged N, whose neighbours hold NaN - a column or row
+    read past the tensors' own would show."""
     B, H, N = 2, 3, 150
     q, k, v, do = oracle.make_inputs(B, H, N, D, seed=D, dtype=dtype, std=1.0 if softmax else 0.5)
     ref = oracle.torch_forward_backward(q, k, v, do, causal, softmax, dtype=torch.float32)
@@ -868,6 +867,7 @@ def test_head_dims_that_are_multiples_of_eight_run_in_place(D, softmax, causal, 
     for i, t in enumerate((q, k, v)):
         buf[:, :N, i] = t.to(DEV).permute(0, 2, 1, 3)
     qd, kd, vd = (buf[:, :N, i].permute(0, 2, 1, 3) for i in range(3))
+    assert all(ops._tma_ready(t) is t for t in (qd, kd, vd))
     out, lse = ops._forward(qd, kd, vd, causal, softmax)
     torch.use_deterministic_algorithms(deterministic)
     try:
@@ -878,6 +878,52 @@ def test_head_dims_that_are_multiples_of_eight_run_in_place(D, softmax, causal, 
     for name, got, want in zip(("O", "dQ", "dK", "dV"), (out, *grads), ref):
         assert got.shape == want.shape
         check(name, got.cpu().float(), want, REL_L2[dtype])
+
+
+@pytest.mark.parametrize("D", [8, 40, 72, 120])
+@pytest.mark.parametrize("softmax,deterministic", [(True, False), (True, True), (False, False), (False, True)])
+def test_posting_entries_leave_a_views_neighbours_alone(D, softmax, deterministic):
+    """Outputs and gradients as views with 16 columns, a row and the other heads beside them: the stores end at the head dim
+    (single-kernel and two-kernel backward, with and without the softmax denominator), ragged N."""
+    lib = _lib.load()
+    B, H, N, dtype, guard = 2, 3, 150, torch.bfloat16, 3.0e38
+    q, k, v, do = oracle.make_inputs(B, H, N, D, seed=D, dtype=dtype, std=1.0 if softmax else 0.5)
+    ref = oracle.torch_forward_backward(q, k, v, do, True, softmax, dtype=torch.float32)
+
+    def view():
+        buf = torch.full((B, N + 1, H, D + 16), guard, dtype=dtype, device=DEV)
+        return buf, buf[:, :N, :, 8:8 + D].permute(0, 2, 1, 3)
+
+    bufs, (qd, kd, vd, dod, out, dq, dk, dv) = zip(*(view() for _ in range(8)))
+    for t, src in zip((qd, kd, vd, dod), (q, k, v, do)):
+        t.copy_(src.to(DEV))
+    columns = 64 if D <= 64 else 128
+    stream = torch.cuda.current_stream().cuda_stream
+    lse = torch.empty((B, H, N), dtype=torch.float32, device=DEV)
+    ws = [torch.empty(lib.rbf_b200_workspace_bytes(B, H, N, columns, int(softmax), i), dtype=torch.uint8, device=DEV)
+          for i in range(2)]
+    rc = lib.rbf_b200_fwd_posting(qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), out.data_ptr(), lse.data_ptr(),
+                                  ws[0].data_ptr(), ws[0].numel(), B, H, N, D, _s3(qd), _s3(kd), _s3(vd), _s3(out), 0, 1,
+                                  int(softmax), 1.0 / math.sqrt(D), stream, 7, None)
+    assert rc == 0, lib.rbf_b200_last_error()
+    lib.rbf_b200_set_deterministic(int(deterministic))
+    try:
+        rc = lib.rbf_b200_bwd_posting(qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), out.data_ptr(), lse.data_ptr(),
+                                      dod.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws[1].data_ptr(),
+                                      ws[1].numel(), B, H, N, D, _s3(qd), _s3(kd), _s3(vd), _s3(out), _s3(dod), _s3(dq),
+                                      _s3(dk), _s3(dv), 0, 1, int(softmax), 1.0 / math.sqrt(D), stream, 7, None)
+    finally:
+        lib.rbf_b200_set_deterministic(0)
+    assert rc == 0, lib.rbf_b200_last_error()
+    code = ctypes.c_uint(0)
+    for w in ws:
+        assert lib.rbf_b200_read_device_status(w.data_ptr(), stream, ctypes.byref(code)) == 0, lib.rbf_b200_last_error()
+    for name, got, want in zip(("O", "dQ", "dK", "dV"), (out, dq, dk, dv), ref):
+        check(name, got.cpu().float(), want, REL_L2[dtype])
+    for buf in bufs:
+        outside = torch.ones(buf.shape, dtype=torch.bool, device=DEV)
+        outside[:, :N, :, 8:8 + D] = False
+        assert (buf[outside] == torch.tensor(guard, dtype=dtype)).all()
 
 
 @pytest.mark.parametrize("D,view", [(64, "dense"), (72, "dense"), (64, "bnhd"), (64, "odd"), (36, "dense"), (64, "mixed")])
