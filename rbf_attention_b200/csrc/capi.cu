@@ -684,7 +684,7 @@ int rbf_b200_layer_norm_fwd(const void* x, const void* gamma, const void* beta, 
 size_t rbf_b200_layer_norm_bwd_workspace_bytes(int64_t rows, int cols) {
   const int sms = sm_count();
   if (sms <= 0 || rows < 0 || !rbf::layer_norm_supported(cols)) return 0;
-  return static_cast<size_t>(rbf::layer_norm_bwd_blocks(rows, sms)) * 2 * cols * sizeof(float);
+  return static_cast<size_t>(rbf::layer_norm_bwd_blocks(rows, cols, sms)) * 2 * cols * sizeof(float);
 }
 
 int rbf_b200_layer_norm_bwd_add(const void* x, const void* dy, const void* dres, const void* gamma, const float* mean,

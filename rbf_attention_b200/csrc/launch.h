@@ -126,7 +126,7 @@ struct LayerNormBwdArgs {
   const void* dres;          // optional (rows, cols): added to dx before it is rounded (may be dx itself)
 };
 bool layer_norm_supported(int cols);
-int layer_norm_bwd_blocks(int64_t rows, int sms);
+int layer_norm_bwd_blocks(int64_t rows, int cols, int sms);
 cudaError_t launch_layer_norm_fwd(const LayerNormArgs& a, int cols, bool bf16, int sms, cudaStream_t stream);
 cudaError_t launch_layer_norm_bwd(const LayerNormBwdArgs& a, int cols, bool bf16, int sms, cudaStream_t stream);
 

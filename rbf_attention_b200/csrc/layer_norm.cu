@@ -69,8 +69,18 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Blocks per SM that the prefetched row leaves registers for.
-constexpr int ln_fwd_blocks(int vecs) { return vecs <= 2 ? 3 : (vecs == 3 ? 2 : 1); }
+// Blocks per SM that the prefetched row leaves registers for, by width (256 columns each). Both grids are as large as what
+// is resident: a second wave of blocks would start with nothing prefetched. Microseconds on the device for 65792 rows (bf16),
+// without the prefetch -> now:
+//   columns              256            512            768            1024
+//   forward         11.5 -> 10.9   38.5 -> 25.8   67.8 -> 37.4   88.4 -> 56.0
+//   with residual   24.7 -> 22.7   69.1 -> 47.2  124.1 -> 69.1  163.4 -> 86.5
+//   backward        35.0 -> 27.2   51.7 -> 47.3   90.6 -> 71.5  101.7 -> 79.2
+//   with skip       51.4 -> 34.5   77.8 -> 54.0  167.5 -> 80.3  205.1 -> 90.6
+// and for 3124 rows forward 2.4 -> 2.3, 2.9 -> 3.0, 4.3 -> 3.4, 5.2 -> 4.2, backward 9.8 -> 10.0, 12.1 -> 10.5,
+// 14.2 -> 10.4, 15.2 -> 11.0.
+// (Four backward blocks per SM whatever their residency: 33.8, 51.8, 80.4, 89.2 and 42.0, 58.7, 89.2, 100.5.)
+constexpr int ln_fwd_blocks(int vecs) { return vecs == 1 ? 4 : vecs == 2 ? 3 : (vecs == 3 ? 2 : 1); }
 constexpr int ln_bwd_blocks(int vecs) { return vecs == 1 ? 3 : (vecs == 2 ? 2 : 1); }
 
 template <bool kBf16, int kVecs>
@@ -83,8 +93,8 @@ __global__ void __launch_bounds__(kLnThreads, ln_fwd_blocks(kVecs)) layer_norm_f
     ln_load8<kBf16>(a.gamma, v * 32 + lane, gamma[v]);
     ln_load8<kBf16>(a.beta, v * 32 + lane, beta[v]);
   }
-  // The next row's loads are under way while a row is reduced and written: 65792 x 512 bf16 47 -> 37 us, with the residual
-  // addition 78 -> 56 us (270 MB: 4.8 TB/s), against eight blocks per SM that load a row when they get to it.
+  // The next row's loads are under way while a row is reduced and written: 65792 x 512 bf16 38.5 -> 25.8 us, with the
+  // residual addition 69 -> 47 us (270 MB: 5.7 TB/s), against warps that load a row when they get to it.
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kLnWarps;
   int64_t row = static_cast<int64_t>(blockIdx.x) * kLnWarps + warp;
   uint4 x_next[kVecs], r_next[kVecs];
@@ -166,7 +176,7 @@ __global__ void __launch_bounds__(kLnThreads, ln_bwd_blocks(kVecs)) layer_norm_b
 #pragma unroll
     for (int j = 0; j < 8; ++j) dg[v][j] = db[v][j] = 0.f;
   }
-  // as in the forward; 65792 x 512 bf16 with the skip gradient 95 -> 76 us for both kernels of the backward
+  // as in the forward; 65792 x 512 bf16 with the skip gradient 78 -> 54 us for both kernels of the backward
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kLnWarps;
   int64_t row = static_cast<int64_t>(blockIdx.x) * kLnWarps + warp;
   uint4 x_next[kVecs], dy_next[kVecs], skip_next[kVecs];
@@ -287,9 +297,9 @@ cudaError_t launch_bwd_t(const LayerNormBwdArgs& a, int grid, cudaStream_t strea
 
 bool layer_norm_supported(int cols) { return cols > 0 && cols % 256 == 0 && cols <= 1024; }
 
-int layer_norm_bwd_blocks(int64_t rows, int sms) {
+int layer_norm_bwd_blocks(int64_t rows, int cols, int sms) {
   const int64_t want = (rows + kLnWarps - 1) / kLnWarps;
-  const int64_t cap = static_cast<int64_t>(sms) * 4;
+  const int64_t cap = static_cast<int64_t>(sms) * ln_bwd_blocks(cols / 256);
   return static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
 }
 
@@ -308,7 +318,7 @@ cudaError_t launch_layer_norm_fwd(const LayerNormArgs& a, int cols, bool bf16, i
 }
 
 cudaError_t launch_layer_norm_bwd(const LayerNormBwdArgs& a, int cols, bool bf16, int sms, cudaStream_t stream) {
-  const int grid = layer_norm_bwd_blocks(a.rows, sms);
+  const int grid = layer_norm_bwd_blocks(a.rows, cols, sms);
   RBF_LN_DISPATCH(launch_bwd_t, a, grid, stream)
 }
 

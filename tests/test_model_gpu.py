@@ -179,7 +179,7 @@ def test_in_place_scaling_of_a_gradient_on_any_alignment(dtype, offset, n):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("rows,cols", [(4113, 512), (77, 256), (1, 1024), (300, 768)])
+@pytest.mark.parametrize("rows,cols", [(4113, 512), (77, 256), (1, 1024), (300, 768), (3700, 256), (2500, 768), (1300, 1024)])
 def test_layer_norm_kernels_match_torch(dtype, rows, cols):
     """``ops.layer_norm`` and its backward against ``F.layer_norm`` in fp64 on the same 16-bit values (rows not a
     multiple of the 8 rows a block walks at a time, a non-zero mean, a non-trivial affine part). Tolerances: y and dx
