@@ -363,89 +363,89 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     // N1028 (453 -> 488 us): three issuers wait in turn on the way from one step to the next.
     bool ok = run;
     while (__all_sync(0xffffffffu, ok) && next_item()) {
-    if (warp == kMmaWarpA) {
-      const SmemDesc k_kmaj = stage_of(make_sdesc_parts(smem_u32(s_k), 16, 1024), I & 1, kTileBytes);
-      const SmemDesc q_kmaj0 = make_sdesc_parts(smem_u32(s_q), 16, 1024);
-      const SmemDesc lslab0 = make_sdesc_slab32(smem_u32(s_lslab));
-      ok = mbar_wait(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item);
-      for (int n = 0; n < cnt && ok; ++n) {
-        const uint32_t g = T + n, st = g % kQStages;
-        ok = mbar_wait(&q_full[st], (g / kQStages) & 1, abort_flag, p.status, kSiteQFull, s_item);
-        // S^T(n) may overwrite S^T(n-1) once every compute warp has stored P^T(n-1)
-        if (ok && g > 0) ok = mbar_wait(p_full, (g - 1) & 1, abort_flag, p.status, kSitePFull, s_item);
-        if (!ok) break;
-        tc_fence_after_sync();
-        if (el) {
-          issue_scores(tmem + kColS, k_kmaj, stage_of(q_kmaj0, st, kTileBytes), stage_of(lslab0, st, kSlabBytes));
-          umma_commit(s_full);
+      if (warp == kMmaWarpA) {
+        const SmemDesc k_kmaj = stage_of(make_sdesc_parts(smem_u32(s_k), 16, 1024), I & 1, kTileBytes);
+        const SmemDesc q_kmaj0 = make_sdesc_parts(smem_u32(s_q), 16, 1024);
+        const SmemDesc lslab0 = make_sdesc_slab32(smem_u32(s_lslab));
+        ok = mbar_wait(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item);
+        for (int n = 0; n < cnt && ok; ++n) {
+          const uint32_t g = T + n, st = g % kQStages;
+          ok = mbar_wait(&q_full[st], (g / kQStages) & 1, abort_flag, p.status, kSiteQFull, s_item);
+          // S^T(n) may overwrite S^T(n-1) once every compute warp has stored P^T(n-1)
+          if (ok && g > 0) ok = mbar_wait(p_full, (g - 1) & 1, abort_flag, p.status, kSitePFull, s_item);
+          if (!ok) break;
+          tc_fence_after_sync();
+          if (el) {
+            issue_scores(tmem + kColS, k_kmaj, stage_of(q_kmaj0, st, kTileBytes), stage_of(lslab0, st, kSlabBytes));
+            umma_commit(s_full);
+          }
         }
-      }
-    } else if (warp == kMmaWarpB) {
-      const SmemDesc v_kmaj = make_sdesc_parts(smem_u32(s_v), 16, 1024);
-      const SmemDesc do_kmaj0 = make_sdesc_parts(smem_u32(s_do), 16, 1024);
-      const SmemDesc do_nmaj0 = make_sdesc_parts(smem_u32(s_do), kTile * 128, 1024);
-      const SmemDesc dslab0 = make_sdesc_slab32(smem_u32(s_dslab));
-      ok = mbar_wait(v_full, I & 1, abort_flag, p.status, kSiteVFull, s_item);
-      for (int n = 0; n < cnt && ok; ++n) {
-        const uint32_t g = T + n, st = g % kDoStages;
-        ok = mbar_wait(&do_full[st], (g / kDoStages) & 1, abort_flag, p.status, kSiteDoFull, s_item);
-        // dP^T(n) may overwrite dP^T(n-1) once every compute warp has stored dS^T(n-1)
-        if (ok && g > 0) ok = mbar_wait(ds_full, (g - 1) & 1, abort_flag, p.status, kSiteDSFull, s_item);
-        if (!ok) break;
-        tc_fence_after_sync();
-        if (el) {
-          issue_scores(tmem + kColDP, v_kmaj, stage_of(do_kmaj0, st, kTileBytes), stage_of(dslab0, st, kSlabBytes));
-          umma_commit(dp_full);
-          if (n == cnt - 1) umma_commit(v_free);
-        }
-        // dV += P^T dO, from zero once the previous item's dV has left
-        ok = mbar_wait(p_full, g & 1, abort_flag, p.status, kSitePFull, s_item);
-        if (ok && n == 0 && I > 0) ok = mbar_wait(dv_free, (I - 1) & 1, abort_flag, p.status, kSiteDVFree, s_item);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const SmemDesc do_n = stage_of(do_nmaj0, st, kTileBytes);
-        if (el) {
+      } else if (warp == kMmaWarpB) {
+        const SmemDesc v_kmaj = make_sdesc_parts(smem_u32(s_v), 16, 1024);
+        const SmemDesc do_kmaj0 = make_sdesc_parts(smem_u32(s_do), 16, 1024);
+        const SmemDesc do_nmaj0 = make_sdesc_parts(smem_u32(s_do), kTile * 128, 1024);
+        const SmemDesc dslab0 = make_sdesc_slab32(smem_u32(s_dslab));
+        ok = mbar_wait(v_full, I & 1, abort_flag, p.status, kSiteVFull, s_item);
+        for (int n = 0; n < cnt && ok; ++n) {
+          const uint32_t g = T + n, st = g % kDoStages;
+          ok = mbar_wait(&do_full[st], (g / kDoStages) & 1, abort_flag, p.status, kSiteDoFull, s_item);
+          // dP^T(n) may overwrite dP^T(n-1) once every compute warp has stored dS^T(n-1)
+          if (ok && g > 0) ok = mbar_wait(ds_full, (g - 1) & 1, abort_flag, p.status, kSiteDSFull, s_item);
+          if (!ok) break;
+          tc_fence_after_sync();
+          if (el) {
+            issue_scores(tmem + kColDP, v_kmaj, stage_of(do_kmaj0, st, kTileBytes), stage_of(dslab0, st, kSlabBytes));
+            umma_commit(dp_full);
+            if (n == cnt - 1) umma_commit(v_free);
+          }
+          // dV += P^T dO, from zero once the previous item's dV has left
+          ok = mbar_wait(p_full, g & 1, abort_flag, p.status, kSitePFull, s_item);
+          if (ok && n == 0 && I > 0) ok = mbar_wait(dv_free, (I - 1) & 1, abort_flag, p.status, kSiteDVFree, s_item);
+          if (!ok) break;
+          tc_fence_after_sync();
+          const SmemDesc do_n = stage_of(do_nmaj0, st, kTileBytes);
+          if (el) {
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk)
-            umma_ts(tmem + kColDV, tmem + kColPT + kk * 8, sdesc_at(do_n, kk * 2048), idesc_acc,
-                    (n > 0 || kk > 0) ? 1u : 0u);
-          umma_commit(&do_empty[st]);
-          if (n == cnt - 1) umma_commit(dv_acc);
+            for (int kk = 0; kk < kTile / 16; ++kk)
+              umma_ts(tmem + kColDV, tmem + kColPT + kk * 8, sdesc_at(do_n, kk * 2048), idesc_acc,
+                      (n > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(&do_empty[st]);
+            if (n == cnt - 1) umma_commit(dv_acc);
+          }
         }
-      }
-    } else {
-      // dK += dS^T Q : A = dS^T tile (K-major: 64-query boxes of 128-byte rows), B = Q read N-major
-      const SmemDesc q_nmaj0 = make_sdesc_parts(smem_u32(s_q), kTile * 128, 1024);
-      const SmemDesc ds_kmaj = make_sdesc_parts(smem_u32(s_ds), 16, 1024);            // rows = keys, K = queries
-      // dQ_partial = dS K : A = the dS^T tile read M-major (rows = keys = reduction index), B = K read N-major
-      const SmemDesc k_nmaj = stage_of(make_sdesc_parts(smem_u32(s_k), kTile * 128, 1024), I & 1, kTileBytes);
-      const SmemDesc ds_mmaj = make_sdesc_parts(smem_u32(s_ds), kTile * 128, 1024);   // rows = reduction (keys)
-      ok = mbar_wait(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item);
-      for (int n = 0; n < cnt && ok; ++n) {
-        const uint32_t g = T + n, st = g % kQStages;
-        ok = mbar_wait(ds_full, g & 1, abort_flag, p.status, kSiteDSFull, s_item);
-        if (ok && n == 0 && I > 0) ok = mbar_wait(dk_free, (I - 1) & 1, abort_flag, p.status, kSiteDKFree, s_item);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const SmemDesc q_n = stage_of(q_nmaj0, st, kTileBytes);
-        if (el) {
+      } else {
+        // dK += dS^T Q : A = dS^T tile (K-major: 64-query boxes of 128-byte rows), B = Q read N-major
+        const SmemDesc q_nmaj0 = make_sdesc_parts(smem_u32(s_q), kTile * 128, 1024);
+        const SmemDesc ds_kmaj = make_sdesc_parts(smem_u32(s_ds), 16, 1024);            // rows = keys, K = queries
+        // dQ_partial = dS K : A = the dS^T tile read M-major (rows = keys = reduction index), B = K read N-major
+        const SmemDesc k_nmaj = stage_of(make_sdesc_parts(smem_u32(s_k), kTile * 128, 1024), I & 1, kTileBytes);
+        const SmemDesc ds_mmaj = make_sdesc_parts(smem_u32(s_ds), kTile * 128, 1024);   // rows = reduction (keys)
+        ok = mbar_wait(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item);
+        for (int n = 0; n < cnt && ok; ++n) {
+          const uint32_t g = T + n, st = g % kQStages;
+          ok = mbar_wait(ds_full, g & 1, abort_flag, p.status, kSiteDSFull, s_item);
+          if (ok && n == 0 && I > 0) ok = mbar_wait(dk_free, (I - 1) & 1, abort_flag, p.status, kSiteDKFree, s_item);
+          if (!ok) break;
+          tc_fence_after_sync();
+          const SmemDesc q_n = stage_of(q_nmaj0, st, kTileBytes);
+          if (el) {
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk)
-            umma_ss(tmem + kColDK, sdesc_at(ds_kmaj, (kk >> 2) * (kTile * 128) + (kk & 3) * 32), sdesc_at(q_n, kk * 2048),
-                    idesc_acc, (n > 0 || kk > 0) ? 1u : 0u);
-          umma_commit(&q_empty[st]);
-          if (n == cnt - 1) umma_commit(dk_acc);   // the item's dK is complete
-        }
-        if (g > 0) ok = mbar_wait(dq_drained, (g - 1) & 1, abort_flag, p.status, kSiteDQDrained, s_item);
-        if (!ok) break;
-        tc_fence_after_sync();
-        if (el) {
+            for (int kk = 0; kk < kTile / 16; ++kk)
+              umma_ss(tmem + kColDK, sdesc_at(ds_kmaj, (kk >> 2) * (kTile * 128) + (kk & 3) * 32), sdesc_at(q_n, kk * 2048),
+                      idesc_acc, (n > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(&q_empty[st]);
+            if (n == cnt - 1) umma_commit(dk_acc);   // the item's dK is complete
+          }
+          if (g > 0) ok = mbar_wait(dq_drained, (g - 1) & 1, abort_flag, p.status, kSiteDQDrained, s_item);
+          if (!ok) break;
+          tc_fence_after_sync();
+          if (el) {
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk)
-            umma_ss(tmem + kColDQ, sdesc_at(ds_mmaj, kk * 2048), sdesc_at(k_nmaj, kk * 2048), idesc_dq, kk > 0);
-          umma_commit(dq_full);                    // dQ_partial readable; the dS^T tile's readers are done
+            for (int kk = 0; kk < kTile / 16; ++kk)
+              umma_ss(tmem + kColDQ, sdesc_at(ds_mmaj, kk * 2048), sdesc_at(k_nmaj, kk * 2048), idesc_dq, kk > 0);
+            umma_commit(dq_full);                    // dQ_partial readable; the dS^T tile's readers are done
+          }
         }
-      }
     }
     T += cnt;
     ++I;
@@ -497,38 +497,38 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     };
     bool ok = run;
     while (ok && next_item()) {
-    const int row0 = k_row0 + wq * 32;             // this warp's key rows
-    for (int n = 0; n < cnt - 1 && ok; ++n) ok = drain_dq(n);
-    // dV and dK are complete before the last dQ_partial, and the next item's products wait for their columns
-    if (ok) ok = mbar_wait_warp(dv_acc, I & 1, abort_flag, p.status, kSiteDVAcc, s_item);
-    if (!ok) break;
-    tc_fence_after_sync();
-    {
-      uint8_t* box = open_box();
+      const int row0 = k_row0 + wq * 32;             // this warp's key rows
+      for (int n = 0; n < cnt - 1 && ok; ++n) ok = drain_dq(n);
+      // dV and dK are complete before the last dQ_partial, and the next item's products wait for their columns
+      if (ok) ok = mbar_wait_warp(dv_acc, I & 1, abort_flag, p.status, kSiteDVAcc, s_item);
+      if (!ok) break;
+      tc_fence_after_sync();
+      {
+        uint8_t* box = open_box();
 #pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        uint32_t acc[32];
-        tmem_ld_x32(tmem + kColDV + lane_sel + hh * 32, acc);
-        tmem_ld_wait();
-        if (hh == 1) {
-          tc_fence_before_sync();
-          mbar_arrive_warp(dv_free);
+        for (int hh = 0; hh < 2; ++hh) {
+          uint32_t acc[32];
+          tmem_ld_x32(tmem + kColDV + lane_sel + hh * 32, acc);
+          tmem_ld_wait();
+          if (hh == 1) {
+            tc_fence_before_sync();
+            mbar_arrive_warp(dv_free);
+          }
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
+            uint32_t o[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              o[i] = pack2<kBf16>(__uint_as_float(acc[q4 * 8 + 2 * i]), __uint_as_float(acc[q4 * 8 + 2 * i + 1]));
+            *reinterpret_cast<uint4*>(box + sw128_offset(lane, hh * 4 + q4)) = make_uint4(o[0], o[1], o[2], o[3]);
+          }
         }
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          uint32_t o[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            o[i] = pack2<kBf16>(__uint_as_float(acc[q4 * 8 + 2 * i]), __uint_as_float(acc[q4 * 8 + 2 * i + 1]));
-          *reinterpret_cast<uint4*>(box + sw128_offset(lane, hh * 4 + q4)) = make_uint4(o[0], o[1], o[2], o[3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (row0 < p.N) tma_store_4d(&tm_dv, box, 0, row0, h, b);
+          tma_store_commit();
         }
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        if (row0 < p.N) tma_store_4d(&tm_dv, box, 0, row0, h, b);
-        tma_store_commit();
-      }
     }
     ok = mbar_wait_warp(dk_acc, I & 1, abort_flag, p.status, kSiteDKAcc, s_item) &&
          mbar_wait_warp(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item) &&
@@ -589,82 +589,82 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
     bool ok = run;
     while (ok && next_item()) {
-    ok = mbar_wait_warp(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item);
-    if (!ok) break;
-    const float neg_ksq = -s_ksq[(I & 1) * kTile + r];
-    float ds_rowsum = 0.f;
-    for (int n = 0; n < cnt; ++n) {
-      ok = mbar_wait_warp(s_full, (T + n) & 1, abort_flag, p.status, kSiteSFull, s_item);
+      ok = mbar_wait_warp(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item);
       if (!ok) break;
-      tc_fence_after_sync();
-      float pr[32];
-      bool dp_ready;
-      {
-        uint32_t raw[32];
-        tmem_ld_x32(tmem + kColS + lane_sel + g * 32, raw);
-        dp_ready = mbar_test(dp_full, (T + n) & 1);
-        tmem_ld_wait();
-        // acc = k.q - L / scale2 ; P = exp2(acc * scale2 - ksq)
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float a0, a1;
-          ffma2_bcast(a0, a1, __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]), p.scale2, neg_ksq);
-          pr[i] = ex2_approx(a0);
-          pr[i + 1] = ex2_approx(a1);
-        }
-      }
-      if (p.causal && n == 0) {
-        // diagonal tile: query column (32g + c) sees key row r iff column >= row
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-          if (g * 32 + c < r) pr[c] = 0.f;
-      }
-      // dP^T(n) has landed, and with it dV(n-1): the P^T columns are free
-      if (!__all_sync(0xffffffffu, dp_ready)) {
-        ok = mbar_wait_warp(dp_full, (T + n) & 1, abort_flag, p.status, kSiteDPFull, s_item);
+      const float neg_ksq = -s_ksq[(I & 1) * kTile + r];
+      float ds_rowsum = 0.f;
+      for (int n = 0; n < cnt; ++n) {
+        ok = mbar_wait_warp(s_full, (T + n) & 1, abort_flag, p.status, kSiteSFull, s_item);
         if (!ok) break;
-      }
-      tc_fence_after_sync();
-      {
-        uint32_t packed[16];
+        tc_fence_after_sync();
+        float pr[32];
+        bool dp_ready;
+        {
+          uint32_t raw[32];
+          tmem_ld_x32(tmem + kColS + lane_sel + g * 32, raw);
+          dp_ready = mbar_test(dp_full, (T + n) & 1);
+          tmem_ld_wait();
+          // acc = k.q - L / scale2 ; P = exp2(acc * scale2 - ksq)
 #pragma unroll
-        for (int i = 0; i < 16; ++i) packed[i] = pack2<kBf16>(pr[2 * i], pr[2 * i + 1]);
-        tmem_st_x16(tmem + kColPT + lane_sel + g * 16, packed);
-      }
-      uint32_t ds_packed[16];
-      bool ds_free;
-      {
-        uint32_t raw[32];
-        tmem_ld_x32(tmem + kColDP + lane_sel + g * 32, raw);     // travels while the P^T store completes
-        tmem_st_wait();
+          for (int i = 0; i < 32; i += 2) {
+            float a0, a1;
+            ffma2_bcast(a0, a1, __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]), p.scale2, neg_ksq);
+            pr[i] = ex2_approx(a0);
+            pr[i + 1] = ex2_approx(a1);
+          }
+        }
+        if (p.causal && n == 0) {
+          // diagonal tile: query column (32g + c) sees key row r iff column >= row
+#pragma unroll
+          for (int c = 0; c < 32; ++c)
+            if (g * 32 + c < r) pr[c] = 0.f;
+        }
+        // dP^T(n) has landed, and with it dV(n-1): the P^T columns are free
+        if (!__all_sync(0xffffffffu, dp_ready)) {
+          ok = mbar_wait_warp(dp_full, (T + n) & 1, abort_flag, p.status, kSiteDPFull, s_item);
+          if (!ok) break;
+        }
+        tc_fence_after_sync();
+        {
+          uint32_t packed[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) packed[i] = pack2<kBf16>(pr[2 * i], pr[2 * i + 1]);
+          tmem_st_x16(tmem + kColPT + lane_sel + g * 16, packed);
+        }
+        uint32_t ds_packed[16];
+        bool ds_free;
+        {
+          uint32_t raw[32];
+          tmem_ld_x32(tmem + kColDP + lane_sel + g * 32, raw);     // travels while the P^T store completes
+          tmem_st_wait();
+          tc_fence_before_sync();
+          mbar_arrive_warp(p_full);
+          // the dS^T tile is free once dK and dQ_partial of the previous step have completed
+          ds_free = T + n == 0 || mbar_test(dq_full, (T + n - 1) & 1);
+          tmem_ld_wait();
+          // acc = v.dO - delta ; dS = P * acc
+          float rs0 = 0.f, rs1 = 0.f;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float d0, d1;
+            fmul2(d0, d1, pr[2 * i], pr[2 * i + 1], __uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1]));
+            fadd2(rs0, rs1, rs0, rs1, d0, d1);
+            ds_packed[i] = pack2<kBf16>(d0, d1);
+          }
+          ds_rowsum += rs0 + rs1;
+        }
+        if (!__all_sync(0xffffffffu, ds_free)) {
+          ok = mbar_wait_warp(dq_full, (T + n - 1) & 1, abort_flag, p.status, kSiteDsFree, s_item);
+          if (!ok) break;
+        }
+        // row r of the [key][query] tile, box g/2, 16-byte chunks 4(g%2) .. +3
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch)
+          *reinterpret_cast<uint4*>(s_ds + (g >> 1) * (kTile * 128) + sw128_offset(r, (g & 1) * 4 + ch)) =
+              make_uint4(ds_packed[ch * 4 + 0], ds_packed[ch * 4 + 1], ds_packed[ch * 4 + 2], ds_packed[ch * 4 + 3]);
         tc_fence_before_sync();
-        mbar_arrive_warp(p_full);
-        // the dS^T tile is free once dK and dQ_partial of the previous step have completed
-        ds_free = T + n == 0 || mbar_test(dq_full, (T + n - 1) & 1);
-        tmem_ld_wait();
-        // acc = v.dO - delta ; dS = P * acc
-        float rs0 = 0.f, rs1 = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float d0, d1;
-          fmul2(d0, d1, pr[2 * i], pr[2 * i + 1], __uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1]));
-          fadd2(rs0, rs1, rs0, rs1, d0, d1);
-          ds_packed[i] = pack2<kBf16>(d0, d1);
-        }
-        ds_rowsum += rs0 + rs1;
-      }
-      if (!__all_sync(0xffffffffu, ds_free)) {
-        ok = mbar_wait_warp(dq_full, (T + n - 1) & 1, abort_flag, p.status, kSiteDsFree, s_item);
-        if (!ok) break;
-      }
-      // row r of the [key][query] tile, box g/2, 16-byte chunks 4(g%2) .. +3
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch)
-        *reinterpret_cast<uint4*>(s_ds + (g >> 1) * (kTile * 128) + sw128_offset(r, (g & 1) * 4 + ch)) =
-            make_uint4(ds_packed[ch * 4 + 0], ds_packed[ch * 4 + 1], ds_packed[ch * 4 + 2], ds_packed[ch * 4 + 3]);
-      tc_fence_before_sync();
-      fence_proxy_async_smem();
-      mbar_arrive_warp(ds_full);
+        fence_proxy_async_smem();
+        mbar_arrive_warp(ds_full);
     }
 
     if (ok) {
