@@ -15,9 +15,9 @@
 // dK = 2g (acc - rowsum(dS^T)[key] * k).
 //
 // Roles: warps 0, 1, 3 MMA issuers (one thread sustains one MMA per ~60 cycles, the tensor pipe retires an N = 64
-// product in 32; five issuers, one per product, measured slower than three), warp 2 TMA producer, warps 4-19 compute (thread = key row; group g owns query columns [32g, 32g+32) of the
-// tile), warps 20-23 drain dQ_partial of every step and dV, dK of every item (thread = query / key row). Compute
-// warpgroups take registers from the others.
+// product in 32; five issuers, one per product, measured slower than three), warp 2 TMA producer, warps 4-19 compute
+// (thread = key row; group g owns query columns [32g, 32g+32) of the tile), warps 20-23 drain dQ_partial of every step
+// and dV, dK of every item (thread = query / key row). Compute warpgroups take registers from the others.
 //   issuer A: S^T(n+1) when P^T(n) is in TMEM (S^T(n) has been read by then)
 //   issuer B: dV(n) when P^T(n) is in TMEM; dP^T(n+1) when dS^T(n) is in shared memory (dP^T(n) has been read by then)
 //   issuer C: dK(n) when dS^T(n) is in shared memory, dQ_partial(n) when also dQ_partial(n-1) has been read by the drain
@@ -97,7 +97,6 @@ enum Site : uint32_t {
 
 struct Params {
   const float* ksq;      // (B*H, n_pad), +inf on padding rows
-  float* dq_acc;         // fp32 (B*H, N, 64), zero-initialised
   DeviceStatus* status;
   unsigned int* work;    // [0] items taken beyond the CTAs' first, [1] CTAs that have left; zero at launch and at its end
   int total_items;       // key tiles x (batch, head) pairs
@@ -189,7 +188,8 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
   constexpr int kItemReaders = 3 + 4 + kNumComputeWarps;
   auto next_item = [&]() -> bool {
     const int slot = I % Smem::kItemSlots;
-    if (!mbar_wait_warp(&item_full[slot], (I / Smem::kItemSlots) & 1, abort_flag, p.status, kSiteItemFull, s_item)) return false;
+    if (!mbar_wait_warp(&item_full[slot], (I / Smem::kItemSlots) & 1, abort_flag, p.status, kSiteItemFull, s_item))
+      return false;
     const int tile = s_items[slot].x;
     bh = s_items[slot].y;
     b = s_items[slot].z;
@@ -748,13 +748,14 @@ static cudaError_t launch_t(const BwdFusedArgs& a, cudaStream_t stream) {
   // the pre-pass has cleared the dQ accumulator
   cudaError_t e = cudaSuccess;
   Params p{};
-  p.ksq = a.ksq; p.dq_acc = a.dq_acc; p.status = a.status;
+  p.ksq = a.ksq; p.status = a.status;
   p.H = a.H; p.N = a.N; p.n_pad = a.n_pad; p.causal = a.causal;
   p.scale2 = a.scale2; p.grad_scale = a.grad_scale; p.slab_w = a.slab_w;
   p.work = a.work;
   p.total_items = ((a.N + kTile - 1) / kTile) * a.B * a.H;
   dim3 grid(p.total_items < a.sm_count ? p.total_items : a.sm_count);
-  kernel<<<grid, kThreads, smem, stream>>>(a.tm_k, a.tm_v, a.tm_q, a.tm_do, a.tm_dk, a.tm_dv, a.tm_lslab, a.tm_dslab, a.tm_dq_acc, p);
+  kernel<<<grid, kThreads, smem, stream>>>(a.tm_k, a.tm_v, a.tm_q, a.tm_do, a.tm_dk, a.tm_dv, a.tm_lslab,
+                                           a.tm_dslab, a.tm_dq_acc, p);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int64_t chunks = static_cast<int64_t>(a.B) * a.H * a.N * 8;
