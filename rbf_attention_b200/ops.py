@@ -301,11 +301,12 @@ class _StatusMonitor:
         if code != 0:
             self._report(code & 0xFFFFFFFF, e.what)
 
-    def _enqueue(self, what, call) -> None:
-        """``call(slot number)`` enqueues what posts a status word there and returns an error code."""
+    def _enqueue(self, what, call, ring) -> None:
+        """``call(slot address)`` enqueues what posts a status word there and returns an error code; ``ring`` is the address
+        of the first slot."""
         entry = self._reserve(what)
         try:
-            rc = call(entry.slot)
+            rc = call(ring + 4 * entry.slot)
             entry.state = _ENQUEUED
         except BaseException:
             # whether something was enqueued is not known: the slot is not used again before the device has been waited for
@@ -334,14 +335,14 @@ class _StatusMonitor:
         if torch._C._cuda_isCurrentStreamCapturing():
             _lib.check(call(0), what)
             return
-        self._enqueue(what, lambda slot: call(self.mapped + 4 * slot))
+        self._enqueue(what, call, self.mapped)
 
     def record(self, ws, what):
         """Posts the status word at the start of ``ws`` with a kernel of its own."""
         if torch.cuda.is_current_stream_capturing():
             return
         self._enqueue(what, lambda slot: _lib.load().rbf_b200_post_device_status(
-            ws.data_ptr(), self.base + 4 * slot, _stream_ptr(ws.device)))
+            ws.data_ptr(), slot, _stream_ptr(ws.device)), self.base)
 
 
 _SYNC_STATUS = os.environ.get("RBF_B200_SYNC_STATUS", "0") not in ("", "0")
