@@ -7,7 +7,7 @@
 // softmax - onehot, scaled by 1 / (rows that count), from there. Rows too long for that are read a second time
 // (with two blocks per SM in flight they are L2 hits). Measured at 65536 x 50304 bf16: 2.89 ms, 4.57 TB/s = 71 % of the
 // copy bandwidth (2.93 ms with maxima, scaling and sums one element at a time; 8192 x 32000: 301 -> 292 us, 3108 x 50304:
-// 200.5 -> 198.4 us, in turn on one box). exp2f() in place of the bare ex2.approx took 11 % longer. Block shapes of 256 to
+// 200.5 -> 198.4 us, in turn on one GPU). exp2f() in place of the bare ex2.approx took 11 % longer. Block shapes of 256 to
 // 512 threads, two to eight per SM, staged or re-read, all land within 10 % of each other; a variant with one block of 1024
 // threads per SM that streams the next row into a second buffer with cp.async while the current one is reduced was slower
 // (3.82 ms) and is not kept.
