@@ -384,7 +384,38 @@ __device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const uint32_t (&r)[8
                "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
+template <int kCount>
+__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t* r) {
+  static_assert(kCount == 8 || kCount == 16 || kCount == 32, "columns of a store");
+  if constexpr (kCount == 32) {
+    tmem_st_x32(taddr, *reinterpret_cast<const uint32_t(*)[32]>(r));
+  } else if constexpr (kCount == 16) {
+    tmem_st_x16(taddr, *reinterpret_cast<const uint32_t(*)[16]>(r));
+  } else {
+    tmem_st_x8(taddr, *reinterpret_cast<const uint32_t(*)[8]>(r));
+  }
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Ties registers to this point of the program: a load that tmem_ld_wait has completed before it is not read earlier by
+// code that the compiler moves (the wait itself names no registers).
+template <int kCount>
+__device__ __forceinline__ void pin_regs(uint32_t* r) {
+  static_assert(kCount % 16 == 0, "whole groups");
+#pragma unroll
+  for (int i = 0; i < kCount; i += 16)
+    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]),
+                 "+r"(r[i + 6]), "+r"(r[i + 7]), "+r"(r[i + 8]), "+r"(r[i + 9]), "+r"(r[i + 10]), "+r"(r[i + 11]),
+                 "+r"(r[i + 12]), "+r"(r[i + 13]), "+r"(r[i + 14]), "+r"(r[i + 15]));
+}
+template <int kCount>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t* r) {
+  static_assert(kCount == 16 || kCount == 32, "columns of a load");
+  if constexpr (kCount == 32) {
+    tmem_ld_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(r));
+  } else {
+    tmem_ld_x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(r));
+  }
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------

@@ -19,7 +19,10 @@
 //                    the N = 64 products, hence two issuing threads.
 // TMEM columns: S_0, S_1 (one key tile wide each), O_0 and O_1 (D columns each), P_0 and P_1 (16-bit pairs, half a key
 // tile wide each): P_t has columns of its own and is consumed from there as the A operand of the second MMA, so the
-// next scores are issued as soon as the current ones are in registers.
+// next scores are issued as soon as the current ones are in registers. (P over the scores it was made from, with key tiles
+// of 128 at D = 128 too and the next scores issued right behind P V, is 14 % slower there: B2 H16 N4096 151 -> 173 us.)
+// Of a tile's exponentials every quarter is computed, packed and stored by itself (B2 H16 N3333 D128 full, against halves:
+// 229 -> 220 us).
 //
 // The key-norm bias never passes through registers or shared-memory loads: the pre-pass stores
 // -|k_j|^2 / 2 as three 16-bit parts per key ("bias slab"), and S_t gets one extra K = 16 MMA step against a
@@ -179,11 +182,11 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   uint64_t* k_empty = k_full + kStages;          // two arrivals: one per issuer
   uint64_t* v_full = k_empty + kStages;
   uint64_t* v_empty = v_full + kStages;          // two arrivals
-  uint64_t* s_full = v_empty + kStages;          // [2]
-  uint64_t* p_full = s_full + 2;                 // [2]
-  uint64_t* o_done = p_full + 2;                 // [2]
+  uint64_t* s_full = v_empty + kStages;          // [2] S_t(j) complete; persistent: and P_t(j-2) V
+  uint64_t* p_full = s_full + 2;                 // [2] P_t(j) stored; persistent: and S_t(j+1) in the group's registers
+  uint64_t* o_done = p_full + 2;                 // [2] P_t(j) V complete (one item per CTA)
   uint64_t* grp_sync = o_done + 2;               // [2] rendezvous of the warps of a query tile
-  uint64_t* s_consumed = grp_sync + 2;           // [2] the softmax group holds S_t(j) in registers
+  uint64_t* s_consumed = grp_sync + 2;           // [2] the group holds S_t(j) in registers (one item per CTA)
   uint64_t* q_free = s_consumed + 2;             // [2] persistent: Q_t may be overwritten (issuer + softmax warps)
   uint64_t* stage_free = q_free + 2;             // [2] persistent: the previous output store has read its staging tile
   uint64_t* item_full = stage_free + 2;          // [kItemSlots] the producer has published the CTA's n-th item number
@@ -340,7 +343,8 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   // Counters that run on across a CTA's items, kept identically by every role that needs them:
   //   G      K/V tiles put through the ring by earlier items (tile j of the item uses stage (G + j) % kStages in
   //          round (G + j) / kStages)
-  //   ct     key tiles query tile t has processed in earlier items (phase of s_full, s_consumed, p_full, o_done)
+  //   md     phases of s_full[t] so far: per item one for its first scores and one for each group of MMAs
+  //   td     phases of p_full[t] so far: per item one for its first scores and one for each P
   //   qn     loads of Q_t by earlier items (phase of q_full, q_free; also of grp_sync and stage_free: one output
   //          store per load)
   if (warp == kLoadWarp) {
@@ -427,7 +431,6 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     sdesc_at(k_desc, (kk >> 2) * kKvBoxBytes + (kk & 3) * 32), idesc_s, kk > 0);
           }
           umma_ss(tmem_s[t], sdesc_at(ones_desc, 0), sdesc_at(slab, 0), idesc_s, 1u);   // + key-norm bias
-          umma_commit(&s_full[t]);
         }
       };
       auto issue_o = [&](int st, uint32_t accumulate) {
@@ -437,7 +440,6 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
           for (int kk = 0; kk < kKeys / 16; ++kk)
             umma_ts(tmem_o[t], tmem_p[t] + kk * 8, sdesc_at(v_desc, kk * 2048), idesc_o, kk > 0 ? 1u : accumulate);
-          umma_commit(&o_done[t]);
         }
       };
       auto wait_k = [&](uint32_t g) {
@@ -446,76 +448,126 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       auto wait_v = [&](uint32_t g) {
         return mbar_wait_warp(&v_full[g % kStages], (g / kStages) & 1, abort_flag, status, kSiteVFull, s_unit);
       };
-      uint32_t G = 0, ct = 0, qn = 0;
-      bool ok = true;
-      for (uint32_t n = 0; ok && (kPersistent || n == 0); ++n) {
-        Item it;
-        if (!read_item(n, ok, it)) break;
-        const int my_nkt = it.nkt(t), nkt_max = it.nkt_max;
-        // Every stage is released by both issuers: by a commit after this tile's last MMA that reads it, or - when
-        // this tile has nothing (left) to do with it - by a plain arrival made only after the stage has been filled,
-        // so that an idle issuer can never arrive twice within one phase.
-        if (my_nkt > 0) {
-          // first scores of the item: Q_t has landed, the first key tile has landed, and the group holds the last
-          // scores of the previous item in registers (it is then busy with their exponentials and its output)
-          ok = mbar_wait_warp(&q_full[t], qn & 1, abort_flag, status, kSiteQFull, s_unit) && wait_k(G);
-          if (ok && ct > 0) ok = mbar_wait_warp(&s_consumed[t], (ct - 1) & 1, abort_flag, status, kSiteSConsumed, s_unit);
-          if (!ok) break;
-          tc_fence_after_sync();
-          issue_s(G % kStages);
-          if (el && kPersistent && my_nkt == 1) umma_commit(&q_free[t]);
-          if (el) umma_commit(&k_empty[G % kStages]);
-        } else {
-          ok = wait_k(G);
-          if (!ok) break;
-          if (el) mbar_arrive(&k_empty[G % kStages]);
-        }
-        for (int j = 0; j < nkt_max && ok; ++j) {
-          const uint32_t g = G + j;
-          const int st = g % kStages;
-          const int st_next = (g + 1) % kStages;
-          bool used_k_next = false;
-          if (j < my_nkt) {
-            if (j + 1 < my_nkt) {
-              // next scores first: they only need S_t(j) to have been read
-              ok = wait_k(g + 1) && mbar_wait_warp(&s_consumed[t], (ct + j) & 1, abort_flag, status, kSiteSConsumed, s_unit);
-              if (!ok) break;
-              tc_fence_after_sync();
-              issue_s(st_next);
-              if (el && kPersistent && j + 2 == my_nkt) umma_commit(&q_free[t]);   // the item's last read of Q_t
-              used_k_next = true;
-            }
-            ok = wait_v(g);
-            ok = ok && mbar_wait_warp(&p_full[t], (ct + j) & 1, abort_flag, status, kSitePFull, s_unit);
+      if constexpr (kPersistent) {
+        uint32_t G = 0, td = 0, qn = 0;
+        bool ok = true;
+        for (uint32_t n = 0; ok && (kPersistent || n == 0); ++n) {
+          Item it;
+          if (!read_item(n, ok, it)) break;
+          const int my_nkt = it.nkt(t), nkt_max = it.nkt_max;
+          // Every stage is released by both issuers: by a commit after this tile's last MMA that reads it, or - when
+          // this tile has nothing (left) to do with it - by a plain arrival made only after the stage has been filled,
+          // so that an idle issuer can never arrive twice within one phase.
+          if (my_nkt > 0) {
+            // First scores of the item: Q_t and the first key tile have landed. (The group has read the previous item's
+            // last scores: it has arrived for the last P, which was waited for before the last P V.)
+            ok = mbar_wait_warp(&q_full[t], qn & 1, abort_flag, status, kSiteQFull, s_unit) && wait_k(G);
             if (!ok) break;
             tc_fence_after_sync();
-            issue_o(st, j > 0 ? 1u : 0u);
-            if (el) umma_commit(&v_empty[st]);
-          } else {
-            ok = wait_v(g);
+            issue_s(G % kStages);
+            if (el) {
+              umma_commit(&s_full[t]);
+              if (kPersistent && my_nkt == 1) umma_commit(&q_free[t]);
+              umma_commit(&k_empty[G % kStages]);
+            }
+            // Group j of the item's MMAs, j = 0 .. my_nkt: P_t(j-1) V and the scores S_t(j+1), once the softmax group has
+            // stored the one and holds S_t(j) in registers. One commit covers both.
+            for (int j = 0; j <= my_nkt; ++j) {
+              ok = mbar_wait_warp(&p_full[t], (td + j) & 1, abort_flag, status, kSitePFull, s_unit);
+              if (!ok) break;
+              tc_fence_after_sync();
+              if (j > 0) {
+                const int st = (G + j - 1) % kStages;
+                ok = wait_v(G + j - 1);
+                if (!ok) break;
+                issue_o(st, j > 1 ? 1u : 0u);
+                if (el) umma_commit(&v_empty[st]);
+              }
+              if (j + 1 < my_nkt) {
+                const int st = (G + j + 1) % kStages;
+                ok = wait_k(G + j + 1);
+                if (!ok) break;
+                issue_s(st);
+                if (el) {
+                  if (kPersistent && j + 2 == my_nkt) umma_commit(&q_free[t]);   // the item's last read of Q_t
+                  umma_commit(&k_empty[st]);
+                }
+              }
+              if (el) umma_commit(&s_full[t]);
+            }
+            if (!ok) break;
+            td += my_nkt + 1;
+          }
+          for (int j = my_nkt; j < nkt_max; ++j) {
+            const int st = (G + j) % kStages;
+            ok = wait_k(G + j);
+            if (!ok) break;
+            if (el) mbar_arrive(&k_empty[st]);
+            ok = wait_v(G + j);
             if (!ok) break;
             if (el) mbar_arrive(&v_empty[st]);
           }
-          if (j + 1 < nkt_max) {
-            if (used_k_next) {
-              if (el) umma_commit(&k_empty[st_next]);
-            } else {
-              ok = wait_k(g + 1);
-              if (!ok) break;
-              if (el) mbar_arrive(&k_empty[st_next]);
+          G += nkt_max;
+          qn += my_nkt > 0 ? 1 : 0;
+        }
+      } else {
+        // One item per CTA, key tiles of 64: the next scores are issued as soon as the group has read the current ones, the
+        // product with V when P is stored (tile for tile the MMAs take as long as the exponentials here, and scores that
+        // waited behind the last product with V cost 12 % at B2 H16 N4096: 151 -> 170 us).
+        const int my_nkt = first_item.nkt(t), nkt_max = first_item.nkt_max;
+        bool ok = wait_k(0);
+        if (my_nkt > 0) {
+          ok = ok && mbar_wait_warp(&q_full[t], 0, abort_flag, status, kSiteQFull, s_unit);
+          if (ok) {
+            tc_fence_after_sync();
+            issue_s(0);
+            if (el) {
+              umma_commit(&s_full[t]);
+              umma_commit(&k_empty[0]);
             }
           }
+        } else if (ok && el) {
+          mbar_arrive(&k_empty[0]);
         }
-        G += nkt_max;
-        ct += my_nkt;
-        qn += my_nkt > 0 ? 1 : 0;
+        for (int j = 0; j < nkt_max && ok; ++j) {
+          const int st = j % kStages;
+          const int st_next = (j + 1) % kStages;
+          if (j + 1 < my_nkt) {
+            // next scores first: they only need S_t(j) to have been read
+            ok = wait_k(j + 1) && mbar_wait_warp(&s_consumed[t], j & 1, abort_flag, status, kSiteSConsumed, s_unit);
+            if (!ok) break;
+            tc_fence_after_sync();
+            issue_s(st_next);
+            if (el) umma_commit(&s_full[t]);
+          }
+          ok = wait_v(j);
+          if (j < my_nkt) {
+            ok = ok && mbar_wait_warp(&p_full[t], j & 1, abort_flag, status, kSitePFull, s_unit);
+            if (!ok) break;
+            tc_fence_after_sync();
+            issue_o(st, j > 0 ? 1u : 0u);
+            if (el) {
+              umma_commit(&o_done[t]);
+              umma_commit(&v_empty[st]);
+            }
+          } else {
+            if (!ok) break;
+            if (el) mbar_arrive(&v_empty[st]);
+          }
+          if (j + 1 < my_nkt) {
+            if (el) umma_commit(&k_empty[st_next]);
+          } else if (j + 1 < nkt_max) {
+            ok = wait_k(j + 1);
+            if (ok && el) mbar_arrive(&k_empty[st_next]);
+          }
+        }
       }
     }
   } else if (warp < kLoadWarp) {
     // ------------------------------------------------------------------ softmax groups
     setmaxnreg_inc<R::kSoftmaxRegs>();
     constexpr int kCols = kKeys / kSplit;            // key columns of a tile handled by one thread
-    constexpr int kChunk = kCols >= 64 && kSplit == 1 ? 64 : 32;   // columns converted and stored to TMEM at a time
+    constexpr int kChunk = kCols / 4;                // a quarter of them: columns loaded and exponentiated at a time
     constexpr int kOCols = D / kSplit;               // output columns rescaled / written by one thread
     const int grp = warp >> 2;                       // warpgroup
     const int t = grp / kSplit;                      // query tile of this group
@@ -526,7 +578,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const bool storer = r == 0 && hf == 0;           // issues the tile's output stores
     constexpr bool kSkipMax = R::kSkipMax;
     static_assert(kSplit == 1 || !kSoftmax, "threads that share a row would have to agree on its maximum and sum");
-    uint32_t ct = 0, qn = 0;
+    uint32_t md = 0, qn = 0;
     bool ok = true;
     bool store_pending = false;                      // storer: a store whose staging tile has not been released yet
     if (D == 64 && kSplit == 1 && t == 1) {
@@ -570,21 +622,22 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         ub = ((acc[0] + acc[1]) + (acc[2] + acc[3])) * (0.5f * scale2);
       }
       if (kPersistent) mbar_arrive_warp(&q_free[t]);   // this warp will not read Q_t of this item (again)
-      for (int j = 0; j < my_nkt; ++j) {
-        ok = ok && mbar_wait_warp(&s_full[t], (ct + j) & 1, abort_flag, status, kSiteSFull, s_unit);
-        if (!ok) break;
-        tc_fence_after_sync();
-
-        // acc = q.k - |k|^2 / 2 for this thread's keys of the tile; the logit in base-2 units is acc * scale2
-        uint32_t raw[kCols];
-        {
+      // acc = q.k - |k|^2 / 2 for this thread's keys of a tile; the logit in base-2 units is acc * scale2
+      uint32_t raw[kCols];
+      uint32_t packed[kCols / 2];                    // P, 16-bit pairs
+      const uint32_t s_addr = tmem_s[t] + lane_sel + col0;
+      // P_t: key column c holds its 16-bit probability in column c / 2
+      const uint32_t p_addr = tmem_p[t] + lane_sel + col0 / 2;
+      auto load_scores = [&]() {
 #pragma unroll
-          for (int c = 0; c < kCols / 32; ++c)
-            tmem_ld_x32(tmem_s[t] + lane_sel + col0 + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
-          tmem_ld_wait();
-          tc_fence_before_sync();
-          mbar_arrive_warp(&s_consumed[t]);
-        }
+        for (int c = 0; c < 4; ++c) tmem_ld<kChunk>(s_addr + c * kChunk, raw + c * kChunk);
+        tmem_ld_wait();
+        pin_regs<kCols>(raw);
+        tc_fence_before_sync();
+      };
+      // tile j, with its scores in registers: the mask and the maximum; p = exp2(acc * scale2 - the result). `wait_o` waits
+      // until P_t(j-1) V has landed (false: the wait ran out, the result is void).
+      auto shift_of = [&](int j, auto&& wait_o) -> float {
         if (causal && (j + 1) * kKeys > r0 + 1) {
           // tiles that reach past the block's first row: key (j * kKeys + col0 + c) is visible to query (r0 + r) iff
           // it is not larger
@@ -593,104 +646,163 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           for (int c = 0; c < kCols; ++c)
             if (c > c_max) raw[c] = 0xff800000u;   // -inf
         }
-
-        float sub;   // p = exp2(acc * scale2 - sub)
-        if constexpr (kSoftmax) {
-          if (!(kSkipMax && safe)) {
-            // four independent three-input maxima: short dependency chains, half the instructions
-            float mx0 = __uint_as_float(raw[0]), mx1 = __uint_as_float(raw[1]), mx2 = __uint_as_float(raw[2]),
-                  mx3 = __uint_as_float(raw[3]);
+        if constexpr (!kSoftmax) return row_bias;
+        if (!(kSkipMax && safe)) {
+          // four independent three-input maxima: short dependency chains, half the instructions
+          float mx0 = __uint_as_float(raw[0]), mx1 = __uint_as_float(raw[1]), mx2 = __uint_as_float(raw[2]),
+                mx3 = __uint_as_float(raw[3]);
 #pragma unroll
-            for (int c = 4; c + 8 <= kCols; c += 8) {
-              mx0 = fmax3(mx0, __uint_as_float(raw[c + 0]), __uint_as_float(raw[c + 1]));
-              mx1 = fmax3(mx1, __uint_as_float(raw[c + 2]), __uint_as_float(raw[c + 3]));
-              mx2 = fmax3(mx2, __uint_as_float(raw[c + 4]), __uint_as_float(raw[c + 5]));
-              mx3 = fmax3(mx3, __uint_as_float(raw[c + 6]), __uint_as_float(raw[c + 7]));
-            }
-            mx0 = fmax3(mx0, __uint_as_float(raw[kCols - 4]), __uint_as_float(raw[kCols - 3]));
-            mx1 = fmax3(mx1, __uint_as_float(raw[kCols - 2]), __uint_as_float(raw[kCols - 1]));
-            const float tile_max = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-            const float m_new = fmaxf(m_used, tile_max * scale2);
-            const bool need = (m_new - m_used) > kRescaleThreshold;
-            float alpha = 1.f;
-            if (need) {
-              alpha = ex2_approx(m_used - m_new);
-              m_used = m_new;
-              l_sum *= alpha;
-            }
-            if (j > 0 && __any_sync(0xffffffffu, need)) {
-              // O_t holds the sum over key tiles < j; wait until the last P V has landed, then rescale this thread's
-              // share of the row.
-              ok = mbar_wait_warp(&o_done[t], (ct + j - 1) & 1, abort_flag, status, kSiteODone, s_unit);
-              if (!ok) break;
-              tc_fence_after_sync();
-#pragma unroll
-              for (int c = 0; c < kOCols / 32; ++c) {
-                uint32_t o[32];
-                tmem_ld_x32(tmem_o[t] + lane_sel + hf * kOCols + c * 32, o);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                tmem_st_x32(tmem_o[t] + lane_sel + hf * kOCols + c * 32, o);
-              }
-            }
-            if constexpr (kSkipMax) safe = __all_sync(0xffffffffu, ub - m_used <= kSafeGap);
+          for (int c = 4; c + 8 <= kCols; c += 8) {
+            mx0 = fmax3(mx0, __uint_as_float(raw[c + 0]), __uint_as_float(raw[c + 1]));
+            mx1 = fmax3(mx1, __uint_as_float(raw[c + 2]), __uint_as_float(raw[c + 3]));
+            mx2 = fmax3(mx2, __uint_as_float(raw[c + 4]), __uint_as_float(raw[c + 5]));
+            mx3 = fmax3(mx3, __uint_as_float(raw[c + 6]), __uint_as_float(raw[c + 7]));
           }
-          sub = m_used;
-        } else {
-          sub = row_bias;
+          mx0 = fmax3(mx0, __uint_as_float(raw[kCols - 4]), __uint_as_float(raw[kCols - 3]));
+          mx1 = fmax3(mx1, __uint_as_float(raw[kCols - 2]), __uint_as_float(raw[kCols - 1]));
+          const float tile_max = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+          const float m_new = fmaxf(m_used, tile_max * scale2);
+          const bool need = (m_new - m_used) > kRescaleThreshold;
+          float alpha = 1.f;
+          if (need) {
+            alpha = ex2_approx(m_used - m_new);
+            m_used = m_new;
+            l_sum *= alpha;
+          }
+          if (j > 0 && __any_sync(0xffffffffu, need)) {
+            // O_t holds the sum over key tiles < j once the last P V has landed: rescale this thread's share of the row
+            if (!wait_o()) return m_used;
+#pragma unroll
+            for (int c = 0; c < kOCols / 32; ++c) {
+              uint32_t o[32];
+              tmem_ld_x32(tmem_o[t] + lane_sel + hf * kOCols + c * 32, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st_x32(tmem_o[t] + lane_sel + hf * kOCols + c * 32, o);
+            }
+          }
+          if constexpr (kSkipMax) safe = __all_sync(0xffffffffu, ub - m_used <= kSafeGap);
         }
+        return m_used;
+      };
+      float ps0, ps1, ps2, ps3;                      // the tile's row sum
+      auto exponentials = [&](int c, float neg_sub) {   // quarter c
+        uint32_t* out = packed + c * (kChunk / 2);
+#pragma unroll
+        for (int i = 0; i < kChunk / 2; i += 2) {
+          float a0, a1, a2, a3;
+          ffma2_bcast(a0, a1, __uint_as_float(raw[c * kChunk + 2 * i + 0]), __uint_as_float(raw[c * kChunk + 2 * i + 1]),
+                      scale2, neg_sub);
+          ffma2_bcast(a2, a3, __uint_as_float(raw[c * kChunk + 2 * i + 2]), __uint_as_float(raw[c * kChunk + 2 * i + 3]),
+                      scale2, neg_sub);
+          const float p0 = ex2_approx(a0), p1 = ex2_approx(a1), p2 = ex2_approx(a2), p3 = ex2_approx(a3);
+          fadd2(ps0, ps1, ps0, ps1, p0, p1);
+          fadd2(ps2, ps3, ps2, ps3, p2, p3);
+          out[i] = pack2<kBf16>(p0, p1);
+          out[i + 1] = pack2<kBf16>(p2, p3);
+        }
+      };
+      auto store_p = [&](int c) { tmem_st<kChunk / 2>(p_addr + c * (kChunk / 2), packed + c * (kChunk / 2)); };
+      auto p_stored = [&]() {
+        l_sum += (ps0 + ps1) + (ps2 + ps3);
+        tmem_st_wait();
+      };
 
-        // P's own columns are free once O_t += P_t V_(j-1) has completed (for the item's first tile: the output of
-        // the previous item has been read, which waited for its last P V)
-        bool waited_o = j == 0;
-        const float neg_sub = -sub;
-        float ps0 = 0.f, ps1 = 0.f, ps2 = 0.f, ps3 = 0.f;
+      if constexpr (kPersistent) {
+        // One wait and one arrival per tile. The wait, at three quarters of the exponentials, is for group j of the item's
+        // MMAs - P_t(j-1) V and S_t(j+1), issued when S_t(j) was in registers -, after which P's columns are free and the
+        // next scores can be loaded: three quarters of them travel under the last quarter's exponentials. Against a wait
+        // for the scores, one for P's columns and two arrivals, each 130 to 220 clocks of a warp's 2900 per tile (traced):
+        // B8 H16 N4096 causal 421 -> 401 us with the pre-pass, B64 H8 N1028 207 -> 198, B4 H12 N1000 full 39.4 -> 37.4.
+        ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, status, kSiteSFull, s_unit);
+        if (!ok) break;
+        ++md;
+        tc_fence_after_sync();
+        load_scores();
+        mbar_arrive_warp(&p_full[t]);
+        for (int j = 0;; ++j, ++md) {
+          bool group_done = false;
+          const float neg_sub = -shift_of(j, [&]() {
+            ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, status, kSiteODone, s_unit);
+            if (ok) tc_fence_after_sync();
+            return group_done = ok;
+          });
+          if (!ok) break;
+          ps0 = ps1 = ps2 = ps3 = 0.f;
 #pragma unroll
-        for (int c = 0; c < kCols / kChunk; ++c) {
-          uint32_t packed[kChunk / 2];
-#pragma unroll
-          for (int i = 0; i < kChunk / 2; i += 2) {
-            float a0, a1, a2, a3;
-            ffma2_bcast(a0, a1, __uint_as_float(raw[c * kChunk + 2 * i + 0]), __uint_as_float(raw[c * kChunk + 2 * i + 1]),
-                        scale2, neg_sub);
-            ffma2_bcast(a2, a3, __uint_as_float(raw[c * kChunk + 2 * i + 2]), __uint_as_float(raw[c * kChunk + 2 * i + 3]),
-                        scale2, neg_sub);
-            const float p0 = ex2_approx(a0), p1 = ex2_approx(a1), p2 = ex2_approx(a2), p3 = ex2_approx(a3);
-            fadd2(ps0, ps1, ps0, ps1, p0, p1);
-            fadd2(ps2, ps3, ps2, ps3, p2, p3);
-            packed[i] = pack2<kBf16>(p0, p1);
-            packed[i + 1] = pack2<kBf16>(p2, p3);
-          }
-          if (!waited_o) {
-            ok = mbar_wait_warp(&o_done[t], (ct + j - 1) & 1, abort_flag, status, kSitePFree, s_unit);
+          for (int c = 0; c < 3; ++c) exponentials(c, neg_sub);
+          if (!group_done) {
+            ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, status, kSiteSFull, s_unit);
             if (!ok) break;
             tc_fence_after_sync();
-            waited_o = true;
           }
-          // key column c holds its 16-bit P in column c / 2 of the tile's P block
-          if constexpr (kChunk == 64) {
-            tmem_st_x32(tmem_p[t] + lane_sel + (col0 + c * kChunk) / 2, packed);
-          } else {
-            tmem_st_x16(tmem_p[t] + lane_sel + (col0 + c * kChunk) / 2, packed);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) store_p(c);
+          const bool last = j + 1 == my_nkt;
+          if (last) {
+            exponentials(3, neg_sub);
+            store_p(3);
+            p_stored();
+            tc_fence_before_sync();
+            mbar_arrive_warp(&p_full[t]);
+            ++md;
+            break;
+          }
+#pragma unroll
+          for (int c = 0; c < 3; ++c) tmem_ld<kChunk>(s_addr + c * kChunk, raw + c * kChunk);
+          exponentials(3, neg_sub);
+          tmem_ld<kChunk>(s_addr + 3 * kChunk, raw + 3 * kChunk);
+          store_p(3);
+          p_stored();
+          tmem_ld_wait();
+          pin_regs<kCols>(raw);
+          tc_fence_before_sync();
+          mbar_arrive_warp(&p_full[t]);
+          if (j == 0 && storer && store_pending) {
+            // the previous item's output store was issued a whole tile ago: its staging tile has been read by now
+            tma_store_wait_read();
+            mbar_arrive(&stage_free[t]);
+            store_pending = false;
           }
         }
         if (!ok) break;
-        l_sum += (ps0 + ps1) + (ps2 + ps3);
-        tmem_st_wait();
-        tc_fence_before_sync();
-        mbar_arrive_warp(&p_full[t]);
-        if (kPersistent && j == 0 && storer && store_pending) {
-          // the previous item's output store was issued a whole tile ago: its staging tile has been read by now
+        if (storer && store_pending) {               // an item of one tile
           tma_store_wait_read();
           mbar_arrive(&stage_free[t]);
           store_pending = false;
         }
+        ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, status, kSiteODoneFinal, s_unit);
+        ++md;
+        if (ok && qn > 0) ok = mbar_wait_warp(&stage_free[t], (qn - 1) & 1, abort_flag, status, kSiteStageFree, s_unit);
+      } else {
+        for (int j = 0; j < my_nkt; ++j) {
+          ok = mbar_wait_warp(&s_full[t], j & 1, abort_flag, status, kSiteSFull, s_unit);
+          if (!ok) break;
+          tc_fence_after_sync();
+          load_scores();
+          mbar_arrive_warp(&s_consumed[t]);
+          auto wait_o = [&]() {
+            ok = mbar_wait_warp(&o_done[t], (j - 1) & 1, abort_flag, status, kSiteODone, s_unit);
+            if (ok) tc_fence_after_sync();
+            return ok;
+          };
+          const float neg_sub = -shift_of(j, wait_o);
+          if (!ok) break;
+          ps0 = ps1 = ps2 = ps3 = 0.f;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) exponentials(c, neg_sub);
+          // P's own columns are free once O_t += P_t V_(j-1) has completed
+          if (j > 0 && !wait_o()) break;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) store_p(c);
+          p_stored();
+          tc_fence_before_sync();
+          mbar_arrive_warp(&p_full[t]);
+        }
+        if (!ok) break;
+        ok = mbar_wait_warp(&o_done[t], (my_nkt - 1) & 1, abort_flag, status, kSiteODoneFinal, s_unit);
       }
-      if (!ok) break;
-
-      ok = mbar_wait_warp(&o_done[t], (ct + my_nkt - 1) & 1, abort_flag, status, kSiteODoneFinal, s_unit);
-      if (ok && kPersistent && qn > 0) ok = mbar_wait_warp(&stage_free[t], (qn - 1) & 1, abort_flag, status, kSiteStageFree, s_unit);
       if (!ok) break;
       tc_fence_after_sync();
       const float inv = kSoftmax ? (1.0f / l_sum) : 1.0f;
@@ -722,7 +834,6 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         store_pending = true;
       }
       if (kSoftmax && hf == 0 && row < N) lse[static_cast<int64_t>(it.bh) * N + row] = m_used + log2f(l_sum);
-      ct += my_nkt;
       ++qn;
     }
     if (storer && store_pending) tma_store_wait_read();   // the CTA may exit once the staging tile has been read

@@ -1,0 +1,38 @@
+"""The forward at the edges of its tiles: items of one and more key tiles, with one or two query tiles, an odd number of
+them, and rows whose maximum rises from key tile to key tile (the accumulated output is rescaled under the products in
+flight). Against the fp32 oracle with the tolerances of the 16-bit operands (2^-9 and 2^-11 relative rounding of P and of the
+result over sums of independent terms)."""
+
+import pytest
+import torch
+
+from oracle import rbf_oracle as oracle
+from rbf_attention_b200 import ops
+
+pytestmark = pytest.mark.gpu
+REL_L2 = {torch.bfloat16: 6e-3, torch.float16: 1e-3}
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("N", [127, 128, 129, 256, 257, 385, 640])
+def test_forward_at_tile_edges(N, D, dtype):
+    for softmax in (True, False):
+        q, k, v, do = oracle.make_inputs(2, 3, N, D, seed=N, dtype=dtype, std=1.0 if softmax else 0.5)
+        if softmax:                     # nearer keys come later: 2^8 is passed several times over the first keys
+            k = (k.float() * torch.linspace(2.5, 0.8, N)[None, None, :, None]).to(dtype)
+        for causal in (True, False):
+            ref = oracle.torch_forward_backward(q, k, v, do, causal, softmax, dtype=torch.float32)[0]
+            out, lse = ops._forward(q.to("cuda"), k.to("cuda"), v.to("cuda"), causal, softmax)
+            again, _ = ops._forward(q.to("cuda"), k.to("cuda"), v.to("cuda"), causal, softmax)
+            ops.check_device_status()
+            rep = oracle.error_report(out.cpu().float(), ref)
+            assert rep["rel_l2"] <= REL_L2[dtype], (softmax, causal, rep)
+            assert torch.equal(out, again)
+            if softmax:
+                qf, kf = q.double(), k.double()
+                scores = (2 * qf @ kf.mT - kf.square().sum(-1)[:, :, None]) / D ** 0.5
+                if causal:
+                    scores = scores.masked_fill(torch.ones(N, N, dtype=torch.bool).triu(1), float("-inf"))
+                want = torch.logsumexp(scores, -1) / torch.tensor(2.0).double().log()
+                assert (lse.cpu().double() - want).abs().max() <= 1e-3
