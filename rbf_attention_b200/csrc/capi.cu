@@ -219,8 +219,8 @@ static int fwd_tf32(const void* q, const void* k, const void* v, void* out, floa
   if (sr != 0) return fail(RBF_B200_ERR_TENSOR_MAP, "cuTensorMapEncodeTiled failed for the key-norm slabs (code %d)", sr);
   a.qsq = ws.row_bias; a.lse = lse; a.status = ws.status;
   a.B = B; a.H = H; a.N = N; a.n_pad = n_pad; a.causal = causal ? 1 : 0; a.scale2 = 2.f * c; a.slab_w = 1.0f;
+  a.status_slot = status_slot;
   e = rbf::launch_fwd_tf32(a, softmax != 0, stream);
-  if (e == cudaSuccess && status_slot != nullptr) e = rbf::launch_post_status(ws.status, status_slot, stream);
   if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "forward launch failed: %s", cudaGetErrorString(e));
   return RBF_B200_OK;
 }

@@ -23,6 +23,7 @@ template <bool kBf16>
 __global__ void __launch_bounds__(256) col_sums_partial_kernel(const uint16_t* __restrict__ x, int64_t ld, int64_t rows,
                                                                int cols, int64_t band, float* __restrict__ partials) {
   __shared__ float s_acc[8][256 + 8];
+  grid_dependents_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = (blockIdx.x * 32 + lane) * 8;
   const int64_t r0 = blockIdx.y * band, r1 = min(r0 + band, rows);
@@ -60,8 +61,8 @@ __global__ void __launch_bounds__(256) col_sums_final_kernel(const float* __rest
   const int col = threadIdx.x & 31, lp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + col;
   float sum = 0.f;
-  if (c < cols)
-    for (int b = lp; b < bands; b += 8) sum += partials[static_cast<int64_t>(b) * cols + c];
+  grid_dependency_wait();
+  if (c < cols) sum = strided_sum(partials + static_cast<int64_t>(lp) * cols + c, 8ll * cols, (bands - lp + 7) / 8);
   s[lp][col] = sum;
   __syncthreads();
   if (threadIdx.x < 32 && c < cols) {
@@ -84,8 +85,7 @@ int col_sums_bands(int64_t rows, int cols, int sms) {
 }
 
 cudaError_t launch_col_sums_final(const float* partials, int bands, int cols, float* out, cudaStream_t stream) {
-  col_sums_final_kernel<<<(cols + 31) / 32, 256, 0, stream>>>(partials, bands, cols, out);
-  return cudaGetLastError();
+  return launch_dependent(col_sums_final_kernel, (cols + 31) / 32, 256, 0, stream, partials, bands, cols, out);
 }
 
 cudaError_t launch_col_sums(const void* x, int64_t ld, int64_t rows, int cols, bool bf16, float* partials, float* out,
@@ -98,8 +98,7 @@ cudaError_t launch_col_sums(const void* x, int64_t ld, int64_t rows, int cols, b
   else col_sums_partial_kernel<false><<<grid, 256, 0, stream>>>(xp, ld, rows, cols, band, partials);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  col_sums_final_kernel<<<(cols + 31) / 32, 256, 0, stream>>>(partials, bands, cols, out);
-  return cudaGetLastError();
+  return launch_col_sums_final(partials, bands, cols, out, stream);
 }
 
 }  // namespace rbf

@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const uint16_t* __restric
                                                        uint16_t* __restrict__ dh, int64_t rows, int cols, int64_t band,
                                                        float* __restrict__ partials) {
   __shared__ float s_acc[8][256 + 8];
+  grid_dependents_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = (blockIdx.x * 32 + lane) * 8;
   const int64_t r0 = blockIdx.y * band, r1 = min(r0 + band, rows);

@@ -278,6 +278,26 @@ inline cudaError_t ensure_dynamic_smem(Kernel kernel, int bytes, PerDeviceFlags&
   return e;
 }
 
+// Launches a kernel that begins with grid_dependency_wait(): it may be set up - blocks resident, barriers and tensor memory
+// ready - before the kernel ahead of it has completed. Every boundary inside a call: about a microsecond of 2 (forward calls
+// replayed back to back: B2 H4 N256 12.3 -> 11.3 us, B4 H8 N1024 23.0 -> 22.0, B2 H12 N1500 D80 37.4 -> 36.1; backward 17.4 ->
+// 16.4, 41.5 -> 40.5, 83.5 -> 82.4).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream,
+                                    const Args&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = dim3(block);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 // SM count of the current device (-1 on error), cached per device.
 inline int device_sm_count() {
   static std::atomic<int> cached[PerDeviceFlags::kMaxDevices];

@@ -168,6 +168,7 @@ template <bool kBf16, int kVecs>
 __global__ void __launch_bounds__(kLnThreads, ln_bwd_blocks(kVecs)) layer_norm_bwd_kernel(const LayerNormBwdArgs a) {
   constexpr int kCols = kVecs * 256;
   extern __shared__ float s_part[];               // [kLnWarps][2][kCols]
+  grid_dependents_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float gamma[kVecs][8], dg[kVecs][8], db[kVecs][8];
 #pragma unroll
@@ -256,8 +257,8 @@ __global__ void __launch_bounds__(256) layer_norm_bwd_final_kernel(const float* 
   const int col = threadIdx.x & 31, lp = threadIdx.x >> 5;
   const int o = blockIdx.x * 32 + col;
   float sum = 0.f;
-  if (o < n_out)
-    for (int p = lp; p < n_blocks; p += 8) sum += partials[static_cast<int64_t>(p) * n_out + o];
+  grid_dependency_wait();
+  if (o < n_out) sum = strided_sum(partials + static_cast<int64_t>(lp) * n_out + o, 8ll * n_out, (n_blocks - lp + 7) / 8);
   s[lp][col] = sum;
   __syncthreads();
   if (threadIdx.x < 32 && o < n_out) {
@@ -289,8 +290,8 @@ cudaError_t launch_bwd_t(const LayerNormBwdArgs& a, int grid, cudaStream_t strea
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int n_out = 2 * kVecs * 256;
-  layer_norm_bwd_final_kernel<<<(n_out + 31) / 32, 256, 0, stream>>>(a.partials, grid, n_out, a.dgamma, a.dbeta);
-  return cudaGetLastError();
+  return launch_dependent(layer_norm_bwd_final_kernel, (n_out + 31) / 32, 256, 0, stream, a.partials, grid, n_out, a.dgamma,
+                          a.dbeta);
 }
 
 }  // namespace

@@ -153,6 +153,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 }
 
 // ---------------------------------------------------------------------------------------------
+// Dependent launches (launch_dependent in launch.h): the next kernel of a call is set up while this one still runs.
+// ---------------------------------------------------------------------------------------------
+// Returns when the kernels before this one in the stream have completed and their writes are visible. A kernel launched with
+// launch_dependent calls it, in every thread, before it touches global memory.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel may be launched once every block has come here (or has exited).
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------------------
 // TMA (tensor maps are passed as __grid_constant__ kernel parameters)
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {

@@ -236,8 +236,6 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
   // the first loads before the CTA-wide synchronisation, so that K, V and the first query tiles travel while TMEM is
   // allocated and the constant slab is written.
   if (warp == kLoadWarp) {
-    unsigned int earlier = 0u;
-    if (lane == 0) earlier = *reinterpret_cast<volatile unsigned int*>(&p.status->code);
     for (int i = lane; i < Smem::kNumBars; i += 32) {
       uint64_t* bar = &bars[i];
       uint32_t count = 1;                          // one MMA commit, TMA producer or publishing thread
@@ -252,15 +250,17 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
       // the loads below complete on barriers that other lanes have just initialised; besides the warp-level
       // synchronisation, order those generic-proxy writes before this thread's async-proxy operations
       fence_proxy_async_smem();
+      tma_prefetch_desc(&tm_k);
+      tma_prefetch_desc(&tm_v);
+      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(&tm_do);
+      tma_prefetch_desc(&tm_lslab);
+      tma_prefetch_desc(&tm_dslab);
+      grid_dependency_wait();                      // the pre-pass: slabs, norms, cleared accumulator, status word, counters
+      const unsigned int earlier = *reinterpret_cast<volatile unsigned int*>(&p.status->code);
       *s_item = static_cast<int>(blockIdx.x);
       *abort_flag = earlier != 0u ? 1 : 0;
       if (earlier == 0u) {
-        tma_prefetch_desc(&tm_k);
-        tma_prefetch_desc(&tm_v);
-        tma_prefetch_desc(&tm_q);
-        tma_prefetch_desc(&tm_do);
-        tma_prefetch_desc(&tm_lslab);
-        tma_prefetch_desc(&tm_dslab);
         set_item(static_cast<int>(blockIdx.x));    // the launch never has more CTAs than items
         load_k();
         load_q(0);
@@ -285,6 +285,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     *reinterpret_cast<uint4*>(s_ones + tid * 32 + 16) = v;
     fence_proxy_async_smem();
   }
+  grid_dependency_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -678,6 +679,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
   }
 
   // ------------------------------------------------------------------ teardown
+  grid_dependents_launch();
   if (*abort_flag) {
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000ll) {
@@ -705,6 +707,7 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict
                                                          const float* __restrict__ delta, int n_pad,
                                                          const DeviceStatus* status, unsigned int* status_slot,
                                                          int head_dim) {
+  grid_dependency_wait();
   if (status_slot != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) post_status_word(status, status_slot);
   // one thread per 8 consecutive elements of a row (D = 64: 8 chunks per row)
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -754,15 +757,13 @@ static cudaError_t launch_t(const BwdFusedArgs& a, cudaStream_t stream) {
   p.work = a.work;
   p.total_items = ((a.N + kTile - 1) / kTile) * a.B * a.H;
   dim3 grid(p.total_items < a.sm_count ? p.total_items : a.sm_count);
-  kernel<<<grid, kThreads, smem, stream>>>(a.tm_k, a.tm_v, a.tm_q, a.tm_do, a.tm_dk, a.tm_dv, a.tm_lslab,
-                                           a.tm_dslab, a.tm_dq_acc, p);
-  e = cudaGetLastError();
+  e = launch_dependent(kernel, grid, kThreads, smem, stream, a.tm_k, a.tm_v, a.tm_q, a.tm_do, a.tm_dk, a.tm_dv, a.tm_lslab,
+                       a.tm_dslab, a.tm_dq_acc, p);
   if (e != cudaSuccess) return e;
   const int64_t chunks = static_cast<int64_t>(a.B) * a.H * a.N * 8;
-  dq_convert_kernel<kBf16><<<static_cast<unsigned>((chunks + 255) / 256), 256, 0, stream>>>(
-      a.dq_acc, a.dq, a.H, a.N, a.dq_strides[0], a.dq_strides[1], a.dq_strides[2], a.grad_scale, chunks, a.q_rows,
+  return launch_dependent(
+      dq_convert_kernel<kBf16>, static_cast<unsigned>((chunks + 255) / 256), 256, 0, stream, a.dq_acc, a.dq, a.H, a.N, a.dq_strides[0], a.dq_strides[1], a.dq_strides[2], a.grad_scale, chunks, a.q_rows,
       a.q_strides[0], a.q_strides[1], a.q_strides[2], a.delta, a.n_pad, a.status, a.status_slot, a.head_dim);
-  return cudaGetLastError();
 }
 
 }  // namespace bwdf

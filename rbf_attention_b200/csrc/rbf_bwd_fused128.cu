@@ -160,7 +160,6 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   // the first loads before the CTA-wide synchronisation, so that they travel while TMEM is allocated and the constant
   // slab is written (behind a synchronisation of its own for the status word: backward call at B4 H16 N2048 266 -> 263 us).
   if (tid == kLoadWarp * 32) {
-    const unsigned int earlier = *reinterpret_cast<volatile unsigned int*>(&p.status->code);
     mbar_init(kv_full, 1);
     for (int s = 0; s < kQStages; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 2); }
     for (int s = 0; s < kDoStages; ++s) { mbar_init(&do_full[s], 1); mbar_init(&do_empty[s], 2); }
@@ -178,14 +177,16 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     mbar_init(grp_sync, kNumComputeWarps);
     fence_mbar_init();
     fence_proxy_async_smem();
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_do);
+    tma_prefetch_desc(&tm_lslab);
+    tma_prefetch_desc(&tm_dslab);
+    grid_dependency_wait();                          // the pre-pass: slabs, cleared accumulator, status word
+    const unsigned int earlier = *reinterpret_cast<volatile unsigned int*>(&p.status->code);
     *abort_flag = earlier != 0u ? 1 : 0;
     if (earlier == 0u) {
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
-      tma_prefetch_desc(&tm_q);
-      tma_prefetch_desc(&tm_do);
-      tma_prefetch_desc(&tm_lslab);
-      tma_prefetch_desc(&tm_dslab);
       mbar_arrive_expect_tx(kv_full, 2 * kKvBytes);
       for (int x = 0; x < 2; ++x) tma_load_4d(s_k + x * kBoxBytes, &tm_k, kv_full, x * 64, k_row0, h, b);
       load_q(0);
@@ -208,6 +209,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     *reinterpret_cast<uint4*>(s_ones + tid * 32 + 16) = v;
     fence_proxy_async_smem();
   }
+  grid_dependency_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -563,6 +565,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   }
 
   // ------------------------------------------------------------------ teardown
+  grid_dependents_launch();
   if (*abort_flag) {
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000ll) {
@@ -583,6 +586,7 @@ __global__ void __launch_bounds__(256) dq_convert128_kernel(const float* __restr
                                                             const DeviceStatus* status, unsigned int* status_slot,
                                                          int head_dim) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  grid_dependency_wait();
   if (status_slot != nullptr && i == 0) post_status_word(status, status_slot);
   if (i >= total_chunks) return;
   const int64_t row = i >> 4;
@@ -628,15 +632,13 @@ static cudaError_t launch_t(const BwdFusedArgs& a, cudaStream_t stream) {
   p.H = a.H; p.N = a.N; p.n_pad = a.n_pad; p.causal = a.causal;
   p.scale2 = a.scale2; p.grad_scale = a.grad_scale; p.slab_w = a.slab_w;
   dim3 grid((a.N + kTile - 1) / kTile, a.B * a.H);
-  kernel<<<grid, kThreads, smem, stream>>>(a.tm_k, a.tm_v, a.tm_q, a.tm_do, a.tm_dk, a.tm_dv, a.tm_lslab, a.tm_dslab,
-                                           p);
-  e = cudaGetLastError();
+  e = launch_dependent(kernel, grid, kThreads, smem, stream, a.tm_k, a.tm_v, a.tm_q, a.tm_do, a.tm_dk, a.tm_dv, a.tm_lslab,
+                       a.tm_dslab, p);
   if (e != cudaSuccess) return e;
   const int64_t chunks = static_cast<int64_t>(a.B) * a.H * a.N * (D / 8);
-  dq_convert128_kernel<kBf16><<<static_cast<unsigned>((chunks + 255) / 256), 256, 0, stream>>>(
-      a.dq_acc, a.dq, a.H, a.N, a.dq_strides[0], a.dq_strides[1], a.dq_strides[2], a.grad_scale, chunks, a.q_rows,
+  return launch_dependent(
+      dq_convert128_kernel<kBf16>, static_cast<unsigned>((chunks + 255) / 256), 256, 0, stream, a.dq_acc, a.dq, a.H, a.N, a.dq_strides[0], a.dq_strides[1], a.dq_strides[2], a.grad_scale, chunks, a.q_rows,
       a.q_strides[0], a.q_strides[1], a.q_strides[2], a.delta, a.n_pad, a.status, a.status_slot, a.head_dim);
-  return cudaGetLastError();
 }
 
 }  // namespace bwdf128

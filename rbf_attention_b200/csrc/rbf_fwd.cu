@@ -275,7 +275,6 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   // is in flight, and issues the first loads before the CTA-wide synchronisation, so that Q and the first key tiles
   // travel while TMEM is allocated and the constant slab is written.
   if (tid == kLoadWarp * 32) {
-    const unsigned int earlier = *reinterpret_cast<volatile unsigned int*>(&status->code);
     mbar_init(&q_full[0], 1);
     mbar_init(&q_full[1], 1);
     for (int s = 0; s < kStages; ++s) {
@@ -298,15 +297,17 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       mbar_init(&item_empty[i], kItemReaders);
     }
     fence_mbar_init();
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+    tma_prefetch_desc(&tm_kslab);
+    grid_dependency_wait();                          // the pre-pass: slabs, norms, status word and counters
+    const unsigned int earlier = *reinterpret_cast<volatile unsigned int*>(&status->code);
     s_items[0].x = first_item.bh;
     *s_unit = static_cast<int>(blockIdx.x);
     mbar_arrive(&item_full[0]);
     *abort_flag = earlier != 0u ? 1 : 0;
     if (earlier == 0u) {
-      tma_prefetch_desc(&tm_q);
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
-      tma_prefetch_desc(&tm_kslab);
       for (int t = 0; t < 2; ++t)
         if (first_item.nkt(t) > 0) load_q(first_item, t);
       for (int j = 0; j < first_item.nkt_max && j < kStages; ++j) {
@@ -327,6 +328,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     *reinterpret_cast<uint4*>(s_ones + tid * 32 + 16) = v;
     fence_proxy_async_smem();
   }
+  grid_dependency_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -872,11 +874,10 @@ static cudaError_t launch_fwd_t(const FwdArgs& a, cudaStream_t stream) {
     if (sms <= 0) return cudaErrorInvalidDevice;
     if (grid > sms) grid = sms;                    // one CTA per SM walks the items w, w + grid, ...
   }
-  kernel<<<grid, fwd::Roles<D, kSoftmax, kBf16>::kThreads, smem, stream>>>(a.tm_q, a.tm_k, a.tm_v, a.tm_o, a.tm_kslab, a.qsq, a.lse, a.status,
+  return launch_dependent(kernel, grid, fwd::Roles<D, kSoftmax, kBf16>::kThreads, smem, stream, a.tm_q, a.tm_k, a.tm_v, a.tm_o, a.tm_kslab, a.qsq, a.lse, a.status,
                                                 a.H, a.N, a.n_pad, a.causal, a.scale2, a.slab_w, heads, blocks,
                                                 // forward work counters: words 18, 19 of the status block (zeroed with it)
                                                 reinterpret_cast<unsigned int*>(a.status) + 18, a.status_slot);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_fwd(const FwdArgs& a, bool bf16, int D, bool softmax, cudaStream_t stream) {

@@ -51,6 +51,7 @@ template <bool kBf16, int D>
 __global__ void __launch_bounds__(256) row_stats_kernel(const RowStatsArgs a) {
   constexpr int kLanesPerRow = D / 8;                 // 8 (D=64) or 16 (D=128)
   constexpr int kRowsPerWarp = 32 / kLanesPerRow;     // 4 or 2
+  grid_dependents_launch();
   if (a.status_to_clear != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 64)
     reinterpret_cast<unsigned int*>(a.status_to_clear)[threadIdx.x] = 0u;   // status word and work counters
   const int lane = threadIdx.x & 31;
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(256) row_stats_f32_kernel(const RowStatsF32Arg
   constexpr int D = 64;
   constexpr int kLanesPerRow = D / 4;                 // 16 lanes x 16 bytes
   constexpr int kRowsPerWarp = 32 / kLanesPerRow;     // 2
+  grid_dependents_launch();
   if (a.status_to_clear != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 64)
     reinterpret_cast<unsigned int*>(a.status_to_clear)[threadIdx.x] = 0u;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -230,6 +232,7 @@ static constexpr int kPrepRowsPerBlock = 8;      // sequence positions per block
 template <bool kBf16, int D>
 __global__ void __launch_bounds__(256) qkv_prep_kernel(const QkvPrepArgs a) {
   constexpr int kLanesPerRow = D / 8;
+  grid_dependents_launch();
   if (a.status_to_clear != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 64)
     reinterpret_cast<unsigned int*>(a.status_to_clear)[threadIdx.x] = 0u;
   const int b = blockIdx.y;
@@ -304,6 +307,7 @@ int qkv_prep_bwd_chunks(int S, int R) { return (S - R + kPrepBwdRows - 1) / kPre
 template <bool kBf16>
 __global__ void __launch_bounds__(256) qkv_prep_bwd_partial_kernel(const QkvPrepBwdArgs a) {
   extern __shared__ float s_cols[];              // groups x (H * D) column sums of this block
+  grid_dependents_launch();
   const int D = a.D;
   const int lanes = D / 8;
   const int cols = a.H * lanes;                  // 16-byte columns of one text row over all heads
@@ -364,6 +368,7 @@ __global__ void __launch_bounds__(1024) qkv_prep_bwd_final_kernel(const QkvPrepB
   const int half = a.D / 2;
   const int n_out = a.H * half;
   const int nw = (n_out + 31) / 32;
+  grid_dependency_wait();
   if (static_cast<int>(blockIdx.x) < nw) {
     __shared__ float s_part[32][33];
     const int col = threadIdx.x & 31, lane_p = threadIdx.x >> 5;
@@ -425,9 +430,8 @@ cudaError_t launch_qkv_prep_bwd(QkvPrepBwdArgs a, bool bf16, cudaStream_t stream
   if (e != cudaSuccess) return e;
   const int nw = (a.H * (a.D / 2) + 31) / 32;
   const int nr = (a.H * a.R * a.D + 1023) / 1024;
-  if (bf16) qkv_prep_bwd_final_kernel<true><<<nw + nr, 1024, 0, stream>>>(a);
-  else qkv_prep_bwd_final_kernel<false><<<nw + nr, 1024, 0, stream>>>(a);
-  return cudaGetLastError();
+  return bf16 ? launch_dependent(qkv_prep_bwd_final_kernel<true>, nw + nr, 1024, 0, stream, a)
+              : launch_dependent(qkv_prep_bwd_final_kernel<false>, nw + nr, 1024, 0, stream, a);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -36,3 +36,25 @@ def test_forward_at_tile_edges(N, D, dtype):
                     scores = scores.masked_fill(torch.ones(N, N, dtype=torch.bool).triu(1), float("-inf"))
                 want = torch.logsumexp(scores, -1) / torch.tensor(2.0).double().log()
                 assert (lse.cpu().double() - want).abs().max() <= 1e-3
+
+
+@pytest.mark.parametrize("N", [64, 65, 127, 129, 300])
+def test_fp32_forward_posts_its_status_word(N):
+    """The word comes from the last block of the kernel itself, also on a workspace of an earlier call."""
+    for seed in range(3):
+        q, k, v, do = oracle.make_inputs(2, 3, N, 64, seed=seed, dtype=torch.float32)
+        ref = oracle.torch_forward_backward(q, k, v, do, True, True, dtype=torch.float32)[0]
+        out, _ = ops._forward(q.to("cuda"), k.to("cuda"), v.to("cuda"), True, True)
+        ops.check_device_status()
+        assert oracle.error_report(out.cpu(), ref)["rel_l2"] <= 6e-3
+
+
+@pytest.mark.parametrize("rows", [1, 63, 64, 65, 64 * 8 + 1, 64 * 13 + 5, 70000])
+def test_column_sums_over_few_and_many_bands(rows):
+    """One fp32 sum per column over the bands' partial sums: the second kernel starts while the first one runs."""
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, 264, generator=g).to(torch.bfloat16)
+    got = ops._column_sums(x.to("cuda")).cpu().double()
+    want = x.double().sum(0)
+    # sums of `rows` terms in any order: the error of an fp32 sum is at most its depth (well below 2^10) times 2^-24 of sum |x|
+    assert ((got - want).abs() <= 2.0 ** -14 * x.double().abs().sum(0)).all()
