@@ -128,6 +128,10 @@ int rbf_b200_bwd_posting(const void* q, const void* k, const void* v, const void
  * caller). Widening: dense fp16 tensors of n elements each, n a multiple of 8, into fp32. */
 int rbf_b200_narrow_f32(int count, const void* const* src, void* const* dst, const int64_t* strides, int B, int H, int N,
                         int D, int checked, unsigned int* flag, void* stream);
+/* The same, and the last block stores flag[0] to `status_slot` (an address that the device can write, NULL: not posted):
+   `flag` is two 32-bit words of device memory, cleared by the call. */
+int rbf_b200_narrow_f32_posting(int count, const void* const* src, void* const* dst, const int64_t* strides, int B, int H,
+                                int N, int D, int checked, unsigned int* flag, void* stream, unsigned int* status_slot);
 int rbf_b200_widen_f16(int count, const void* const* src, void* const* dst, int64_t n, void* stream);
 
 /* Device-side address of `host_slots` (page-locked host memory mapped into the current device's address space). */

@@ -66,6 +66,11 @@ SIGNATURES = {
         [ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p), _c_i64p] + [ctypes.c_int] * 5
         + [ctypes.c_void_p, ctypes.c_void_p],
     ),
+    "rbf_b200_narrow_f32_posting": (
+        ctypes.c_int,
+        [ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p), _c_i64p] + [ctypes.c_int] * 5
+        + [ctypes.c_void_p] * 3,
+    ),
     "rbf_b200_widen_f16": (
         ctypes.c_int,
         [ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p), ctypes.c_int64, ctypes.c_void_p],
@@ -139,6 +144,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 def load() -> ctypes.CDLL:
@@ -161,6 +167,22 @@ def load() -> ctypes.CDLL:
         raise RuntimeError(f"librbf_b200.so has ABI version {got}, this package expects {ABI_VERSION}")
     _lib = lib
     return lib
+
+
+def host():
+    """The extension that takes tensors (csrc/host.cpp). Raises if it is not built."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as extension
+        except ImportError as e:
+            raise RuntimeError(
+                f"{os.path.join(os.path.dirname(LIB_PATH), '_host.so')} is missing or does not load ({e}): build it with "
+                "`python -m rbf_attention_b200.build` (this package has no fallback path)"
+            ) from e
+        _host = extension
+    return _host
 
 
 def strides3(t) -> ctypes.Array:

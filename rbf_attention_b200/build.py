@@ -1,4 +1,5 @@
-"""Builds librbf_b200.so in-tree with nvcc for sm_100a (no torch headers, no libcuda link dependency).
+"""Builds librbf_b200.so in-tree with nvcc for sm_100a (no torch headers, no libcuda link dependency) and _host.so, the
+CPython extension on top of it that ops.py calls (torch headers).
 
 Usage: ``python -m rbf_attention_b200.build [--force] [--verbose]``.
 """
@@ -8,11 +9,14 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "librbf_b200.so")
+HOST = os.path.join(HERE, "_host.so")
+HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 SOURCES = ["capi.cu", "rbf_prep.cu", "rbf_fwd.cu", "rbf_fwd_tf32.cu", "rbf_bwd.cu", "rbf_bwd_fused.cu",
            "rbf_bwd_fused128.cu", "ce_loss.cu", "layer_norm.cu", "col_sums.cu", "gelu.cu", "narrow.cu"]
 NVCC_FLAGS = [
@@ -40,8 +44,23 @@ def _stale(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _host_command() -> list[str]:
+    """g++ on host.cpp against the installed torch, linked to the library beside it."""
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include"), sysconfig.get_paths()["include"]]
+    # the compiler that nvcc takes for host code: one with a C++ runtime of its own does not mix with torch's libraries
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in includes), HOST_SOURCE,
+            "-o", HOST, f"-L{os.path.join(root, 'lib')}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10",
+            "-lc10_cuda", f"-L{HERE}", "-l:librbf_b200.so", "-Wl,-rpath,$ORIGIN"]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compiles every translation unit to an object and links the shared library. Returns its path."""
+    """Compiles every translation unit to an object, links the shared library and builds the extension. Returns the
+    library's path."""
     deps = _deps()
     objs = []
     jobs = []
@@ -59,12 +78,14 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if verbose or r.returncode != 0:
             sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
         if r.returncode != 0:
-            raise RuntimeError(f"nvcc failed for {cmd[-3]}")
+            raise RuntimeError(f"build failed: {' '.join(cmd)}")
 
     with ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
         list(pool.map(run, jobs))
     if jobs or force or _stale(LIB, objs):
         run([_nvcc(), "-shared", "-o", LIB, *objs, "-lcudart"])
+    if force or _stale(HOST, [HOST_SOURCE, *_deps()[-1:]]):
+        run(_host_command())
     return LIB
 
 

@@ -818,7 +818,13 @@ int rbf_b200_scale_unless_one(void* x, const float* factor, int64_t n, int dtype
 
 int rbf_b200_narrow_f32(int count, const void* const* src, void* const* dst, const int64_t* strides, int B, int H, int N,
                         int D, int checked, unsigned int* flag, void* stream_v) {
+  return rbf_b200_narrow_f32_posting(count, src, dst, strides, B, H, N, D, checked, flag, stream_v, nullptr);
+}
+
+int rbf_b200_narrow_f32_posting(int count, const void* const* src, void* const* dst, const int64_t* strides, int B, int H,
+                                int N, int D, int checked, unsigned int* flag, void* stream_v, unsigned int* status_slot) {
   g_last_error[0] = 0;
+  if (status_slot != nullptr && flag == nullptr) return fail(RBF_B200_ERR_BAD_ARGUMENT, "nothing to post: flag is NULL");
   if (count <= 0 || count > rbf::kMaxNarrow || checked < 0 || checked > count)
     return fail(RBF_B200_ERR_BAD_ARGUMENT, "1 to %d tensors, of which at most that many are checked", rbf::kMaxNarrow);
   if (B <= 0 || H <= 0 || N <= 0 || D <= 0 || D % 8 != 0)
@@ -841,8 +847,10 @@ int rbf_b200_narrow_f32(int count, const void* const* src, void* const* dst, con
   }
   a.chunks = static_cast<int64_t>(B) * H * N * (D / 8);
   if ((a.chunks + 255) / 256 > 0x7fffffffll) return fail(RBF_B200_ERR_BAD_ARGUMENT, "the tensors are too large");
-  a.H = H; a.N = N; a.D = D; a.count = count; a.checked = checked; a.flag = flag;
-  const cudaError_t e = rbf::launch_narrow(a, static_cast<cudaStream_t>(stream_v));
+  a.H = H; a.N = N; a.D = D; a.count = count; a.checked = checked; a.flag = flag; a.status_slot = status_slot;
+  cudaError_t e = cudaSuccess;
+  if (status_slot != nullptr) e = cudaMemsetAsync(flag, 0, 2 * sizeof(unsigned int), static_cast<cudaStream_t>(stream_v));
+  if (e == cudaSuccess) e = rbf::launch_narrow(a, static_cast<cudaStream_t>(stream_v));
   if (e != cudaSuccess) return fail(RBF_B200_ERR_LAUNCH, "narrowing launch failed: %s", cudaGetErrorString(e));
   return RBF_B200_OK;
 }

@@ -140,6 +140,7 @@ struct NarrowArgs {
   int64_t chunks;            // B * H * N * D / 8
   int H, N, D, count, checked;
   unsigned int* flag;
+  unsigned int* status_slot;   // optional: flag[0] goes here from the last block; flag[1] counts the blocks that have left
 };
 struct WidenArgs {
   const void* src[kMaxNarrow];

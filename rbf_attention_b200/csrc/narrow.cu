@@ -31,6 +31,13 @@ __global__ void __launch_bounds__(256) narrow_kernel(const NarrowArgs a) {
     for (int j = 0; j < 4; ++j) bad |= (w[j] & 0x7fffu) == 0x7c00u || (w[j] & 0x7fff0000u) == 0x7c000000u;   // an infinity
   }
   if (t < a.checked && __any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) *a.flag = 1u;
+  if (a.status_slot == nullptr) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&a.flag[1], 1u) == gridDim.x * gridDim.y - 1) {
+    __threadfence();
+    post_status_word(reinterpret_cast<const DeviceStatus*>(a.flag), a.status_slot);
+  }
 }
 
 __global__ void __launch_bounds__(256) widen_kernel(const WidenArgs a) {

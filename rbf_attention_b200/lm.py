@@ -10,6 +10,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import ops
 from .attention import CustomCausalAttention
 
 
@@ -39,10 +40,9 @@ def apply_layer_norm(ln: nn.LayerNorm, x: torch.Tensor) -> torch.Tensor:
     (``ops.layer_norm``, a warp per row; PyTorch's kernels reach a sixth of the memory bandwidth at 512 columns),
     anything else through PyTorch."""
     if x.is_cuda and len(ln.normalized_shape) == 1 and ln.elementwise_affine:
-        from . import ops
-
-        if ops.layer_norm_supported(x, ln.weight, ln.bias):
-            return ops.layer_norm(x, ln.weight, ln.bias, ln.eps)
+        weight, bias = ln.weight, ln.bias           # once: a module's parameters are found through __getattr__
+        if ops.layer_norm_supported(x, weight, bias):
+            return ops.layer_norm(x, weight, bias, ln.eps)
     return ln(x)
 
 
@@ -53,10 +53,9 @@ def apply_add_layer_norm(ln: nn.LayerNorm, x: torch.Tensor, delta):
         return x, apply_layer_norm(ln, x)
     if x.is_cuda and len(ln.normalized_shape) == 1 and ln.elementwise_affine and delta.shape == x.shape \
             and delta.dtype == x.dtype:
-        from . import ops
-
-        if ops.layer_norm_supported(x, ln.weight, ln.bias):
-            return ops.add_layer_norm(x, delta, ln.weight, ln.bias, ln.eps)
+        weight, bias = ln.weight, ln.bias
+        if ops.layer_norm_supported(x, weight, bias):
+            return ops.add_layer_norm(x, delta, weight, bias, ln.eps)
     x = x + delta
     return x, ln(x)
 
@@ -69,8 +68,6 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int
     logits = logits.reshape(-1, logits.shape[-1])
     targets = targets.reshape(-1)
     if logits.is_cuda:
-        from . import ops
-
         return ops.cross_entropy(logits, targets, ignore_index)
     return F.cross_entropy(logits, targets, ignore_index=ignore_index)
 
@@ -106,11 +103,10 @@ class TransformerBlock(nn.Module):
         """``self.ff(x)`` (Linear, GELU, Linear) with the activation, its backward and the bias gradients of both
         projections from the library."""
         if x.is_cuda:
-            from . import ops
-
-            exact_gelu = isinstance(self.ff[1], nn.GELU) and self.ff[1].approximate == "none"
-            hidden = ops.linear_gelu(self.ff[0], x) if exact_gelu else self.ff[1](ops.linear(self.ff[0], x))
-            return ops.linear(self.ff[2], hidden)
+            up, act, down = self.ff[0], self.ff[1], self.ff[2]
+            exact_gelu = isinstance(act, nn.GELU) and act.approximate == "none"
+            hidden = ops.linear_gelu(up, x) if exact_gelu else act(ops.linear(up, x))
+            return ops.linear(down, hidden)
         return self.ff(x)
 
 

@@ -11,7 +11,6 @@ from __future__ import annotations
 
 import collections
 import ctypes
-import functools
 import math
 import os
 import threading
@@ -23,8 +22,6 @@ from torch.autograd import forward_ad
 from . import _lib
 
 _DTYPE_CODE = {torch.bfloat16: 0, torch.float16: 1}
-_F32_CODE = 2          # forward only: fp32 tensors on TF32 operands, head dim 64
-
 
 _PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
 
@@ -106,40 +103,16 @@ def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     return t if ok else t.contiguous()
 
 
-def _compute_dtype(q: torch.Tensor) -> torch.dtype:
-    if q.dtype in _DTYPE_CODE:
-        return q.dtype
-    if q.dtype == torch.float32:
-        # fp32 inputs: the forward at head dims up to 64 runs on TF32 operands (see _forward); everything else - the
-        # backward, head dims above 64 - runs with fp16 tensor-core operands (11-bit significand, like the TF32 the
-        # reference's Triton path uses for them, rbf_attention.py:183) and fp32 accumulation. There fp16's range
-        # limit applies: |x| must stay below 65504, which attention activations do by orders of magnitude.
-        return torch.float16
-    raise ValueError(f"unsupported dtype {q.dtype} (bfloat16, float16 or float32)")
-
-
 def _padded_head_dim(D: int) -> int:
     """Head dim the kernels run at: 64 or 128. Other head dims up to 128 run zero-padded to the next of the two, which
     is exact: zero columns add nothing to q.k, to |k|^2 or to |q|^2, and zero value columns give zero output columns
     (the reference pads to the next power of two inside its kernels, rbf_attention.py:661). The softmax scale keeps
-    using the caller's D. Multiples of 8 in 16-bit types are padded by the kernels' own loads (``_columns``)."""
+    using the caller's D. Multiples of 8 in 16-bit types are padded by the kernels' own loads."""
     if D <= 64:
         return 64
     if D <= 128:
         return 128
     raise ValueError(f"head dim {D} is not supported (at most 128)")
-
-
-def _columns(D: int, dtype: torch.dtype) -> int:
-    """Columns the tensors of a call get: their own where the kernels' loads can pad them (16-bit rows of a multiple of 16
-    bytes), else those the kernels run at. At head dim 80 (B2 H12 N1500, fp16) padding and slicing with separate passes
-    were 20 of the 28 launches and half the device time of a training pass."""
-    return D if dtype != torch.float32 and D % 8 == 0 else _padded_head_dim(D)
-
-
-def _pad_d(t: torch.Tensor, Dp: int) -> torch.Tensor:
-    D = t.shape[-1]
-    return t if D == Dp else torch.nn.functional.pad(t, (0, Dp - D))
 
 
 def _device_index(device: torch.device) -> int:
@@ -172,22 +145,6 @@ class _OnDevice:
         if self.prev >= 0:
             torch._C._cuda_setDevice(self.prev)
         return False
-
-
-@functools.lru_cache(maxsize=256)
-def _workspace_bytes(B, H, N, D, softmax, backward) -> int:
-    return _lib.load().rbf_b200_workspace_bytes(B, H, N, D, int(softmax), int(backward))
-
-
-@functools.lru_cache(maxsize=256)
-def _dense_strides3(H, N, D) -> ctypes.Array:
-    return _lib.I64x3(H * N * D, N * D, D)
-
-
-def _workspace(B, H, N, D, softmax, backward, device) -> torch.Tensor:
-    nbytes = _workspace_bytes(B, H, N, D, bool(softmax), backward)
-    # torch's caching allocator returns 512-byte aligned blocks, which satisfies the 256-byte rule
-    return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
 # States of a status entry: its slot is taken but its call has not returned yet; the call's kernels are enqueued and will
@@ -369,79 +326,39 @@ def _narrow(tensors, checked: int, mon, what: str):
     """fp32 (B, H, N, D) tensors as fp16 operands, in one launch that also looks whether one of the first ``checked``
     leaves fp16's range (reported like a status word: by a later call). What the kernel's 16-byte loads cannot take goes
     through PyTorch's conversion."""
-    B, H, N, D = tensors[0].shape
-    ok = D % 8 == 0 and D > 0 and all(
-        t.dtype == torch.float32 and t.shape == tensors[0].shape and t.device == tensors[0].device and t.stride(3) == 1 and t.data_ptr() % 16 == 0 and all(e <= 1 or st % 4 == 0 for e, st in zip((B, H, N), t.stride()))
-        for t in tensors)
-    if not ok:
+    prepared = _lib.host().narrow_f32(tensors, checked)
+    if prepared is None:
         halves = [t.to(torch.float16) for t in tensors]
         mon.record_range_check(halves[:checked], what)
         return halves
-    n = len(tensors)
-    dev = tensors[0].device
-    halves = [torch.empty((B, H, N, D), dtype=torch.float16, device=dev) for _ in tensors]
-    flag = torch.zeros(4, dtype=torch.uint8, device=dev)
-    pointers, strides = ctypes.c_void_p * n, (ctypes.c_int64 * (3 * n))(*(st for t in tensors for st in t.stride()[:3]))
-    with _OnDevice(dev):
-        rc = _lib.load().rbf_b200_narrow_f32(n, pointers(*(t.data_ptr() for t in tensors)),
-                                             pointers(*(t.data_ptr() for t in halves)), strides, B, H, N, D, checked,
-                                             flag.data_ptr(), _stream_ptr(dev))
-        _lib.check(rc, "rbf_b200_narrow_f32")
-        mon.record(flag, "range:" + what)
+    enqueue, halves = prepared
+    mon.launch("range:" + what, enqueue)
     return halves
 
 
 def _widen(tensors):
     """Dense fp16 tensors of one shape as fp32, in one launch."""
-    count = tensors[0].numel()
-    if count % 8 != 0:
-        return [t.float() for t in tensors]
-    out = [torch.empty(t.shape, dtype=torch.float32, device=t.device) for t in tensors]
-    pointers = ctypes.c_void_p * len(out)
-    with _OnDevice(out[0].device):
-        rc = _lib.load().rbf_b200_widen_f16(len(out), pointers(*(t.data_ptr() for t in tensors)),
-                                            pointers(*(t.data_ptr() for t in out)), count, _stream_ptr(out[0].device))
-    _lib.check(rc, "rbf_b200_widen_f16")
-    return out
+    return _lib.host().widen_f16(tensors)
 
 
-_PHASE_ALL = 7          # pre-pass and both main kernels (include/rbf_b200.h)
-
-
-def _strides3(t: torch.Tensor, dense) -> ctypes.Array:
-    return dense if t.is_contiguous() else _lib.strides3(t)
+def _first_columns(t: torch.Tensor, D: int) -> torch.Tensor:
+    return t if t.shape[-1] == D else t[..., :D].contiguous()
 
 
 def _forward(q, k, v, is_causal: bool, softmax: bool):
     _validate("q", q)
-    _validate("k", k, q)
-    _validate("v", v, q)
-    B, H, N, D0 = q.shape
-    D = _padded_head_dim(D0)
-    lib = _lib.load()
-    # fp32 tensors at head dim <= 64: TF32 operands, as the reference's Triton path uses for them (fp32's exponent range)
-    tf32 = q.dtype == torch.float32 and D == 64
-    cdt = torch.float32 if tf32 else _compute_dtype(q)
-    code = _F32_CODE if tf32 else _DTYPE_CODE[cdt]
-    Dc = _columns(D0, cdt)
+    D = q.shape[3]
     mon = _monitor(q.device)
     mon.poll()
-    narrowed = q.dtype == torch.float32 and not tf32
-    ins = _narrow((q, k, v), 3, mon, "rbf_b200_fwd") if narrowed else (q, k, v)
-    qc, kc, vc = (_tma_ready(_pad_d(t, Dc)) for t in ins)
-    out = torch.empty((B, H, N, Dc), dtype=cdt, device=q.device)
-    lse = torch.empty((B, H, N), dtype=torch.float32, device=q.device) if softmax else None
-    ws = _workspace(B, H, N, D, softmax, False, q.device)
-    dense = _dense_strides3(H, N, Dc)
-    with _OnDevice(q.device):
-        mon.launch("rbf_b200_fwd", lambda slot: lib.rbf_b200_fwd_posting(
-            qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(),
-            lse.data_ptr() if softmax else None, ws.data_ptr(), ws.numel(),
-            B, H, N, Dc, _strides3(qc, dense), _strides3(kc, dense), _strides3(vc, dense), dense,
-            code, int(bool(is_causal)), int(softmax), 1.0 / math.sqrt(D0), _stream_ptr(q.device), _PHASE_ALL, slot,
-        ))
-    if Dc != D0:
-        out = out[..., :D0].contiguous()
+    # fp32 tensors at head dim <= 64: TF32 operands, as the reference's Triton path uses for them (fp32's exponent range)
+    narrowed = q.dtype == torch.float32 and _padded_head_dim(D) != 64
+    if narrowed:
+        _validate("k", k, q)
+        _validate("v", v, q)
+        q, k, v = _narrow((q, k, v), 3, mon, "rbf_b200_fwd")
+    enqueue, out, lse = _lib.host().attention_fwd(q, k, v, is_causal, softmax)
+    mon.launch("rbf_b200_fwd", enqueue)
+    out = _first_columns(out, D)
     if narrowed:
         (out,) = _widen([out])
     return out, lse
@@ -449,48 +366,22 @@ def _forward(q, k, v, is_causal: bool, softmax: bool):
 
 def _backward(q, k, v, out, lse, dout, is_causal: bool, sm_scale: float, softmax: bool):
     _validate("q", q)
-    _validate("k", k, q)
-    _validate("v", v, q)
-    _validate("dout", dout, q)
-    B, H, N, D0 = q.shape
-    D = _padded_head_dim(D0)
-    lib = _lib.load()
-    cdt = _compute_dtype(q)
-    Dc = _columns(D0, cdt)
+    D = q.shape[3]
     mon = _monitor(q.device)
     mon.poll()
     # the non-softmax variant takes the forward output when the caller has it: the single-kernel backward needs it
-    have_out = out is not None
-    ins = (q, k, v, dout, out) if have_out else (q, k, v, dout)
-    if cdt != q.dtype:
-        ins = _narrow(ins, 4, mon, "rbf_b200_bwd")
-    elif have_out and out.dtype != cdt:
-        ins = (q, k, v, dout, out.to(cdt))
-    qc, kc, vc, doc, *oc = (_tma_ready(_pad_d(t, Dc)) for t in ins)
-    oc = oc[0] if have_out else None
-    dq = torch.empty((B, H, N, Dc), dtype=cdt, device=q.device)
-    dk = torch.empty_like(dq)
-    dv = torch.empty_like(dq)
-    ws = _workspace(B, H, N, D, softmax, True, q.device)
-    z3 = _lib.I64x3(0, 0, 0)
-    # torch.use_deterministic_algorithms(True) selects the backward whose summation order is fixed
-    lib.rbf_b200_set_deterministic(int(torch.are_deterministic_algorithms_enabled()))
-    dense = _dense_strides3(H, N, Dc)
-    with _OnDevice(q.device):
-        mon.launch("rbf_b200_bwd", lambda slot: lib.rbf_b200_bwd_posting(
-            qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
-            oc.data_ptr() if have_out else None, lse.data_ptr() if softmax else None, doc.data_ptr(),
-            dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(),
-            B, H, N, Dc, _strides3(qc, dense), _strides3(kc, dense), _strides3(vc, dense),
-            _strides3(oc, dense) if have_out else z3, _strides3(doc, dense),
-            dense, dense, dense,
-            _DTYPE_CODE[cdt], int(bool(is_causal)), int(softmax), float(sm_scale), _stream_ptr(q.device), _PHASE_ALL, slot,
-        ))
-    if Dc != D0:
-        dq, dk, dv = (t[..., :D0].contiguous() for t in (dq, dk, dv))
-    if cdt != q.dtype:
-        dq, dk, dv = _widen([dq, dk, dv])
-    return dq, dk, dv
+    narrowed = q.dtype == torch.float32
+    if narrowed:
+        _padded_head_dim(D)
+        _validate("k", k, q)
+        _validate("v", v, q)
+        _validate("dout", dout, q)
+        q, k, v, dout, *rest = _narrow((q, k, v, dout) if out is None else (q, k, v, dout, out), 4, mon, "rbf_b200_bwd")
+        out = rest[0] if rest else None
+    enqueue, *grads = _lib.host().attention_bwd(q, k, v, out, lse, dout, is_causal, sm_scale, softmax)
+    mon.launch("rbf_b200_bwd", enqueue)
+    grads = [_first_columns(g, D) for g in grads]
+    return tuple(_widen(grads) if narrowed else grads)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -641,11 +532,6 @@ torch.library.register_autograd(
 # "rbf_non_softmax" attention types with SuSiE positions, the torch ops of rbf_attention.py:1659-1688 and :1761
 # (split, broadcast adds, concatenation, transpose copy) and their autograd.
 # ---------------------------------------------------------------------------------------------
-def _bhsd_view(t: torch.Tensor) -> torch.Tensor:
-    """(B, S, H, D) memory seen as (B, H, S, D), no copy."""
-    return t.permute(0, 2, 1, 3)
-
-
 def _susie_block_fwd(
     qkv: torch.Tensor,
     pos_weight: torch.Tensor,
@@ -656,49 +542,10 @@ def _susie_block_fwd(
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """qkv (B, S, 3 H D), pos_weight (H, D/2), reg_pos_emb (H, R, D) or None, table (>= S - R, D) ->
     (out (B, S, H D), L (B, H, S) fp32 [empty when softmax is False], qk (2, B, S, H, D) = the prepared q', k')."""
-    if not qkv.is_cuda:
-        raise RuntimeError("qkv must be a CUDA tensor: rbf_attention_b200 has no CPU path")
-    if qkv.dtype not in _DTYPE_CODE:
-        raise ValueError(f"unsupported dtype {qkv.dtype} (bfloat16 or float16)")
-    B, S, E3 = qkv.shape
-    E = E3 // 3
-    H = num_heads
-    D = E // H
-    R = 0 if reg_pos_emb is None else reg_pos_emb.shape[-2]
-    if D not in (64, 128):
-        raise ValueError(f"head dim {D} is not supported (64 or 128)")
-    lib = _lib.load()
-    dev = qkv.device
-    qkv = qkv.contiguous()
-    params_fp32 = pos_weight.dtype == torch.float32
-    if not params_fp32 and pos_weight.dtype != qkv.dtype:
-        raise ValueError("pos_weight must be float32 or have the dtype of qkv")
-    pw = pos_weight.contiguous()
-    rp = None if R == 0 else reg_pos_emb.to(pw.dtype).contiguous()
-    table = table.to(device=dev, dtype=torch.float32).contiguous()
-    if table.shape[0] < S - R:
-        raise ValueError(f"the position table holds {table.shape[0]} rows, {S - R} text positions are needed")
-    qk = torch.empty((2, B, S, H, D), dtype=qkv.dtype, device=dev)
-    out = torch.empty((B, S, E), dtype=qkv.dtype, device=dev)
-    lse = torch.empty((B, H, S) if softmax else (0,), dtype=torch.float32, device=dev)
-    q, k = _bhsd_view(qk[0]), _bhsd_view(qk[1])
-    v = _bhsd_view(qkv.view(B, S, 3, H, D)[:, :, 2])
-    o = _bhsd_view(out.view(B, S, H, D))
-    ws = _workspace(B, H, S, D, softmax, False, dev)
-    scale = 1.0 / math.sqrt(D)
-    mon = _monitor(dev)
+    enqueue, out, lse, qk = _lib.host().block_fwd(qkv, pos_weight, reg_pos_emb, table, num_heads, softmax)
+    mon = _monitor(out.device)
     mon.poll()
-    with _OnDevice(dev):
-        stream = _stream_ptr(dev)
-        rc = lib.rbf_b200_qkv_prep(
-            qkv.data_ptr(), pw.data_ptr(), None if rp is None else rp.data_ptr(), int(params_fp32), table.data_ptr(),
-            q.data_ptr(), k.data_ptr(), _lib.strides3(q), _lib.strides3(k), ws.data_ptr(), ws.numel(),
-            B, S, H, D, R, _DTYPE_CODE[qkv.dtype], int(softmax), scale, stream)
-        _lib.check(rc, "rbf_b200_qkv_prep")
-        mon.launch("rbf_b200_fwd (attention block)", lambda slot: lib.rbf_b200_fwd_posting(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr() if softmax else None,
-            ws.data_ptr(), ws.numel(), B, H, S, D, _lib.strides3(q), _lib.strides3(k), _lib.strides3(v),
-            _lib.strides3(o), _DTYPE_CODE[qkv.dtype], 1, int(softmax), scale, stream, 2, slot))
+    mon.launch("rbf_b200_fwd (attention block)", enqueue)
     return out, lse, qk
 
 
@@ -728,42 +575,11 @@ def _susie_block_bwd(
     softmax: bool,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """-> (dqkv (B, S, 3 H D), d_pos_weight (H, D/2) fp32, d_reg_pos_emb (H, R, D) fp32)."""
-    _, B, S, H, D = qk.shape
-    E = H * D
-    R = num_registers
-    lib = _lib.load()
-    dev = qkv.device
-    dt = _DTYPE_CODE[qkv.dtype]
-    qkv = qkv.contiguous()
-    dout = dout.to(qkv.dtype).contiguous()
-    table = table.to(device=dev, dtype=torch.float32).contiguous()
-    q, k = _bhsd_view(qk[0]), _bhsd_view(qk[1])
-    v = _bhsd_view(qkv.view(B, S, 3, H, D)[:, :, 2])
-    o = _bhsd_view(out.view(B, S, H, D))
-    do = _bhsd_view(dout.view(B, S, H, D))
-    dqkv = torch.empty((B, S, 3, H, D), dtype=qkv.dtype, device=dev)
-    dq, dk, dv = (_bhsd_view(dqkv[:, :, i]) for i in range(3))
-    d_pw = torch.empty((H, D // 2), dtype=torch.float32, device=dev)
-    d_rp = torch.empty((H, R, D), dtype=torch.float32, device=dev)
-    ws = _workspace(B, H, S, D, softmax, True, dev)
-    nb2 = lib.rbf_b200_qkv_prep_bwd_workspace_bytes(B, S, H, D, R)
-    ws2 = torch.empty(nb2, dtype=torch.uint8, device=dev)
-    mon = _monitor(dev)
+    enqueue, dqkv, d_pw, d_rp = _lib.host().block_bwd(qkv, qk, out, lse, dout, table, num_registers, softmax)
+    mon = _monitor(qkv.device)
     mon.poll()
-    lib.rbf_b200_set_deterministic(int(torch.are_deterministic_algorithms_enabled()))
-    with _OnDevice(dev):
-        stream = _stream_ptr(dev)
-        mon.launch("rbf_b200_bwd (attention block)", lambda slot: lib.rbf_b200_bwd_posting(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr() if softmax else None,
-            do.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(), B, H, S, D,
-            _lib.strides3(q), _lib.strides3(k), _lib.strides3(v), _lib.strides3(o), _lib.strides3(do),
-            _lib.strides3(dq), _lib.strides3(dk), _lib.strides3(dv), dt, 1, int(softmax), 1.0 / math.sqrt(D), stream,
-            _PHASE_ALL, slot))
-        rc = lib.rbf_b200_qkv_prep_bwd(
-            dq.data_ptr(), dk.data_ptr(), _lib.strides3(dq), _lib.strides3(dk), table.data_ptr(), d_pw.data_ptr(),
-            d_rp.data_ptr() if R > 0 else None, ws2.data_ptr(), nb2, B, S, H, D, R, dt, stream)
-        _lib.check(rc, "rbf_b200_qkv_prep_bwd")
-    return dqkv.view(B, S, 3 * E), d_pw, d_rp
+    mon.launch("rbf_b200_bwd (attention block)", enqueue)
+    return dqkv, d_pw, d_rp
 
 
 susie_block_bwd = torch.library.custom_op("rbf_attn_b200::susie_block_bwd", mutates_args=())(_susie_block_bwd)
@@ -901,20 +717,7 @@ def exclusive_self_attention(o, v):
 # ---------------------------------------------------------------------------------------------
 def _column_sums(x: torch.Tensor) -> torch.Tensor:
     """fp32 sums over the rows of a 16-bit CUDA matrix (rows, cols), cols a multiple of 8."""
-    if x.dim() != 2 or not x.is_cuda or x.dtype not in _DTYPE_CODE or x.shape[1] % 8 != 0:
-        raise ValueError("column_sums: a 16-bit CUDA matrix whose width is a multiple of 8")
-    ok = x.stride(1) == 1 and x.stride(0) >= x.shape[1] and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
-    xc = x if ok else x.contiguous()
-    rows, cols = xc.shape
-    lib = _lib.load()
-    out = torch.empty(cols, dtype=torch.float32, device=x.device)
-    with _OnDevice(x.device):
-        nbytes = lib.rbf_b200_column_sums_workspace_bytes(rows, cols)
-        ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
-        rc = lib.rbf_b200_column_sums(xc.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), rows, cols,
-                                      xc.stride(0) if rows > 1 else cols, _DTYPE_CODE[x.dtype], _stream_ptr(x.device))
-    _lib.check(rc, "rbf_b200_column_sums")
-    return out
+    return _lib.host().column_sums(x)
 
 
 column_sums = torch.library.custom_op("rbf_attn_b200::column_sums", mutates_args=())(_column_sums)
@@ -950,15 +753,7 @@ class _LinearBiasSum(torch.autograd.Function):
 
 def _gelu_fwd(h: torch.Tensor) -> torch.Tensor:
     """Exact (erf) GELU of a 16-bit CUDA tensor whose element count is a multiple of 8."""
-    if not h.is_cuda or h.dtype not in _DTYPE_CODE or h.numel() % 8 != 0:
-        raise ValueError("gelu_fwd: a 16-bit CUDA tensor with a multiple of 8 elements")
-    hc = h.contiguous()
-    out = torch.empty_like(hc)
-    with _OnDevice(h.device):
-        rc = _lib.load().rbf_b200_gelu_fwd(hc.data_ptr(), out.data_ptr(), hc.numel(), _DTYPE_CODE[h.dtype],
-                                           _stream_ptr(h.device))
-    _lib.check(rc, "rbf_b200_gelu_fwd")
-    return out
+    return _lib.host().gelu_fwd(h)
 
 
 gelu_fwd = torch.library.custom_op("rbf_attn_b200::gelu_fwd", mutates_args=())(_gelu_fwd)
@@ -971,19 +766,7 @@ def _(h):
 
 def _gelu_bwd(h: torch.Tensor, dy: torch.Tensor, with_bias: bool) -> tuple[torch.Tensor, torch.Tensor]:
     """dh = dy * gelu'(h) for (..., cols) tensors and, with ``with_bias``, its fp32 sum over all leading dims."""
-    cols = h.shape[-1]
-    hc, gc = h.contiguous(), dy.to(h.dtype).contiguous()
-    rows = hc.numel() // cols
-    lib = _lib.load()
-    dh = torch.empty_like(hc)
-    dbias = torch.empty(cols if with_bias else 0, dtype=torch.float32, device=h.device)
-    with _OnDevice(h.device):
-        nbytes = lib.rbf_b200_column_sums_workspace_bytes(rows, cols) if with_bias else 0
-        ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=h.device)
-        rc = lib.rbf_b200_gelu_bwd(hc.data_ptr(), gc.data_ptr(), dh.data_ptr(), dbias.data_ptr() if with_bias else None,
-                                   ws.data_ptr(), ws.numel(), rows, cols, _DTYPE_CODE[h.dtype], _stream_ptr(h.device))
-    _lib.check(rc, "rbf_b200_gelu_bwd")
-    return dh, dbias
+    return _lib.host().gelu_bwd(h, dy, with_bias)
 
 
 gelu_bwd = torch.library.custom_op("rbf_attn_b200::gelu_bwd", mutates_args=())(_gelu_bwd)
@@ -1023,18 +806,22 @@ class _LinearGelu(torch.autograd.Function):
 def linear_gelu(module: torch.nn.Linear, x: torch.Tensor) -> torch.Tensor:
     """``F.gelu(module(x))`` (exact form) on the library's kernels for 16-bit CUDA activations; anything else through
     PyTorch."""
-    if (x.is_cuda and x.dtype in _DTYPE_CODE and module.bias is not None and module.weight.dtype == x.dtype
-            and module.out_features % 8 == 0):
-        return _LinearGelu.apply(x, module.weight, module.bias)
+    if x.is_cuda and x.dtype in _DTYPE_CODE:
+        weight, bias = module.weight, module.bias
+        if bias is not None and weight.dtype == x.dtype and module.out_features % 8 == 0:
+            if _direct(x) and not _needs_grad(x, weight, bias):
+                return _gelu_fwd(torch.nn.functional.linear(x, weight, bias))
+            return _LinearGelu.apply(x, weight, bias)
     return torch.nn.functional.gelu(module(x))
 
 
 def linear(module: torch.nn.Linear, x: torch.Tensor) -> torch.Tensor:
     """``module(x)``; for 16-bit CUDA activations and a bias, the bias gradient comes from the library's column-sum
     kernel instead of PyTorch's generic reduction."""
-    if (x.is_cuda and x.dtype in _DTYPE_CODE and module.bias is not None and module.weight.dtype == x.dtype
-            and module.out_features % 8 == 0 and torch.is_grad_enabled() and module.bias.requires_grad):
-        return _LinearBiasSum.apply(x, module.weight, module.bias)
+    if torch.is_grad_enabled() and x.is_cuda and x.dtype in _DTYPE_CODE:
+        weight, bias = module.weight, module.bias
+        if bias is not None and weight.dtype == x.dtype and module.out_features % 8 == 0 and bias.requires_grad:
+            return _LinearBiasSum.apply(x, weight, bias)
     return module(x)
 
 
@@ -1051,21 +838,7 @@ def layer_norm_supported(x: torch.Tensor, weight, bias) -> bool:
 def _layer_norm_fwd(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
                    eps: float) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """y = (x - mean) * rstd * weight + bias over the last dim; returns (y, mean, rstd), the statistics in fp32."""
-    if not layer_norm_supported(x, weight, bias):
-        raise ValueError("layer_norm_fwd: 16-bit CUDA tensors with 256, 512, 768 or 1024 columns")
-    cols = x.shape[-1]
-    xc = x.contiguous()
-    rows = xc.numel() // cols
-    y = torch.empty_like(xc)
-    mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-    rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-    wc, bc = weight.contiguous(), bias.contiguous()
-    with _OnDevice(x.device):
-        rc = _lib.load().rbf_b200_layer_norm_fwd(xc.data_ptr(), wc.data_ptr(), bc.data_ptr(), y.data_ptr(),
-                                                 mean.data_ptr(), rstd.data_ptr(), rows, cols, float(eps),
-                                                 _DTYPE_CODE[x.dtype], _stream_ptr(x.device))
-    _lib.check(rc, "rbf_b200_layer_norm_fwd")
-    return y, mean, rstd
+    return _lib.host().layer_norm_fwd(x, None, weight, bias, eps)[1:]
 
 
 layer_norm_fwd = torch.library.custom_op("rbf_attn_b200::layer_norm_fwd", mutates_args=())(_layer_norm_fwd)
@@ -1080,21 +853,7 @@ def _(x, weight, bias, eps):
 
 def _layer_norm_bwd(x: torch.Tensor, dy: torch.Tensor, weight: torch.Tensor, mean: torch.Tensor,
                    rstd: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    cols = x.shape[-1]
-    xc, dyc, wc = x.contiguous(), dy.to(x.dtype).contiguous(), weight.contiguous()
-    rows = xc.numel() // cols
-    lib = _lib.load()
-    dx = torch.empty_like(xc)
-    dgamma = torch.empty(cols, dtype=torch.float32, device=x.device)
-    dbeta = torch.empty(cols, dtype=torch.float32, device=x.device)
-    with _OnDevice(x.device):
-        nbytes = lib.rbf_b200_layer_norm_bwd_workspace_bytes(rows, cols)
-        ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
-        rc = lib.rbf_b200_layer_norm_bwd(xc.data_ptr(), dyc.data_ptr(), wc.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
-                                         dx.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), ws.data_ptr(), ws.numel(),
-                                         rows, cols, _DTYPE_CODE[x.dtype], _stream_ptr(x.device))
-    _lib.check(rc, "rbf_b200_layer_norm_bwd")
-    return dx, dgamma.to(weight.dtype), dbeta.to(weight.dtype)
+    return _lib.host().layer_norm_bwd(x, dy, None, weight, mean, rstd)
 
 
 layer_norm_bwd = torch.library.custom_op("rbf_attn_b200::layer_norm_bwd", mutates_args=())(_layer_norm_bwd)
@@ -1151,24 +910,7 @@ def _add_layer_norm_fwd(x: torch.Tensor, residual: torch.Tensor, weight: torch.T
                        eps: float) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """s = x + residual (rounded to the dtype, as the separate addition leaves it) and y = LayerNorm(s) from one pass;
     returns (s, y, mean, rstd)."""
-    if not layer_norm_supported(x, weight, bias):
-        raise ValueError("add_layer_norm_fwd: 16-bit CUDA tensors with 256, 512, 768 or 1024 columns")
-    if residual.shape != x.shape or residual.dtype != x.dtype or residual.device != x.device:
-        raise ValueError(f"residual must have the shape, dtype and device of x: {tuple(residual.shape)} {residual.dtype} "
-                         f"against {tuple(x.shape)} {x.dtype}")
-    cols = x.shape[-1]
-    xc, rc_ = x.contiguous(), residual.contiguous()
-    rows = xc.numel() // cols
-    s, y = torch.empty_like(xc), torch.empty_like(xc)
-    mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-    rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-    wc, bc = weight.contiguous(), bias.contiguous()
-    with _OnDevice(x.device):
-        rc = _lib.load().rbf_b200_add_layer_norm_fwd(xc.data_ptr(), rc_.data_ptr(), s.data_ptr(), wc.data_ptr(),
-                                                     bc.data_ptr(), y.data_ptr(), mean.data_ptr(), rstd.data_ptr(), rows,
-                                                     cols, float(eps), _DTYPE_CODE[x.dtype], _stream_ptr(x.device))
-    _lib.check(rc, "rbf_b200_add_layer_norm_fwd")
-    return s, y, mean, rstd
+    return _lib.host().layer_norm_fwd(x, residual, weight, bias, eps)
 
 
 add_layer_norm_fwd = torch.library.custom_op("rbf_attn_b200::add_layer_norm_fwd", mutates_args=())(_add_layer_norm_fwd)
@@ -1186,25 +928,7 @@ def _layer_norm_bwd_add(x: torch.Tensor, dy: torch.Tensor, dres: torch.Tensor, w
                        rstd: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """The LayerNorm backward with ``dres`` (the gradient reaching x along the skip path) added to dx before the
     rounding: (dx, dgamma, dbeta)."""
-    cols = x.shape[-1]
-    xc, dyc, wc = x.contiguous(), dy.to(x.dtype).contiguous(), weight.contiguous()
-    drc = dres.to(x.dtype).contiguous()
-    if drc.shape != xc.shape:
-        raise ValueError(f"dres must have the shape of x: {tuple(dres.shape)} against {tuple(x.shape)}")
-    rows = xc.numel() // cols
-    lib = _lib.load()
-    dx = torch.empty_like(xc)
-    dgamma = torch.empty(cols, dtype=torch.float32, device=x.device)
-    dbeta = torch.empty(cols, dtype=torch.float32, device=x.device)
-    with _OnDevice(x.device):
-        nbytes = lib.rbf_b200_layer_norm_bwd_workspace_bytes(rows, cols)
-        ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
-        rc = lib.rbf_b200_layer_norm_bwd_add(xc.data_ptr(), dyc.data_ptr(), drc.data_ptr(), wc.data_ptr(), mean.data_ptr(),
-                                             rstd.data_ptr(), dx.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(),
-                                             ws.data_ptr(), ws.numel(), rows, cols, _DTYPE_CODE[x.dtype],
-                                             _stream_ptr(x.device))
-    _lib.check(rc, "rbf_b200_layer_norm_bwd_add")
-    return dx, dgamma.to(weight.dtype), dbeta.to(weight.dtype)
+    return _lib.host().layer_norm_bwd(x, dy, dres, weight, mean, rstd)
 
 
 layer_norm_bwd_add = torch.library.custom_op("rbf_attn_b200::layer_norm_bwd_add", mutates_args=())(_layer_norm_bwd_add)
