@@ -18,8 +18,8 @@
 //                    (TMEM x smem). One thread sustains one MMA per ~58 cycles, slower than the tensor pipe retires
 //                    the N = 64 products, hence two issuing threads.
 // TMEM columns: S_0, S_1 (one key tile wide each), O_0 and O_1 (D columns each), P_0 and P_1 (16-bit pairs, half a key
-// tile wide each): P_t has columns of its own and is consumed from there as the A operand of the second MMA, so the
-// next scores are issued as soon as the current ones are in registers. (P over the scores it was made from, with key tiles
+// tile wide each; two buffers each at D = 128): P_t has columns of its own and is consumed from there as the A operand of the
+// second MMA, so the next scores are issued as soon as the current ones are in registers. (P over the scores it was made from, with key tiles
 // of 128 at D = 128 too and the next scores issued right behind P V, is 14 % slower there: B2 H16 N4096 151 -> 173 us.)
 // Of a tile's exponentials every quarter is computed, packed and stored by itself (B2 H16 N3333 D128 full, against halves:
 // 229 -> 220 us).
@@ -43,7 +43,7 @@ namespace fwd {
 
 static constexpr float kRescaleThreshold = 8.0f;
 // Keys per streamed tile: 128 at D = 64; 64 at D = 128, where the narrower score tile leaves TMEM columns for P of
-// its own (2 x 64 S + 2 x 32 P + 2 x 128 O), so that the next scores run under the current tile's exponentials.
+// its own (2 x 64 S + 4 x 32 P + 2 x 128 O), so that the next scores run under the current tile's exponentials.
 template <int D>
 struct KeyTile {
   static constexpr int kKeys = (D == 64) ? 128 : 64;
@@ -162,10 +162,11 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   constexpr int kBoxes = D / 64;                 // 64-column TMA boxes per tile row
   constexpr int kBoxBytes = kTile * 128;         // one query / output box: 128 rows x 128 bytes
   constexpr int kKvBoxBytes = kKeys * 128;       // one key / value box
+  constexpr int kPCols = kKeys / 2;              // TMEM columns of a P tile
   constexpr uint32_t kTileBytes = L::kTileBytes;
   constexpr uint32_t kKvBytes = L::kKvBytes;
   constexpr int kSlabBytes = L::kSlabBytes;
-  // P has TMEM columns of its own (D = 64: 2 x 128 S + 2 x 64 O + 2 x 64 P; D = 128: 2 x 64 S + 2 x 32 P + 2 x 128 O):
+  // P has TMEM columns of its own (D = 64: 2 x 128 S + 2 x 64 O + 2 x 64 P; D = 128: 2 x 64 S + 4 x 32 P + 2 x 128 O):
   // S_t(j+1) is issued as soon as the softmax group holds S_t(j) in registers and runs under the exponentials.
 
   extern __shared__ uint8_t smem_raw[];
@@ -340,7 +341,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   }
   const uint32_t tmem_s[2] = {tmem, tmem + kKeys};
   const uint32_t tmem_o[2] = {tmem + 256, tmem + 256 + D};
-  const uint32_t tmem_p[2] = {D == 64 ? tmem + 384 : tmem + 128, D == 64 ? tmem + 448 : tmem + 160};
+  const uint32_t tmem_p[2] = {D == 64 ? tmem + 384 : tmem + 128, D == 64 ? tmem + 448 : tmem + 192};
 
   // Counters that run on across a CTA's items, kept identically by every role that needs them:
   //   G      K/V tiles put through the ring by earlier items (tile j of the item uses stage (G + j) % kStages in
@@ -435,13 +436,13 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           umma_ss(tmem_s[t], sdesc_at(ones_desc, 0), sdesc_at(slab, 0), idesc_s, 1u);   // + key-norm bias
         }
       };
-      auto issue_o = [&](int st, uint32_t accumulate) {
+      auto issue_o = [&](int st, uint32_t accumulate, uint32_t p) {
         SmemDesc v_desc = v_desc0;
         v_desc.lo += static_cast<uint32_t>(st) * (kKvBytes >> 4);
         if (el) {
 #pragma unroll
           for (int kk = 0; kk < kKeys / 16; ++kk)
-            umma_ts(tmem_o[t], tmem_p[t] + kk * 8, sdesc_at(v_desc, kk * 2048), idesc_o, kk > 0 ? 1u : accumulate);
+            umma_ts(tmem_o[t], p + kk * 8, sdesc_at(v_desc, kk * 2048), idesc_o, kk > 0 ? 1u : accumulate);
         }
       };
       auto wait_k = [&](uint32_t g) {
@@ -482,7 +483,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const int st = (G + j - 1) % kStages;
                 ok = wait_v(G + j - 1);
                 if (!ok) break;
-                issue_o(st, j > 1 ? 1u : 0u);
+                issue_o(st, j > 1 ? 1u : 0u, tmem_p[t]);
                 if (el) umma_commit(&v_empty[st]);
               }
               if (j + 1 < my_nkt) {
@@ -547,7 +548,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             ok = ok && mbar_wait_warp(&p_full[t], j & 1, abort_flag, status, kSitePFull, s_unit);
             if (!ok) break;
             tc_fence_after_sync();
-            issue_o(st, j > 0 ? 1u : 0u);
+            issue_o(st, j > 0 ? 1u : 0u, tmem_p[t] + (j & 1) * kPCols);
             if (el) {
               umma_commit(&o_done[t]);
               umma_commit(&v_empty[st]);
@@ -705,7 +706,9 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           out[i + 1] = pack2<kBf16>(p2, p3);
         }
       };
-      auto store_p = [&](int c) { tmem_st<kChunk / 2>(p_addr + c * (kChunk / 2), packed + c * (kChunk / 2)); };
+      auto store_p = [&](int c, uint32_t buffer = 0) {
+        tmem_st<kChunk / 2>(p_addr + buffer + c * (kChunk / 2), packed + c * (kChunk / 2));
+      };
       auto p_stored = [&]() {
         l_sum += (ps0 + ps1) + (ps2 + ps3);
         tmem_st_wait();
@@ -794,10 +797,10 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           ps0 = ps1 = ps2 = ps3 = 0.f;
 #pragma unroll
           for (int c = 0; c < 4; ++c) exponentials(c, neg_sub);
-          // P's own columns are free once O_t += P_t V_(j-1) has completed
-          if (j > 0 && !wait_o()) break;
+          // P's buffer is free: P_t(j-2) V went to the tensor core before the scores that have been waited for (with one
+          // buffer and a wait for P_t(j-1) V: B2 H16 N3333 full 220 us, now 213; B2 H12 N1500 D80 36.2, now 34.8)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) store_p(c);
+          for (int c = 0; c < 4; ++c) store_p(c, (j & 1) * kPCols);
           p_stored();
           tc_fence_before_sync();
           mbar_arrive_warp(&p_full[t]);
