@@ -19,7 +19,9 @@
 // reduce-adds into L2, measured; a step's 32 KB of dQ therefore takes as long as its MMAs and must overlap them.)
 //
 // TMEM columns: S^T [0,64), dP^T [64,128), P^T [128,160), dQ^T [160,224), dS^T [224,256), dV [256,384), dK [384,512).
-// Roles: warps 0, 1, 3 MMA issuers (A: S^T(n+1), dV(n); B: dP^T(n+1), dK(n); C: dQ^T(n)), warp 2 TMA producer,
+// Roles: warps 0, 1, 3 MMA issuers (A: S^T; B: dP^T(n), dV(n); C: dK(n), dQ^T(n), in an order in which three waits and two
+// arrivals of the compute warps per step are enough: five and four before, backward call at B2 H12 N1500 D80 83.0 -> 80.9 us,
+// level from N = 3333 on), warp 2 TMA producer,
 // warps 4-19 compute (thread = key row, group g owns query columns [16g, 16g+16) of the step), warps 20-23 drain
 // dQ^T (thread = head-dim index).
 #include "common.cuh"
@@ -68,7 +70,7 @@ struct Smem {
   static constexpr int kOnes = kDSlab + kDoStages * kSlabBytes;
   static constexpr int kRowsum = kOnes + kOnesBytes;         // [4 groups][128] floats
   static constexpr int kBars = kRowsum + 4 * kTile * 4;
-  static constexpr int kNumBars = 1 + 2 * kQStages + 2 * kDoStages + 2 * kDsStages + 11;
+  static constexpr int kNumBars = 1 + 2 * kQStages + 2 * kDoStages + 9;
   static constexpr int kMisc = kBars + kNumBars * 8;
   static constexpr int kTotal = kMisc + 16;
   static constexpr int kDynamic = kTotal + 1024;
@@ -79,8 +81,7 @@ static constexpr int kColS = 0, kColDP = 64, kColPT = 128, kColDQ = 160, kColDST
 
 enum Site : uint32_t {
   kSiteKV = 96, kSiteQFull, kSiteDoFull, kSiteQEmpty, kSiteDoEmpty, kSiteSFull, kSiteDPFull, kSitePFull, kSiteDSFull,
-  kSiteDQFull, kSiteDQDrained, kSiteAccDone, kSiteGroup, kSiteSConsumed, kSiteDPConsumed, kSiteDVDone, kSiteDsFree,
-  kSiteDrain
+  kSiteDQFull, kSiteDQDrained, kSiteAccDone, kSiteGroup, kSiteDsFree
 };
 
 struct Params {
@@ -111,22 +112,18 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Smem::kBars);
   uint64_t* kv_full = bars;
   uint64_t* q_full = kv_full + 1;            // [kQStages] Q step tile + L slab landed
-  uint64_t* q_empty = q_full + kQStages;     // two arrivals: S^T (issuer A) and dK (issuer B) have completed
+  uint64_t* q_empty = q_full + kQStages;     // dK has completed (it follows S^T)
   uint64_t* do_full = q_empty + kQStages;    // [kDoStages] dO step tile + delta slab landed
-  uint64_t* do_empty = do_full + kDoStages;  // two arrivals: dV (issuer A) and dP^T (issuer B)
-  uint64_t* s_full = do_empty + kDoStages;
-  uint64_t* s_consumed = s_full + 1;
-  uint64_t* dp_full = s_consumed + 1;
-  uint64_t* dp_consumed = dp_full + 1;
-  uint64_t* p_full = dp_consumed + 1;
-  uint64_t* dv_done = p_full + 1;
-  uint64_t* ds_full = dv_done + 1;           // [kDsStages] the dS^T tile of a step is written
-  uint64_t* ds_free = ds_full + kDsStages;   // [kDsStages] dQ^T (issuer C) has read the shared-memory tile
-  uint64_t* dq_full = ds_free + kDsStages;   // dQ^T of the step is complete in TMEM
+  uint64_t* do_empty = do_full + kDoStages;  // dV has completed (it follows dP^T)
+  uint64_t* s_full = do_empty + kDoStages;   // S^T(n) complete
+  uint64_t* dp_full = s_full + 1;            // dP^T(n) and dV(n-1) complete: the P^T columns may be overwritten
+  uint64_t* p_full = dp_full + 1;            // P^T(n) stored to TMEM, S^T(n) read
+  uint64_t* ds_full = p_full + 1;            // dS^T(n) stored to TMEM and to shared memory, dP^T(n) read
+  uint64_t* dk_done = ds_full + 1;           // dK(n) and dQ^T(n-1) complete: both copies of dS^T may be overwritten
+  uint64_t* dq_full = dk_done + 1;           // dQ^T of the step is complete in TMEM
   uint64_t* dq_drained = dq_full + 1;
   uint64_t* acc_done = dq_drained + 1;       // three arrivals
   uint64_t* grp_sync = acc_done + 1;
-  uint64_t* dk_done = grp_sync + 1;          // dK (issuer B) has read the TMEM copy of dS^T
   uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(smem + Smem::kMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Smem::kMisc + 4);
 
@@ -161,15 +158,12 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   // slab is written (behind a synchronisation of its own for the status word: backward call at B4 H16 N2048 266 -> 263 us).
   if (tid == kLoadWarp * 32) {
     mbar_init(kv_full, 1);
-    for (int s = 0; s < kQStages; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 2); }
-    for (int s = 0; s < kDoStages; ++s) { mbar_init(&do_full[s], 1); mbar_init(&do_empty[s], 2); }
+    for (int s = 0; s < kQStages; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
+    for (int s = 0; s < kDoStages; ++s) { mbar_init(&do_full[s], 1); mbar_init(&do_empty[s], 1); }
     mbar_init(s_full, 1);
-    mbar_init(s_consumed, kNumComputeWarps);   // one arrival per warp
     mbar_init(dp_full, 1);
-    mbar_init(dp_consumed, kNumComputeWarps);
-    mbar_init(p_full, kNumComputeWarps);
-    mbar_init(dv_done, 1);
-    for (int s = 0; s < kDsStages; ++s) { mbar_init(&ds_full[s], kNumComputeWarps); mbar_init(&ds_free[s], 1); }
+    mbar_init(p_full, kNumComputeWarps);       // one arrival per warp
+    mbar_init(ds_full, kNumComputeWarps);
     mbar_init(dk_done, 1);
     mbar_init(dq_full, 1);
     mbar_init(dq_drained, 4);
@@ -268,91 +262,68 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         const SmemDesc k_kmaj = make_sdesc_parts(smem_u32(s_k), 16, 1024);
         const SmemDesc q_kmaj0 = make_sdesc_parts(smem_u32(s_q), 16, 1024);
         const SmemDesc lslab0 = make_sdesc_slab32(smem_u32(s_lslab));
-        const SmemDesc do_nmaj0 = make_sdesc_parts(smem_u32(s_do), kQBoxBytes, 1024);   // 64-column groups 8 KB apart
-        if (ok) ok = wait_q(0);
-        if (ok) {
-          tc_fence_after_sync();
-          if (el) {
-            issue_scores(tmem + kColS, k_kmaj, q_kmaj0, lslab0);
-            umma_commit(s_full);
-            umma_commit(&q_empty[0]);
-          }
-        }
         for (int n = 0; n < cnt && ok; ++n) {
-          if (n + 1 < cnt) {
-            const int st = (n + 1) % kQStages;
-            ok = wait_q(n + 1) && mbar_wait_warp(s_consumed, n & 1, abort_flag, p.status, kSiteSConsumed);
-            if (!ok) break;
-            tc_fence_after_sync();
-            if (el) {
-              issue_scores(tmem + kColS, k_kmaj, stage_of(q_kmaj0, st, kQTileBytes), stage_of(lslab0, st, kSlabBytes));
-              umma_commit(s_full);
-              umma_commit(&q_empty[st]);
-            }
-          }
-          // dV += P^T dO
-          ok = mbar_wait_warp(p_full, n & 1, abort_flag, p.status, kSitePFull);
+          const int st = n % kQStages;
+          ok = wait_q(n);
+          // S^T(n) may overwrite S^T(n-1) once every compute warp has stored P^T(n-1)
+          if (ok && n > 0) ok = mbar_wait_warp(p_full, (n - 1) & 1, abort_flag, p.status, kSitePFull);
           if (!ok) break;
           tc_fence_after_sync();
-          const SmemDesc do_n = stage_of(do_nmaj0, n % kDoStages, kQTileBytes);
           if (el) {
-#pragma unroll
-            for (int kk = 0; kk < kQStep / 16; ++kk)
-              umma_ts(tmem + kColDV, tmem + kColPT + kk * 8, sdesc_at(do_n, kk * 2048), idesc_acc,
-                      (n > 0 || kk > 0) ? 1u : 0u);
-            umma_commit(dv_done);
-            umma_commit(&do_empty[n % kDoStages]);
+            issue_scores(tmem + kColS, k_kmaj, stage_of(q_kmaj0, st, kQTileBytes), stage_of(lslab0, st, kSlabBytes));
+            umma_commit(s_full);
           }
         }
       } else if (warp == kMmaWarpB) {
         const SmemDesc v_kmaj = make_sdesc_parts(smem_u32(s_v), 16, 1024);
         const SmemDesc do_kmaj0 = make_sdesc_parts(smem_u32(s_do), 16, 1024);
         const SmemDesc dslab0 = make_sdesc_slab32(smem_u32(s_dslab));
-        const SmemDesc q_nmaj0 = make_sdesc_parts(smem_u32(s_q), kQBoxBytes, 1024);
-        if (ok) ok = wait_do(0);
-        if (ok) {
-          tc_fence_after_sync();
-          if (el) {
-            issue_scores(tmem + kColDP, v_kmaj, do_kmaj0, dslab0);
-            umma_commit(dp_full);
-            umma_commit(&do_empty[0]);
-          }
-        }
+        const SmemDesc do_nmaj0 = make_sdesc_parts(smem_u32(s_do), kQBoxBytes, 1024);   // 64-column groups 8 KB apart
         for (int n = 0; n < cnt && ok; ++n) {
-          if (n + 1 < cnt) {
-            const int st = (n + 1) % kDoStages;
-            ok = wait_do(n + 1) && mbar_wait_warp(dp_consumed, n & 1, abort_flag, p.status, kSiteDPConsumed);
-            if (!ok) break;
-            tc_fence_after_sync();
-            if (el) {
-              issue_scores(tmem + kColDP, v_kmaj, stage_of(do_kmaj0, st, kQTileBytes), stage_of(dslab0, st, kSlabBytes));
-              umma_commit(dp_full);
-              umma_commit(&do_empty[st]);
-            }
-          }
-          // dK += dS^T Q
-          ok = mbar_wait_warp(&ds_full[n % kDsStages], (n / kDsStages) & 1, abort_flag, p.status, kSiteDSFull);
+          const int st = n % kDoStages;
+          ok = wait_do(n);
+          // dP^T(n) may overwrite dP^T(n-1) once every compute warp has stored dS^T(n-1)
+          if (ok && n > 0) ok = mbar_wait_warp(ds_full, (n - 1) & 1, abort_flag, p.status, kSiteDSFull);
           if (!ok) break;
           tc_fence_after_sync();
-          // A = the TMEM copy of dS^T (16-bit pairs, 32 columns): only Q is fetched from shared memory
+          if (el) {
+            issue_scores(tmem + kColDP, v_kmaj, stage_of(do_kmaj0, st, kQTileBytes), stage_of(dslab0, st, kSlabBytes));
+            umma_commit(dp_full);                    // and dV(n-1)
+          }
+          // dV += P^T dO
+          ok = mbar_wait_warp(p_full, n & 1, abort_flag, p.status, kSitePFull);
+          if (!ok) break;
+          tc_fence_after_sync();
+          const SmemDesc do_n = stage_of(do_nmaj0, st, kQTileBytes);
+          if (el) {
+#pragma unroll
+            for (int kk = 0; kk < kQStep / 16; ++kk)
+              umma_ts(tmem + kColDV, tmem + kColPT + kk * 8, sdesc_at(do_n, kk * 2048), idesc_acc,
+                      (n > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(&do_empty[st]);
+          }
+        }
+      } else {
+        // dK += dS^T Q: A = the TMEM copy of dS^T (16-bit pairs, 32 columns), so that only Q is fetched from shared memory
+        const SmemDesc q_nmaj0 = make_sdesc_parts(smem_u32(s_q), kQBoxBytes, 1024);
+        // dQ^T = K^T dS^T : A = K tile read M-major (rows = keys = reduction index, 64-wide d groups 16 KB apart),
+        // B = the dS^T tile read N-major
+        const SmemDesc k_mmaj = make_sdesc_parts(smem_u32(s_k), kBoxBytes, 1024);
+        const SmemDesc ds_nmaj = make_sdesc_parts(smem_u32(s_ds), kBoxBytes, 1024);
+        for (int n = 0; n < cnt && ok; ++n) {
+          ok = mbar_wait_warp(ds_full, n & 1, abort_flag, p.status, kSiteDSFull);
+          if (!ok) break;
+          tc_fence_after_sync();
           const SmemDesc q_n = stage_of(q_nmaj0, n % kQStages, kQTileBytes);
           if (el) {
 #pragma unroll
             for (int kk = 0; kk < kQStep / 16; ++kk)
               umma_ts(tmem + kColDK, tmem + kColDST + kk * 8, sdesc_at(q_n, kk * 2048), idesc_acc,
                       (n > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(dk_done);                    // and dQ^T(n-1)
             umma_commit(&q_empty[n % kQStages]);
-            umma_commit(dk_done);
           }
-        }
-      } else {
-        // dQ^T = K^T dS^T : A = K tile read M-major (rows = keys = reduction index, 64-wide d groups 16 KB apart),
-        // B = the dS^T tile read N-major
-        const SmemDesc k_mmaj = make_sdesc_parts(smem_u32(s_k), kBoxBytes, 1024);
-        const SmemDesc ds_nmaj = make_sdesc_parts(smem_u32(s_ds), kBoxBytes, 1024);
-        for (int n = 0; n < cnt && ok; ++n) {
-          ok = mbar_wait_warp(&ds_full[n % kDsStages], (n / kDsStages) & 1, abort_flag, p.status, kSiteDSFull);
-          if (ok && n > 0) ok = mbar_wait_warp(dq_drained, (n - 1) & 1, abort_flag, p.status, kSiteDQDrained);
+          if (n > 0) ok = mbar_wait_warp(dq_drained, (n - 1) & 1, abort_flag, p.status, kSiteDQDrained);
           if (!ok) break;
           tc_fence_after_sync();
           if (el) {
@@ -361,7 +332,6 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
               umma_ss(tmem + kColDQ, sdesc_at(k_mmaj, kk * 2048),
                       sdesc_at(ds_nmaj, (n % kDsStages) * kDsBytes + kk * 2048), idesc_dq, kk > 0);
             umma_commit(dq_full);                    // dQ^T readable
-            umma_commit(&ds_free[n % kDsStages]);    // the shared-memory tile's reader is done
           }
         }
       }
@@ -432,12 +402,12 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       if (!ok) break;
       tc_fence_after_sync();
       float pr[16];
+      bool dp_ready;
       {
         uint32_t raw[16];
         tmem_ld_x16(tmem + kColS + lane_sel + g * 16, raw);
+        dp_ready = mbar_test(dp_full, n & 1);
         tmem_ld_wait();
-        tc_fence_before_sync();
-        mbar_arrive_warp(s_consumed);
         // acc = k.q - L / scale2 ; P = exp2(acc * scale2 - ksq)
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
@@ -454,31 +424,30 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         for (int c = 0; c < 16; ++c)
           if (q0 + g * 16 + c < k_row0 + r) pr[c] = 0.f;
       }
+      // dP^T(n) has landed, and with it dV(n-1): the P^T columns are free
+      if (!__all_sync(0xffffffffu, dp_ready)) {
+        ok = mbar_wait_warp(dp_full, n & 1, abort_flag, p.status, kSiteDPFull);
+        if (!ok) break;
+      }
+      tc_fence_after_sync();
       {
         uint32_t packed[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) packed[i] = pack2<kBf16>(pr[2 * i], pr[2 * i + 1]);
-        if (n > 0) {   // the P^T columns are free once dV of the previous step has completed
-          ok = mbar_wait_warp(dv_done, (n - 1) & 1, abort_flag, p.status, kSiteDVDone);
-          if (!ok) break;
-          tc_fence_after_sync();
-        }
         tmem_st_x8(tmem + kColPT + lane_sel + g * 8, packed);
+      }
+      uint32_t ds_packed[8];
+      bool ds_free;
+      {
+        uint32_t raw[16];
+        tmem_ld_x16(tmem + kColDP + lane_sel + g * 16, raw);       // travels while the P^T store completes
         tmem_st_wait();
         tc_fence_before_sync();
         mbar_arrive_warp(p_full);
-      }
-
-      ok = mbar_wait_warp(dp_full, n & 1, abort_flag, p.status, kSiteDPFull);
-      if (!ok) break;
-      tc_fence_after_sync();
-      uint32_t ds_packed[8];
-      {
-        uint32_t raw[16];
-        tmem_ld_x16(tmem + kColDP + lane_sel + g * 16, raw);
+        // the TMEM copy of dS^T is free once dK(n-1) has completed, this step's shared-memory buffer once dQ^T(n-2) has,
+        // which went to the tensor core before it
+        ds_free = n == 0 || mbar_test(dk_done, (n - 1) & 1);
         tmem_ld_wait();
-        tc_fence_before_sync();
-        mbar_arrive_warp(dp_consumed);
         // acc = v.dO - delta ; dS = P * acc
         float rs0 = 0.f, rs1 = 0.f;
 #pragma unroll
@@ -490,26 +459,22 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         }
         ds_rowsum += rs0 + rs1;
       }
-      if (n >= kDsStages) {   // the dS^T buffer is free once dK and dQ^T of its previous step have completed
-        ok = mbar_wait_warp(&ds_free[n % kDsStages], ((n / kDsStages) - 1) & 1, abort_flag, p.status, kSiteDsFree);
+      if (!__all_sync(0xffffffffu, ds_free)) {
+        ok = mbar_wait_warp(dk_done, (n - 1) & 1, abort_flag, p.status, kSiteDsFree);
         if (!ok) break;
       }
+      tc_fence_after_sync();
+      // second copy for dK = dS^T Q, which takes its A operand from TMEM
+      tmem_st_x8(tmem + kColDST + lane_sel + g * 8, ds_packed);
       // row r of the [key][query] tile: 16-byte chunks 2g and 2g + 1
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch)
         *reinterpret_cast<uint4*>(s_ds + (n % kDsStages) * kDsBytes + sw128_offset(r, g * 2 + ch)) =
             make_uint4(ds_packed[ch * 4 + 0], ds_packed[ch * 4 + 1], ds_packed[ch * 4 + 2], ds_packed[ch * 4 + 3]);
       fence_proxy_async_smem();
-      // second copy for dK = dS^T Q, which takes its A operand from TMEM; free once dK of the previous step is done
-      if (n > 0) {
-        ok = mbar_wait_warp(dk_done, (n - 1) & 1, abort_flag, p.status, kSiteDsFree);
-        if (!ok) break;
-        tc_fence_after_sync();
-      }
-      tmem_st_x8(tmem + kColDST + lane_sel + g * 8, ds_packed);
       tmem_st_wait();
       tc_fence_before_sync();
-      mbar_arrive_warp(&ds_full[n % kDsStages]);
+      mbar_arrive_warp(ds_full);
     }
 
     uint32_t grp_phase = 0;
