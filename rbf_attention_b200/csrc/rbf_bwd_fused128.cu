@@ -128,7 +128,11 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Smem::kMisc + 4);
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  // The roles' branches and the MMAs' tensor-memory addresses go through a shuffle from lane 0, which the compiler knows to
+  // be the same in every lane: what the issuing warps compute from them stays in uniform registers. Backward call, in turn on
+  // one box: B2 H16 N4096 causal 430-459 -> 417-421 us, B2 H16 N3333 full 494 -> 487. (At head dim 64, whose issuers loop over
+  // item sizes read from shared memory, it changes nothing or costs 1 %.)
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
   const int bh = blockIdx.y;
   const int b = bh / p.H, h = bh % p.H;
@@ -207,7 +211,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = *tmem_base_s;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_base_s, 0);
   if (*abort_flag) {
     if (warp == kMmaWarpA) tmem_dealloc(tmem, 512);
     return;

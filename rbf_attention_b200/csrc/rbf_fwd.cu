@@ -201,7 +201,11 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   constexpr int kItemReaders = 2 + 8 * kSplit;   // two issuing warps, one arrival per softmax warp
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  // D = 128: the roles' branches and the tensor-memory addresses from lane 0's registers, known to the compiler as the same in
+  // every lane, so that the issuing warps' operands stay in uniform registers (forward call, in turn on one box: B2 H16 N4096
+  // causal 155-176 -> 142-146 us, B2 H16 N3333 full 223-257 -> 206-225). D = 64, with its loop over items read from shared
+  // memory: 399 -> 402 us at B8 H16 N4096, not done.
+  const int warp = D == 128 ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5;
   const int lane = tid & 31;
   const int total = heads * blocks;
   // The last CTA to leave puts the work counters back to zero for the next launch on this workspace and posts the
@@ -333,7 +337,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = *tmem_base_s;
+  const uint32_t tmem = D == 128 ? __shfl_sync(0xffffffffu, *tmem_base_s, 0) : *tmem_base_s;
   if (*abort_flag) {
     if (warp == kMmaWarp0) tmem_dealloc(tmem, 512);
     leave(queue);
