@@ -91,7 +91,7 @@ struct Smem {
   static constexpr int kStage = kPersistent ? kOnes + kTile * 32 : kQ;
   static constexpr int kBars = kOnes + kTile * 32 + (kPersistent ? 2 * kTileBytes : 0);
   static constexpr int kItemSlots = 4;                     // ring of work item numbers, producer -> all other roles
-  static constexpr int kNumBars = 2 + 4 * kStages + 10 + 4 + 2 * kItemSlots;
+  static constexpr int kNumBars = 2 + 4 * kStages + 12 + 4 + 2 * kItemSlots;
   static constexpr int kMisc = kBars + kNumBars * 8;        // tmem base, abort flag
   static constexpr int kTotal = kMisc + 16 + 16 * kItemSlots;
   static constexpr int kDynamic = kTotal + 1024;            // slack for 1024-byte alignment
@@ -190,7 +190,8 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   uint64_t* v_empty = v_full + kStages;          // two arrivals
   uint64_t* s_full = v_empty + kStages;          // [2] S_t(j) complete; persistent: and P_t(j-2) V
   uint64_t* p_full = s_full + 2;                 // [2] P_t(j) stored; persistent: and S_t(j+1) in the group's registers
-  uint64_t* o_done = p_full + 2;                 // [2] P_t(j) V complete (one item per CTA)
+  uint64_t* p_odd = p_full + 2;                  // [2] one item per CTA: p_full of the odd tiles (see there)
+  uint64_t* o_done = p_odd + 2;                  // [2] P_t(j) V complete (one item per CTA)
   uint64_t* grp_sync = o_done + 2;               // [2] rendezvous of the warps of a query tile
   uint64_t* s_consumed = grp_sync + 2;           // [2] the group holds S_t(j) in registers (one item per CTA)
   uint64_t* q_free = s_consumed + 2;             // [2] persistent: Q_t may be overwritten (issuer + softmax warps)
@@ -296,6 +297,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     for (int t = 0; t < 2; ++t) {
       mbar_init(&s_full[t], 1);
       mbar_init(&p_full[t], 4 * kSplit);     // one arrival per softmax warp of the tile
+      mbar_init(&p_odd[t], 4 * kSplit);
       mbar_init(&o_done[t], 1);
       mbar_init(&grp_sync[t], 4 * kSplit);
       mbar_init(&s_consumed[t], 4 * kSplit);
@@ -554,7 +556,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           }
           ok = wait_v(j);
           if (j < my_nkt) {
-            ok = ok && mbar_wait_warp(&p_full[t], j & 1, abort_flag, status, kSitePFull, s_unit);
+            ok = ok && mbar_wait_warp((j & 1) ? &p_odd[t] : &p_full[t], (j >> 1) & 1, abort_flag, status, kSitePFull, s_unit);
             if (!ok) break;
             tc_fence_after_sync();
             issue_o(st, j > 0 ? 1u : 0u, tmem_p[t] + (j & 1) * kPCols);
@@ -797,6 +799,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           load_scores();
           mbar_arrive_warp(&s_consumed[t]);
           auto wait_o = [&]() {
+            // (phase j - 2 has passed: S_t(j) went to the tensor core behind P_t(j-2) V)
             ok = mbar_wait_warp(&o_done[t], (j - 1) & 1, abort_flag, status, kSiteODone, s_unit);
             if (ok) tc_fence_after_sync();
             return ok;
@@ -812,10 +815,15 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           for (int c = 0; c < 4; ++c) store_p(c, (j & 1) * kPCols);
           p_stored();
           tc_fence_before_sync();
-          mbar_arrive_warp(&p_full[t]);
+          // A warp can be here for tile j + 1 while another one of its group still works on tile j (the scores S_t(j+1) only need
+          // S_t(j) to have been read by all), but not for tile j + 2: the arrivals of odd and even tiles are counted apart.
+          mbar_arrive_warp((j & 1) ? &p_odd[t] : &p_full[t]);
         }
         if (!ok) break;
-        ok = mbar_wait_warp(&o_done[t], (my_nkt - 1) & 1, abort_flag, status, kSiteODoneFinal, s_unit);
+        // The last two products may be under way: their phases one after the other (a wait for the last one's parity alone
+        // would be content with the phase two before it).
+        if (my_nkt > 1) ok = mbar_wait_warp(&o_done[t], (my_nkt - 2) & 1, abort_flag, status, kSiteODoneFinal, s_unit);
+        ok = ok && mbar_wait_warp(&o_done[t], (my_nkt - 1) & 1, abort_flag, status, kSiteODoneFinal, s_unit);
       }
       if (!ok) break;
       tc_fence_after_sync();

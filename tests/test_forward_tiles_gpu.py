@@ -58,3 +58,20 @@ def test_column_sums_over_few_and_many_bands(rows):
     want = x.double().sum(0)
     # sums of `rows` terms in any order: the error of an fp32 sum is at most its depth (well below 2^10) times 2^-24 of sum |x|
     assert ((got - want).abs() <= 2.0 ** -14 * x.double().abs().sum(0)).all()
+
+
+@pytest.mark.parametrize("D,causal,dtype", [(128, False, torch.float16), (128, True, torch.bfloat16), (64, False, torch.float16)])
+def test_forward_repeats_bitwise_under_load(D, causal, dtype):
+    """Warps of a query tile drift apart by up to a key tile; what one of them has arrived for must not be counted for another,
+    and a wait for a product must not be content with an earlier one. 2, 16 heads x 3333 rows: three rounds of CTAs."""
+    q, k, v, _ = oracle.make_inputs(2, 16, 3333, D, seed=3, dtype=dtype)
+    k = (k.float() * torch.linspace(1.5, 0.9, 3333)[None, None, :, None]).to(dtype)
+    q, k, v = (t.to("cuda") for t in (q, k, v))
+    first, lse = ops._forward(q, k, v, causal, True)
+    for _ in range(40):
+        out, again = ops._forward(q, k, v, causal, True)
+        assert torch.equal(out, first) and torch.equal(again, lse)
+    ops.check_device_status()
+    ref = oracle.torch_forward_backward(q[1:, 15:].cpu(), k[1:, 15:].cpu(), v[1:, 15:].cpu(), v[1:, 15:].cpu(), causal, True,
+                                        dtype=torch.float32)[0]
+    assert oracle.error_report(first[1:, 15:].cpu().float(), ref)["rel_l2"] <= REL_L2[dtype]
