@@ -174,13 +174,13 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
         const int row0 = (first + n) * kTile;
         const int s1 = n % C::kB1Stages, s2 = n % C::kB2Stages;
         if (n >= C::kB1Stages &&
-            !mbar_wait(&b1_empty[s1], ((n / C::kB1Stages) - 1) & 1, abort_flag, p.status, kSiteB1Empty))
+            !mbar_wait(&b1_empty[s1], ((n / C::kB1Stages) - 1) & 1, abort_flag, kSiteB1Empty))
           break;
         mbar_arrive_expect_tx(&b1_full[s1], kTileBytes);
         for (int x = 0; x < kBoxes; ++x)
           tma_load_4d(s_b1 + s1 * kTileBytes + x * kBoxBytes, &tm_b1, &b1_full[s1], x * 64, row0, h, b);
         if (n >= C::kB2Stages &&
-            !mbar_wait(&b2_empty[s2], ((n / C::kB2Stages) - 1) & 1, abort_flag, p.status, kSiteB2Empty))
+            !mbar_wait(&b2_empty[s2], ((n / C::kB2Stages) - 1) & 1, abort_flag, kSiteB2Empty))
           break;
         mbar_arrive_expect_tx(&b2_full[s2], kTileBytes);
         for (int x = 0; x < kBoxes; ++x)
@@ -211,10 +211,10 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
         }
       };
       auto wait_b1 = [&](int n) {
-        return mbar_wait(&b1_full[n % C::kB1Stages], (n / C::kB1Stages) & 1, abort_flag, p.status, kSiteB1Full);
+        return mbar_wait(&b1_full[n % C::kB1Stages], (n / C::kB1Stages) & 1, abort_flag, kSiteB1Full);
       };
       auto wait_b2 = [&](int n) {
-        return mbar_wait(&b2_full[n % C::kB2Stages], (n / C::kB2Stages) & 1, abort_flag, p.status, kSiteB2Full);
+        return mbar_wait(&b2_full[n % C::kB2Stages], (n / C::kB2Stages) & 1, abort_flag, kSiteB2Full);
       };
       auto issue_s = [&](int n) {
         const int sb = n % C::kSBufs;
@@ -226,7 +226,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
         umma_commit(dp_full);
       };
 
-      bool ok = mbar_wait(a_full, 0, abort_flag, p.status, kSiteAFull);
+      bool ok = mbar_wait(a_full, 0, abort_flag, kSiteAFull);
       if (ok) ok = wait_b1(0);
       if (ok) {
         tc_fence_after_sync();
@@ -247,12 +247,12 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
       for (int n = 0; n < cnt && ok; ++n) {
         const int sb = n % C::kSBufs;
         if (kHasAccP) {
-          ok = mbar_wait(&p_full[sb], (n / C::kSBufs) & 1, abort_flag, p.status, kSitePFull);
+          ok = mbar_wait(&p_full[sb], (n / C::kSBufs) & 1, abort_flag, kSitePFull);
           if (!ok) break;
           tc_fence_after_sync();
           issue_acc(tmem + C::kColAccP, tmem + C::kColS + sb * kTile, b2 + (n % C::kB2Stages) * kTileBytes, n > 0);
         }
-        ok = mbar_wait(ds_full, n & 1, abort_flag, p.status, kSiteDSFull);
+        ok = mbar_wait(ds_full, n & 1, abort_flag, kSiteDSFull);
         if (!ok) break;
         tc_fence_after_sync();
         issue_acc(tmem + C::kColAccS, tmem + C::kColDP, b1 + (n % C::kB1Stages) * kTileBytes, n > 0);
@@ -295,7 +295,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
     uint32_t grp_phase = 0;
     auto group_sync = [&]() -> bool {
       mbar_arrive_warp(grp_sync);
-      const bool done = mbar_wait_warp(grp_sync, grp_phase & 1, abort_flag, p.status, kSiteGroup);
+      const bool done = mbar_wait_warp(grp_sync, grp_phase & 1, abort_flag, kSiteGroup);
       ++grp_phase;
       return done;
     };
@@ -317,7 +317,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
       const int sb = n % C::kSBufs;
       float cs_next = 0.f, cd_next = 0.f;
       if (n + 1 < cnt) fetch_col(n + 1, cs_next, cd_next);
-      ok = group_sync() && mbar_wait_warp(&s_full[sb], (n / C::kSBufs) & 1, abort_flag, p.status, kSiteSFull);
+      ok = group_sync() && mbar_wait_warp(&s_full[sb], (n / C::kSBufs) & 1, abort_flag, kSiteSFull);
       if (!ok) break;
       tc_fence_after_sync();
       const float* vbuf = s_vec + (n & 1) * 2 * kTile;
@@ -360,7 +360,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
         mbar_arrive_warp(&p_full[sb]);
       }
 
-      ok = mbar_wait_warp(dp_full, n & 1, abort_flag, p.status, kSiteDPFull);
+      ok = mbar_wait_warp(dp_full, n & 1, abort_flag, kSiteDPFull);
       if (!ok) break;
       tc_fence_after_sync();
       // dS = P * (dP - delta): read dP in four 32-column chunks, then write the packed dS over dP's columns
@@ -400,7 +400,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
       }
     }
 
-    if (ok) ok = mbar_wait_warp(acc_done, 0, abort_flag, p.status, kSiteAccDone);
+    if (ok) ok = mbar_wait_warp(acc_done, 0, abort_flag, kSiteAccDone);
     if (ok) {
       tc_fence_after_sync();
       // All MMAs are complete: the B1 ring is free and serves as staging for the TMA stores.
@@ -467,6 +467,7 @@ rbf_bwd_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_constant_
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (tid == 0) record_timeout(abort_flag, p.status, status_unit());
   if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
 }
 

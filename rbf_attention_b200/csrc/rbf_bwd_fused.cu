@@ -188,7 +188,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
   constexpr int kItemReaders = 3 + 4 + kNumComputeWarps;
   auto next_item = [&]() -> bool {
     const int slot = I % Smem::kItemSlots;
-    if (!mbar_wait_warp(&item_full[slot], (I / Smem::kItemSlots) & 1, abort_flag, p.status, kSiteItemFull, s_item))
+    if (!mbar_wait_warp(&item_full[slot], (I / Smem::kItemSlots) & 1, abort_flag, kSiteItemFull))
       return false;
     const int tile = s_items[slot].x;
     bh = s_items[slot].y;
@@ -303,23 +303,23 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
       while (true) {
         if (I > 0) {
           // the K buffer's previous user is two items back
-          if (I > 1) ok = mbar_wait(&k_free[I & 1], ((I >> 1) - 1) & 1, abort_flag, p.status, kSiteKFree, s_item);
+          if (I > 1) ok = mbar_wait(&k_free[I & 1], ((I >> 1) - 1) & 1, abort_flag, kSiteKFree);
           if (!ok) break;
           load_k();
         }
         for (int n = I == 0 ? 2 : 0; n < cnt; ++n) {
           const uint32_t g = T + n;
           if (g >= kQStages)
-            ok = mbar_wait(&q_empty[g % kQStages], ((g / kQStages) - 1) & 1, abort_flag, p.status, kSiteQEmpty, s_item);
+            ok = mbar_wait(&q_empty[g % kQStages], ((g / kQStages) - 1) & 1, abort_flag, kSiteQEmpty);
           if (!ok) break;
           load_q(n);
           if (n == 0) {
-            ok = mbar_wait(v_free, (I - 1) & 1, abort_flag, p.status, kSiteVFree, s_item);
+            ok = mbar_wait(v_free, (I - 1) & 1, abort_flag, kSiteVFree);
             if (!ok) break;
             load_v();
           }
           if (g >= kDoStages)
-            ok = mbar_wait(&do_empty[g % kDoStages], ((g / kDoStages) - 1) & 1, abort_flag, p.status, kSiteDoEmpty, s_item);
+            ok = mbar_wait(&do_empty[g % kDoStages], ((g / kDoStages) - 1) & 1, abort_flag, kSiteDoEmpty);
           if (!ok) break;
           load_do(n);
         }
@@ -334,7 +334,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
         if (more) set_item(item);
         const int slot = I % Smem::kItemSlots;
         if (I >= Smem::kItemSlots &&
-            !mbar_wait(&item_empty[slot], ((I / Smem::kItemSlots) - 1) & 1, abort_flag, p.status, kSiteItemEmpty, s_item))
+            !mbar_wait(&item_empty[slot], ((I / Smem::kItemSlots) - 1) & 1, abort_flag, kSiteItemEmpty))
           break;
         if (more) *s_item = item;
         publish_item(more);
@@ -368,12 +368,12 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
         const SmemDesc k_kmaj = stage_of(make_sdesc_parts(smem_u32(s_k), 16, 1024), I & 1, kTileBytes);
         const SmemDesc q_kmaj0 = make_sdesc_parts(smem_u32(s_q), 16, 1024);
         const SmemDesc lslab0 = make_sdesc_slab32(smem_u32(s_lslab));
-        ok = mbar_wait(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item);
+        ok = mbar_wait(&k_full[I & 1], (I >> 1) & 1, abort_flag, kSiteKFull);
         for (int n = 0; n < cnt && ok; ++n) {
           const uint32_t g = T + n, st = g % kQStages;
-          ok = mbar_wait(&q_full[st], (g / kQStages) & 1, abort_flag, p.status, kSiteQFull, s_item);
+          ok = mbar_wait(&q_full[st], (g / kQStages) & 1, abort_flag, kSiteQFull);
           // S^T(n) may overwrite S^T(n-1) once every compute warp has stored P^T(n-1)
-          if (ok && g > 0) ok = mbar_wait(p_full, (g - 1) & 1, abort_flag, p.status, kSitePFull, s_item);
+          if (ok && g > 0) ok = mbar_wait(p_full, (g - 1) & 1, abort_flag, kSitePFull);
           if (!ok) break;
           tc_fence_after_sync();
           if (el) {
@@ -386,12 +386,12 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
         const SmemDesc do_kmaj0 = make_sdesc_parts(smem_u32(s_do), 16, 1024);
         const SmemDesc do_nmaj0 = make_sdesc_parts(smem_u32(s_do), kTile * 128, 1024);
         const SmemDesc dslab0 = make_sdesc_slab32(smem_u32(s_dslab));
-        ok = mbar_wait(v_full, I & 1, abort_flag, p.status, kSiteVFull, s_item);
+        ok = mbar_wait(v_full, I & 1, abort_flag, kSiteVFull);
         for (int n = 0; n < cnt && ok; ++n) {
           const uint32_t g = T + n, st = g % kDoStages;
-          ok = mbar_wait(&do_full[st], (g / kDoStages) & 1, abort_flag, p.status, kSiteDoFull, s_item);
+          ok = mbar_wait(&do_full[st], (g / kDoStages) & 1, abort_flag, kSiteDoFull);
           // dP^T(n) may overwrite dP^T(n-1) once every compute warp has stored dS^T(n-1)
-          if (ok && g > 0) ok = mbar_wait(ds_full, (g - 1) & 1, abort_flag, p.status, kSiteDSFull, s_item);
+          if (ok && g > 0) ok = mbar_wait(ds_full, (g - 1) & 1, abort_flag, kSiteDSFull);
           if (!ok) break;
           tc_fence_after_sync();
           if (el) {
@@ -400,8 +400,8 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
             if (n == cnt - 1) umma_commit(v_free);
           }
           // dV += P^T dO, from zero once the previous item's dV has left
-          ok = mbar_wait(p_full, g & 1, abort_flag, p.status, kSitePFull, s_item);
-          if (ok && n == 0 && I > 0) ok = mbar_wait(dv_free, (I - 1) & 1, abort_flag, p.status, kSiteDVFree, s_item);
+          ok = mbar_wait(p_full, g & 1, abort_flag, kSitePFull);
+          if (ok && n == 0 && I > 0) ok = mbar_wait(dv_free, (I - 1) & 1, abort_flag, kSiteDVFree);
           if (!ok) break;
           tc_fence_after_sync();
           const SmemDesc do_n = stage_of(do_nmaj0, st, kTileBytes);
@@ -421,11 +421,11 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
         // dQ_partial = dS K : A = the dS^T tile read M-major (rows = keys = reduction index), B = K read N-major
         const SmemDesc k_nmaj = stage_of(make_sdesc_parts(smem_u32(s_k), kTile * 128, 1024), I & 1, kTileBytes);
         const SmemDesc ds_mmaj = make_sdesc_parts(smem_u32(s_ds), kTile * 128, 1024);   // rows = reduction (keys)
-        ok = mbar_wait(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item);
+        ok = mbar_wait(&k_full[I & 1], (I >> 1) & 1, abort_flag, kSiteKFull);
         for (int n = 0; n < cnt && ok; ++n) {
           const uint32_t g = T + n, st = g % kQStages;
-          ok = mbar_wait(ds_full, g & 1, abort_flag, p.status, kSiteDSFull, s_item);
-          if (ok && n == 0 && I > 0) ok = mbar_wait(dk_free, (I - 1) & 1, abort_flag, p.status, kSiteDKFree, s_item);
+          ok = mbar_wait(ds_full, g & 1, abort_flag, kSiteDSFull);
+          if (ok && n == 0 && I > 0) ok = mbar_wait(dk_free, (I - 1) & 1, abort_flag, kSiteDKFree);
           if (!ok) break;
           tc_fence_after_sync();
           const SmemDesc q_n = stage_of(q_nmaj0, st, kTileBytes);
@@ -437,7 +437,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
             umma_commit(&q_empty[st]);
             if (n == cnt - 1) umma_commit(dk_acc);   // the item's dK is complete
           }
-          if (g > 0) ok = mbar_wait(dq_drained, (g - 1) & 1, abort_flag, p.status, kSiteDQDrained, s_item);
+          if (g > 0) ok = mbar_wait(dq_drained, (g - 1) & 1, abort_flag, kSiteDQDrained);
           if (!ok) break;
           tc_fence_after_sync();
           if (el) {
@@ -470,7 +470,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
       return my_boxes + (uses++ & 1) * kDqBoxBytes;
     };
     auto drain_dq = [&](int n) -> bool {
-      if (!mbar_wait_warp(dq_full, (T + n) & 1, abort_flag, p.status, kSiteDQFull, s_item)) return false;
+      if (!mbar_wait_warp(dq_full, (T + n) & 1, abort_flag, kSiteDQFull)) return false;
       tc_fence_after_sync();
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
@@ -501,7 +501,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
       const int row0 = k_row0 + wq * 32;             // this warp's key rows
       for (int n = 0; n < cnt - 1 && ok; ++n) ok = drain_dq(n);
       // dV and dK are complete before the last dQ_partial, and the next item's products wait for their columns
-      if (ok) ok = mbar_wait_warp(dv_acc, I & 1, abort_flag, p.status, kSiteDVAcc, s_item);
+      if (ok) ok = mbar_wait_warp(dv_acc, I & 1, abort_flag, kSiteDVAcc);
       if (!ok) break;
       tc_fence_after_sync();
       {
@@ -531,9 +531,9 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
           tma_store_commit();
         }
     }
-    ok = mbar_wait_warp(dk_acc, I & 1, abort_flag, p.status, kSiteDKAcc, s_item) &&
-         mbar_wait_warp(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item) &&
-         mbar_wait_warp(&rs_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteRowsum, s_item);
+    ok = mbar_wait_warp(dk_acc, I & 1, abort_flag, kSiteDKAcc) &&
+         mbar_wait_warp(&k_full[I & 1], (I >> 1) & 1, abort_flag, kSiteKFull) &&
+         mbar_wait_warp(&rs_full[I & 1], (I >> 1) & 1, abort_flag, kSiteRowsum);
     if (!ok) break;
     tc_fence_after_sync();
     {
@@ -590,12 +590,12 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
     bool ok = run;
     while (ok && next_item()) {
-      ok = mbar_wait_warp(&k_full[I & 1], (I >> 1) & 1, abort_flag, p.status, kSiteKFull, s_item);
+      ok = mbar_wait_warp(&k_full[I & 1], (I >> 1) & 1, abort_flag, kSiteKFull);
       if (!ok) break;
       const float neg_ksq = -s_ksq[(I & 1) * kTile + r];
       float ds_rowsum = 0.f;
       for (int n = 0; n < cnt; ++n) {
-        ok = mbar_wait_warp(s_full, (T + n) & 1, abort_flag, p.status, kSiteSFull, s_item);
+        ok = mbar_wait_warp(s_full, (T + n) & 1, abort_flag, kSiteSFull);
         if (!ok) break;
         tc_fence_after_sync();
         float pr[32];
@@ -622,7 +622,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
         }
         // dP^T(n) has landed, and with it dV(n-1): the P^T columns are free
         if (!__all_sync(0xffffffffu, dp_ready)) {
-          ok = mbar_wait_warp(dp_full, (T + n) & 1, abort_flag, p.status, kSiteDPFull, s_item);
+          ok = mbar_wait_warp(dp_full, (T + n) & 1, abort_flag, kSiteDPFull);
           if (!ok) break;
         }
         tc_fence_after_sync();
@@ -655,7 +655,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
           ds_rowsum += rs0 + rs1;
         }
         if (!__all_sync(0xffffffffu, ds_free)) {
-          ok = mbar_wait_warp(dq_full, (T + n - 1) & 1, abort_flag, p.status, kSiteDsFree, s_item);
+          ok = mbar_wait_warp(dq_full, (T + n - 1) & 1, abort_flag, kSiteDsFree);
           if (!ok) break;
         }
         // row r of the [key][query] tile, box g/2, 16-byte chunks 4(g%2) .. +3
@@ -687,6 +687,7 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (tid == 0) record_timeout(abort_flag, p.status, *s_item);
   if (warp == kMmaWarpA) tmem_dealloc(*tmem_base_s, 512);
   if (queue && tid == 0) {
     // the last CTA to leave puts the work counters back to zero for the next launch on this workspace

@@ -226,9 +226,9 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       static_assert(kQStages == kDoStages, "the first loads fill both rings");
       for (int n = kQStages; n < cnt; ++n) {
         const uint32_t par = ((n / kQStages) - 1) & 1;
-        if (!mbar_wait(&q_empty[n % kQStages], par, abort_flag, p.status, kSiteQEmpty)) break;
+        if (!mbar_wait(&q_empty[n % kQStages], par, abort_flag, kSiteQEmpty)) break;
         load_q(n);
-        if (!mbar_wait(&do_empty[n % kDoStages], par, abort_flag, p.status, kSiteDoEmpty)) break;
+        if (!mbar_wait(&do_empty[n % kDoStages], par, abort_flag, kSiteDoEmpty)) break;
         load_do(n);
       }
     }
@@ -255,12 +255,12 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         umma_ss(dst, sdesc_at(ones_desc, 0), sdesc_at(slab, 0), idesc_s, 1u);
       };
       auto wait_q = [&](int n) {
-        return mbar_wait_warp(&q_full[n % kQStages], (n / kQStages) & 1, abort_flag, p.status, kSiteQFull);
+        return mbar_wait_warp(&q_full[n % kQStages], (n / kQStages) & 1, abort_flag, kSiteQFull);
       };
       auto wait_do = [&](int n) {
-        return mbar_wait_warp(&do_full[n % kDoStages], (n / kDoStages) & 1, abort_flag, p.status, kSiteDoFull);
+        return mbar_wait_warp(&do_full[n % kDoStages], (n / kDoStages) & 1, abort_flag, kSiteDoFull);
       };
-      bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status, kSiteKV);
+      bool ok = mbar_wait_warp(kv_full, 0, abort_flag, kSiteKV);
 
       if (warp == kMmaWarpA) {
         const SmemDesc k_kmaj = make_sdesc_parts(smem_u32(s_k), 16, 1024);
@@ -270,7 +270,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
           const int st = n % kQStages;
           ok = wait_q(n);
           // S^T(n) may overwrite S^T(n-1) once every compute warp has stored P^T(n-1)
-          if (ok && n > 0) ok = mbar_wait_warp(p_full, (n - 1) & 1, abort_flag, p.status, kSitePFull);
+          if (ok && n > 0) ok = mbar_wait_warp(p_full, (n - 1) & 1, abort_flag, kSitePFull);
           if (!ok) break;
           tc_fence_after_sync();
           if (el) {
@@ -287,7 +287,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
           const int st = n % kDoStages;
           ok = wait_do(n);
           // dP^T(n) may overwrite dP^T(n-1) once every compute warp has stored dS^T(n-1)
-          if (ok && n > 0) ok = mbar_wait_warp(ds_full, (n - 1) & 1, abort_flag, p.status, kSiteDSFull);
+          if (ok && n > 0) ok = mbar_wait_warp(ds_full, (n - 1) & 1, abort_flag, kSiteDSFull);
           if (!ok) break;
           tc_fence_after_sync();
           if (el) {
@@ -295,7 +295,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
             umma_commit(dp_full);                    // and dV(n-1)
           }
           // dV += P^T dO
-          ok = mbar_wait_warp(p_full, n & 1, abort_flag, p.status, kSitePFull);
+          ok = mbar_wait_warp(p_full, n & 1, abort_flag, kSitePFull);
           if (!ok) break;
           tc_fence_after_sync();
           const SmemDesc do_n = stage_of(do_nmaj0, st, kQTileBytes);
@@ -315,7 +315,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         const SmemDesc k_mmaj = make_sdesc_parts(smem_u32(s_k), kBoxBytes, 1024);
         const SmemDesc ds_nmaj = make_sdesc_parts(smem_u32(s_ds), kBoxBytes, 1024);
         for (int n = 0; n < cnt && ok; ++n) {
-          ok = mbar_wait_warp(ds_full, n & 1, abort_flag, p.status, kSiteDSFull);
+          ok = mbar_wait_warp(ds_full, n & 1, abort_flag, kSiteDSFull);
           if (!ok) break;
           tc_fence_after_sync();
           const SmemDesc q_n = stage_of(q_nmaj0, n % kQStages, kQTileBytes);
@@ -327,7 +327,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
             umma_commit(dk_done);                    // and dQ^T(n-1)
             umma_commit(&q_empty[n % kQStages]);
           }
-          if (n > 0) ok = mbar_wait_warp(dq_drained, (n - 1) & 1, abort_flag, p.status, kSiteDQDrained);
+          if (n > 0) ok = mbar_wait_warp(dq_drained, (n - 1) & 1, abort_flag, kSiteDQDrained);
           if (!ok) break;
           tc_fence_after_sync();
           if (el) {
@@ -349,7 +349,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     float* acc_col = p.dq_acc + static_cast<int64_t>(bh) * p.N * D + wq * 32 + lane;
     bool ok = true;
     for (int n = 0; n < cnt; ++n) {
-      ok = mbar_wait_warp(dq_full, n & 1, abort_flag, p.status, kSiteDQFull);
+      ok = mbar_wait_warp(dq_full, n & 1, abort_flag, kSiteDQFull);
       if (!ok) break;
       tc_fence_after_sync();
       const int q0 = (first + n) * kQStep;
@@ -384,7 +384,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     // c |k_r|^2 of this thread's key row, from the resident K tile; rows past N (zero-filled by the load) get
     // +infinity, i.e. weight exp2(-inf) = 0
     float neg_ksq = -INFINITY;
-    bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status, kSiteKV);
+    bool ok = mbar_wait_warp(kv_full, 0, abort_flag, kSiteKV);
     if (ok && k_row0 + r < p.N) {
       float acc = 0.f;
 #pragma unroll 1
@@ -402,7 +402,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     }
 
     for (int n = 0; n < cnt && ok; ++n) {
-      ok = mbar_wait_warp(s_full, n & 1, abort_flag, p.status, kSiteSFull);
+      ok = mbar_wait_warp(s_full, n & 1, abort_flag, kSiteSFull);
       if (!ok) break;
       tc_fence_after_sync();
       float pr[16];
@@ -430,7 +430,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       }
       // dP^T(n) has landed, and with it dV(n-1): the P^T columns are free
       if (!__all_sync(0xffffffffu, dp_ready)) {
-        ok = mbar_wait_warp(dp_full, n & 1, abort_flag, p.status, kSiteDPFull);
+        ok = mbar_wait_warp(dp_full, n & 1, abort_flag, kSiteDPFull);
         if (!ok) break;
       }
       tc_fence_after_sync();
@@ -464,7 +464,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         ds_rowsum += rs0 + rs1;
       }
       if (!__all_sync(0xffffffffu, ds_free)) {
-        ok = mbar_wait_warp(dk_done, (n - 1) & 1, abort_flag, p.status, kSiteDsFree);
+        ok = mbar_wait_warp(dk_done, (n - 1) & 1, abort_flag, kSiteDsFree);
         if (!ok) break;
       }
       tc_fence_after_sync();
@@ -484,11 +484,11 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     uint32_t grp_phase = 0;
     auto group_sync = [&]() -> bool {
       mbar_arrive_warp(grp_sync);
-      const bool done = mbar_wait_warp(grp_sync, grp_phase & 1, abort_flag, p.status, kSiteGroup);
+      const bool done = mbar_wait_warp(grp_sync, grp_phase & 1, abort_flag, kSiteGroup);
       ++grp_phase;
       return done;
     };
-    if (ok) ok = mbar_wait_warp(acc_done, 0, abort_flag, p.status, kSiteAccDone);
+    if (ok) ok = mbar_wait_warp(acc_done, 0, abort_flag, kSiteAccDone);
     if (ok) {
       tc_fence_after_sync();
       s_rowsum[g * kTile + r] = ds_rowsum;      // every group holds a quarter of rowsum(dS^T)
@@ -542,6 +542,7 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (tid == 0) record_timeout(abort_flag, p.status, status_unit());
   if (warp == kMmaWarpA) tmem_dealloc(tmem, 512);
 }
 

@@ -249,7 +249,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       return false;
     }
     const int slot = n % kItemSlots;
-    if (!mbar_wait_warp(&item_full[slot], (n / kItemSlots) & 1, abort_flag, status, kSiteItemFull, s_unit)) {
+    if (!mbar_wait_warp(&item_full[slot], (n / kItemSlots) & 1, abort_flag, kSiteItemFull)) {
       ok_ref = false;
       return false;
     }
@@ -373,7 +373,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (n != 0) {
           for (int t = 0; t < 2 && ok; ++t) {
             if (it.nkt(t) == 0) continue;
-            if (qn[t] > 0) ok = mbar_wait(&q_free[t], (qn[t] - 1) & 1, abort_flag, status, kSiteQFree, s_unit);
+            if (qn[t] > 0) ok = mbar_wait(&q_free[t], (qn[t] - 1) & 1, abort_flag, kSiteQFree);
             if (ok) load_q(it, t);
           }
         }
@@ -382,12 +382,12 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           if (n == 0 && j < kStages) continue;       // issued before the CTA-wide synchronisation
           const int st = g % kStages;
           const uint32_t par = ((g / kStages) - 1) & 1;
-          if (g >= kStages && !mbar_wait(&k_empty[st], par, abort_flag, status, kSiteKEmpty, s_unit)) {
+          if (g >= kStages && !mbar_wait(&k_empty[st], par, abort_flag, kSiteKEmpty)) {
             ok = false;
             break;
           }
           load_keys(it, j, st);
-          if (g >= kStages && !mbar_wait(&v_empty[st], par, abort_flag, status, kSiteVEmpty, s_unit)) {
+          if (g >= kStages && !mbar_wait(&v_empty[st], par, abort_flag, kSiteVEmpty)) {
             ok = false;
             break;
           }
@@ -407,7 +407,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         const int slot = (n + 1) % kItemSlots;
         if (n + 1 >= kItemSlots &&
-            !mbar_wait(&item_empty[slot], (((n + 1) / kItemSlots) - 1) & 1, abort_flag, status, kSiteItemEmpty, s_unit))
+            !mbar_wait(&item_empty[slot], (((n + 1) / kItemSlots) - 1) & 1, abort_flag, kSiteItemEmpty))
           break;
         s_items[slot].x = more ? it.bh : -1;
         s_items[slot].y = it.b;
@@ -457,10 +457,10 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
       };
       auto wait_k = [&](uint32_t g) {
-        return mbar_wait_warp(&k_full[g % kStages], (g / kStages) & 1, abort_flag, status, kSiteKFull, s_unit);
+        return mbar_wait_warp(&k_full[g % kStages], (g / kStages) & 1, abort_flag, kSiteKFull);
       };
       auto wait_v = [&](uint32_t g) {
-        return mbar_wait_warp(&v_full[g % kStages], (g / kStages) & 1, abort_flag, status, kSiteVFull, s_unit);
+        return mbar_wait_warp(&v_full[g % kStages], (g / kStages) & 1, abort_flag, kSiteVFull);
       };
       if constexpr (kPersistent) {
         uint32_t G = 0, td = 0, qn = 0;
@@ -475,7 +475,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           if (my_nkt > 0) {
             // First scores of the item: Q_t and the first key tile have landed. (The group has read the previous item's
             // last scores: it has arrived for the last P, which was waited for before the last P V.)
-            ok = mbar_wait_warp(&q_full[t], qn & 1, abort_flag, status, kSiteQFull, s_unit) && wait_k(G);
+            ok = mbar_wait_warp(&q_full[t], qn & 1, abort_flag, kSiteQFull) && wait_k(G);
             if (!ok) break;
             tc_fence_after_sync();
             issue_s(G % kStages);
@@ -487,7 +487,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // Group j of the item's MMAs, j = 0 .. my_nkt: P_t(j-1) V and the scores S_t(j+1), once the softmax group has
             // stored the one and holds S_t(j) in registers. One commit covers both.
             for (int j = 0; j <= my_nkt; ++j) {
-              ok = mbar_wait_warp(&p_full[t], (td + j) & 1, abort_flag, status, kSitePFull, s_unit);
+              ok = mbar_wait_warp(&p_full[t], (td + j) & 1, abort_flag, kSitePFull);
               if (!ok) break;
               tc_fence_after_sync();
               if (j > 0) {
@@ -531,7 +531,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const int my_nkt = first_item.nkt(t), nkt_max = first_item.nkt_max;
         bool ok = wait_k(0);
         if (my_nkt > 0) {
-          ok = ok && mbar_wait_warp(&q_full[t], 0, abort_flag, status, kSiteQFull, s_unit);
+          ok = ok && mbar_wait_warp(&q_full[t], 0, abort_flag, kSiteQFull);
           if (ok) {
             tc_fence_after_sync();
             issue_s(0);
@@ -548,7 +548,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           const int st_next = (j + 1) % kStages;
           if (j + 1 < my_nkt) {
             // next scores first: they only need S_t(j) to have been read
-            ok = wait_k(j + 1) && mbar_wait_warp(&s_consumed[t], j & 1, abort_flag, status, kSiteSConsumed, s_unit);
+            ok = wait_k(j + 1) && mbar_wait_warp(&s_consumed[t], j & 1, abort_flag, kSiteSConsumed);
             if (!ok) break;
             tc_fence_after_sync();
             issue_s(st_next);
@@ -556,7 +556,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           }
           ok = wait_v(j);
           if (j < my_nkt) {
-            ok = ok && mbar_wait_warp((j & 1) ? &p_odd[t] : &p_full[t], (j >> 1) & 1, abort_flag, status, kSitePFull, s_unit);
+            ok = ok && mbar_wait_warp((j & 1) ? &p_odd[t] : &p_full[t], (j >> 1) & 1, abort_flag, kSitePFull);
             if (!ok) break;
             tc_fence_after_sync();
             issue_o(st, j > 0 ? 1u : 0u, tmem_p[t] + (j & 1) * kPCols);
@@ -618,7 +618,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       float ub = INFINITY;
       bool safe = false;                             // warp-wide: no row of this warp can overflow any more
       if (kSkipMax) {
-        ok = mbar_wait_warp(&q_full[t], qn & 1, abort_flag, status, kSiteQFull, s_unit);
+        ok = mbar_wait_warp(&q_full[t], qn & 1, abort_flag, kSiteQFull);
         if (!ok) break;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};         // independent sums: the chain is on every item's critical path
 #pragma unroll
@@ -731,7 +731,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // next scores can be loaded: three quarters of them travel under the last quarter's exponentials. Against a wait
         // for the scores, one for P's columns and two arrivals, each 130 to 220 clocks of a warp's 2900 per tile (traced):
         // B8 H16 N4096 causal 421 -> 401 us with the pre-pass, B64 H8 N1028 207 -> 198, B4 H12 N1000 full 39.4 -> 37.4.
-        ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, status, kSiteSFull, s_unit);
+        ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, kSiteSFull);
         if (!ok) break;
         ++md;
         tc_fence_after_sync();
@@ -740,7 +740,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int j = 0;; ++j, ++md) {
           bool group_done = false;
           const float neg_sub = -shift_of(j, [&]() {
-            ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, status, kSiteODone, s_unit);
+            ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, kSiteODone);
             if (ok) tc_fence_after_sync();
             return group_done = ok;
           });
@@ -749,7 +749,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
           for (int c = 0; c < 3; ++c) exponentials(c, neg_sub);
           if (!group_done) {
-            ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, status, kSiteSFull, s_unit);
+            ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, kSiteSFull);
             if (!ok) break;
             tc_fence_after_sync();
           }
@@ -788,19 +788,19 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           mbar_arrive(&stage_free[t]);
           store_pending = false;
         }
-        ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, status, kSiteODoneFinal, s_unit);
+        ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, kSiteODoneFinal);
         ++md;
-        if (ok && qn > 0) ok = mbar_wait_warp(&stage_free[t], (qn - 1) & 1, abort_flag, status, kSiteStageFree, s_unit);
+        if (ok && qn > 0) ok = mbar_wait_warp(&stage_free[t], (qn - 1) & 1, abort_flag, kSiteStageFree);
       } else {
         for (int j = 0; j < my_nkt; ++j) {
-          ok = mbar_wait_warp(&s_full[t], j & 1, abort_flag, status, kSiteSFull, s_unit);
+          ok = mbar_wait_warp(&s_full[t], j & 1, abort_flag, kSiteSFull);
           if (!ok) break;
           tc_fence_after_sync();
           load_scores();
           mbar_arrive_warp(&s_consumed[t]);
           auto wait_o = [&]() {
             // (phase j - 2 has passed: S_t(j) went to the tensor core behind P_t(j-2) V)
-            ok = mbar_wait_warp(&o_done[t], (j - 1) & 1, abort_flag, status, kSiteODone, s_unit);
+            ok = mbar_wait_warp(&o_done[t], (j - 1) & 1, abort_flag, kSiteODone);
             if (ok) tc_fence_after_sync();
             return ok;
           };
@@ -822,8 +822,8 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (!ok) break;
         // The last two products may be under way: their phases one after the other (a wait for the last one's parity alone
         // would be content with the phase two before it).
-        if (my_nkt > 1) ok = mbar_wait_warp(&o_done[t], (my_nkt - 2) & 1, abort_flag, status, kSiteODoneFinal, s_unit);
-        ok = ok && mbar_wait_warp(&o_done[t], (my_nkt - 1) & 1, abort_flag, status, kSiteODoneFinal, s_unit);
+        if (my_nkt > 1) ok = mbar_wait_warp(&o_done[t], (my_nkt - 2) & 1, abort_flag, kSiteODoneFinal);
+        ok = ok && mbar_wait_warp(&o_done[t], (my_nkt - 1) & 1, abort_flag, kSiteODoneFinal);
       }
       if (!ok) break;
       tc_fence_after_sync();
@@ -848,7 +848,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       tc_fence_before_sync();                        // the output has been read: the next item may accumulate into O_t
       fence_proxy_async_smem();
       mbar_arrive_warp(&grp_sync[t]);
-      ok = mbar_wait_warp(&grp_sync[t], qn & 1, abort_flag, status, kSiteGroup, s_unit);
+      ok = mbar_wait_warp(&grp_sync[t], qn & 1, abort_flag, kSiteGroup);
       if (!ok) break;
       if (storer) {
         for (int x = 0; x < kBoxes; ++x) tma_store_4d(&tm_o, stage + x * kBoxBytes, x * 64, r0, it.h, it.b);
@@ -872,6 +872,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (tid == 0) record_timeout(abort_flag, status, *s_unit);
   if (warp == kMmaWarp0) tmem_dealloc(tmem, 512);
   leave(queue);
 }

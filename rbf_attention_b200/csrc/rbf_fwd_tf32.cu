@@ -210,8 +210,8 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         umma_ss_tf32(tmem_s, sdesc_at(ones_desc, 0), sdesc_at(slab, 0), idesc_s, 1u);   // + key-norm bias
         umma_commit(s_full);
       };
-      bool ok = nkt > 0 && mbar_wait(q_full, 0, abort_flag, status, kSiteQFull) &&
-                mbar_wait(&k_full[0], 0, abort_flag, status, kSiteKvFull);
+      bool ok = nkt > 0 && mbar_wait(q_full, 0, abort_flag, kSiteQFull) &&
+                mbar_wait(&k_full[0], 0, abort_flag, kSiteKvFull);
       if (ok) {
         tc_fence_after_sync();
         issue_s(0);
@@ -219,7 +219,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       for (int j = 0; j < nkt && ok; ++j) {
         const int st = j % kStages;
         // p_full: P of tile j is in TMEM and the transposed V tile in shared memory
-        ok = mbar_wait(p_full, j & 1, abort_flag, status, kSitePFull);
+        ok = mbar_wait(p_full, j & 1, abort_flag, kSitePFull);
         if (!ok) break;
         tc_fence_after_sync();
         // a K step is 8 keys: 8 TMEM columns of P, 32 bytes of the K-major V^T rows (two boxes of 32 keys)
@@ -231,13 +231,13 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         umma_commit(&stage_free[st]);
         if (j + 1 < nkt) {
           // the scores were read before P was written, so S may be overwritten now
-          ok = mbar_wait(&k_full[(j + 1) % kStages], ((j + 1) / kStages) & 1, abort_flag, status, kSiteKvFull);
+          ok = mbar_wait(&k_full[(j + 1) % kStages], ((j + 1) / kStages) & 1, abort_flag, kSiteKvFull);
           if (!ok) break;
           tc_fence_after_sync();
           issue_s((j + 1) % kStages);
         }
         if (j + kStages < nkt) {
-          ok = mbar_wait(&stage_free[st], (j / kStages) & 1, abort_flag, status, kSiteStageFree);
+          ok = mbar_wait(&stage_free[st], (j / kStages) & 1, abort_flag, kSiteStageFree);
           if (!ok) break;
           load_stage(j + kStages);
         }
@@ -254,7 +254,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (!kSoftmax && nkt > 0) row_bias = qsq[static_cast<int64_t>(bh) * n_pad + row];
     bool ok = true;
     for (int j = 0; j < nkt; ++j) {
-      ok = mbar_wait_warp(s_full, j & 1, abort_flag, status, kSiteSFull);
+      ok = mbar_wait_warp(s_full, j & 1, abort_flag, kSiteSFull);
       if (!ok) break;
       tc_fence_after_sync();
       uint32_t raw[kKeys];
@@ -281,7 +281,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           l_sum *= alpha;
         }
         if (j > 0 && __any_sync(0xffffffffu, need)) {
-          ok = mbar_wait_warp(o_done, (j - 1) & 1, abort_flag, status, kSiteODone);
+          ok = mbar_wait_warp(o_done, (j - 1) & 1, abort_flag, kSiteODone);
           if (!ok) break;
           tc_fence_after_sync();
 #pragma unroll
@@ -308,7 +308,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       l_sum += ps;
       // P's columns are free once O += P V of the previous tile has completed
       if (j > 0) {
-        ok = mbar_wait_warp(o_done, (j - 1) & 1, abort_flag, status, kSiteODone);
+        ok = mbar_wait_warp(o_done, (j - 1) & 1, abort_flag, kSiteODone);
         if (!ok) break;
         tc_fence_after_sync();
       }
@@ -318,7 +318,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // 128-byte swizzle; thread = (key, half of the d chunks); the previous tile's MMAs have released V^T (o_done)
       {
         const int st = j % kStages;
-        ok = mbar_wait_warp(&v_full[st], (j / kStages) & 1, abort_flag, status, kSiteVFull);
+        ok = mbar_wait_warp(&v_full[st], (j / kStages) & 1, abort_flag, kSiteVFull);
         if (!ok) break;
         const int key = tid & 63, half = tid >> 6;
         const uint8_t* src = s_v + st * kKvBytes;
@@ -340,7 +340,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       tc_fence_before_sync();
       mbar_arrive_warp(p_full);
     }
-    if (ok && nkt > 0) ok = mbar_wait_warp(o_done, (nkt - 1) & 1, abort_flag, status, kSiteODone);
+    if (ok && nkt > 0) ok = mbar_wait_warp(o_done, (nkt - 1) & 1, abort_flag, kSiteODone);
     if (ok && nkt > 0) {
       tc_fence_after_sync();
       const float inv = kSoftmax ? (1.0f / l_sum) : 1.0f;
@@ -358,7 +358,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       fence_proxy_async_smem();
       mbar_arrive_warp(grp_sync);
-      ok = mbar_wait_warp(grp_sync, 0, abort_flag, status, kSiteGroup);
+      ok = mbar_wait_warp(grp_sync, 0, abort_flag, kSiteGroup);
       if (ok && r == 0) {
         for (int x = 0; x < 2; ++x) tma_store_4d(&tm_o, stage + x * kBoxBytes, x * 32, r0, h, b);
         tma_store_commit();
@@ -376,6 +376,7 @@ rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (tid == 0) record_timeout(abort_flag, status, status_unit());
   if (warp == 0) tmem_dealloc(tmem, 256);
   leave();
 }

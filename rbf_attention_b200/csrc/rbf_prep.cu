@@ -521,7 +521,7 @@ cudaError_t launch_xsa(const XsaArgs& a, bool backward, bool bf16, int D, cudaSt
   return bf16 ? launch_xsa_t<true, 128>(a, backward, stream) : launch_xsa_t<false, 128>(a, backward, stream);
 }
 
-__global__ void __launch_bounds__(32) wait_selftest_kernel(DeviceStatus* status, long long limit) {
+__global__ void __launch_bounds__(32) wait_selftest_kernel(DeviceStatus* status, uint32_t limit) {
   __shared__ uint64_t bar;
   __shared__ int abort_flag;
   if (threadIdx.x == 0) {
@@ -532,12 +532,13 @@ __global__ void __launch_bounds__(32) wait_selftest_kernel(DeviceStatus* status,
   __syncwarp();
   // Nothing ever arrives on `bar`. The warp's wait, with a limit of its own for every lane: all lanes leave it together,
   // with the same answer and the status recorded (a unit of 0xffffff says that they did not agree).
-  const bool ran_out = !mbar_wait_warp_limit(&bar, 0, &abort_flag, status, kSiteSelfTest, limit + 64 * threadIdx.x);
+  const bool ran_out = !mbar_wait_warp_limit(&bar, 0, &abort_flag, kSiteSelfTest, limit + 64 * threadIdx.x);
   const bool agree = __all_sync(0xffffffffu, ran_out);
   // One thread's wait: it raises the flag again.
   if (threadIdx.x == 0) {
+    record_timeout(&abort_flag, status, status_unit());
     abort_flag = 0;
-    const bool second = !mbar_wait_limit(&bar, 0, &abort_flag, status, kSiteSelfTest, limit);
+    const bool second = !mbar_wait_limit(&bar, 0, &abort_flag, kSiteSelfTest, limit);
     if (!agree || !second || abort_flag == 0) status->code = (kSiteSelfTest << 24) | 0xffffffu;
   }
   __syncwarp();
@@ -554,7 +555,7 @@ cudaError_t launch_post_status(const DeviceStatus* status, unsigned int* host_sl
 }
 
 cudaError_t launch_wait_selftest(DeviceStatus* status, long long limit, cudaStream_t stream) {
-  wait_selftest_kernel<<<1, 32, 0, stream>>>(status, limit);
+  wait_selftest_kernel<<<1, 32, 0, stream>>>(status, static_cast<uint32_t>(limit < kWaitCycleLimit ? limit : kWaitCycleLimit));
   return cudaGetLastError();
 }
 
