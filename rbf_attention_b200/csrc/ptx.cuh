@@ -131,16 +131,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 // The same wait by a whole converged warp: every lane gets the same answer. Lanes that decided for themselves could part
 // at a wait that runs out, one leaving for the end of the kernel while another goes on to a __syncwarp or a warp-wide
 // tensor-memory instruction and stands there without limit.
+// (One poll in the code, in the loop, not a first one before it: forward B64 H8 N1028 187 -> 184.5 us.)
 __device__ __forceinline__ bool mbar_wait_warp_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t site,
                                                      uint32_t limit) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   const uint32_t t0 = clock32();
+#pragma unroll 1
   while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
-    const bool late = clock32() - t0 > limit;
-    if (__any_sync(0xffffffffu, late || *abort_flag != 0)) {
-      if (late && *abort_flag == 0) *abort_flag = static_cast<int>(site);
-      return false;
-    }
+    if (clock32() - t0 > limit) *abort_flag = static_cast<int>(site);
+    if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
   }
   return true;
 }
