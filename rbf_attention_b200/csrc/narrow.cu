@@ -1,8 +1,9 @@
 // fp32 tensors on the fp16-operand kernels: narrowing of a call's inputs and widening of its gradients, one launch each.
 // Roofline: HBM / launch latency. PyTorch took one launch per tensor and direction, and the check whether an input left
 // fp16's range another five per tensor (an isinf, an any and an or, with temporaries): 40 launches and 157 us of device
-// time in a training pass at B2 H8 N1024 D64, against 10 launches with these two kernels (the range flag's clearing and its
-// posting are two of them); that pass: 426 -> 276 us (502 us with the calls going through the operators).
+// time in a training pass at B2 H8 N1024 D64, against 8 launches with these two kernels (the range flag's clearing is one of
+// them; the narrowing's last block posts it). That pass: 426 us with PyTorch's launches, 276 us with these kernels and a
+// posting launch of its own, 145-164 us now, with the calls prepared in the extension as well.
 #include <cuda_fp16.h>
 
 #include "launch.h"
