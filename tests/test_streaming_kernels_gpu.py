@@ -1,0 +1,37 @@
+"""GELU at the edges of its grids: a thread's second chunk missing, grids below, at and above what is resident."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n", [8, 2048, 2056, 4096, 4104, 148 * 6 * 4096, 148 * 6 * 4096 + 2056])
+def test_gelu_forward_chunks(n, dtype):
+    """Within one rounding step of the erf form in fp64 (2^-8 / 2^-11 relative, 3e-7 absolute for the approximation of the
+    normal distribution function), every element written, none beyond."""
+    from rbf_attention_b200 import ops
+
+    g = torch.Generator(device=DEV).manual_seed(n)
+    h = (torch.randn(n, generator=g, device=DEV) * 2).to(dtype)
+    want = F.gelu(h.double())
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert ((ops.gelu_fwd(h).double() - want).abs() <= rel * want.abs() + 3e-7).all()
+
+
+@pytest.mark.parametrize("rows, cols", [(1, 256), (7, 256), (64, 2048), (65, 264), (4097, 512), (6001, 2048), (700, 40960)])
+def test_gelu_backward_bands(rows, cols):
+    """dh within one rounding step of fp64; the bias gradient within fp32 summation error (2^-23 times the rows a lane
+    adds, at most 1e-5) of the sum of the stored dh."""
+    from rbf_attention_b200 import ops
+
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    h = (torch.randn((rows, cols), generator=g, device=DEV) * 2).bfloat16()
+    dy = torch.randn((rows, cols), generator=g, device=DEV).bfloat16()
+    x = h.double().requires_grad_(True)
+    F.gelu(x).backward(dy.double())
+    dh, db = ops.gelu_bwd(h, dy, True)
+    assert ((dh.double() - x.grad).abs() <= 2.0 ** -8 * x.grad.abs() + 3e-7 * dy.double().abs()).all()
+    assert ((db.double() - dh.double().sum(0)).abs() <= 1e-5 * dh.double().abs().sum(0) + 1e-6).all()
