@@ -5,9 +5,12 @@
 // one read and one write. Roofline: HBM. A block owns a row: pass 1 reads it from DRAM with an online maximum / sum
 // and keeps it in shared memory (100 KB per row at the benchmark's vocabulary, two blocks per SM), pass 2 writes
 // softmax - onehot, scaled by 1 / (rows that count), from there. Rows too long for that are read a second time
-// (with two blocks per SM in flight they are L2 hits). Measured at 65536 x 50304 bf16: 2.89 ms, 4.57 TB/s = 71 % of the
-// copy bandwidth (2.93 ms with maxima, scaling and sums one element at a time; 8192 x 32000: 301 -> 292 us, 3108 x 50304:
-// 200.5 -> 198.4 us, in turn on one GPU). exp2f() in place of the bare ex2.approx took 11 % longer. Block shapes of 256 to
+// (with two blocks per SM in flight they are L2 hits). While a staged row is reduced and written, the block's next row is
+// on its way into L2, and neither is kept there afterwards. Measured at 65536 x 50304 bf16: 2.47 ms, 5.33 TB/s = 83 % of
+// the copy bandwidth, without the next row's prefetch 2.88 ms (8192 x 32000: 292 -> 271 us, 8192 x 50304: 418 -> 372 us,
+// 3108 x 50304: 201 -> 185 us, 16384 x 4096: 192 -> 176 us, in turn on one GPU). Asked for at the start of a row instead of
+// behind its pass 1 the prefetch brings nothing (2.96 ms), one slice per warp inside pass 2 less (2.72 ms); for rows that are
+// read twice it evicts the second read (8192 x 128256: 1.15 -> 1.35 ms) and is left out. exp2f() in place of the bare ex2.approx took 11 % longer. Block shapes of 256 to
 // 512 threads, two to eight per SM, staged or re-read, all land within 10 % of each other; a variant with one block of 1024
 // threads per SM that streams the next row into a second buffer with cp.async while the current one is reduced was slower
 // (3.82 ms) and is not kept.
@@ -29,6 +32,10 @@ __device__ __forceinline__ float ce_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// Brings a row (16-byte aligned, a multiple of 16 bytes) into L2; nothing waits for it.
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 constexpr float kLn2 = 0.6931471805599453f;
 
@@ -91,12 +98,16 @@ __global__ void __launch_bounds__(kCeThreads, 2) cross_entropy_kernel(const Cros
   const float scale = *a.grad_scale;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
+  auto counted = [&](int64_t t) { return t != a.ignore_index && t >= 0 && t < a.cols; };
+  int64_t t_next = blockIdx.x < a.rows ? a.targets[blockIdx.x] : 0;
   for (int row = blockIdx.x; row < a.rows; row += gridDim.x) {
     const T* x = static_cast<const T*>(a.logits) + static_cast<int64_t>(row) * a.ld;
     T* dx = static_cast<T*>(a.dlogits) + static_cast<int64_t>(row) * a.ld_out;
-    const int64_t t = a.targets[row];
-    const bool counts = t != a.ignore_index && t >= 0 && t < a.cols;
-    if (!counts) {                                // no loss, zero gradient: the row is not read
+    const int64_t t = t_next;
+    const bool more = static_cast<int>(gridDim.x) < a.rows - row;
+    if (more) t_next = a.targets[row + gridDim.x];
+    const bool next_counts = more && counted(t_next);
+    if (!counted(t)) {                                // no loss, zero gradient: the row is not read
       if constexpr (kVec) {
         for (int c = threadIdx.x; c < a.cols / V; c += kCeThreads) reinterpret_cast<uint4*>(dx)[c] = make_uint4(0, 0, 0, 0);
       } else {
@@ -110,7 +121,7 @@ __global__ void __launch_bounds__(kCeThreads, 2) cross_entropy_kernel(const Cros
     if constexpr (kVec) {
 #pragma unroll 4                                    // two blocks per SM: 4 x 16 bytes per thread keep 64 KB in flight
       for (int c = threadIdx.x; c < a.cols / V; c += kCeThreads) {
-        const uint4 raw = reinterpret_cast<const uint4*>(x)[c];
+        const uint4 raw = kStage ? __ldcs(reinterpret_cast<const uint4*>(x) + c) : reinterpret_cast<const uint4*>(x)[c];
         if constexpr (kStage) s_row[c] = raw;
         const T* e = reinterpret_cast<const T*>(&raw);
         float xv[V];
@@ -142,6 +153,11 @@ __global__ void __launch_bounds__(kCeThreads, 2) cross_entropy_kernel(const Cros
         }
         if (m != -INFINITY) s += ce_ex2(y - m);
       }
+    }
+    if constexpr (kStage) {
+      // the block's next row comes into L2 while this one is reduced and written: its pass 1 then waits for L2 only
+      if (threadIdx.x == kCeThreads - 32 && next_counts)
+        prefetch_l2(static_cast<const T*>(a.logits) + (row + static_cast<int64_t>(gridDim.x)) * a.ld, a.cols * sizeof(T));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -201,7 +217,8 @@ __global__ void __launch_bounds__(kCeThreads, 2) cross_entropy_kernel(const Cros
           for (int j = 0; j < 4; ++j) w[j] = pack2<kDtype == 0>(p[(2 * j) % V], p[(2 * j + 1) % V]);
           out = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        reinterpret_cast<uint4*>(dx)[c] = out;
+        if constexpr (kStage) __stcs(reinterpret_cast<uint4*>(dx) + c, out);
+        else reinterpret_cast<uint4*>(dx)[c] = out;
       }
     } else {
       for (int c = threadIdx.x; c < a.cols; c += kCeThreads) {

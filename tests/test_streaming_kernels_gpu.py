@@ -1,4 +1,5 @@
-"""GELU at the edges of its grids: a thread's second chunk missing, grids below, at and above what is resident."""
+"""GELU and cross entropy at the edges of their grids: a thread's second chunk missing, grids below, at and above what is
+resident, rows that are brought into L2 ahead, rows that do not count among them."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -35,3 +36,29 @@ def test_gelu_backward_bands(rows, cols):
     dh, db = ops.gelu_bwd(h, dy, True)
     assert ((dh.double() - x.grad).abs() <= 2.0 ** -8 * x.grad.abs() + 3e-7 * dy.double().abs()).all()
     assert ((db.double() - dh.double().sum(0)).abs() <= 1e-5 * dh.double().abs().sum(0) + 1e-6).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows, cols", [(1, 64), (295, 1000), (296, 1000), (297, 1000), (900, 4104), (640, 28920), (610, 57864)])
+def test_cross_entropy_rows_brought_in_ahead(rows, cols, dtype):
+    """Loss and gradient against fp64 with every third row ignored (the block's next row may or may not count), rows of
+    odd widths for the staged, the re-read and (1000 columns of a wider tensor) the strided case. Gradients within one
+    rounding step of the dtype (fp32: the exponential's 2^-21) of softmax / count, plus what a loss sum error of 1e-6 gives."""
+    from rbf_attention_b200 import ops
+
+    g = torch.Generator(device=DEV).manual_seed(rows + cols)
+    x = (torch.randn((rows, cols + 24), generator=g, device=DEV) * 3).to(dtype)[:, :cols]
+    t = torch.randint(0, cols, (rows,), generator=g, device=DEV)
+    t[1::3] = -100
+    ref_in = x.double().requires_grad_(True)
+    ref = F.cross_entropy(ref_in, t, ignore_index=-100)
+    ref.backward()
+    a = x.detach().requires_grad_(True)
+    loss = ops.cross_entropy(a, t)
+    loss.backward()
+    assert abs(loss.item() - ref.item()) <= 2e-6 * abs(ref.item()) + 1e-6
+    rel = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -18}[dtype]
+    tiny = 6e-8 if dtype == torch.float16 else 2e-6 / rows          # fp16 subnormals: spacing 2^-24
+    err = (a.grad.double() - ref_in.grad).abs()
+    assert (err <= rel * ref_in.grad.abs() + tiny).all()
+    assert (a.grad[1::3] == 0).all()
