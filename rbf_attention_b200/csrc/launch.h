@@ -36,7 +36,6 @@ struct RowStatsArgs {
   int head_dim;           // columns of the tensors, a multiple of 8 up to the kernel's D
   float scale;
   float qsq_pad;
-  int iters;              // set by the launcher
   DeviceStatus* status_to_clear;  // optional: the 256-byte status block (status word, work counters) is zeroed
 };
 cudaError_t launch_row_stats(const RowStatsArgs& a, bool bf16, int D, cudaStream_t stream);

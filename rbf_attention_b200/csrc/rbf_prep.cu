@@ -47,8 +47,16 @@ __device__ __forceinline__ uint4 load_chunk(const void* base, const int64_t* s, 
                                          static_cast<int64_t>(row) * s[2] + part * 8);
 }
 
-template <bool kBf16, int D>
-__global__ void __launch_bounds__(256) row_stats_kernel(const RowStatsArgs a) {
+// Bytes in flight bound it: a row's tensors are asked for together (forward: two rows at a time), and registers are kept to
+// what leaves seven blocks on an SM. Against one tensor after the other, forward and backward in one kernel (36 registers),
+// microseconds, forward and backward call:
+//   B8 H16 N4096 D64   26.9 -> 23.2, 68.8 -> 60.3      B2 H32 N16384 D128  101 -> 89, 212 -> 191
+//   B4 H16 N8192 D64 without softmax  39.1 -> 31.5, 77.5 -> 69.1      B4 H8 N1024 D64  4.9 -> 3.6, 8.2 -> 6.3
+// (Forward four rows at a time 23.6; backward two rows at six blocks 61.4, four at five 76.9; two or eight rows per lane
+// instead of four 61-64 and 69 in the backward; a row's stores spread over its lanes, every lane computing them, 73.5.)
+constexpr int kStatIters = 4;                    // rows per lane group
+template <bool kBf16, int D, bool kBack>         // kBack: O and dO are there (and only then an accumulator to clear)
+__global__ void __launch_bounds__(256, 7) row_stats_kernel(const RowStatsArgs a) {
   constexpr int kLanesPerRow = D / 8;                 // 8 (D=64) or 16 (D=128)
   constexpr int kRowsPerWarp = 32 / kLanesPerRow;     // 4 or 2
   grid_dependents_launch();
@@ -60,58 +68,64 @@ __global__ void __launch_bounds__(256) row_stats_kernel(const RowStatsArgs a) {
   const int part = lane % kLanesPerRow;               // 16-byte chunk of the row
   const int bh = blockIdx.y;
   const int b = bh / a.H, h = bh % a.H;
-  const int rows_per_block = 8 * kRowsPerWarp * a.iters;
+  const int rows_per_block = 8 * kRowsPerWarp * kStatIters;
   const int row_begin = blockIdx.x * rows_per_block;
   const int64_t out_base = static_cast<int64_t>(bh) * a.n_pad;
 
-  if (a.zero_rows != nullptr) {
-    // clear this block's rows of the fp32 accumulator: the writes ride along with a kernel that mostly reads
-    const int rows_here = min(rows_per_block, a.N - row_begin);
-    if (rows_here > 0) {
-      float4* dst = reinterpret_cast<float4*>(a.zero_rows + (static_cast<int64_t>(bh) * a.N + row_begin) * D);
-      const int n4 = rows_here * (D / 4);
-      for (int i = threadIdx.x; i < n4; i += 256) dst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  for (int it = 0; it < a.iters; ++it) {
-    const int row = row_begin + (it * 8 + warp) * kRowsPerWarp + sub;
-    const bool valid = row < a.N;
-    float ksq = 0.f, qsq = 0.f, delta = 0.f;
-    if (valid && part * 8 < a.head_dim) {
-      if (a.k != nullptr) {
-        const uint4 v = load_chunk(a.k, a.ks, b, h, row, part);
-        ksq = dot8<kBf16>(v, v);
+  constexpr int kBatch = kBack ? 1 : 2;
+#pragma unroll 1
+  for (int it0 = 0; it0 < kStatIters; it0 += kBatch) {
+    // the batch's loads first, then row after row
+    uint4 kv[kBatch], ov[kBatch], gv[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int row = row_begin + ((it0 + u) * 8 + warp) * kRowsPerWarp + sub;
+      kv[u] = ov[u] = gv[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (row < a.N && part * 8 < a.head_dim) {
+        if (kBack) {
+          ov[u] = load_chunk(a.o, a.os, b, h, row, part);
+          gv[u] = load_chunk(a.dout, a.dos, b, h, row, part);
+        }
+        if (a.k != nullptr) kv[u] = load_chunk(a.k, a.ks, b, h, row, part);
       }
-      if (a.q != nullptr) {
-        const uint4 v = load_chunk(a.q, a.qs, b, h, row, part);
-        qsq = dot8<kBf16>(v, v);
-      }
-      if (a.o != nullptr) {
-        const uint4 x = load_chunk(a.o, a.os, b, h, row, part);
-        const uint4 y = load_chunk(a.dout, a.dos, b, h, row, part);
-        delta = dot8<kBf16>(x, y);
+      if (kBack && a.zero_rows != nullptr && row < a.N) {
+        // the fp32 accumulator's row: these writes ride along with a kernel that mostly reads
+        float4* dst = reinterpret_cast<float4*>(a.zero_rows + (static_cast<int64_t>(bh) * a.N + row) * D) + part;
+        dst[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+        dst[kLanesPerRow] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
 #pragma unroll
-    for (int o = kLanesPerRow / 2; o > 0; o >>= 1) {
-      ksq += __shfl_xor_sync(0xffffffffu, ksq, o);
-      qsq += __shfl_xor_sync(0xffffffffu, qsq, o);
-      delta += __shfl_xor_sync(0xffffffffu, delta, o);
-    }
-    if (part == 0 && row < a.n_pad) {
-      if (a.ksq_out != nullptr) a.ksq_out[out_base + row] = valid ? ksq * a.scale : INFINITY;
-      if (a.qsq_out != nullptr) a.qsq_out[out_base + row] = valid ? qsq * a.scale : a.qsq_pad;
-      if (a.delta_out != nullptr) a.delta_out[out_base + row] = delta;
-      float lse = INFINITY;
-      if (a.lse != nullptr && valid) lse = a.lse[static_cast<int64_t>(bh) * a.N + row];
-      if (a.lse_pad_out != nullptr) a.lse_pad_out[out_base + row] = lse;
-      const float inv = 1.0f / (a.scale2 * a.slab_w);
-      if (a.kslab_out != nullptr) store_slab_row<kBf16>(a.kslab_out, out_base + row, valid ? -ksq * a.scale * inv : -a.slab_big);
-      const float row_stat = a.lslab_from_qsq ? qsq * a.scale : lse;
-      if (a.lslab_out != nullptr)
-        store_slab_row<kBf16>(a.lslab_out, out_base + row, valid ? -row_stat * inv : -a.slab_big);
-      if (a.dslab_out != nullptr)
-        store_slab_row<kBf16>(a.dslab_out, out_base + row, a.dslab_zero ? 0.f : -delta / a.slab_w);
+    for (int u = 0; u < kBatch; ++u) {
+      const int row = row_begin + ((it0 + u) * 8 + warp) * kRowsPerWarp + sub;
+      const bool valid = row < a.N;
+      float ksq = dot8<kBf16>(kv[u], kv[u]), qsq = 0.f, delta = 0.f;
+      if (a.q != nullptr && valid && part * 8 < a.head_dim) {
+        const uint4 v = load_chunk(a.q, a.qs, b, h, row, part);
+        qsq = dot8<kBf16>(v, v);
+      }
+      if (kBack) delta = dot8<kBf16>(ov[u], gv[u]);
+#pragma unroll
+      for (int o = kLanesPerRow / 2; o > 0; o >>= 1) {
+        ksq += __shfl_xor_sync(0xffffffffu, ksq, o);
+        qsq += __shfl_xor_sync(0xffffffffu, qsq, o);
+        delta += __shfl_xor_sync(0xffffffffu, delta, o);
+      }
+      if (part == 0 && row < a.n_pad) {
+        if (a.ksq_out != nullptr) a.ksq_out[out_base + row] = valid ? ksq * a.scale : INFINITY;
+        if (a.qsq_out != nullptr) a.qsq_out[out_base + row] = valid ? qsq * a.scale : a.qsq_pad;
+        if (a.delta_out != nullptr) a.delta_out[out_base + row] = delta;
+        float lse = INFINITY;
+        if (a.lse != nullptr && valid) lse = a.lse[static_cast<int64_t>(bh) * a.N + row];
+        if (a.lse_pad_out != nullptr) a.lse_pad_out[out_base + row] = lse;
+        const float inv = 1.0f / (a.scale2 * a.slab_w);
+        if (a.kslab_out != nullptr) store_slab_row<kBf16>(a.kslab_out, out_base + row, valid ? -ksq * a.scale * inv : -a.slab_big);
+        const float row_stat = a.lslab_from_qsq ? qsq * a.scale : lse;
+        if (a.lslab_out != nullptr)
+          store_slab_row<kBf16>(a.lslab_out, out_base + row, valid ? -row_stat * inv : -a.slab_big);
+        if (a.dslab_out != nullptr)
+          store_slab_row<kBf16>(a.dslab_out, out_base + row, a.dslab_zero ? 0.f : -delta / a.slab_w);
+      }
     }
   }
 }
@@ -119,10 +133,10 @@ __global__ void __launch_bounds__(256) row_stats_kernel(const RowStatsArgs a) {
 template <bool kBf16, int D>
 static cudaError_t launch_row_stats_t(RowStatsArgs a, cudaStream_t stream) {
   constexpr int kRowsPerWarp = 32 / (D / 8);
-  a.iters = 4;
-  const int rows_per_block = 8 * kRowsPerWarp * a.iters;
+  const int rows_per_block = 8 * kRowsPerWarp * kStatIters;
   dim3 grid((a.n_pad + rows_per_block - 1) / rows_per_block, a.B * a.H);
-  row_stats_kernel<kBf16, D><<<grid, 256, 0, stream>>>(a);
+  if (a.o != nullptr) row_stats_kernel<kBf16, D, true><<<grid, 256, 0, stream>>>(a);
+  else row_stats_kernel<kBf16, D, false><<<grid, 256, 0, stream>>>(a);
   return cudaGetLastError();
 }
 
@@ -251,6 +265,11 @@ __global__ void __launch_bounds__(256) qkv_prep_kernel(const QkvPrepArgs a) {
     const bool valid = in_range && s < a.S;
     float ksq = 0.f, qsq = 0.f;
     if (valid) {
+      // the rows are asked for ahead of the parameters: B64 S1028 H8 D64 65 -> 55 us, B4 S4100 H8 D64 fp16 13.1 as before
+      const uint16_t* src = reinterpret_cast<const uint16_t*>(a.qkv) + (static_cast<int64_t>(b) * a.S + s) * 3 * E +
+                            static_cast<int64_t>(h) * D + part * 8;
+      const uint4 qv = *reinterpret_cast<const uint4*>(src);
+      const uint4 kv = *reinterpret_cast<const uint4*>(src + E);
       float e[8];
       if (s < a.R) {
         load_param8(a.reg_pos, (static_cast<int64_t>(h) * a.R + s) * D + part * 8, a.params_fp32, kBf16, e);
@@ -262,10 +281,6 @@ __global__ void __launch_bounds__(256) qkv_prep_kernel(const QkvPrepArgs a) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) e[j] *= tv[j];
       }
-      const uint16_t* src = reinterpret_cast<const uint16_t*>(a.qkv) + (static_cast<int64_t>(b) * a.S + s) * 3 * E +
-                            static_cast<int64_t>(h) * D + part * 8;
-      const uint4 qv = *reinterpret_cast<const uint4*>(src);
-      const uint4 kv = *reinterpret_cast<const uint4*>(src + E);
       const uint4 qn = add_round8<kBf16>(qv, e, qsq);
       const uint4 kn = add_round8<kBf16>(kv, e, ksq);
       *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.q_out) + b * a.qo[0] + h * a.qo[1] +

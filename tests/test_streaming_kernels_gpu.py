@@ -1,5 +1,5 @@
-"""GELU and cross entropy at the edges of their grids: a thread's second chunk missing, grids below, at and above what is
-resident, rows that are brought into L2 ahead, rows that do not count among them."""
+"""GELU, cross entropy and the pre-passes at the edges of their grids: a thread's second chunk missing, grids below, at and above
+what is resident, rows that are brought into L2 ahead, rows that do not count among them, ragged lengths."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -62,3 +62,27 @@ def test_cross_entropy_rows_brought_in_ahead(rows, cols, dtype):
     err = (a.grad.double() - ref_in.grad).abs()
     assert (err <= rel * ref_in.grad.abs() + tiny).all()
     assert (a.grad[1::3] == 0).all()
+
+
+@pytest.mark.parametrize("softmax", [True, False])
+@pytest.mark.parametrize("D", [64, 72, 128])
+@pytest.mark.parametrize("N", [1, 31, 33, 63, 65, 97, 129])
+def test_row_statistics_at_ragged_lengths(N, D, softmax):
+    """The pre-passes' rows that fill part of a batch, a warp's group or a block: outputs and gradients against the fp32 oracle
+    (2^-11 relative rounding of operands, P, dS and results over sums of independent terms), on a workspace that a longer call
+    has left behind."""
+    from oracle import rbf_oracle as oracle
+    from rbf_attention_b200 import ops
+
+    for n in (2 * N + 200, N):
+        q, k, v, do = oracle.make_inputs(2, 3, n, D, seed=n, dtype=torch.float16, std=1.0 if softmax else 0.3)
+        ref = oracle.torch_forward_backward(q, k, v, do, True, softmax, dtype=torch.float32)
+        qd, kd, vd, dod = (x.to(DEV) for x in (q, k, v, do))
+        out, lse = ops._forward(qd, kd, vd, True, softmax)
+        grads = ops._backward(qd, kd, vd, out, lse, dod, True, D ** -0.5, softmax)
+        ops.check_device_status()
+        for got, want in zip((out, *grads[:3]), (ref[0], *ref[-3:])):
+            rep = oracle.error_report(got.cpu().float(), want)
+            # a single key: dq and dk are exactly zero, their error that of dP and delta, two fp32 sums of up to 128 products
+            # in different orders: 2^-24 * 128 * 4 * 4 times 2 D^-0.5 |k| <= 2 * 0.125 * 5
+            assert rep["rel_l2"] <= 3e-3 or n == 1 and rep["max_abs"] <= 1.6e-4, rep
