@@ -101,14 +101,14 @@ struct Params {
   DeviceStatus* status;
   unsigned int* work;    // [0] items taken beyond the CTAs' first, [1] CTAs that have left; zero at launch and at its end
   int total_items;       // key tiles x (batch, head) pairs
+  int plain_heads, group;   // order of the items (decode_item)
   int H, N, n_pad, causal;
   float scale2, grad_scale, slab_w;
 };
 
 // The launch is persistent and its items overlap: a CTA per SM, each starting with item blockIdx.x and taking further
-// (key tile, batch-head) items from a global counter in the order a plain grid would run them (key tile fastest,
-// heaviest causal tile first). TMEM, the barriers (their phases run on) and the Q / dO rings carry on from item to item;
-// K and the key norms have two buffers, V is reloaded as soon as the item's last dP^T has read it, and the drain warps
+// (key tile, batch-head) items from a global counter, in decode_item's order. TMEM, the barriers (their phases run on) and
+// the Q / dO rings carry on from item to item; K and the key norms have two buffers, V is reloaded as soon as the item's last dP^T has read it, and the drain warps
 // bring dK and dV out, so that the compute warps - the critical resource - go straight on to the next item's scores.
 template <bool kBf16>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -179,10 +179,11 @@ rbf_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     cnt = n_tiles - first;
   };
   auto set_item = [&](int item) {
-    bh = item / n_tiles;
+    int tile;
+    decode_item(item, n_tiles, p.plain_heads, p.group, bh, tile);
     b = bh / p.H;
     h = bh % p.H;
-    set_tile(item - bh * n_tiles);
+    set_tile(tile);
   };
   // The next item as the issuer, drain and compute warps see it; false at the end of the sequence or when the launch is
   // being abandoned.
@@ -759,7 +760,10 @@ static cudaError_t launch_t(const BwdFusedArgs& a, cudaStream_t stream) {
   p.H = a.H; p.N = a.N; p.n_pad = a.n_pad; p.causal = a.causal;
   p.scale2 = a.scale2; p.grad_scale = a.grad_scale; p.slab_w = a.slab_w;
   p.work = a.work;
-  p.total_items = ((a.N + kTile - 1) / kTile) * a.B * a.H;
+  const int n_tiles = (a.N + kTile - 1) / kTile;
+  p.total_items = n_tiles * a.B * a.H;
+  p.group = item_group(n_tiles, a.B * a.H, a.causal, a.sm_count);
+  p.plain_heads = a.B * a.H - p.group;
   dim3 grid(p.total_items < a.sm_count ? p.total_items : a.sm_count);
   e = launch_dependent(kernel, grid, kThreads, smem, stream, a.tm_k, a.tm_v, a.tm_q, a.tm_do, a.tm_dk, a.tm_dv, a.tm_lslab,
                        a.tm_dslab, a.tm_dq_acc, p);

@@ -88,6 +88,7 @@ struct Params {
   float* dq_acc;         // fp32 (B, H, N, 128), zero-initialised
   DeviceStatus* status;
   int H, N, n_pad, causal;
+  int plain_heads, group;   // order of the items (decode_item)
   float scale2, grad_scale, slab_w;
 };
 
@@ -134,9 +135,9 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   // item sizes read from shared memory, it changes nothing or costs 1 %.)
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
-  const int bh = blockIdx.y;
+  int bh, kt;                                      // key tile; tile 0 is the heaviest under the causal mask
+  decode_item(blockIdx.x, (p.N + kTile - 1) / kTile, p.plain_heads, p.group, bh, kt);
   const int b = bh / p.H, h = bh % p.H;
-  const int kt = blockIdx.x;                       // key tile; tile 0 is the heaviest under the causal mask
   const int k_row0 = kt * kTile;
   const int n_steps_all = (p.N + kQStep - 1) / kQStep;
   const int first = p.causal ? 2 * kt : 0;         // first 64-query step that sees these keys
@@ -601,7 +602,10 @@ static cudaError_t launch_t(const BwdFusedArgs& a, cudaStream_t stream) {
   p.dq_acc = a.dq_acc; p.status = a.status;
   p.H = a.H; p.N = a.N; p.n_pad = a.n_pad; p.causal = a.causal;
   p.scale2 = a.scale2; p.grad_scale = a.grad_scale; p.slab_w = a.slab_w;
-  dim3 grid((a.N + kTile - 1) / kTile, a.B * a.H);
+  const int n_tiles = (a.N + kTile - 1) / kTile;
+  dim3 grid(n_tiles * a.B * a.H);
+  p.group = item_group(n_tiles, a.B * a.H, a.causal, a.sm_count);
+  p.plain_heads = a.B * a.H - p.group;
   e = launch_dependent(kernel, grid, kThreads, smem, stream, a.tm_k, a.tm_v, a.tm_q, a.tm_do, a.tm_dk, a.tm_dv, a.tm_lslab,
                        a.tm_dslab, p);
   if (e != cudaSuccess) return e;

@@ -86,3 +86,23 @@ def test_row_statistics_at_ragged_lengths(N, D, softmax):
             # a single key: dq and dk are exactly zero, their error that of dP and delta, two fp32 sums of up to 128 products
             # in different orders: 2^-24 * 128 * 4 * 4 times 2 D^-0.5 |k| <= 2 * 0.125 * 5
             assert rep["rel_l2"] <= 3e-3 or n == 1 and rep["max_abs"] <= 1.6e-4, rep
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B, H, N", [(1, 1, 700), (5, 20, 300), (2, 85, 129), (3, 67, 64), (1, 38, 900)])
+def test_backward_items_in_groups_of_heads(B, H, N, D):
+    """Every (key tile, head) item is worked on once, whatever the number of heads leaves for the first group (few heads, one
+    group, a short first group, one key tile): gradients of each head by itself against the fp32 oracle."""
+    from oracle import rbf_oracle as oracle
+    from rbf_attention_b200 import ops
+
+    q, k, v, do = oracle.make_inputs(B, H, N, D, seed=N, dtype=torch.float16, std=1.0)
+    qd, kd, vd, dod = (x.to(DEV) for x in (q, k, v, do))
+    for causal in (True, False):
+        ref = oracle.torch_forward_backward(q, k, v, do, causal, True, dtype=torch.float32)[-3:]
+        out, lse = ops._forward(qd, kd, vd, causal, True)
+        grads = ops._backward(qd, kd, vd, out, lse, dod, causal, D ** -0.5, True)
+        ops.check_device_status()
+        for got, want in zip(grads[:3], ref):
+            err = (got.cpu().float() - want).flatten(2).norm(dim=2) / want.flatten(2).norm(dim=2)
+            assert err.max().item() <= 3e-3       # 2^-11 relative rounding of operands, P, dS and results
