@@ -91,7 +91,7 @@ struct Smem {
   static constexpr int kStage = kPersistent ? kOnes + kTile * 32 : kQ;
   static constexpr int kBars = kOnes + kTile * 32 + (kPersistent ? 2 * kTileBytes : 0);
   static constexpr int kItemSlots = 4;                     // ring of work item numbers, producer -> all other roles
-  static constexpr int kNumBars = 2 + 4 * kStages + 12 + 4 + 2 * kItemSlots;
+  static constexpr int kNumBars = 2 + 4 * kStages + 14 + 4 + 2 * kItemSlots;
   static constexpr int kMisc = kBars + kNumBars * 8;        // tmem base, abort flag
   static constexpr int kTotal = kMisc + 16 + 16 * kItemSlots;
   static constexpr int kDynamic = kTotal + 1024;            // slack for 1024-byte alignment
@@ -188,11 +188,16 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   uint64_t* k_empty = k_full + kStages;          // two arrivals: one per issuer
   uint64_t* v_full = k_empty + kStages;
   uint64_t* v_empty = v_full + kStages;          // two arrivals
-  uint64_t* s_full = v_empty + kStages;          // [2] S_t(j) complete; persistent: and P_t(j-2) V
+  uint64_t* s_full = v_empty + kStages;          // [2] S_t(j) complete; persistent: and P_t(j-2) V, but not an item's last
   uint64_t* p_full = s_full + 2;                 // [2] P_t(j) stored; persistent: and S_t(j+1) in the group's registers
   uint64_t* p_odd = p_full + 2;                  // [2] one item per CTA: p_full of the odd tiles (see there)
-  uint64_t* o_done = p_odd + 2;                  // [2] P_t(j) V complete (one item per CTA)
-  uint64_t* grp_sync = o_done + 2;               // [2] rendezvous of the warps of a query tile
+  // [2] the item's last P_t V complete; one item per CTA: P_t(j) V of the even tiles complete, o_odd: of the odd tiles. The
+  // warps wait for these phases late or not at all, so the next phase of the same barrier must not complete before they have
+  // looked (a wait that comes after it stands until it runs out): it takes P of the next item or of the tile after next, that
+  // is their own arrival.
+  uint64_t* o_done = p_odd + 2;
+  uint64_t* o_odd = o_done + 2;
+  uint64_t* grp_sync = o_odd + 2;                // [2] rendezvous of the warps of a query tile
   uint64_t* s_consumed = grp_sync + 2;           // [2] the group holds S_t(j) in registers (one item per CTA)
   uint64_t* q_free = s_consumed + 2;             // [2] persistent: Q_t may be overwritten (issuer + softmax warps)
   uint64_t* stage_free = q_free + 2;             // [2] persistent: the previous output store has read its staging tile
@@ -299,6 +304,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       mbar_init(&p_full[t], 4 * kSplit);     // one arrival per softmax warp of the tile
       mbar_init(&p_odd[t], 4 * kSplit);
       mbar_init(&o_done[t], 1);
+      mbar_init(&o_odd[t], 1);
       mbar_init(&grp_sync[t], 4 * kSplit);
       mbar_init(&s_consumed[t], 4 * kSplit);
       mbar_init(&q_free[t], 1 + 4 * kSplit);
@@ -357,10 +363,10 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   // Counters that run on across a CTA's items, kept identically by every role that needs them:
   //   G      K/V tiles put through the ring by earlier items (tile j of the item uses stage (G + j) % kStages in
   //          round (G + j) / kStages)
-  //   md     phases of s_full[t] so far: per item one for its first scores and one for each group of MMAs
+  //   md     phases of s_full[t] so far: per item one for its first scores and one for each group of MMAs but the last
   //   td     phases of p_full[t] so far: per item one for its first scores and one for each P
-  //   qn     loads of Q_t by earlier items (phase of q_full, q_free; also of grp_sync and stage_free: one output
-  //          store per load)
+  //   qn     loads of Q_t by earlier items (phase of q_full, q_free; also of o_done, grp_sync and stage_free: one output
+  //          per load)
   if (warp == kLoadWarp) {
     // ------------------------------------------------------------------ TMA producer
     setmaxnreg_dec<R::kOtherRegs>();
@@ -485,7 +491,8 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
               umma_commit(&k_empty[G % kStages]);
             }
             // Group j of the item's MMAs, j = 0 .. my_nkt: P_t(j-1) V and the scores S_t(j+1), once the softmax group has
-            // stored the one and holds S_t(j) in registers. One commit covers both.
+            // stored the one and holds S_t(j) in registers. One commit covers both. (The last group's is a barrier of its
+            // own: the next item's first scores may complete before every warp of the group has seen it.)
             for (int j = 0; j <= my_nkt; ++j) {
               ok = mbar_wait_warp(&p_full[t], (td + j) & 1, abort_flag, kSitePFull);
               if (!ok) break;
@@ -507,7 +514,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                   umma_commit(&k_empty[st]);
                 }
               }
-              if (el) umma_commit(&s_full[t]);
+              if (el) umma_commit(j < my_nkt ? &s_full[t] : &o_done[t]);
             }
             if (!ok) break;
             td += my_nkt + 1;
@@ -561,7 +568,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             tc_fence_after_sync();
             issue_o(st, j > 0 ? 1u : 0u, tmem_p[t] + (j & 1) * kPCols);
             if (el) {
-              umma_commit(&o_done[t]);
+              umma_commit((j & 1) ? &o_odd[t] : &o_done[t]);
               umma_commit(&v_empty[st]);
             }
           } else {
@@ -788,10 +795,13 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           mbar_arrive(&stage_free[t]);
           store_pending = false;
         }
-        ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, kSiteODoneFinal);
-        ++md;
+        ok = mbar_wait_warp(&o_done[t], qn & 1, abort_flag, kSiteODoneFinal);
         if (ok && qn > 0) ok = mbar_wait_warp(&stage_free[t], (qn - 1) & 1, abort_flag, kSiteStageFree);
       } else {
+        // P_t(j) V complete. Its barrier's phase before is that of P_t(j-2) V, which is over when S_t(j) has been seen.
+        auto wait_product = [&](int j, uint32_t site) {
+          return mbar_wait_warp((j & 1) ? &o_odd[t] : &o_done[t], (j >> 1) & 1, abort_flag, site);
+        };
         for (int j = 0; j < my_nkt; ++j) {
           ok = mbar_wait_warp(&s_full[t], j & 1, abort_flag, kSiteSFull);
           if (!ok) break;
@@ -799,8 +809,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           load_scores();
           mbar_arrive_warp(&s_consumed[t]);
           auto wait_o = [&]() {
-            // (phase j - 2 has passed: S_t(j) went to the tensor core behind P_t(j-2) V)
-            ok = mbar_wait_warp(&o_done[t], (j - 1) & 1, abort_flag, kSiteODone);
+            ok = wait_product(j - 1, kSiteODone);
             if (ok) tc_fence_after_sync();
             return ok;
           };
@@ -820,10 +829,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           mbar_arrive_warp((j & 1) ? &p_odd[t] : &p_full[t]);
         }
         if (!ok) break;
-        // The last two products may be under way: their phases one after the other (a wait for the last one's parity alone
-        // would be content with the phase two before it).
-        if (my_nkt > 1) ok = mbar_wait_warp(&o_done[t], (my_nkt - 2) & 1, abort_flag, kSiteODoneFinal);
-        ok = ok && mbar_wait_warp(&o_done[t], (my_nkt - 1) & 1, abort_flag, kSiteODoneFinal);
+        ok = wait_product(my_nkt - 1, kSiteODoneFinal);
       }
       if (!ok) break;
       tc_fence_after_sync();
