@@ -382,6 +382,8 @@ PyObject* block_fwd(const Args& a) {
   const int64_t B = qkv.size(0), S = qkv.size(1), E = qkv.size(2) / 3, D = E / H;
   const int64_t R = reg ? reg->size(-2) : 0;
   TORCH_CHECK_VALUE(D == 64 || D == 128, "head dim ", D, " is not supported (64 or 128)");
+  // the kernels walk qkv, and k behind q, by H * D columns
+  TORCH_CHECK(qkv.size(2) == 3 * H * D, "qkv ", qkv.sizes(), " is not (B, S, 3 x ", H, " heads x ", D, ")");
   TORCH_CHECK_VALUE(pos_weight.scalar_type() == at::kFloat || pos_weight.scalar_type() == qkv.scalar_type(),
                     "pos_weight must be float32 or have the dtype of qkv");
   const at::Device dev = qkv.device();
