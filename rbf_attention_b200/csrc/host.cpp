@@ -429,16 +429,30 @@ PyObject* block_bwd(const Args& a) {
   const Tensor qk = a.tensor(1, "qk"), out = a.tensor(2, "out"), lse = a.tensor(3, "lse");
   const int64_t R = a.integer(6);
   const bool softmax = a.flag(7);
-  TORCH_CHECK_VALUE(qk.dim() == 5, "qk must have shape (2, B, S, H, D), got ", qk.sizes());
+  TORCH_CHECK(qkv.is_cuda(), "qkv must be a CUDA tensor: rbf_attention_b200 has no CPU path");
+  TORCH_CHECK_VALUE(is_16bit(qkv), "unsupported dtype ", qkv.scalar_type(), " (bfloat16 or float16)");
+  TORCH_CHECK_VALUE(qk.dim() == 5 && qk.size(0) == 2, "qk must have shape (2, B, S, H, D), got ", qk.sizes());
   const int64_t B = qk.size(1), S = qk.size(2), H = qk.size(3), D = qk.size(4), E = H * D;
   const at::Device dev = qkv.device();
   const at::ScalarType type = qkv.scalar_type();
+  TORCH_CHECK_VALUE(D == 64 || D == 128, "head dim ", D, " is not supported (64 or 128)");
+  TORCH_CHECK_VALUE(R >= 0 && R <= S, R, " registers in a sequence of ", S);
+  // the kernels walk every tensor by qk's sizes
+  TORCH_CHECK(qkv.numel() == 3 * B * S * E && out.numel() == B * S * E && dout.numel() == B * S * E &&
+                  (!softmax || lse.numel() == B * H * S) && table.numel() >= (S - R) * D,
+              "qkv ", qkv.sizes(), ", out ", out.sizes(), ", lse ", lse.sizes(), ", dout ", dout.sizes(), " or table ",
+              table.sizes(), " does not go with qk ", qk.sizes());
+  TORCH_CHECK_VALUE(qk.scalar_type() == type && out.scalar_type() == type && (!softmax || lse.scalar_type() == at::kFloat),
+                    "qk and out must have the dtype of qkv and lse float32, got ", qk.scalar_type(), ", ", out.scalar_type(),
+                    ", ", lse.scalar_type(), " with ", type);
+  TORCH_CHECK_VALUE(qk.device() == dev && out.device() == dev && dout.device() == dev && (!softmax || lse.device() == dev),
+                    "qkv, qk, out, lse and dout must be on one device");
   const c10::cuda::CUDAGuard guard(dev);
   qkv = qkv.contiguous();
   dout = (dout.scalar_type() == type ? dout : dout.to(type)).contiguous();
   if (table.device() != dev || table.scalar_type() != at::kFloat) table = table.to(dev, at::kFloat);
   table = table.contiguous();
-  const Tensor qk_c = qk.contiguous(), out_c = out.contiguous();
+  const Tensor qk_c = qk.contiguous(), out_c = out.contiguous(), lse_c = softmax ? lse.contiguous() : lse;
   const Tensor dqkv = empty({B, S, 3 * E}, type, dev), d_pw = empty({H, D / 2}, at::kFloat, dev),
                d_rp = empty({H, R, D}, at::kFloat, dev);
   const Tensor ws = workspace(rbf_b200_workspace_bytes(B, H, S, D, softmax, 1), dev);
@@ -460,7 +474,7 @@ PyObject* block_bwd(const Args& a) {
     {
       const Unlocked unlocked;
       const int rc =
-          rbf_b200_bwd_posting(q, k, v, out_c.const_data_ptr(), softmax ? lse.const_data_ptr<float>() : nullptr,
+          rbf_b200_bwd_posting(q, k, v, out_c.const_data_ptr(), softmax ? lse_c.const_data_ptr<float>() : nullptr,
                                dout.const_data_ptr(), dq, dk, dk + E * item, ws.data_ptr(), ws.nbytes(), B, H, S, D, packed.s,
                                packed.s, fused.s, packed.s, packed.s, fused.s, fused.s, fused.s, code, 1, softmax, scale, stream,
                                RBF_B200_PHASE_ALL, slot);

@@ -37,3 +37,32 @@ def test_the_block_takes_three_times_its_heads_columns(heads, rest):
     for call in (_lib.host().block_fwd, torch.ops.rbf_attn_b200.susie_block_fwd, ops.susie_block_attention):
         with pytest.raises((RuntimeError, ValueError)):
             call(qkv, pw, None, table, heads, True)
+
+
+def _block_backward(softmax):
+    B, S, H, D = 2, 20, 3, 64
+    lse = _zeros(*((B, H, S) if softmax else (0,)), dtype=torch.float32)
+    return dict(qkv=_zeros(B, S, 3 * H * D), qk=_zeros(2, B, S, H, D), out=_zeros(B, S, H * D), lse=lse,
+                dout=_zeros(B, S, H * D), table=_zeros(S, D, dtype=torch.float32), num_registers=2, softmax=softmax)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("softmax", [True, False])
+def test_the_blocks_backward_takes_tensors_of_one_size(softmax):
+    op = torch.ops.rbf_attn_b200.susie_block_bwd
+    good = _block_backward(softmax)
+    dqkv, d_pw, d_rp = op(**good)
+    assert dqkv.shape == good["qkv"].shape and d_pw.shape == (3, 32) and d_rp.shape == (3, 2, 64)
+    lse = good["lse"]
+    bad = [{name: good[name][:, :-1]} for name in ("qkv", "out", "dout", "qk")] + [{name: good[name][:1]} for name in
+           ("qkv", "out", "dout", "qk")] + [{name: good[name][..., :-8]} for name in ("qkv", "out", "dout")]
+    bad += [{"qk": good["qk"][0]}, {"qk": good["qk"][..., :32]}, {"qk": good["qk"].half()}, {"out": good["out"].float()},
+            {"table": good["table"][:17]}, {"num_registers": 21}, {"num_registers": -1}, {"qkv": good["qkv"].float()},
+            {"dout": good["dout"].cpu()}, {"out": good["out"].cpu()}, {"qkv": good["qkv"].cpu()}]
+    if softmax:
+        bad += [{"lse": lse[:, :, :-1]}, {"lse": lse[:0]}, {"lse": lse.double()}, {"lse": lse.cpu()}]
+    for change in bad:
+        with pytest.raises((RuntimeError, ValueError)):
+            op(**{**good, **change})
+    op(**{**good, "dout": good["dout"].float(), "qkv": good["qkv"].view(40, -1), "table": good["table"][:18]})
+    ops.check_device_status()
