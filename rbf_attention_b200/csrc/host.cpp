@@ -536,6 +536,7 @@ PyObject* gelu_bwd(const Args& a) {
   Tensor h = a.tensor(0, "h"), dy = a.tensor(1, "dy");
   const bool with_bias = a.flag(2);
   TORCH_CHECK_VALUE(h.is_cuda() && is_16bit(h), "gelu_bwd: a 16-bit CUDA tensor");
+  TORCH_CHECK_VALUE(h.dim() > 0 && h.size(-1) > 0, "gelu_bwd: no columns in ", h.sizes());
   TORCH_CHECK_VALUE(dy.numel() == h.numel() && dy.device() == h.device(), "gelu_bwd: dy must have the size and device of h");
   const c10::cuda::CUDAGuard guard(h.device());
   const at::ScalarType type = h.scalar_type();
@@ -607,6 +608,7 @@ PyObject* layer_norm_bwd(const Args& a) {
   Optional dres = a.optional(2, "dres");
   const Tensor weight = a.tensor(3, "weight"), mean = a.tensor(4, "mean"), rstd = a.tensor(5, "rstd");
   TORCH_CHECK(x.is_cuda(), "x must be a CUDA tensor: rbf_attention_b200 has no CPU path");
+  TORCH_CHECK_VALUE(x.dim() > 0 && x.size(-1) > 0, "layer_norm_bwd: no columns in ", x.sizes());
   const c10::cuda::CUDAGuard guard(x.device());
   const at::ScalarType type = x.scalar_type();
   const at::Device dev = x.device();

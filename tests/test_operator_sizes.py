@@ -66,3 +66,14 @@ def test_the_blocks_backward_takes_tensors_of_one_size(softmax):
             op(**{**good, **change})
     op(**{**good, "dout": good["dout"].float(), "qkv": good["qkv"].view(40, -1), "table": good["table"][:18]})
     ops.check_device_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(4, 0), (0,), (2, 3, 0), ()])
+def test_gradients_over_no_columns_are_refused(shape):
+    x, w, stat = _zeros(*shape), _zeros(0), _zeros(4, dtype=torch.float32)
+    op = torch.ops.rbf_attn_b200
+    for call in (lambda: op.gelu_bwd(x, x, True), lambda: op.gelu_bwd(x, x, False), lambda: op.layer_norm_bwd(x, x, w, stat, stat),
+                 lambda: op.layer_norm_bwd_add(x, x, x, w, stat, stat)):
+        with pytest.raises(ValueError, match="no columns"):
+            call()
