@@ -239,6 +239,11 @@ PyObject* attention_bwd(const Args& a) {
   TORCH_CHECK_VALUE(is_16bit(q), "unsupported dtype ", type, " (bfloat16, float16 or float32)");
   const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D0 = q.size(3);
   const int64_t D = padded_head_dim(D0), Dc = columns_of(D0, type);
+  TORCH_CHECK_VALUE(!out || (out->sizes() == q.sizes() && out->device() == q.device()),
+                    "out must have the shape and device of q, ", q.sizes());
+  TORCH_CHECK_VALUE(!softmax || !lse || (lse->numel() == B * H * N && lse->scalar_type() == at::kFloat &&
+                                         lse->device() == q.device()),
+                    "L must be (B, H, N) float32 on the device of q");
   const c10::cuda::CUDAGuard guard(q.device());
   const Tensor qc = tma_ready(pad_columns(q, Dc)), kc = tma_ready(pad_columns(k, Dc)), vc = tma_ready(pad_columns(v, Dc)),
                doc = tma_ready(pad_columns(dout, Dc));
@@ -248,7 +253,7 @@ PyObject* attention_bwd(const Args& a) {
                dv = empty({B, H, N, Dc}, type, q.device());
   const Tensor ws = workspace(rbf_b200_workspace_bytes(B, H, N, D, softmax, 1), q.device());
   Optional l;
-  if (softmax) l = lse;
+  if (softmax && lse) l = lse->contiguous();
   void* stream = stream_of(q);
   Enqueue call = [=](unsigned int* slot) {
     const c10::cuda::CUDAGuard on(dq.device());
@@ -387,6 +392,10 @@ PyObject* block_fwd(const Args& a) {
   TORCH_CHECK_VALUE(pos_weight.scalar_type() == at::kFloat || pos_weight.scalar_type() == qkv.scalar_type(),
                     "pos_weight must be float32 or have the dtype of qkv");
   const at::Device dev = qkv.device();
+  TORCH_CHECK_VALUE(pos_weight.numel() == H * (D / 2) && pos_weight.device() == dev, "pos_weight must be (", H, ", ", D / 2,
+                    ") on the device of qkv, got ", pos_weight.sizes());
+  TORCH_CHECK_VALUE(R == 0 || (reg->numel() == H * R * D && reg->device() == dev), "reg_pos_emb must be (", H, ", R, ", D,
+                    ") on the device of qkv");
   const c10::cuda::CUDAGuard guard(dev);
   qkv = qkv.contiguous();
   const Tensor pw = pos_weight.contiguous();
@@ -394,8 +403,8 @@ PyObject* block_fwd(const Args& a) {
   if (R > 0) rp = (reg->scalar_type() == pw.scalar_type() ? *reg : reg->to(pw.scalar_type())).contiguous();
   if (table.device() != dev || table.scalar_type() != at::kFloat) table = table.to(dev, at::kFloat);
   table = table.contiguous();
-  TORCH_CHECK_VALUE(table.size(0) >= S - R, "the position table holds ", table.size(0), " rows, ", S - R,
-                    " text positions are needed");
+  TORCH_CHECK_VALUE(table.size(0) >= S - R && table.numel() >= (S - R) * D, "the position table holds ", table.size(0),
+                    " rows, ", S - R, " text positions of ", D, " columns are needed");
   const at::ScalarType type = qkv.scalar_type();
   const Tensor qk = empty({2, B, S, H, D}, type, dev), out = empty({B, S, E}, type, dev);
   const Tensor lse = softmax ? empty({B, H, S}, at::kFloat, dev) : empty({0}, at::kFloat, dev);
@@ -577,6 +586,10 @@ PyObject* layer_norm_fwd(const Args& a) {
                           residual->device() == x.device(),
                       "residual must have the shape, dtype and device of x: ", residual->sizes(), " ",
                       residual->scalar_type(), " against ", x.sizes(), " ", x.scalar_type());
+  TORCH_CHECK_VALUE(weight.numel() == x.size(-1) && bias.numel() == x.size(-1) && weight.device() == x.device() &&
+                        bias.device() == x.device(),
+                    name, ": weight and bias must have the columns and the device of x, got ", weight.sizes(), " and ",
+                    bias.sizes(), " with ", x.sizes());
   const c10::cuda::CUDAGuard guard(x.device());
   const at::ScalarType type = x.scalar_type();
   const at::Device dev = x.device();
@@ -612,21 +625,30 @@ PyObject* layer_norm_bwd(const Args& a) {
   const c10::cuda::CUDAGuard guard(x.device());
   const at::ScalarType type = x.scalar_type();
   const at::Device dev = x.device();
+  const int64_t cols = x.size(-1), rows = x.numel() / cols;
+  TORCH_CHECK_VALUE(is_16bit(x) && weight.scalar_type() == type && mean.scalar_type() == at::kFloat &&
+                        rstd.scalar_type() == at::kFloat,
+                    "layer_norm_bwd: 16-bit x and weight of one type, mean and rstd float32");
+  TORCH_CHECK_VALUE(dy.numel() == x.numel() && weight.numel() == cols && mean.numel() == rows && rstd.numel() == rows,
+                    "layer_norm_bwd: dy ", dy.sizes(), ", weight ", weight.sizes(), ", mean ", mean.sizes(), " or rstd ",
+                    rstd.sizes(), " does not go with x ", x.sizes());
+  TORCH_CHECK_VALUE(dy.device() == dev && weight.device() == dev && mean.device() == dev && rstd.device() == dev &&
+                        (!dres || dres->device() == dev),
+                    "layer_norm_bwd: tensors on several devices");
   x = x.contiguous();
   dy = (dy.scalar_type() == type ? dy : dy.to(type)).contiguous();
-  const Tensor wc = weight.contiguous();
+  const Tensor wc = weight.contiguous(), mean_c = mean.contiguous(), rstd_c = rstd.contiguous();
   if (dres) {
     dres = (dres->scalar_type() == type ? *dres : dres->to(type)).contiguous();
     TORCH_CHECK_VALUE(dres->sizes() == x.sizes(), "dres must have the shape of x: ", dres->sizes(), " against ", x.sizes());
   }
-  const int64_t cols = x.size(-1), rows = x.numel() / cols;
   const Tensor dx = empty(x.sizes(), type, dev), dgamma = empty({cols}, at::kFloat, dev), dbeta = empty({cols}, at::kFloat, dev);
   const Tensor ws = workspace(std::max<size_t>(rbf_b200_layer_norm_bwd_workspace_bytes(rows, cols), 16), dev);
   int rc;
   {
     const Unlocked unlocked;
     rc = rbf_b200_layer_norm_bwd_add(x.const_data_ptr(), dy.const_data_ptr(), dres ? dres->const_data_ptr() : nullptr,
-                                     wc.const_data_ptr(), mean.const_data_ptr<float>(), rstd.const_data_ptr<float>(),
+                                     wc.const_data_ptr(), mean_c.const_data_ptr<float>(), rstd_c.const_data_ptr<float>(),
                                      dx.data_ptr(), dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), ws.data_ptr(),
                                      ws.nbytes(), rows, cols, dtype_code(type), stream_of(x));
   }

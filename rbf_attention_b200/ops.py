@@ -674,9 +674,15 @@ def _(o, v):
 
 @torch.library.custom_op("rbf_attn_b200::xsa_bwd", mutates_args=())
 def xsa_bwd(g: torch.Tensor, o: torch.Tensor, v: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    _validate("o", o)
+    _validate("v", v, o)
+    g = g.to(o.dtype)
+    _validate("g", g, o)
+    if o.dtype not in _DTYPE_CODE:
+        raise ValueError(f"unsupported dtype {o.dtype} (bfloat16 or float16)")
     B, H, N, D = o.shape
     lib = _lib.load()
-    gc, oc, vc = _tma_ready(g.to(o.dtype)), _tma_ready(o), _tma_ready(v)
+    gc, oc, vc = _tma_ready(g), _tma_ready(o), _tma_ready(v)
     d_o = torch.empty((B, H, N, D), dtype=o.dtype, device=o.device)
     d_v = torch.empty_like(d_o)
     with _OnDevice(o.device):

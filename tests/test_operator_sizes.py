@@ -77,3 +77,68 @@ def test_gradients_over_no_columns_are_refused(shape):
                  lambda: op.layer_norm_bwd_add(x, x, x, w, stat, stat)):
         with pytest.raises(ValueError, match="no columns"):
             call()
+
+
+def _refused(call, good, bad):
+    call(**good)
+    for change in bad:
+        with pytest.raises((RuntimeError, ValueError)):
+            call(**{**good, **change})
+    ops.check_device_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_attention_gradients_take_an_output_and_statistics_of_q(dtype):
+    t, lse = _zeros(2, 3, 70, 64, dtype=dtype), _zeros(2, 3, 70, dtype=torch.float32)
+    good = dict(q=t, k=t, v=t, out=t, L=lse, dout=t, is_causal=True, sm_scale=0.125)
+    outs = [{"out": o} for o in (t[:, :, :-1], t[:1], t[..., :32], t[0], t.cpu())]
+    _refused(torch.ops.rbf_attn_v5.scaled_bwd, good, outs + [{"L": x} for x in (lse[:, :, :-1], lse[:1], lse.half(), lse.cpu())])
+    wide = torch.zeros(2, 3, 140, device=DEV)[:, :, ::2]
+    torch.ops.rbf_attn_v5.scaled_bwd(**{**good, "L": wide, "out": t.half()})
+    good = {name: good[name] for name in ("q", "k", "v", "out", "dout", "is_causal", "sm_scale")}
+    _refused(torch.ops.rbf_attn_v5.non_softmax_bwd_with_out, good, outs)
+
+
+@pytest.mark.gpu
+def test_statistics_in_any_layout_give_the_same_gradients():
+    g = torch.Generator(device=DEV).manual_seed(0)
+    q, k, v, do = ((torch.randn(2, 3, 70, 64, generator=g, device=DEV) * 0.5).half() for _ in range(4))
+    out, lse = torch.ops.rbf_attn_v5.scaled_fwd(q, k, v, True)
+    strided = torch.stack((lse, -lse), -1)[..., 0]
+    want = torch.ops.rbf_attn_v5.scaled_bwd(q, k, v, out, lse, do, True, 0.125)
+    for a, b in zip(torch.ops.rbf_attn_v5.scaled_bwd(q, k, v, out, strided, do, True, 0.125), want):
+        assert (a.double() - b.double()).norm() <= 1e-3 * b.double().norm()         # the order of dQ's fp32 additions
+
+
+@pytest.mark.gpu
+def test_the_block_takes_positions_of_its_heads():
+    good = dict(qkv=_zeros(2, 20, 3 * 2 * 64), pos_weight=_zeros(2, 32), reg_pos_emb=_zeros(2, 4, 64),
+                table=_zeros(16, 64, dtype=torch.float32), num_heads=2, softmax=True)
+    _refused(torch.ops.rbf_attn_b200.susie_block_fwd, good,
+             [{"pos_weight": _zeros(1, 32)}, {"pos_weight": _zeros(2, 16)}, {"pos_weight": good["pos_weight"].cpu()},
+              {"reg_pos_emb": _zeros(1, 4, 64)}, {"reg_pos_emb": _zeros(2, 4, 32)}, {"reg_pos_emb": good["reg_pos_emb"].cpu()},
+              {"table": good["table"][:15]}, {"table": good["table"][:, :32]}])
+
+
+@pytest.mark.gpu
+def test_layer_norms_take_parameters_and_gradients_of_their_columns():
+    x, w, stat = _zeros(6, 512), _zeros(512), _zeros(6, dtype=torch.float32)
+    params = [{name: t} for name in ("weight", "bias") for t in (w[:256], _zeros(1024), w.cpu(), w.float())]
+    op = torch.ops.rbf_attn_b200
+    _refused(op.layer_norm_fwd, dict(x=x, weight=w, bias=w, eps=1e-5), params)
+    _refused(op.add_layer_norm_fwd, dict(x=x, residual=x, weight=w, bias=w, eps=1e-5), params + [{"residual": x[:5]}])
+    bad = [{"dy": x[:5]}, {"dy": x[:, :256]}, {"dy": x.cpu()}, {"weight": w[:256]}, {"weight": w.float()}, {"weight": w.cpu()},
+           {"x": x.float()}]
+    bad += [{name: t} for name in ("mean", "rstd") for t in (stat[:5], stat.half(), stat.cpu())]
+    good = dict(x=x, dy=x, weight=w, mean=stat, rstd=stat)
+    _refused(op.layer_norm_bwd, good, bad)
+    _refused(op.layer_norm_bwd_add, dict(good, dres=x), bad + [{"dres": x[:5]}, {"dres": x.cpu()}])
+
+
+@pytest.mark.gpu
+def test_exclusive_self_attention_takes_one_shape():
+    t = _zeros(2, 3, 50, 64)
+    bad = [{"v": t[:, :, :-1]}, {"v": t[:1]}, {"v": t.half()}, {"v": t.cpu()}]
+    _refused(torch.ops.rbf_attn_b200.xsa_fwd, dict(o=t, v=t), bad)
+    _refused(torch.ops.rbf_attn_b200.xsa_bwd, dict(g=t, o=t, v=t), bad + [{"g": t[:, :, :-1]}, {"g": t.cpu()}])
