@@ -170,7 +170,7 @@ cudaError_t launch_gelu_fwd(const void* h, void* out, int64_t n, bool bf16, int 
 
 cudaError_t launch_gelu_bwd(const void* h, const void* dy, void* dh, int64_t rows, int cols, bool bf16, float* partials,
                             float* dbias, int sms, cudaStream_t stream) {
-  if (rows == 0) return cudaSuccess;
+  if (rows == 0) return dbias != nullptr ? cudaMemsetAsync(dbias, 0, cols * sizeof(float), stream) : cudaSuccess;
   const int col_blocks = (cols + 255) / 256;
   int bands = col_sums_bands(rows, cols, sms);
   const int one_wave = sms * kGeluBwdBlocks / col_blocks;      // (of few bands a wave may be far from full)
