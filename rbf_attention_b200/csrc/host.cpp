@@ -21,6 +21,7 @@
 #include <cmath>
 #include <functional>
 #include <optional>
+#include <utility>
 #include <vector>
 
 #include "../../include/rbf_b200.h"
@@ -126,10 +127,15 @@ void check(int rc, const char* what) {
   TORCH_CHECK(false, what, ": ", name, ": ", rbf_b200_last_error());
 }
 
-// The interpreter's lock is not held while a call enqueues: a full launch queue blocks, and what it waits for may need it.
+// The interpreter's lock is not held while a call copies, allocates or enqueues: a full launch queue blocks, an allocation may
+// wait for the device, and what they wait for may need it. An entry point takes its arguments with the lock, does the rest
+// without it and takes it back for the results.
 struct Unlocked {
   PyThreadState* state = PyEval_SaveThread();
-  ~Unlocked() { PyEval_RestoreThread(state); }
+  void lock() {
+    if (state != nullptr) PyEval_RestoreThread(std::exchange(state, nullptr));
+  }
+  ~Unlocked() { lock(); }
 };
 
 // ------------------------------------------------------------------ tensors
@@ -204,6 +210,7 @@ PyObject* attention_fwd(const Args& a) {
   TORCH_CHECK_VALUE(is_16bit(q) || (type == at::kFloat && D == 64), "unsupported dtype ", type,
                     " (bfloat16, float16 or float32)");
   const int64_t Dc = columns_of(D0, type);
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(q.device());
   const Tensor qc = tma_ready(pad_columns(q, Dc)), kc = tma_ready(pad_columns(k, Dc)), vc = tma_ready(pad_columns(v, Dc));
   const Tensor out = empty({B, H, N, Dc}, type, q.device());
@@ -220,6 +227,7 @@ PyObject* attention_fwd(const Args& a) {
                                 strides3(kc), strides3(vc), strides3(out), dtype_code(type), causal, softmax, scale, stream,
                                 RBF_B200_PHASE_ALL, slot);
   };
+  unlocked.lock();
   return tuple(callable(std::move(call)), wrap(out), wrap(lse));
 }
 
@@ -244,6 +252,7 @@ PyObject* attention_bwd(const Args& a) {
   TORCH_CHECK_VALUE(!softmax || !lse || (lse->numel() == B * H * N && lse->scalar_type() == at::kFloat &&
                                          lse->device() == q.device()),
                     "L must be (B, H, N) float32 on the device of q");
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(q.device());
   const Tensor qc = tma_ready(pad_columns(q, Dc)), kc = tma_ready(pad_columns(k, Dc)), vc = tma_ready(pad_columns(v, Dc)),
                doc = tma_ready(pad_columns(dout, Dc));
@@ -267,6 +276,7 @@ PyObject* attention_bwd(const Args& a) {
                                 oc ? strides3(*oc) : none, strides3(doc), strides3(dq), strides3(dk), strides3(dv),
                                 dtype_code(type), causal, softmax, scale, stream, RBF_B200_PHASE_ALL, slot);
   };
+  unlocked.lock();
   return tuple(callable(std::move(call)), wrap(dq), wrap(dk), wrap(dv));
 }
 
@@ -316,6 +326,7 @@ PyObject* narrow_f32(const Args& a) {
   }
   if (!ok) Py_RETURN_NONE;
   const at::Device dev = first.device();
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(dev);
   std::vector<Tensor> halves;
   for (size_t i = 0; i < src.size(); ++i) halves.push_back(empty({B, H, N, D}, at::kHalf, dev));
@@ -331,6 +342,7 @@ PyObject* narrow_f32(const Args& a) {
     return rbf_b200_narrow_f32_posting(static_cast<int>(src.size()), from.data(), to.data(), strides.data(), B, H, N, D, checked,
                                        static_cast<unsigned int*>(flag.data_ptr()), stream, slot);
   };
+  unlocked.lock();
   return tuple(callable(std::move(call)), wrap_all(halves));
 }
 
@@ -341,6 +353,7 @@ PyObject* widen_f16(const Args& a) {
   TORCH_CHECK_VALUE(!src.empty(), "widen_f16: no tensors");
   const int64_t count = src[0].numel();
   const at::Device dev = src[0].device();
+  Unlocked unlocked;
   std::vector<const void*> from;
   std::vector<void*> to;
   std::vector<Tensor> out;
@@ -353,14 +366,13 @@ PyObject* widen_f16(const Args& a) {
     from.push_back(t.const_data_ptr());
     to.push_back(out.back().data_ptr());
   }
-  if (!ok) return wrap_all(out);
-  const c10::cuda::CUDAGuard guard(dev);
-  int rc;
-  {
-    const Unlocked unlocked;
+  int rc = RBF_B200_OK;
+  if (ok) {
+    const c10::cuda::CUDAGuard guard(dev);
     rc = rbf_b200_widen_f16(static_cast<int>(src.size()), from.data(), to.data(), count, stream_of(src[0]));
   }
   check(rc, "rbf_b200_widen_f16");
+  unlocked.lock();
   return wrap_all(out);
 }
 
@@ -396,6 +408,7 @@ PyObject* block_fwd(const Args& a) {
                     ") on the device of qkv, got ", pos_weight.sizes());
   TORCH_CHECK_VALUE(R == 0 || (reg->numel() == H * R * D && reg->device() == dev), "reg_pos_emb must be (", H, ", R, ", D,
                     ") on the device of qkv");
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(dev);
   qkv = qkv.contiguous();
   const Tensor pw = pos_weight.contiguous();
@@ -428,6 +441,7 @@ PyObject* block_fwd(const Args& a) {
                                 B, H, S, D, packed.s, packed.s, fused.s, packed.s, code, 1, softmax, scale, stream,
                                 RBF_B200_PHASE_MAIN, slot);
   };
+  unlocked.lock();
   return tuple(callable(std::move(call)), wrap(out), wrap(lse), wrap(qk));
 }
 
@@ -456,6 +470,7 @@ PyObject* block_bwd(const Args& a) {
                     ", ", lse.scalar_type(), " with ", type);
   TORCH_CHECK_VALUE(qk.device() == dev && out.device() == dev && dout.device() == dev && (!softmax || lse.device() == dev),
                     "qkv, qk, out, lse and dout must be on one device");
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(dev);
   qkv = qkv.contiguous();
   dout = (dout.scalar_type() == type ? dout : dout.to(type)).contiguous();
@@ -495,6 +510,7 @@ PyObject* block_bwd(const Args& a) {
     check(rc2, "rbf_b200_qkv_prep_bwd");     // raised, not returned: the backward is enqueued and posts its word
     return static_cast<int>(RBF_B200_OK);
   };
+  unlocked.lock();
   return tuple(callable(std::move(call)), wrap(dqkv), wrap(d_pw), wrap(d_rp));
 }
 
@@ -505,6 +521,7 @@ PyObject* column_sums(const Args& a) {
   Tensor x = a.tensor(0, "x");
   TORCH_CHECK_VALUE(x.dim() == 2 && x.is_cuda() && is_16bit(x) && x.size(1) % 8 == 0,
                     "column_sums: a 16-bit CUDA matrix whose width is a multiple of 8");
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(x.device());
   const bool ok = x.stride(1) == 1 && x.stride(0) >= x.size(1) && x.stride(0) % 8 == 0 &&
                   reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 16 == 0;
@@ -512,13 +529,10 @@ PyObject* column_sums(const Args& a) {
   const int64_t rows = x.size(0), cols = x.size(1);
   const Tensor out = empty({cols}, at::kFloat, x.device());
   const Tensor ws = workspace(std::max<size_t>(rbf_b200_column_sums_workspace_bytes(rows, cols), 16), x.device());
-  int rc;
-  {
-    const Unlocked unlocked;
-    rc = rbf_b200_column_sums(x.const_data_ptr(), out.data_ptr<float>(), ws.data_ptr(), ws.nbytes(), rows, cols,
-                              rows > 1 ? x.stride(0) : cols, dtype_code(x.scalar_type()), stream_of(x));
-  }
+  const int rc = rbf_b200_column_sums(x.const_data_ptr(), out.data_ptr<float>(), ws.data_ptr(), ws.nbytes(), rows, cols,
+                                      rows > 1 ? x.stride(0) : cols, dtype_code(x.scalar_type()), stream_of(x));
   check(rc, "rbf_b200_column_sums");
+  unlocked.lock();
   return wrap(out);
 }
 
@@ -527,15 +541,13 @@ PyObject* gelu_fwd(const Args& a) {
   Tensor h = a.tensor(0, "h");
   TORCH_CHECK_VALUE(h.is_cuda() && is_16bit(h) && h.numel() % 8 == 0,
                     "gelu_fwd: a 16-bit CUDA tensor with a multiple of 8 elements");
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(h.device());
   h = h.contiguous();
   const Tensor out = empty(h.sizes(), h.scalar_type(), h.device());
-  int rc;
-  {
-    const Unlocked unlocked;
-    rc = rbf_b200_gelu_fwd(h.const_data_ptr(), out.data_ptr(), h.numel(), dtype_code(h.scalar_type()), stream_of(h));
-  }
+  const int rc = rbf_b200_gelu_fwd(h.const_data_ptr(), out.data_ptr(), h.numel(), dtype_code(h.scalar_type()), stream_of(h));
   check(rc, "rbf_b200_gelu_fwd");
+  unlocked.lock();
   return wrap(out);
 }
 
@@ -547,6 +559,7 @@ PyObject* gelu_bwd(const Args& a) {
   TORCH_CHECK_VALUE(h.is_cuda() && is_16bit(h), "gelu_bwd: a 16-bit CUDA tensor");
   TORCH_CHECK_VALUE(h.dim() > 0 && h.size(-1) > 0, "gelu_bwd: no columns in ", h.sizes());
   TORCH_CHECK_VALUE(dy.numel() == h.numel() && dy.device() == h.device(), "gelu_bwd: dy must have the size and device of h");
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(h.device());
   const at::ScalarType type = h.scalar_type();
   h = h.contiguous();
@@ -556,13 +569,11 @@ PyObject* gelu_bwd(const Args& a) {
   const Tensor dbias = empty({with_bias ? cols : 0}, at::kFloat, h.device());
   const size_t bytes = with_bias ? rbf_b200_column_sums_workspace_bytes(rows, cols) : 0;
   const Tensor ws = workspace(std::max<size_t>(bytes, 16), h.device());
-  int rc;
-  {
-    const Unlocked unlocked;
-    rc = rbf_b200_gelu_bwd(h.const_data_ptr(), dy.const_data_ptr(), dh.data_ptr(), with_bias ? dbias.data_ptr<float>() : nullptr,
-                           ws.data_ptr(), ws.nbytes(), rows, cols, dtype_code(type), stream_of(h));
-  }
+  const int rc = rbf_b200_gelu_bwd(h.const_data_ptr(), dy.const_data_ptr(), dh.data_ptr(),
+                                   with_bias ? dbias.data_ptr<float>() : nullptr, ws.data_ptr(), ws.nbytes(), rows, cols,
+                                   dtype_code(type), stream_of(h));
   check(rc, "rbf_b200_gelu_bwd");
+  unlocked.lock();
   return tuple(wrap(dh), wrap(dbias));
 }
 
@@ -590,6 +601,7 @@ PyObject* layer_norm_fwd(const Args& a) {
                         bias.device() == x.device(),
                     name, ": weight and bias must have the columns and the device of x, got ", weight.sizes(), " and ",
                     bias.sizes(), " with ", x.sizes());
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(x.device());
   const at::ScalarType type = x.scalar_type();
   const at::Device dev = x.device();
@@ -602,15 +614,12 @@ PyObject* layer_norm_fwd(const Args& a) {
   }
   const Tensor y = empty(x.sizes(), type, dev), mean = empty({rows}, at::kFloat, dev), rstd = empty({rows}, at::kFloat, dev);
   const Tensor wc = weight.contiguous(), bc = bias.contiguous();
-  int rc;
-  {
-    const Unlocked unlocked;
-    rc = rbf_b200_add_layer_norm_fwd(x.const_data_ptr(), residual ? residual->const_data_ptr() : nullptr,
-                                     sum ? sum->data_ptr() : nullptr, wc.const_data_ptr(), bc.const_data_ptr(), y.data_ptr(),
-                                     mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, cols, eps, dtype_code(type),
-                                     stream_of(x));
-  }
+  const int rc = rbf_b200_add_layer_norm_fwd(x.const_data_ptr(), residual ? residual->const_data_ptr() : nullptr,
+                                             sum ? sum->data_ptr() : nullptr, wc.const_data_ptr(), bc.const_data_ptr(),
+                                             y.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, cols, eps,
+                                             dtype_code(type), stream_of(x));
   check(rc, residual ? "rbf_b200_add_layer_norm_fwd" : "rbf_b200_layer_norm_fwd");
+  unlocked.lock();
   return tuple(wrap(sum), wrap(y), wrap(mean), wrap(rstd));
 }
 
@@ -622,6 +631,7 @@ PyObject* layer_norm_bwd(const Args& a) {
   const Tensor weight = a.tensor(3, "weight"), mean = a.tensor(4, "mean"), rstd = a.tensor(5, "rstd");
   TORCH_CHECK(x.is_cuda(), "x must be a CUDA tensor: rbf_attention_b200 has no CPU path");
   TORCH_CHECK_VALUE(x.dim() > 0 && x.size(-1) > 0, "layer_norm_bwd: no columns in ", x.sizes());
+  Unlocked unlocked;
   const c10::cuda::CUDAGuard guard(x.device());
   const at::ScalarType type = x.scalar_type();
   const at::Device dev = x.device();
@@ -644,17 +654,15 @@ PyObject* layer_norm_bwd(const Args& a) {
   }
   const Tensor dx = empty(x.sizes(), type, dev), dgamma = empty({cols}, at::kFloat, dev), dbeta = empty({cols}, at::kFloat, dev);
   const Tensor ws = workspace(std::max<size_t>(rbf_b200_layer_norm_bwd_workspace_bytes(rows, cols), 16), dev);
-  int rc;
-  {
-    const Unlocked unlocked;
-    rc = rbf_b200_layer_norm_bwd_add(x.const_data_ptr(), dy.const_data_ptr(), dres ? dres->const_data_ptr() : nullptr,
-                                     wc.const_data_ptr(), mean_c.const_data_ptr<float>(), rstd_c.const_data_ptr<float>(),
-                                     dx.data_ptr(), dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), ws.data_ptr(),
-                                     ws.nbytes(), rows, cols, dtype_code(type), stream_of(x));
-  }
+  const int rc =
+      rbf_b200_layer_norm_bwd_add(x.const_data_ptr(), dy.const_data_ptr(), dres ? dres->const_data_ptr() : nullptr,
+                                  wc.const_data_ptr(), mean_c.const_data_ptr<float>(), rstd_c.const_data_ptr<float>(),
+                                  dx.data_ptr(), dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), ws.data_ptr(), ws.nbytes(),
+                                  rows, cols, dtype_code(type), stream_of(x));
   check(rc, dres ? "rbf_b200_layer_norm_bwd_add" : "rbf_b200_layer_norm_bwd");
-  const at::ScalarType wtype = weight.scalar_type();
-  return tuple(wrap(dx), wrap(dgamma.to(wtype)), wrap(dbeta.to(wtype)));
+  const Tensor dgamma_out = dgamma.to(type), dbeta_out = dbeta.to(type);      // the type of weight
+  unlocked.lock();
+  return tuple(wrap(dx), wrap(dgamma_out), wrap(dbeta_out));
 }
 
 // ------------------------------------------------------------------ module
