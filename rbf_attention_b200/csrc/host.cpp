@@ -12,6 +12,8 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -665,6 +667,16 @@ PyObject* layer_norm_bwd(const Args& a) {
   return tuple(wrap(dx), wrap(dgamma_out), wrap(dbeta_out));
 }
 
+// (device index) -> whether the current stream of that device, which is the one that a call on its tensors uses, is being
+// captured into a graph. (The question without a device is answered for the thread's current one.)
+PyObject* capturing(const Args& a) {
+  a.expect(1);
+  const int64_t index = a.integer(0);
+  if (c10::cuda::device_count() == 0) Py_RETURN_FALSE;
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(index));
+  return PyBool_FromLong(c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None);
+}
+
 // ------------------------------------------------------------------ module
 template <PyObject* (*kFn)(const Args&)>
 PyObject* entry(PyObject* self, PyObject* const* argv, Py_ssize_t n) {
@@ -684,7 +696,8 @@ PyMethodDef methods[] = {
     method<narrow_f32>("narrow_f32"),         method<widen_f16>("widen_f16"),
     method<column_sums>("column_sums"),       method<gelu_fwd>("gelu_fwd"),
     method<gelu_bwd>("gelu_bwd"),             method<layer_norm_fwd>("layer_norm_fwd"),
-    method<layer_norm_bwd>("layer_norm_bwd"), {nullptr, nullptr, 0, nullptr}};
+    method<layer_norm_bwd>("layer_norm_bwd"), method<capturing>("capturing"),
+    {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -177,6 +177,7 @@ class _StatusMonitor:
 
     def __init__(self, device):
         self.device = device
+        self.index = _device_index(device)
         self.host = torch.zeros(self.SLOTS, dtype=torch.int32).pin_memory()
         self.slots = memoryview(self.host.numpy())      # same memory: reading a slot costs 0.05 us instead of 3
         self.base = self.host.data_ptr()
@@ -289,17 +290,18 @@ class _StatusMonitor:
     def launch(self, what, call) -> None:
         """``call(slot address)`` enqueues a call whose last kernel posts its status word there (0: no posting, while a
         CUDA graph is being captured) and returns its error code."""
-        if torch._C._cuda_isCurrentStreamCapturing():
+        if _lib.host().capturing(self.index):
             _lib.check(call(0), what)
             return
         self._enqueue(what, call, self.mapped)
 
     def record(self, ws, what):
         """Posts the status word at the start of ``ws`` with a kernel of its own."""
-        if torch.cuda.is_current_stream_capturing():
+        if _lib.host().capturing(self.index):
             return
-        self._enqueue(what, lambda slot: _lib.load().rbf_b200_post_device_status(
-            ws.data_ptr(), slot, _stream_ptr(ws.device)), self.base)
+        with _OnDevice(self.device):
+            self._enqueue(what, lambda slot: _lib.load().rbf_b200_post_device_status(
+                ws.data_ptr(), slot, _stream_ptr(ws.device)), self.base)
 
 
 _SYNC_STATUS = os.environ.get("RBF_B200_SYNC_STATUS", "0") not in ("", "0")
