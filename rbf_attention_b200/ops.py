@@ -817,7 +817,7 @@ def linear_gelu(module: torch.nn.Linear, x: torch.Tensor) -> torch.Tensor:
     if x.is_cuda and x.dtype in _DTYPE_CODE:
         weight, bias = module.weight, module.bias
         if bias is not None and weight.dtype == x.dtype and module.out_features % 8 == 0:
-            if _direct(x) and not _needs_grad(x, weight, bias):
+            if _direct(x, weight, bias) and not _needs_grad(x, weight, bias):
                 return _gelu_fwd(torch.nn.functional.linear(x, weight, bias))
             return _LinearGelu.apply(x, weight, bias)
     return torch.nn.functional.gelu(module(x))
