@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(256) col_sums_partial_kernel(const uint16_t* _
 }
 
 // out[c] = sum over bands of partials[band][c]: 32 columns x 8 band-lanes per block of 256
-__global__ void __launch_bounds__(256) col_sums_final_kernel(const float* __restrict__ partials, int bands, int cols,
+__global__ void __launch_bounds__(256) col_sums_final_kernel(const float* partials, int bands, int cols,
                                                              float* __restrict__ out) {
   __shared__ float s[8][33];
   const int col = threadIdx.x & 31, lp = threadIdx.x >> 5;

@@ -281,7 +281,8 @@ inline cudaError_t ensure_dynamic_smem(Kernel kernel, int bytes, PerDeviceFlags&
 // Launches a kernel that begins with grid_dependency_wait(): it may be set up - blocks resident, barriers and tensor memory
 // ready - before the kernel ahead of it has completed. Every boundary inside a call: about a microsecond of 2 (forward calls
 // replayed back to back: B2 H4 N256 12.3 -> 11.3 us, B4 H8 N1024 23.0 -> 22.0, B2 H12 N1500 D80 37.4 -> 36.1; backward 17.4 ->
-// 16.4, 41.5 -> 40.5, 83.5 -> 82.4).
+// 16.4, 41.5 -> 40.5, 83.5 -> 82.4). Memory may change while such a kernel runs, so none of its inputs is a `const
+// __restrict__` pointer: that would allow loads which the wait does not order.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream,
                                     const Args&... args) {

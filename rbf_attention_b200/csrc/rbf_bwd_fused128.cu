@@ -549,11 +549,11 @@ rbf_bwd_fused128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 
 // dq[b,h,n,:] = scale * acc[b,h,n,:]  (acc fp32 contiguous, dq 16-bit with strides); one thread per 8 elements
 template <bool kBf16>
-__global__ void __launch_bounds__(256) dq_convert128_kernel(const float* __restrict__ acc, void* __restrict__ dq,
+__global__ void __launch_bounds__(256) dq_convert128_kernel(const float* acc, void* dq,
                                                             int H, int N, int64_t sb, int64_t sh, int64_t sn,
                                                             float scale, int64_t total_chunks,
-                                                            const void* __restrict__ q, int64_t qsb, int64_t qsh,
-                                                            int64_t qsn, const float* __restrict__ delta, int n_pad,
+                                                            const void* q, int64_t qsb, int64_t qsh,
+                                                            int64_t qsn, const float* delta, int n_pad,
                                                             const DeviceStatus* status, unsigned int* status_slot,
                                                          int head_dim) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;

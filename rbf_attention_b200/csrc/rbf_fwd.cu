@@ -153,7 +153,7 @@ template <int D, bool kSoftmax, bool kBf16>
 __global__ void __launch_bounds__(Roles<D, kSoftmax, kBf16>::kThreads, 1)
 rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
-               const __grid_constant__ CUtensorMap tm_kslab, const float* __restrict__ qsq,
+               const __grid_constant__ CUtensorMap tm_kslab, const float* qsq,
                float* __restrict__ lse, DeviceStatus* status, int H, int N, int n_pad, int causal, float scale2,
                float slab_w, int heads, int blocks, unsigned int* work, unsigned int* status_slot) {
   using L = Smem<D>;

@@ -88,7 +88,7 @@ template <bool kSoftmax>
 __global__ void __launch_bounds__(kThreads, 1)
 rbf_fwd_tf32_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
-                    const __grid_constant__ CUtensorMap tm_kslab, const float* __restrict__ qsq,
+                    const __grid_constant__ CUtensorMap tm_kslab, const float* qsq,
                     float* __restrict__ lse, DeviceStatus* status, int H, int N, int n_pad, int causal, float scale2,
                     unsigned int* work, unsigned int* status_slot) {
   extern __shared__ uint8_t smem_raw[];
