@@ -173,6 +173,8 @@ def host():
     """The extension that takes tensors (csrc/host.cpp). Raises if it is not built."""
     global _host
     if _host is None:
+        import torch
+
         load()
         try:
             from . import _host as extension
@@ -181,6 +183,9 @@ def host():
                 f"{os.path.join(os.path.dirname(LIB_PATH), '_host.so')} is missing or does not load ({e}): build it with "
                 "`python -m rbf_attention_b200.build` (this package has no fallback path)"
             ) from e
+        if extension.torch_version != torch.__version__:
+            raise RuntimeError(f"_host.so was built for torch {extension.torch_version}, this is {torch.__version__}: build it "
+                               "again with `python -m rbf_attention_b200.build`")
         _host = extension
     return _host
 

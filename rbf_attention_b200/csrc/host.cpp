@@ -703,4 +703,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host() {
+  PyObject* m = PyModule_Create(&module);
+  // the torch that this file was compiled against: no other one has the interface it calls
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", RBF_TORCH_VERSION) != 0) Py_CLEAR(m);
+  return m;
+}
