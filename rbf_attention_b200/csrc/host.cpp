@@ -187,6 +187,9 @@ void validate(const char* name, const Tensor& t, const Tensor* like) {
   TORCH_CHECK_VALUE(t.device() == like->device(), name, " is on ", t.device(), ", q is on ", like->device());
 }
 
+// Head dim the kernels run at. Others up to 128 run zero-padded to the next of the two, which is exact: zero columns add
+// nothing to q.k, to |k|^2 or to |q|^2, and zero value columns give zero output columns (the reference pads to the next power
+// of two inside its kernels, rbf_attention.py:661). The softmax scale keeps using the caller's head dim.
 int64_t padded_head_dim(int64_t d) {
   TORCH_CHECK_VALUE(d <= 128, "head dim ", d, " is not supported (at most 128)");
   return d <= 64 ? 64 : 128;
@@ -195,6 +198,26 @@ int64_t padded_head_dim(int64_t d) {
 int64_t columns_of(int64_t d, at::ScalarType t) { return t != at::kFloat && d % 8 == 0 ? d : padded_head_dim(d); }
 
 const int64_t* strides3(const Tensor& t) { return t.strides().data(); }
+
+// The same two rules for calls that are prepared in Python: (name, tensor, tensor that it has to go with or None), (tensor)
+PyObject* validate_entry(const Args& a) {
+  a.expect(3);
+  const char* name = PyUnicode_AsUTF8(a.v[0]);
+  if (name == nullptr) throw python_error();
+  const Optional like = a.optional(2, "like");
+  validate(name, a.tensor(1, name), like ? &*like : nullptr);
+  Py_RETURN_NONE;
+}
+
+PyObject* tma_ready_entry(const Args& a) {
+  a.expect(1);
+  const Tensor t = a.tensor(0, "t");
+  TORCH_CHECK_VALUE(t.dim() == 4, "t must have shape (B, H, N, D), got ", t.sizes());
+  Unlocked unlocked;
+  const Tensor ready = tma_ready(t);
+  unlocked.lock();
+  return wrap(ready);
+}
 
 // ------------------------------------------------------------------ attention operators
 // (q, k, v, causal, softmax) -> (enqueue, out, lse or None). 16-bit tensors, or fp32 at head dims up to 64; `out` has the
@@ -316,6 +339,7 @@ PyObject* narrow_f32(const Args& a) {
   const Tensor& first = src[0];
   if (first.dim() != 4) Py_RETURN_NONE;
   const int64_t B = first.size(0), H = first.size(1), N = first.size(2), D = first.size(3);
+  padded_head_dim(D);                              // refused before anything is enqueued
   bool ok = D > 0 && D % 8 == 0;
   std::vector<int64_t> strides;
   for (const Tensor& t : src) {
@@ -697,6 +721,7 @@ PyMethodDef methods[] = {
     method<column_sums>("column_sums"),       method<gelu_fwd>("gelu_fwd"),
     method<gelu_bwd>("gelu_bwd"),             method<layer_norm_fwd>("layer_norm_fwd"),
     method<layer_norm_bwd>("layer_norm_bwd"), method<capturing>("capturing"),
+    method<validate_entry>("validate"),       method<tma_ready_entry>("tma_ready"),
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -71,48 +71,14 @@ def _needs_grad(*tensors) -> bool:
 
 
 def _validate(name: str, t: torch.Tensor, like: torch.Tensor | None = None) -> None:
-    if not isinstance(t, torch.Tensor):
-        raise TypeError(f"{name} must be a tensor")
-    if t.dim() != 4:
-        raise ValueError(f"{name} must have shape (B, H, N, D), got {tuple(t.shape)}")
-    if not t.is_cuda:
-        raise RuntimeError(f"{name} must be a CUDA tensor: rbf_attention_b200 has no CPU path")
-    if like is not None:
-        if t.shape != like.shape:
-            raise ValueError(f"{name} shape {tuple(t.shape)} differs from q shape {tuple(like.shape)}")
-        if t.dtype != like.dtype:
-            raise ValueError(f"{name} dtype {t.dtype} differs from q dtype {like.dtype}")
-        if t.device != like.device:
-            raise ValueError(f"{name} is on {t.device}, q is on {like.device}")
+    """(B, H, N, D) on a GPU and, if given, with the shape, dtype and device of ``like``."""
+    _lib.host().validate(name, t, like)
 
 
 def _tma_ready(t: torch.Tensor) -> torch.Tensor:
-    """Returns ``t`` if the TMA engine can address it in place (unit stride on D, 16-byte aligned base,
-    strides of dims b, h, n multiples of 16 bytes), else a contiguous copy. The reference assumes
+    """Returns ``t`` if the TMA engine can address it in place, else a contiguous copy. The reference assumes
     ``stride(-1) == 1`` without checking (rbf_attention.py:111-138)."""
-    B, H, N, D = t.shape
-    per16 = 16 // t.element_size()
-    ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0
-    if ok and D % per16 == 0 and t.is_contiguous():
-        return t
-    for ext, s in zip((B, H, N), t.stride()[:3]):
-        if ext > 1 and (s <= 0 or s % per16 != 0):
-            ok = False
-    if N > 1 and t.stride(2) < D:
-        ok = False
-    return t if ok else t.contiguous()
-
-
-def _padded_head_dim(D: int) -> int:
-    """Head dim the kernels run at: 64 or 128. Other head dims up to 128 run zero-padded to the next of the two, which
-    is exact: zero columns add nothing to q.k, to |k|^2 or to |q|^2, and zero value columns give zero output columns
-    (the reference pads to the next power of two inside its kernels, rbf_attention.py:661). The softmax scale keeps
-    using the caller's D. Multiples of 8 in 16-bit types are padded by the kernels' own loads."""
-    if D <= 64:
-        return 64
-    if D <= 128:
-        return 128
-    raise ValueError(f"head dim {D} is not supported (at most 128)")
+    return _lib.host().tma_ready(t)
 
 
 def _device_index(device: torch.device) -> int:
@@ -353,7 +319,7 @@ def _forward(q, k, v, is_causal: bool, softmax: bool):
     mon = _monitor(q.device)
     mon.poll()
     # fp32 tensors at head dim <= 64: TF32 operands, as the reference's Triton path uses for them (fp32's exponent range)
-    narrowed = q.dtype == torch.float32 and _padded_head_dim(D) != 64
+    narrowed = q.dtype == torch.float32 and D > 64
     if narrowed:
         _validate("k", k, q)
         _validate("v", v, q)
@@ -374,7 +340,6 @@ def _backward(q, k, v, out, lse, dout, is_causal: bool, sm_scale: float, softmax
     # the non-softmax variant takes the forward output when the caller has it: the single-kernel backward needs it
     narrowed = q.dtype == torch.float32
     if narrowed:
-        _padded_head_dim(D)
         _validate("k", k, q)
         _validate("v", v, q)
         _validate("dout", dout, q)

@@ -142,3 +142,32 @@ def test_exclusive_self_attention_takes_one_shape():
     bad = [{"v": t[:, :, :-1]}, {"v": t[:1]}, {"v": t.half()}, {"v": t.cpu()}]
     _refused(torch.ops.rbf_attn_b200.xsa_fwd, dict(o=t, v=t), bad)
     _refused(torch.ops.rbf_attn_b200.xsa_bwd, dict(g=t, o=t, v=t), bad + [{"g": t[:, :, :-1]}, {"g": t.cpu()}])
+
+
+def test_the_extensions_rules_are_the_ones_python_uses(built_library):
+    with pytest.raises(TypeError, match="k must be a tensor"):
+        ops._validate("k", None)
+    with pytest.raises(ValueError, match="q must have shape"):
+        ops._validate("q", torch.zeros(3, 64))
+    with pytest.raises(RuntimeError, match="q must be a CUDA tensor"):
+        ops._validate("q", torch.zeros(1, 2, 3, 64))
+    dense = torch.zeros(2, 3, 40, 64, dtype=torch.bfloat16)
+    heads_last = dense.permute(0, 2, 1, 3)
+    assert ops._tma_ready(dense) is dense and ops._tma_ready(heads_last) is heads_last
+    for t in (dense[..., 1:], dense[..., ::2], dense[:, :, :1].expand(2, 3, 40, 64), torch.zeros(2, 3, 40, 36).half()[..., :33]):
+        ready = ops._tma_ready(t)
+        assert ready.is_contiguous() and ready.shape == t.shape and ready is not t
+    with pytest.raises(ValueError, match="at most 128"):
+        _lib.host().narrow_f32([torch.zeros(1, 1, 4, 136)], 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_head_dims_above_128_are_refused_before_anything_runs(dtype):
+    t = _zeros(1, 2, 16, 136, dtype=dtype)
+    mon = ops._monitor(t.device)
+    ops.check_device_status()
+    for call in (lambda: ops._forward(t, t, t, True, True), lambda: ops._backward(t, t, t, t, t[..., 0].float(), t, True, 0.1, True)):
+        with pytest.raises(ValueError, match="at most 128"):
+            call()
+    assert len(mon.free) == mon.SLOTS
