@@ -471,7 +471,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if constexpr (kPersistent) {
         uint32_t G = 0, td = 0, qn = 0;
         bool ok = true;
-        for (uint32_t n = 0; ok && (kPersistent || n == 0); ++n) {
+        for (uint32_t n = 0; ok; ++n) {
           Item it;
           if (!read_item(n, ok, it)) break;
           const int my_nkt = it.nkt(t), nkt_max = it.nkt_max;
@@ -487,7 +487,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             issue_s(G % kStages);
             if (el) {
               umma_commit(&s_full[t]);
-              if (kPersistent && my_nkt == 1) umma_commit(&q_free[t]);
+              if (my_nkt == 1) umma_commit(&q_free[t]);
               umma_commit(&k_empty[G % kStages]);
             }
             // Group j of the item's MMAs, j = 0 .. my_nkt: P_t(j-1) V and the scores S_t(j+1), once the softmax group has
@@ -510,7 +510,7 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (!ok) break;
                 issue_s(st);
                 if (el) {
-                  if (kPersistent && j + 2 == my_nkt) umma_commit(&q_free[t]);   // the item's last read of Q_t
+                  if (j + 2 == my_nkt) umma_commit(&q_free[t]);   // the item's last read of Q_t
                   umma_commit(&k_empty[st]);
                 }
               }
@@ -738,6 +738,8 @@ rbf_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // next scores can be loaded: three quarters of them travel under the last quarter's exponentials. Against a wait
         // for the scores, one for P's columns and two arrivals, each 130 to 220 clocks of a warp's 2900 per tile (traced):
         // B8 H16 N4096 causal 421 -> 401 us with the pre-pass, B64 H8 N1028 207 -> 198, B4 H12 N1000 full 39.4 -> 37.4.
+        // (The scores on their way and the packed quarter do not all fit: 104 bytes of spill stores in the bf16 softmax
+        // kernel, 72 to 76 in the others, 68 in the bf16 one before.)
         ok = mbar_wait_warp(&s_full[t], md & 1, abort_flag, kSiteSFull);
         if (!ok) break;
         ++md;

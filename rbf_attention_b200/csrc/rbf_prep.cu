@@ -48,7 +48,7 @@ __device__ __forceinline__ uint4 load_chunk(const void* base, const int64_t* s, 
 }
 
 // Bytes in flight bound it: a row's tensors are asked for together (forward: two rows at a time), and registers are kept to
-// what leaves seven blocks on an SM. Against one tensor after the other, forward and backward in one kernel (36 registers),
+// what leaves seven blocks on an SM (32, which costs the backward's kernel 8 bytes of spills). Against one tensor after the other, forward and backward in one kernel (36 registers),
 // microseconds, forward and backward call:
 //   B8 H16 N4096 D64   26.9 -> 23.2, 68.8 -> 60.3      B2 H32 N16384 D128  101 -> 89, 212 -> 191
 //   B4 H16 N8192 D64 without softmax  39.1 -> 31.5, 77.5 -> 69.1      B4 H8 N1024 D64  4.9 -> 3.6, 8.2 -> 6.3
