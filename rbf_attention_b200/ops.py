@@ -144,6 +144,7 @@ class _StatusMonitor:
     def __init__(self, device):
         self.device = device
         self.index = _device_index(device)
+        self.capturing = _lib.host().capturing
         self.host = torch.zeros(self.SLOTS, dtype=torch.int32).pin_memory()
         self.slots = memoryview(self.host.numpy())      # same memory: reading a slot costs 0.05 us instead of 3
         self.base = self.host.data_ptr()
@@ -256,14 +257,14 @@ class _StatusMonitor:
     def launch(self, what, call) -> None:
         """``call(slot address)`` enqueues a call whose last kernel posts its status word there (0: no posting, while a
         CUDA graph is being captured) and returns its error code."""
-        if _lib.host().capturing(self.index):
+        if self.capturing(self.index):
             _lib.check(call(0), what)
             return
         self._enqueue(what, call, self.mapped)
 
     def record(self, ws, what):
         """Posts the status word at the start of ``ws`` with a kernel of its own."""
-        if _lib.host().capturing(self.index):
+        if self.capturing(self.index):
             return
         with _OnDevice(self.device):
             self._enqueue(what, lambda slot: _lib.load().rbf_b200_post_device_status(
@@ -314,7 +315,8 @@ def _first_columns(t: torch.Tensor, D: int) -> torch.Tensor:
 
 
 def _forward(q, k, v, is_causal: bool, softmax: bool):
-    _validate("q", q)
+    host = _lib.host()
+    host.validate("q", q, None)
     D = q.shape[3]
     mon = _monitor(q.device)
     mon.poll()
@@ -324,7 +326,7 @@ def _forward(q, k, v, is_causal: bool, softmax: bool):
         _validate("k", k, q)
         _validate("v", v, q)
         q, k, v = _narrow((q, k, v), 3, mon, "rbf_b200_fwd")
-    enqueue, out, lse = _lib.host().attention_fwd(q, k, v, is_causal, softmax)
+    enqueue, out, lse = host.attention_fwd(q, k, v, is_causal, softmax)
     mon.launch("rbf_b200_fwd", enqueue)
     out = _first_columns(out, D)
     if narrowed:
@@ -333,7 +335,8 @@ def _forward(q, k, v, is_causal: bool, softmax: bool):
 
 
 def _backward(q, k, v, out, lse, dout, is_causal: bool, sm_scale: float, softmax: bool):
-    _validate("q", q)
+    host = _lib.host()
+    host.validate("q", q, None)
     D = q.shape[3]
     mon = _monitor(q.device)
     mon.poll()
@@ -345,7 +348,7 @@ def _backward(q, k, v, out, lse, dout, is_causal: bool, sm_scale: float, softmax
         _validate("dout", dout, q)
         q, k, v, dout, *rest = _narrow((q, k, v, dout) if out is None else (q, k, v, dout, out), 4, mon, "rbf_b200_bwd")
         out = rest[0] if rest else None
-    enqueue, *grads = _lib.host().attention_bwd(q, k, v, out, lse, dout, is_causal, sm_scale, softmax)
+    enqueue, *grads = host.attention_bwd(q, k, v, out, lse, dout, is_causal, sm_scale, softmax)
     mon.launch("rbf_b200_bwd", enqueue)
     grads = [_first_columns(g, D) for g in grads]
     return tuple(_widen(grads) if narrowed else grads)
