@@ -296,7 +296,9 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, unsign
   config.stream = stream;
   config.attrs = &attr;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();      // reported here, and not again by whoever asks next
+  return e;
 }
 
 // SM count of the current device (-1 on error), cached per device.
